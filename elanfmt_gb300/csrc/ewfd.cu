@@ -234,7 +234,8 @@ struct ewf_handle {
     int ty = TY;        // two-kernel step: CTA tile height in rows (autotuned)
     bool pdl = true;    // two-kernel step: kernels launched as programmatic dependents (off if capture refuses)
     int l2pf = 0;       // two-kernel step: L2 prefetch distance of the velocity kernel in planes (autotuned)
-    bool fdiv = false;  // div_spacing verified for (float) dx, dy, dz
+    int fdiv = 0;       // StepArgs::fdiv of this handle's spacings
+    bool src_plane1 = false;  // a fused source entry that plane 2's thread applies on plane 1
     struct Snapshots *snap = nullptr;  // queued snapshot writer (created on first use)
 };
 
@@ -373,9 +374,10 @@ static StepArgs<T> make_args(const ewf_handle *h, int which = -1)
     a.by = (T)h->p.by;
     a.bz = (T)h->p.bz;
     a.third = (T)1.0 / (T)3.0;
-    a.fdiv = h->fdiv ? 1 : 0;
+    a.fdiv = h->fdiv;
     a.l2pf = h->l2pf;
     a.vdamp = (T)h->p.vdamp;
+    a.vdamp_on = a.vdamp != T(0) ? 1 : 0;
     a.bc1 = h->p.free_surface == EWF_FS_BC1 ? 1 : 0;
     a.smu_on = h->p.surface_mu > 0.0 ? 1 : 0;
     a.smu = (T)h->p.surface_mu;
@@ -384,7 +386,8 @@ static StepArgs<T> make_args(const ewf_handle *h, int which = -1)
 
 // ------------------------------------------------------------------------------------------
 // device check of div_spacing: every significand of three binades of x (2^-90, 2^0, 2^99, both
-// signs) against IEEE division; the range argument in ewfd_kernels.cuh carries the result to
+// signs) against IEEE division, and of five small ones (the subnormals, and normal x around those
+// whose quotients are subnormal); the range argument in ewfd_kernels.cuh carries the result to
 // the whole range
 // ------------------------------------------------------------------------------------------
 namespace ewf {
@@ -433,6 +436,15 @@ bool ewf_fdiv_verified(float d)
     ok = ok && hbad == 0;
     cache[key] = ok;
     return ok;
+}
+
+// Correction steps of the FP64 division by d (div_fast): 1 when |r d - 1| <= 2^-54 for r = RN(1/d)
+// (exact in one FMA), else 2; 0 outside the range of d the range test of x is made for.
+static int fdiv_f64_steps(double d)
+{
+    if (!(d >= 0x1p-100 && d <= 0x1p100)) return 0;
+    const double r = 1.0 / d;
+    return std::fabs(std::fma(r, d, -1.0)) <= 0x1p-54 ? 1 : 2;
 }
 
 static int dev_zero(ewf_handle *h, void *alloc)
@@ -589,6 +601,10 @@ extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
     }
     if (p->model == EWF_MODEL_ORTHO && h->esz == 4)
         h->fdiv = ewf_fdiv_verified((float)p->dx) && ewf_fdiv_verified((float)p->dy) && ewf_fdiv_verified((float)p->dz);
+    if (p->model == EWF_MODEL_ORTHO && h->esz == 8) {
+        const int sx_ = fdiv_f64_steps(p->dx), sy_ = fdiv_f64_steps(p->dy), sz_ = fdiv_f64_steps(p->dz);
+        h->fdiv = (sx_ && sy_ && sz_) ? std::max(sx_, std::max(sy_, sz_)) : 0;
+    }
     for (int q = 0; q < 9; ++q) CKH(alloc_box(h, &h->f_alloc[q]));
     if (h->dbuf)
         for (int q = 0; q < 9; ++q) CKH(alloc_box(h, &h->g_alloc[q]));

@@ -53,8 +53,9 @@ struct StepArgs {
     T c66, bx, by, bz;  // isotropic scalars (OK4:405-407)
     T c44, c55;         // per-component-weight scheme: shear moduli of yz and xz
     T third;            // (T)1/(T)3 of BC1
-    int fdiv;           // 1: div_spacing may take the reciprocal path for dx, dy, dz (verified)
+    int fdiv;           // FP32: 1 if div_fast is verified for dx, dy, dz; FP64: its correction steps (1 or 2); 0: IEEE division
     T vdamp;            // linear velocity damping (16 km scheme), 0 = off
+    int vdamp_on;       // vdamp != 0 (an integer: a test of T takes the FP64 pipe in the FP64 form)
     int bc1;            // 1: BC1 after the stress update (stress_store, inject_entry); 0: none
     int smu_on;         // isotropic 1-D PML scheme: shear modulus smu instead of c66 on plane k = 1
     T smu;
@@ -132,27 +133,121 @@ __device__ __forceinline__ T lds(const T *p)
 
 // ---------------------------------------------------------------------------------------------
 // Division by a grid spacing.  The orthorhombic shear terms divide velocity differences by dx,
-// dy, dz (ANISO:327-352), and six IEEE divisions per cell cost a sixth of the stress kernel's
-// time.  div_spacing returns the same correctly rounded quotient through the reciprocal with
-// Markstein's correction step (P. Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", IBM J. Res. Develop. 34(1), 1990): with r = RN(1/d),
-// q = RN(x r), the residual e = x - q d is exact in one FMA, and RN(q + e r) is the quotient.
-// For x = 0 or 2^-90 <= |x| <= 2^100 and 2^-10 <= d <= 2^30 every intermediate stays normal
-// (the residual exact), so the result scales exactly with the binade of x; the library checks
-// it against IEEE division over whole binades of x for each spacing on the device before it
-// sets `ok` (ewfd.cu, fdiv_verified).  Other x, and unverified spacings, take IEEE division.
+// dy, dz (ANISO:327-352), six divisions per cell.  div_fast returns the same correctly rounded
+// quotient through the reciprocal with Markstein's correction step (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1), 1990):
+// with r = RN(1/d), q = RN(x r), the residual x - q d is exact in one FMA, and q plus the residual
+// times r, rounded once, is the quotient.  The residual is taken with the opposite sign
+// (n = q d - x) so that an exact quotient keeps the sign of its zero: n = +0 then, and q - n r = q.
+//
+// FP32: for x = 0 or 2^-90 <= |x| <= 2^100 and 2^-10 <= d <= 2^30 every intermediate stays normal,
+// so the result scales exactly with the binade of x; the library checks it against IEEE division
+// over whole binades of x for each spacing on the device before it sets `ok` (ewfd.cu,
+// fdiv_verified).  Smaller x (the numerical precursor ahead of a wavefront) go through
+// div_small: x 2^64 is in that range again, and its quotient is scaled back with one rounding on
+// the subnormal grid.
+// FP64: Markstein's theorem makes one step exact when q is within one unit in the last place of
+// x / d.  The error of q is at most half a unit (its rounding) plus |r d - 1| |x / d|, less than
+// |r d - 1| 2^53 units (the reciprocal's): below one when |r d - 1| <= 2^-54, which the host computes
+// exactly for each spacing (fdiv_f64_steps); otherwise a first step brings q there and a second
+// one finishes.  The FP64 pipe (two lanes per SM and cycle) bounds the FP64 form: three or five
+// operations for a quotient in place of the compiler's division took the orthorhombic stress update
+// on 128^3 from 719 to 340 us.
+// Other x, and spacings outside those ranges, take IEEE division.
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float div_fast(float x, float d, float r)
+{
+    const float q = __fmul_rn(x, r);
+    const float n = __fmaf_rn(q, d, -x);
+    return __fmaf_rn(-n, r, q);
+}
+__device__ __forceinline__ double div_fast(double x, double d, double r, bool two)
+{
+    double q = __dmul_rn(x, r);
+    double n = __fma_rn(q, d, -x);
+    q = __fma_rn(-n, r, q);
+    if (two) {
+        n = __fma_rn(q, d, -x);
+        q = __fma_rn(-n, r, q);
+    }
+    return q;
+}
+
+// FP32, |x| < 2^100: div_fast with x scaled by 2^64 where |x| < 2^-90.  y is the scaled quotient, one
+// rounding to 24 bits, in units of 2^-149 (the subnormal grid): rounding y to an integer rounds the
+// quotient itself unless y is a half-integer that the first rounding produced; the residual's sign
+// then says on which side the quotient lies.  From 2^23 on y is an integer (a normal result).
+__device__ __forceinline__ float div_small(float x, float d, float r)
+{
+    const bool tiny = (__float_as_uint(x) & 0x7fffffffu) < 0x12800000u;
+    const float xs = tiny ? __fmul_rn(x, 0x1p64f) : x;
+    const float q = div_fast(xs, d, r);
+    const float n = __fmaf_rn(q, d, -xs);  // sign of (rounded - exact) quotient
+    const float y = __fmul_rn(q, 0x1p85f);
+    float Y = rintf(y);
+    if (fabsf(y - Y) == 0.5f && n != 0.f) Y = y - copysignf(0.5f, n);
+    return tiny ? copysignf(__fmul_rn(Y, 0x1p-149f), x) : q;
+}
+
+// Range test of div_fast over several x: div_key maps x = 0 to the largest key and |x| in increasing
+// order below it, so one minimum tests the lower ends together and one maximum the upper ends.
+__device__ __forceinline__ unsigned div_mag(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned div_mag(double x)
+{
+    // the high word; a subnormal whose high word is zero counts as 1 (zero itself stays 0)
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return hi | (__double2loint(x) != 0 ? 1u : 0u);
+}
+template <typename T>
+__device__ __forceinline__ bool div_in_range(unsigned key_min, unsigned mag_max)
+{
+    if (sizeof(T) == 4) return key_min >= 0x12800000u - 1u && mag_max <= 0x71800000u;  // 2^-90 .. 2^100
+    return key_min >= 0x0fb00000u && mag_max <= 0x70000000u;                           // above 2^-773, below 2^769
+}
+
 __device__ __forceinline__ float div_spacing(float x, float d, float r, bool ok)
 {
-    const unsigned ax = __float_as_uint(x) & 0x7fffffffu;
-    if (ok && (ax == 0u || ax - 0x12800000u <= 0x71800000u - 0x12800000u)) {  // 2^-90 .. 2^100
-        const float q = __fmul_rn(x, r);
-        const float e = __fmaf_rn(-q, d, x);
-        return e == 0.f ? q : __fmaf_rn(e, r, q);  // e = 0: q is exact (and keeps the sign of -0)
-    }
-    return __fdiv_rn(x, d);
+    const unsigned m = div_mag(x);
+    if (!ok || m > 0x71800000u) return __fdiv_rn(x, d);
+    return div_in_range<float>(m - 1u, m) ? div_fast(x, d, r) : div_small(x, d, r);
 }
 __device__ __forceinline__ double div_spacing(double x, double d, double, bool) { return x / d; }
+
+// The six shear quotients of a cell: x[0..5] by dy dx dz dx dz dy.  One range test covers all six, so
+// the common case is a single block of independent chains instead of six branches: 333 -> 300
+// instructions per cell of the orthorhombic stress update.  Cells with an x below 2^-90 take
+// div_small for all six (a shell of them travels ahead of every wavefront: 128^3 over its first 200
+// steps, stress 51 us with IEEE division there, 38 us with div_small).
+template <typename T>
+__device__ __forceinline__ void div_shear(const T (&x)[6], T dx, T dy, T dz, T rdx, T rdy, T rdz, int fdiv, T (&q)[6])
+{
+    unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+        const unsigned m = div_mag(x[e]);
+        lo = min(lo, m - 1u);
+        hi = max(hi, m);
+    }
+    const T d[6] = {dy, dx, dz, dx, dz, dy}, r[6] = {rdy, rdx, rdz, rdx, rdz, rdy};
+    if (fdiv != 0 && div_in_range<T>(lo, hi)) {
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int e = 0; e < 6; ++e) q[e] = div_fast(x[e], d[e], r[e]);
+        } else if (fdiv == 1) {
+#pragma unroll
+            for (int e = 0; e < 6; ++e) q[e] = div_fast(x[e], d[e], r[e], false);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 6; ++e) q[e] = div_fast(x[e], d[e], r[e], true);
+        }
+    } else if (sizeof(T) == 4 && fdiv != 0 && hi <= 0x71800000u) {
+#pragma unroll
+        for (int e = 0; e < 6; ++e) q[e] = (T)div_small((float)x[e], (float)d[e], (float)r[e]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 6; ++e) q[e] = x[e] / d[e];
+    }
+}
 
 // ---------------------------------------------------------------------------------------------
 // Stress update.  Isotropic: OK4:285-331.  Orthorhombic: ANISO:287-356.  BC1: OK4:271-283.
@@ -307,16 +402,12 @@ __device__ __forceinline__ void stress_math(const StepArgs<T> &a, const StressIn
         o[1] = q.s[1] * W + dt * (q.c[3] * Vxx + q.c[1] * Vyy + q.c[5] * Vzz);
         o[2] = q.s[2] * W + dt * (q.c[4] * Vxx + q.c[5] * Vyy + q.c[2] * Vzz);
         // ANISO:327-352 (shear derivatives divide by the spacing)
-        const bool fd = a.fdiv != 0;
-        const T dVx_dy = div_spacing(q.vx - q.vx_jm, a.dy, a.rdy, fd);
-        const T dVy_dx = div_spacing(q.vy - q.vy_im, a.dx, a.rdx, fd);
-        o[3] = q.s[3] * W + dt * q.c[6] * (dVy_dx + dVx_dy);
-        const T dVx_dz = div_spacing(q.vx - vx_m, a.dz, a.rdz, fd);
-        const T dVz_dx = div_spacing(vz_k - q.vz_im, a.dx, a.rdx, fd);
-        o[4] = q.s[4] * W + dt * q.c[7] * (dVz_dx + dVx_dz);
-        const T dVy_dz = div_spacing(q.vy - vy_m, a.dz, a.rdz, fd);
-        const T dVz_dy = div_spacing(vz_k - q.vz_jm, a.dy, a.rdy, fd);
-        o[5] = q.s[5] * W + dt * q.c[8] * (dVy_dz + dVz_dy);
+        const T x[6] = {q.vx - q.vx_jm, q.vy - q.vy_im, q.vx - vx_m, vz_k - q.vz_im, q.vy - vy_m, vz_k - q.vz_jm};
+        T d[6];  // dVx/dy dVy/dx dVx/dz dVz/dx dVy/dz dVz/dy
+        div_shear<T>(x, a.dx, a.dy, a.dz, a.rdx, a.rdy, a.rdz, a.fdiv, d);
+        o[3] = q.s[3] * W + dt * q.c[6] * (d[1] + d[0]);
+        o[4] = q.s[4] * W + dt * q.c[7] * (d[3] + d[2]);
+        o[5] = q.s[5] * W + dt * q.c[8] * (d[4] + d[5]);
         w_xy = (i > 0 && j > 0);
         w_xz = (i > 0 && k > 0);
         w_yz = (j > 0 && k > 0);
@@ -537,7 +628,7 @@ __device__ __forceinline__ T vel_update(const StepArgs<T> &a, T V, T dS, T w_or_
     if (!KAHAN) {
         if (MODEL == MODEL_ISO) return w_or_W * (V * a.rdt + b * dS) * a.dt;
         const T r = (V * a.rdt * w_or_W + b * dS) * a.dt;
-        return a.vdamp != T(0) ? r - a.vdamp * V : r;  // 16kmst.cu:337-349
+        return a.vdamp_on ? r - a.vdamp * V : r;  // 16kmst.cu:337-349
     }
     const T aa = w_or_W;
     const T inc = (MODEL == MODEL_ISO) ? aa * (b * dS) * a.dt : b * dS * a.dt;
