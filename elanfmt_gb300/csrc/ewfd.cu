@@ -171,6 +171,8 @@ static bool slot_used(int model, int q)
 // ------------------------------------------------------------------------------------------
 // handle
 // ------------------------------------------------------------------------------------------
+constexpr size_t REC_TABLE_MAX = (size_t)1 << 24;  // plane offsets of the velocity kernel's receiver table (64 MB)
+
 struct ewf_handle {
     ewf_params p;
     std::string workdir;
@@ -220,8 +222,10 @@ struct ewf_handle {
     std::vector<int32_t> h_rec;  // n*4 (i,j,k,comp)
     double *d_traces = nullptr;
     int *d_it = nullptr;     // step counter: [0] (one-pass, wavefront forms); [it & 1] (two-kernel step)
-    int *d_rcol = nullptr;   // two-kernel step: first receiver entry per column (nx*ny, -1 none)
-    int4 *d_rent = nullptr;  // its entries: (k, component, trace row, next entry)
+    uint2 *d_rgrp = nullptr;  // two-kernel step: receiver tables of the velocity kernel (RecFuse)
+    int *d_roff = nullptr;
+    int2 *d_rent = nullptr;
+    int rec_kmin = 0, rec_kmax = -1;
     bool rec_fuse = true;    // the velocity kernel samples every receiver (else k_record does)
     int it = 0;
     void *d_stage = nullptr;
@@ -395,9 +399,9 @@ __global__ void k_fdiv_check(float d, float r, unsigned *bad)
 {
     const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= (1u << 23)) return;
-    const unsigned expo[3] = {37u, 127u, 226u};
+    const unsigned expo[8] = {37u, 127u, 226u, 0u, 1u, 4u, 7u, 20u};
     unsigned nbad = 0;
-    for (int b = 0; b < 3; ++b)
+    for (int b = 0; b < 8; ++b)
         for (unsigned sgn = 0; sgn < 2; ++sgn) {
             const float x = __uint_as_float((sgn << 31) | (expo[b] << 23) | m);
             if (__float_as_uint(div_spacing(x, d, r, true)) != __float_as_uint(__fdiv_rn(x, d))) ++nbad;
@@ -486,7 +490,8 @@ extern "C" void ewf_destroy(ewf_handle *h)
     cudaFree(h->d_rec_comp);
     cudaFree(h->d_traces);
     cudaFree(h->d_it);
-    cudaFree(h->d_rcol);
+    cudaFree(h->d_rgrp);
+    cudaFree(h->d_roff);
     cudaFree(h->d_rent);
     cudaFree(h->d_stage);
     delete h->splan;
@@ -874,20 +879,24 @@ extern "C" int ewf_set_sources(ewf_handle *h, int32_t n, const int32_t *cijk, co
     // covers the rest: cells on the staggered arrays' last planes, and grids too thin for BC1's
     // plane-2 copy)
     StressSrc f{};
-    bool fuse = n > 0 && h->p.nz >= 3;
+    bool fuse = n > 0 && h->p.nz >= 3, plane1 = false;
     f.i0 = f.j0 = INT32_MAX;
     f.i1 = f.j1 = f.k1 = -1;
+    f.k0 = INT32_MAX;
     for (const SrcEntry &q : v) {
         if (q.i >= h->p.nx || q.j >= h->p.ny || q.k >= h->p.nz) fuse = false;
         f.i0 = std::min(f.i0, q.i);
         f.i1 = std::max(f.i1, q.i);
         f.j0 = std::min(f.j0, q.j);
         f.j1 = std::max(f.j1, q.j);
+        f.k0 = std::min(f.k0, fused_src_plane(q.comp, q.k));
         f.k1 = std::max(f.k1, fused_src_plane(q.comp, q.k));
+        if (fused_src_plane(q.comp, q.k) != q.k) plane1 = true;
     }
     if (fuse) {
         f.src = h->d_src;
         f.nsrc = n;
+        if (n <= SRC_INLINE) std::copy(v.begin(), v.end(), f.e);
     } else {
         f = StressSrc{};
     }
@@ -964,30 +973,66 @@ extern "C" int ewf_set_receivers(ewf_handle *h, int32_t n, const int32_t *ijkc)
     h->graph_dirty = true;
     // the two-kernel step's velocity kernel samples the receivers itself when every one is a
     // velocity component on a cell its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz)
-    cudaFree(h->d_rcol);
+    cudaFree(h->d_rgrp);
+    cudaFree(h->d_roff);
     cudaFree(h->d_rent);
-    h->d_rcol = nullptr;
+    h->d_rgrp = nullptr;
+    h->d_roff = nullptr;
     h->d_rent = nullptr;
     bool fuse = true;
+    int kmin = INT32_MAX, kmax = -1;
+    std::vector<int> order((size_t)n);
     for (int r = 0; r < n; ++r) {
         const int i = ijkc[4 * r], j = ijkc[4 * r + 1], k = ijkc[4 * r + 2], c = ijkc[4 * r + 3];
         if (c > EWF_F_VZ || i < 1 || j < 1 || k < 1 || i >= h->p.nx || j >= h->p.ny || k >= h->p.nz) fuse = false;
+        kmin = std::min(kmin, k);
+        kmax = std::max(kmax, k);
+        order[r] = r;
     }
-    h->rec_fuse = fuse;
     if (fuse && n > 0) {
-        const size_t ncol = (size_t)h->p.nx * h->p.ny;
-        std::vector<int> first(ncol, -1);
-        std::vector<int4> ent((size_t)n);
-        for (int r = n - 1; r >= 0; --r) {  // chained in list order
-            const size_t col = (size_t)ijkc[4 * r] + (size_t)ijkc[4 * r + 1] * h->p.nx;
-            ent[r] = make_int4(ijkc[4 * r + 2], ijkc[4 * r + 3], r, first[col]);
-            first[col] = r;
+        // entries by column (row by row), then plane; one slot of plane offsets per column
+        auto col = [&](int r) { return (size_t)ijkc[4 * r] + (size_t)ijkc[4 * r + 1] * h->p.nx; };
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+            return col(x) != col(y) ? col(x) < col(y) : ijkc[4 * x + 2] < ijkc[4 * y + 2];
+        });
+        size_t slots = 0;
+        for (int q = 0; q < n; ++q) slots += (q == 0 || col(order[q]) != col(order[q - 1]));
+        const size_t span = (size_t)(kmax - kmin + 1);
+        if (slots * (span + 1) > REC_TABLE_MAX) {
+            fuse = false;  // receivers all over a volume: k_record
+        } else {
+            const int ngx = (h->p.nx + 31) / 32;
+            std::vector<uint2> grp((size_t)ngx * h->p.ny, make_uint2(0u, 0u));
+            std::vector<int> off(slots * (span + 1));
+            std::vector<int2> ent((size_t)n);
+            int slot = -1;
+            for (int q = 0; q < n; ++q) {
+                const int r = order[q], i = ijkc[4 * r], j = ijkc[4 * r + 1];
+                if (q == 0 || col(r) != col(order[q - 1])) {
+                    ++slot;
+                    uint2 &g = grp[(size_t)j * ngx + i / 32];
+                    if (!g.x) g.y = (unsigned)slot;
+                    g.x |= 1u << (i & 31);
+                    int *o = &off[(size_t)slot * (span + 1)];
+                    int e = q;
+                    for (size_t k = 0; k <= span; ++k) {
+                        while (e < n && col(order[e]) == col(r) && ijkc[4 * order[e] + 2] < kmin + (int)k) ++e;
+                        o[k] = e;
+                    }
+                }
+                ent[q] = make_int2(ijkc[4 * r + 3], r);
+            }
+            CK(cudaMalloc(&h->d_rgrp, grp.size() * sizeof(uint2)));
+            CK(cudaMalloc(&h->d_roff, off.size() * sizeof(int)));
+            CK(cudaMalloc(&h->d_rent, ent.size() * sizeof(int2)));
+            CK(cudaMemcpy(h->d_rgrp, grp.data(), grp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(h->d_roff, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(h->d_rent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
         }
-        CK(cudaMalloc(&h->d_rcol, ncol * sizeof(int)));
-        CK(cudaMalloc(&h->d_rent, (size_t)n * sizeof(int4)));
-        CK(cudaMemcpy(h->d_rcol, first.data(), ncol * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->d_rent, ent.data(), (size_t)n * sizeof(int4), cudaMemcpyHostToDevice));
     }
+    h->rec_kmin = kmin;
+    h->rec_kmax = kmax;
+    h->rec_fuse = fuse;
     return EWF_OK;
 }
 
@@ -1052,8 +1097,12 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
     ss.order = h->p.src_order;
     RecFuse rf{};
     if (h->rec_fuse) {  // receivers sampled and the counter advanced by the velocity kernel
-        rf.col_first = h->d_rcol;
+        rf.grp = h->d_rgrp;
+        rf.off = h->d_roff;
         rf.ent = h->d_rent;
+        rf.ngx = (h->p.nx + 31) / 32;
+        rf.kmin = h->rec_kmin;
+        rf.kmax = h->rec_kmax;
         rf.traces = h->d_traces;
         rf.trace_len = h->p.nt;
         rf.it_rd = it_rd;

@@ -71,29 +71,41 @@ struct SrcEntry {
 // entry's column applies it right after its stores of the entry's plane -- for sxz / syz on plane
 // 1, after plane 2, whose update BC1 copies onto plane 1 -- with k_inject's arithmetic
 // (inject_entry), so the result is bit-identical to the separate launch.  [i0, i1] x [j0, j1]
-// bounds the entries' columns, so every other thread skips them with one test per plane.
+// bounds the entries' columns and [k0, k1] their planes, so every other thread skips them with one
+// test per plane.  The entries travel in the kernel's parameters (e) when there are few: read from
+// memory, a plane's pass over six of them was a chain of loads that outlasted the rest of a small
+// grid's launch.
+constexpr int SRC_INLINE = 8;  // the 6 entries of a moment tensor, and room for a pressure source
 struct StressSrc {
-    const SrcEntry *src;  // nsrc entries, every one inside the stress kernel's cells (i < nx, j < ny, k < nz)
-    int nsrc;             // 0: none (k_inject applies the sources, if any)
+    SrcEntry e[SRC_INLINE];
+    const SrcEntry *src;  // more than SRC_INLINE entries: all of them, in device memory
+    int nsrc;             // 0: none (k_inject applies the sources, if any); every entry has i < nx, j < ny, k < nz
     const double *stf;
     int nstf;
     const int *it_ptr;
     int order;            // 0: before BC1 (OK4), 1: after (ANISO)
     int i0, i1, j0, j1;   // bounding box of the entries' columns
-    int k1;               // last effective plane of any entry
+    int k0, k1;           // first and last effective plane of any entry
 };
 
 // Receivers sampled by the velocity kernel itself (the two-kernel step): the thread that owns a
 // receiver's column writes the trace sample right after its update of the receiver's plane, the
 // value k_record would read (the new velocity where the update writes the cell, the old one where
-// it does not).  col_first[j*nx + i] is the first entry of the column's receivers (-1: none),
-// entries are (k, component, trace row, next entry of the column or -1).  The step counter is read
-// at it_rd and, by one thread of the launch, written plus one at it_wr (a second location, so no
-// thread of the launch can read the new value).  col_first null: k_record samples; it_wr null:
-// k_record advances the counter.
+// it does not).  grp[j*ngx + i/32] = {mask, base}: bit i%32 of the mask marks a column with
+// receivers, whose slot is base plus the number of lower bits set; off[slot*(kmax-kmin+2) + k-kmin]
+// and the next element delimit the plane's entries ent[] = (component, trace row).  One broadcast
+// load per warp finds the columns and two more a plane's entries, however many a column holds (a
+// linked list per column cost a dependent load per entry and plane: 24 of them down a borehole
+// string were 7 us of a 40 x 40 x 32 grid's 10 us launch).  The step counter is read at it_rd and,
+// by one thread of the launch, written plus one at it_wr (a second location, so no thread of the
+// launch can read the new value).  grp null: k_record samples; it_wr null: k_record advances the
+// counter.
 struct RecFuse {
-    const int *col_first;
-    const int4 *ent;
+    const uint2 *grp;
+    const int *off;
+    const int2 *ent;
+    int ngx;
+    int kmin, kmax;
     double *traces;
     int trace_len;
     const int *it_rd;
@@ -416,10 +428,16 @@ __device__ __forceinline__ void stress_math(const StepArgs<T> &a, const StressIn
 
 // Stores the new stresses of cell c (plane k; sys: state plane pitch), with BC1 (when a.bc1):
 // szz = 0 on plane 0 and, from the freshly updated plane 2, sxz / syz on plane 1 (OK4:279-282).
-template <typename T>
+// BC1OWN: plane 1's shear cells that BC1 rewrites are stored by plane 2's thread alone, so planes 1
+// and 2 may belong to different CTAs (chunks of one or two planes).
+template <typename T, bool BC1OWN = false>
 __device__ __forceinline__ void stress_store(const StepArgs<T> &a, long long c, long long sys, int k, int i, int j,
                                              bool row_bc, const T (&o)[6], bool w_xy, bool w_xz, bool w_yz)
 {
+    if (BC1OWN && k == 1 && a.bc1) {
+        w_xz = w_xz && !(i > 0 && row_bc);
+        w_yz = w_yz && !(j > 0);
+    }
     a.f[3][c] = o[0];
     a.f[4][c] = o[1];
     a.f[5][c] = (k == 0 && row_bc && a.bc1) ? T(0) : o[2];
@@ -464,7 +482,7 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int X, int j
     // point sources on this column (SRC: the two-kernel step's stress kernel)
     bool src_col = false;
     T s_src = T(0);
-    if (SRC && ss.nsrc > 0 && i >= ss.i0 && i <= ss.i1 && j >= ss.j0 && j <= ss.j1 && k0 <= ss.k1) {
+    if (SRC && ss.nsrc > 0 && i >= ss.i0 && i <= ss.i1 && j >= ss.j0 && j <= ss.j1 && k0 <= ss.k1 && k1 > ss.k0) {
         const int it = *ss.it_ptr;
         src_col = it >= 0 && it < ss.nstf;  // the host validates the step range; never read past Src
         if (src_col) s_src = (T)ss.stf[it];
@@ -477,11 +495,18 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int X, int j
         T o[6];
         bool w_xy, w_xz, w_yz;
         stress_math<T, MODEL, DAMP>(a, q, cd, i, j, k, vx_m, vy_m, vz_k, wz_k, o, w_xy, w_xz, w_yz);
-        stress_store<T>(a, c, sys, k, i, j, row_bc, o, w_xy, w_xz, w_yz);
-        if (SRC && src_col && k <= ss.k1) {
-            for (int e = 0; e < ss.nsrc; ++e) {
-                const SrcEntry q_e = ss.src[e];
-                if (q_e.i == i && q_e.j == j && fused_src_plane(q_e.comp, q_e.k) == k) inject_entry(a, q_e, s_src, ss.order);
+        stress_store<T, SRC>(a, c, sys, k, i, j, row_bc, o, w_xy, w_xz, w_yz);
+        if (SRC && src_col && k >= ss.k0 && k <= ss.k1) {
+            if (ss.nsrc <= SRC_INLINE) {
+#pragma unroll
+                for (int e = 0; e < SRC_INLINE; ++e)
+                    if (e < ss.nsrc && ss.e[e].i == i && ss.e[e].j == j && fused_src_plane(ss.e[e].comp, ss.e[e].k) == k)
+                        inject_entry(a, ss.e[e], s_src, ss.order);
+            } else {
+                for (int e = 0; e < ss.nsrc; ++e) {
+                    const SrcEntry q_e = ss.src[e];
+                    if (q_e.i == i && q_e.j == j && fused_src_plane(q_e.comp, q_e.k) == k) inject_entry(a, q_e, s_src, ss.order);
+                }
             }
         }
         if (MODEL == MODEL_ISO && DAMP == DAMP_PML1D) wz_k = q.w;
@@ -754,10 +779,13 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
         if (pf_row) pf_row += c - (long long)threadIdx.x + (long long)a.l2pf * sys;
     }
     // receivers on this column (REC: the two-kernel step's velocity kernel)
-    int r_first = -1, r_it = 0;
-    if (REC && rf.col_first) {
-        r_first = rf.col_first[(long long)j * a.nx + i];
-        if (r_first >= 0) r_it = *rf.it_rd;
+    int slot = -1, r_it = 0;
+    if (REC && rf.grp && k0 <= rf.kmax && k1 > rf.kmin) {
+        const uint2 g = rf.grp[j * rf.ngx + (i >> 5)];
+        if ((g.x >> (i & 31)) & 1u) {
+            r_it = *rf.it_rd;
+            if (r_it >= 0 && r_it < rf.trace_len) slot = (int)g.y + __popc(g.x & ((1u << (i & 31)) - 1u));
+        }
     }
 
     for (int k = k0; k < k1; ++k, c += sys) {
@@ -768,17 +796,16 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
         T v[3], cp[3] = {KAHAN ? q.cp[0] : T(0), KAHAN ? q.cp[1] : T(0), KAHAN ? q.cp[2] : T(0)};
         vel_math<T, MODEL, DAMP, KAHAN>(a, q, vd, szz_m, sxz_k, syz_k, v, cp);
         vel_store<T, KAHAN>(a, c, k, i, j, v, cp);
-        if (REC && r_first >= 0 && r_it >= 0 && r_it < rf.trace_len) {
-            for (int e = r_first; e >= 0;) {
-                const int4 re = rf.ent[e];
-                if (re.x == k) {
-                    // the cell's value after the update: vel_store's ranges decide new or old
-                    const bool upd = re.y == 0 ? (j < a.ny - 1 && k < a.nz - 1)
-                                   : re.y == 1 ? (i < a.nx - 1 && k < a.nz - 1) : (i < a.nx - 1 && j < a.ny - 1);
-                    const T val = re.y == 0 ? (upd ? v[0] : q.v[0]) : re.y == 1 ? (upd ? v[1] : q.v[1]) : (upd ? v[2] : q.v[2]);
-                    rf.traces[(long long)re.z * rf.trace_len + r_it] = (double)val;
-                }
-                e = re.w;
+        if (REC && slot >= 0 && k >= rf.kmin && k <= rf.kmax) {
+            const int *po = rf.off + (long long)slot * (rf.kmax - rf.kmin + 2) + (k - rf.kmin);
+            const int e1 = po[1];
+            for (int e = po[0]; e < e1; ++e) {
+                const int2 re = rf.ent[e];
+                // the cell's value after the update: vel_store's ranges decide new or old
+                const bool upd = re.x == 0 ? (j < a.ny - 1 && k < a.nz - 1)
+                               : re.x == 1 ? (i < a.nx - 1 && k < a.nz - 1) : (i < a.nx - 1 && j < a.ny - 1);
+                const T val = re.x == 0 ? (upd ? v[0] : q.v[0]) : re.x == 1 ? (upd ? v[1] : q.v[1]) : (upd ? v[2] : q.v[2]);
+                rf.traces[(long long)re.y * rf.trace_len + r_it] = (double)val;
             }
         }
         szz_m = q.szz;
