@@ -547,6 +547,23 @@ static bool band_fits(const ewf_handle *h, int rows);
 // rows per CTA of the band kernel for a one-pass kernel choice (0: not the band kernel)
 static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (onepass == EWF_ONEPASS_BAND8 ? 8 : 0); }
 
+// Launch shape of the two-kernel step until the autotuner or a caller sets another.  A thread marches
+// kchunk planes one after the other, about a memory latency each, so a grid that does not fill the
+// GPU several times over runs faster in short chunks, and longer ones save the loads a chunk starts
+// with.  The line: one plane per chunk up to 0.5 M cells, then one more plane per 0.5 M cells, at
+// most 6 (three waves of resident warps at every size below that).  CTAs of 4 rows leave the
+// shortest tail at every size measured.  us per step of 16 planes x 8 rows and of this rule: ortho
+// 40x40x32 17.2 (4 planes) and 8.7, iso 128^3 40.0 (4 planes) and 38.9, Kahan 192^3 206.2 and 203.7.
+// The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
+// 320x320x256 641 -> 631) and not below (128^3: 55.8 and 56.1).
+static void split_default_shape(ewf_handle *h)
+{
+    const double cells = (double)h->p.nx * h->p.ny * h->p.nz;
+    if (h->p.kchunk == 0) h->kchunk = (int)std::min(6.0, std::max(1.0, std::floor(cells / 5e5 + 0.5)));
+    h->ty = 4;
+    h->l2pf = cells >= 1.2e7 ? 3 : 0;
+}
+
 extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
 {
     if (!out) return ewf_fail(EWF_ERR_ARG, "out is NULL");
@@ -573,6 +590,7 @@ extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
     h->box_elems = (size_t)h->sy * pz;
     h->base_off = h->hx + (long long)h->sx * 1 + h->sy * 1;
     h->kchunk = p->kchunk > 0 ? p->kchunk : 16;
+    if (p->fused == EWF_STEP_SPLIT) split_default_shape(h);
     h->gsteps = p->graph_steps == 0 ? 64 : (p->graph_steps < 0 ? 0 : p->graph_steps);
     if ((p->fused == EWF_STEP_FUSED || p->fused == EWF_STEP_SPLIT) && (h->gsteps & 1))
         h->gsteps += 1;  // graphs replay buffer pairs (one-pass) / step-counter pairs (two-kernel step)
@@ -901,6 +919,7 @@ extern "C" int ewf_set_sources(ewf_handle *h, int32_t n, const int32_t *cijk, co
         f = StressSrc{};
     }
     h->src_fuse = f;
+    h->src_plane1 = fuse && plane1;
     return EWF_OK;
 }
 
@@ -1082,6 +1101,10 @@ static void launch_on(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st
     cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// Planes per CTA of the two-kernel step.  A shear source entry on plane 1 is applied by the thread of
+// plane 2 (fused_src_plane), which then has to be the one that stores plane 1 too.
+static int split_kchunk(const ewf_handle *h) { return h->src_plane1 ? std::max(h->kchunk, 4) : h->kchunk; }
+
 // One step of the two-kernel form; `parity` = the step number's parity: the step counter of this
 // step is d_it[parity], the next step's d_it[1 - parity].
 template <typename T, int MODEL, int DAMP, bool KAHAN>
@@ -1130,7 +1153,8 @@ typedef void (*step_fn)(const ewf_handle *, cudaEvent_t *, int parity);
 template <typename T, int MODEL, int DAMP, bool KAHAN>
 static void step_entry(const ewf_handle *h, cudaEvent_t *ev, int parity)
 {
-    const StepArgs<T> a = make_args<T>(h, 0);
+    StepArgs<T> a = make_args<T>(h, 0);
+    a.kchunk = split_kchunk(h);
     launch_step_t<T, MODEL, DAMP, KAHAN>(h, a, ev, parity);
 }
 
@@ -1571,7 +1595,7 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
     if (!h || nsteps < 1) return ewf_fail(EWF_ERR_ARG, "bad argument");
     int st = inputs_ready(h);
     if (st) return st;
-    static const int cand[] = {4, 6, 8, 12, 16, 24, 32, 48, 64};
+    static const int cand[] = {1, 2, 3, 4, 6, 8, 12, 16, 32};
     const int steps = std::min(nsteps, h->p.nt - 1);
     if (steps < 1) return ewf_fail(EWF_ERR_ARG, "nt too small to tune");
     if (h->nsrc > 0 && h->nstf < (size_t)steps + 1) return ewf_fail(EWF_ERR_STATE, "source time function too short");
@@ -1615,10 +1639,10 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
         if (!split && ty != h->ty) continue;
         if (ty > (h->esz == 4 ? SPLIT_MAX_TY : TY)) continue;
         for (int kc : cand) {
-            if (kc > h->p.nz && kc != cand[0]) continue;
-            if (h->wave && kc > 16) continue;
+            if (kc > h->p.nz) continue;
+            if (h->wave && (kc < 4 || kc > 16)) continue;
             for (int vi = 0; vi < nvar; ++vi) {
-                h->kchunk = std::max(4, std::min(kc, h->p.nz));
+                h->kchunk = kc;
                 h->ty = ty;
                 if (h->wave) {
                     h->wave_lag_pct = lag_pct[vi];
@@ -1657,7 +1681,8 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
         h->l2pf = best_pf;
     }
     h->graph_dirty = true;
-    if (kchunk) *kchunk = best_k;
+    // what ewf_params.kchunk takes: shorter chunks are this handle's own (and the default's for such grids)
+    if (kchunk) *kchunk = std::max(4, best_k);
     return ewf_reset(h);
 }
 
