@@ -22,6 +22,7 @@
 #include <cstring>
 #include <mutex>
 #include <set>
+#include <utility>
 
 #include "ewf_umma.h"
 #include "ewfd.h"
@@ -41,34 +42,38 @@ __device__ __forceinline__ float gelu_grad(float x)
 }
 
 // ---------------------------------------------------------------------------------------------
-// tcgen05 GEMM: C[M,N] = A[M,K] . B[N,K]^T on the 5th-generation tensor cores.  Persistent: one
-// CTA per SM walks the 128 x BN tiles of C (BN = 256, or 128 when N is not a multiple of 256).
-// Two fp32 accumulators of 128 lanes x BN columns in tensor memory, so the epilogue of one tile
-// overlaps the MMAs of the next.  Warp roles, 192 threads:
-//   warp 0, one lane: TMA producer -- per k-stage one 2-D bulk tensor copy per operand (128-byte
-//     swizzle, ewf_umma.h) into the next free slot of a 4-stage ring, completing on that slot's
-//     "full" mbarrier; the ring runs on across tiles;
+// tcgen05 GEMM: C[M,N] = A[M,K] . B[N,K]^T on the 5th-generation tensor cores; A and B are stored either
+// K-major as written or transposed ([K, M], [K, N]: TA, TB), so gradients need no transposed copies.
+// Persistent: one CTA per SM walks the work items (job, K split, 128 x BN tile of C) of one or several
+// independent products.  Two fp32 accumulators of 128 lanes x BN columns in tensor memory, so the
+// epilogue of one item overlaps the MMAs of the next.  Warp roles, 320 threads:
+//   warp 0, one lane: TMA producer -- per k-stage the operands' boxes (128-byte swizzle, ewf_umma.h)
+//     into the next free slot of a ring of stages, completing on that slot's "full" mbarrier; the ring
+//     runs on across items; rows and K beyond a matrix's end read as zeros;
 //   warp 1, one lane: MMA issuer -- waits for a free accumulator ("acc_empty"), then per stage for
 //     "full", issues 4 tcgen05.mma (K = 16 each) and commits them to the slot's "empty" mbarrier
-//     (freeing it for the producer); after the tile's last stage commits "acc_full";
-//   warps 2-5: epilogue -- wait for "acc_full", read the accumulator with tcgen05.ld (warp w owns
-//     TMEM lanes 32 (w % 4) ..), add the bias, GELU, write the requested outputs, release the
-//     accumulator ("acc_empty", one arrival per warp).  When only the fp32 C is wanted and every
-//     SM has two tiles or more, each warp stages 32 rows x 64 columns in shared memory and writes
-//     them with one TMA store (row-contiguous, asynchronous); otherwise every lane stores its row.
-// K beyond the last full stage would be read as zeros (the tensor map's out-of-bounds fill); the
-// host accepts K multiples of 32.  Every mbarrier wait is bounded (g_umma_wait_limit polls): on
-// timeout the wait raises g_umma_err and gives up (the outputs of that launch are then invalid,
-// ewf_mlp_status reports it), and no later wait of the launch waits at all.  Before the CTA frees
-// its tensor memory and returns, the producer waits (again bounded, with a fixed limit) for the
-// last TMA loads it issued and the MMA issuer for every MMA it issued, whether or not a wait
-// gave up.  Test hook (ewf_mlp_test_hold): the MMA issuer of CTA 0 withholds the accumulator-
-// ready signal of one of its tiles, so the epilogue's wait on it runs out.
+//     (freeing it for the producer); after the item's last stage commits "acc_full";
+//   warps 2-9: epilogue -- wait for "acc_full", read the accumulator with tcgen05.ld (a pair of
+//     warps per quarter of the TMEM lanes, each half of the columns), add the bias, GELU or its
+//     gradient, release the accumulator ("acc_empty", one arrival per warp).  Every output goes
+//     through 32 rows x 32 columns of shared memory, swizzled so that neither the writes nor the TMA
+//     store that sends them off meet bank conflicts; the store clips rows beyond M.
+// What bounds it at the network's K = 512, where a tile has 8 k-stages: few rows, latency (launch, first
+// loads, epilogue); hidden layers of many rows, the GELU's erff; the output layer, the operands' way
+// from L2 and the output bytes.  With four epilogue warps storing a row per lane, and now: 128 x 512 x
+// 512 24.9 and 8.5 us, 8192 x 512 x 512 25.1 and 15.7, 8192 x 10240 x 512 140 and 93.
+// Every mbarrier wait is bounded (g_umma_wait_limit polls): on timeout the wait raises g_umma_err and
+// gives up (the outputs of that launch are then invalid, ewf_mlp_status reports it), and no later wait
+// of the launch waits at all.  Before the CTA frees its tensor memory and returns, the producer waits
+// (again bounded, with a fixed limit) for the last TMA loads it issued and the MMA issuer for every MMA
+// it issued, whether or not a wait gave up.  Test hook (ewf_mlp_test_hold): the MMA issuers of the
+// CTAs whose first tiles make up the first 256 columns withhold the accumulator-ready signal of one
+// of their items, so the epilogue's wait on it runs out.
 // ---------------------------------------------------------------------------------------------
 __device__ int g_umma_err = 0;
 constexpr int kWaitPolls = 1 << 22;
 __device__ int g_umma_wait_limit = kWaitPolls;
-__device__ int g_umma_hold = -1;  // tile (CTA-local index) of CTA 0 whose acc_full is withheld; -1: none
+__device__ int g_umma_hold = -1;  // item (CTA-local index) whose acc_full is withheld; -1: none
 
 __device__ __forceinline__ void mbar_init(uint64_t *b, uint32_t count)
 {
@@ -139,37 +144,91 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
                  : "memory");
 }
 
+// tcgen05.fence::before pairs with the mbarrier arrive that releases an accumulator
+constexpr int GEMM_THREADS = ewf_umma::THREADS + ewf_umma::MORE_EPILOGUE;
+constexpr int EPI_WARPS = (GEMM_THREADS - 64) / 32;
+constexpr int EPI_BOX = 32;                                    // rows and columns of an output box
+constexpr int EPI_BUF = EPI_BOX * EPI_BOX * 4;
+
+// Shared memory of a tile width: the operand ring and the epilogue's buffers, one or two per warp.  256
+// columns: four stages and one buffer (three stages and two: 8192 x 10240 x 512 98 us instead of 93 --
+// what bounds it is the operand traffic from L2, 393 KB a tile, not the epilogue's wait for a box).
 template <int BN>
-__global__ void __launch_bounds__(ewf_umma::THREADS, 1)
-    k_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const __grid_constant__ CUtensorMap mapC, int tma_c,
-             const float *__restrict__ bias, float *__restrict__ Cf, __nv_bfloat16 *__restrict__ Cb, float *__restrict__ Pre,
-             int M, int N, int K, int act)
+struct Shape {
+    static constexpr int STAGES = BN == 64 ? 8 : BN == 128 ? 5 : 4;
+    static constexpr int BUFS = BN == 128 ? 2 : 1;
+    static constexpr int RING = STAGES * ewf_umma::stage_bytes(BN);
+    static constexpr int SMEM = RING + EPI_WARPS * BUFS * EPI_BUF + 1024;  // + alignment slack
+    static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
+};
+
+enum {
+    OUT_F32 = 1, OUT_BF16 = 2, OUT_PRE = 4,  // outputs: fp32, bf16, the fp32 value before the activation
+    ACT_GELU = 8,
+    ACT_GRAD = 16,                           // bf16(value) * GELU'(gpre): the gradient through the activation
+    BF16_DIRECT = 32                         // the bf16 output is not 16-byte aligned: plain stores
+};
+
+// One product.  Maps of unused outputs are never read.
+template <int NOUT>
+struct GemmJob {
+    CUtensorMap a, b, out[NOUT];  // out: fp32 (and, NOUT = 3, bf16, pre), dimensions N, M, K splits
+    const float *bias, *gpre;
+    __nv_bfloat16 *cb;
+    int M, N, tiles_n, item0;     // the job's items start at item0
+    int nk, nk_split;             // k-stages, and of one split
+    int flags;
+};
+template <int NJ, int NOUT>
+struct GemmArgs {
+    GemmJob<NOUT> job[NJ];
+    int njobs, items;
+};
+
+__device__ __forceinline__ float gelu_grad_bf16(float x, float pre)
+{
+    return __bfloat162float(__float2bfloat16_rn(x)) * gelu_grad(pre);
+}
+
+// Sends the warp's 32 x 32 staged values off (one lane), after the writes of every lane.
+__device__ __forceinline__ void epi_store(const CUtensorMap *map, const void *buf, int n, int m, int z, int lane)
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"((uint64_t)map),
+                     "r"(n), "r"(m), "r"(z), "r"(smem_u32(buf))
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+template <int BN, bool TA, bool TB, int NJ, int NOUT>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant__ GemmArgs<NJ, NOUT> g)
 {
     namespace U = ewf_umma;
-    constexpr int STAGE = U::a_bytes() + BN * U::ROW_BYTES;
+    constexpr int STAGE = U::stage_bytes(BN), NS = Shape<BN>::STAGES, BUFS = Shape<BN>::BUFS;
+    constexpr int COLS = 2 * BN;  // tensor-memory columns: two accumulators
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[U::STAGES], empty[U::STAGES], acc_full[2], acc_empty[2], mma_drain;
+    __shared__ uint64_t full[NS], empty[NS], acc_full[2], acc_empty[2], mma_drain;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int tiles_n = N / BN, tiles = (M / U::BM) * tiles_n;
-    const int nk = (K + U::BK - 1) / U::BK;
 
     if (tid == 0) {
-        for (int s = 0; s < U::STAGES; ++s) {
+        for (int s = 0; s < NS; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);  // one arrival per epilogue warp
+            mbar_init(&acc_empty[b], EPI_WARPS);  // one arrival per epilogue warp
         }
         mbar_init(&mma_drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(2 * BN)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -178,43 +237,78 @@ __global__ void __launch_bounds__(ewf_umma::THREADS, 1)
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     bool ok = true;
+    // a dependent launch may start setting up; nothing of an earlier launch is read or written before it has completed
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    struct Item {
+        int job, m0, n0, z, kt0, kt1;
+    };
+    auto item_of = [&](int t) {
+        Item it;
+        it.job = 0;
+        while (NJ > 1 && it.job + 1 < g.njobs && t >= g.job[it.job + 1].item0) ++it.job;
+        const GemmJob<NOUT> &J = g.job[it.job];
+        t -= J.item0;
+        const int tiles = ((J.M + U::BM - 1) / U::BM) * J.tiles_n;
+        it.z = t / tiles;
+        t -= it.z * tiles;
+        it.m0 = (t / J.tiles_n) * U::BM;
+        it.n0 = (t % J.tiles_n) * BN;
+        it.kt0 = it.z * J.nk_split;
+        it.kt1 = min(it.kt0 + J.nk_split, J.nk);
+        return it;
+    };
 
     if (warp == 0) {
-        if (lane == 0) {  // TMA producer: every k-stage of every tile of this CTA, one ring
-            int g = 0;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-                const int m0 = (t / tiles_n) * U::BM, n0 = (t % tiles_n) * BN;
-                for (int kt = 0; kt < nk; ++kt, ++g) {
-                    const int s = U::ring_slot(g);
-                    if (U::ring_needs_free(g) && !mbar_wait(&empty[s], U::ring_free_parity(g))) { ok = false; break; }
-                    uint8_t *As = smem + s * STAGE;
+        if (lane == 0) {  // TMA producer: every k-stage of every item of this CTA, one ring
+            int q = 0;
+            for (int t = blockIdx.x; t < g.items && ok; t += gridDim.x) {
+                const Item it = item_of(t);
+                const GemmJob<NOUT> &J = g.job[it.job];
+                for (int kt = it.kt0; kt < it.kt1; ++kt, ++q) {
+                    const int s = U::ring_slot(q, NS);
+                    if (U::ring_needs_free(q, NS) && !mbar_wait(&empty[s], U::ring_free_parity(q, NS))) { ok = false; break; }
+                    uint8_t *As = smem + s * STAGE, *Bs = As + U::a_bytes();
                     mbar_expect_tx(&full[s], STAGE);
-                    tma_load_2d(As, &mapA, kt * U::BK, m0, &full[s]);
-                    tma_load_2d(As + U::a_bytes(), &mapB, kt * U::BK, n0, &full[s]);
+                    if (TA) {
+                        for (int r = 0; r < U::BM; r += U::MN_ATOM)
+                            tma_load_2d(As + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, &J.a, it.m0 + r, kt * U::BK, &full[s]);
+                    } else {
+                        tma_load_2d(As, &J.a, kt * U::BK, it.m0, &full[s]);
+                    }
+                    if (TB) {
+                        for (int r = 0; r < BN; r += U::MN_ATOM)
+                            tma_load_2d(Bs + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, &J.b, it.n0 + r, kt * U::BK, &full[s]);
+                    } else {
+                        tma_load_2d(Bs, &J.b, kt * U::BK, it.n0, &full[s]);
+                    }
                 }
             }
             // the loads issued last into each slot land before the CTA's shared memory goes
-            for (int q = (g > U::STAGES ? g - U::STAGES : 0); q < g; ++q)
-                mbar_drain(&full[U::ring_slot(q)], U::ring_full_parity(q));
+            for (int p = (q > NS ? q - NS : 0); p < q; ++p)
+                mbar_drain(&full[U::ring_slot(p, NS)], U::ring_full_parity(p, NS));
         }
     } else if (warp == 1) {
         if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = U::instr_desc_bf16_f32(U::BM, BN);
-            const int hold = blockIdx.x == 0 ? *(volatile int *)&g_umma_hold : -1;
-            int g = 0, i = 0;
-            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++i) {
+            const uint32_t idesc = U::instr_desc_bf16_f32(U::BM, BN, TA, TB);
+            const int hold = blockIdx.x < 256 / BN ? *(volatile int *)&g_umma_hold : -1;
+            int q = 0, i = 0;
+            for (int t = blockIdx.x; t < g.items && ok; t += gridDim.x, ++i) {
+                const Item it = item_of(t);
                 const int b = U::acc_buf(i);
                 if (U::acc_needs_free(i) && !mbar_wait(&acc_empty[b], U::acc_free_parity(i))) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)(b * BN);
-                for (int kt = 0; kt < nk; ++kt, ++g) {
-                    const int s = U::ring_slot(g);
-                    if (!mbar_wait(&full[s], U::ring_full_parity(g))) { ok = false; break; }
+                for (int kt = it.kt0; kt < it.kt1; ++kt, ++q) {
+                    const int s = U::ring_slot(q, NS);
+                    if (!mbar_wait(&full[s], U::ring_full_parity(q, NS))) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a0 = smem_u32(smem + s * STAGE), b0 = a0 + U::a_bytes();
                     for (int j = 0; j < U::BK / U::MMA_K; ++j)
-                        umma_bf16(d, U::smem_desc_sw128(a0 + 32 * j), U::smem_desc_sw128(b0 + 32 * j), idesc,
-                                  (kt > 0 || j > 0) ? 1u : 0u);
+                        umma_bf16(d, TA ? U::smem_desc_sw128_mn(a0 + U::MN_K_STEP * j) : U::smem_desc_sw128(a0 + 32 * j),
+                                  TB ? U::smem_desc_sw128_mn(b0 + U::MN_K_STEP * j) : U::smem_desc_sw128(b0 + 32 * j), idesc,
+                                  (kt > it.kt0 || j > 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
                 }
                 if (!ok) break;
@@ -224,123 +318,137 @@ __global__ void __launch_bounds__(ewf_umma::THREADS, 1)
             umma_commit(&mma_drain);
             mbar_drain(&mma_drain, 0);
         }
-    } else {  // epilogue warps 2..5: TMEM lane quarter q = warp % 4
-        const int q = warp & 3;
-        int i = 0;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
-            const int b = U::acc_buf(i);
+    } else {  // epilogue warps 2..9: TMEM lane quarter warp % 4, half of the columns each
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        uint8_t *const bufs = smem + Shape<BN>::RING + (warp - 2) * (BUFS * EPI_BUF);
+        int i = 0, nb = 0;
+        // the next staging buffer, free once the store before last (BUFS = 2) or the last one has read it
+        auto next_buf = [&]() {
+            if (lane == 0) {
+                if (BUFS == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            }
+            __syncwarp();
+            return bufs + (BUFS == 2 ? (nb++ & 1) * EPI_BUF : 0);
+        };
+        for (int t = blockIdx.x; t < g.items; t += gridDim.x, ++i) {
+            const Item it = item_of(t);
+            const GemmJob<NOUT> &J = g.job[it.job];
+            const int b = U::acc_buf(i), flags = J.flags;
             const bool got = !umma_failed() && mbar_wait(&acc_full[b], U::acc_full_parity(i));
             tc_fence_after();
-            const int m0 = (t / tiles_n) * U::BM, n0 = (t % tiles_n) * BN;
-            const int row = m0 + 32 * q + lane;
-            if (tma_c) {
-                // stage 32 rows x 64 columns of this warp in shared memory, store them with one TMA box
-                float *buf = reinterpret_cast<float *>(smem + U::STAGES * STAGE) + (warp - 2) * (32 * 64);
+            const int mrow = it.m0 + 32 * quarter, row = mrow + lane;
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 64) {
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    __syncwarp();
-#pragma unroll 1
-                    for (int h = 0; h < 64; h += 16) {
-                        uint32_t v[16];
-                        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + c0 + h), v);
+            for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += EPI_BOX) {
+                const int n = it.n0 + c0;
+                float x[EPI_BOX];
 #pragma unroll
-                        for (int e = 0; e < 16; e += 4) {
-                            float x0 = got ? __uint_as_float(v[e]) : __int_as_float(0x7fc00000);
-                            float x1 = got ? __uint_as_float(v[e + 1]) : __int_as_float(0x7fc00000);
-                            float x2 = got ? __uint_as_float(v[e + 2]) : __int_as_float(0x7fc00000);
-                            float x3 = got ? __uint_as_float(v[e + 3]) : __int_as_float(0x7fc00000);
-                            if (bias) {
-                                x0 += bias[n0 + c0 + h + e];
-                                x1 += bias[n0 + c0 + h + e + 1];
-                                x2 += bias[n0 + c0 + h + e + 2];
-                                x3 += bias[n0 + c0 + h + e + 3];
-                            }
-                            if (act == 1) {
-                                x0 = gelu(x0);
-                                x1 = gelu(x1);
-                                x2 = gelu(x2);
-                                x3 = gelu(x3);
-                            }
-                            *reinterpret_cast<float4 *>(buf + lane * 64 + h + e) = make_float4(x0, x1, x2, x3);
-                        }
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                for (int h = 0; h < EPI_BOX; h += 16) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(b * BN + c0 + h), v);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) x[h + e] = got ? __uint_as_float(v[e]) : __int_as_float(0x7fc00000);
+                }
+                if (c0 + EPI_BOX == (half + 1) * (BN / 2)) {  // this warp's part of the accumulator is in registers
+                    tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) {
-                        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                                         (uint64_t)&mapC),
-                                     "r"(n0 + c0), "r"(m0 + 32 * q), "r"(smem_u32(buf))
-                                     : "memory");
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+                }
+                if (n >= J.N) continue;  // a tile past the last column (N not a multiple of BN)
+                if (J.bias) {
+#pragma unroll
+                    for (int e = 0; e < EPI_BOX; ++e) x[e] += __ldg(J.bias + n + e);
+                }
+                // staged rows: 16-byte chunk q of row r at chunk q ^ (r % 8) (fp32) or q ^ (r / 2 % 4) (bf16)
+                if (NOUT == 3 && (flags & OUT_PRE)) {
+                    uint8_t *buf = next_buf();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        *reinterpret_cast<float4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+                    epi_store(&J.out[NOUT - 1], buf, n, mrow, it.z, lane);
+                }
+                if (NOUT == 3 && (flags & ACT_GELU)) {
+#pragma unroll
+                    for (int e = 0; e < EPI_BOX; ++e) x[e] = gelu(x[e]);
+                }
+                if (NOUT == 3 && (flags & ACT_GRAD)) {
+                    const float4 *p = reinterpret_cast<const float4 *>(J.gpre + (size_t)min(row, J.M - 1) * J.N + n);
+#pragma unroll
+                    for (int e = 0; e < EPI_BOX; e += 4) {
+                        const float4 pv = p[e / 4];
+                        x[e] = gelu_grad_bf16(x[e], pv.x);
+                        x[e + 1] = gelu_grad_bf16(x[e + 1], pv.y);
+                        x[e + 2] = gelu_grad_bf16(x[e + 2], pv.z);
+                        x[e + 3] = gelu_grad_bf16(x[e + 3], pv.w);
                     }
                 }
-            } else {
-    #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + c0), v);
-                    float x[16];
-    #pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        x[e] = got ? __uint_as_float(v[e]) : __int_as_float(0x7fc00000);
-                        if (bias) x[e] += bias[n0 + c0 + e];
+                if (flags & OUT_F32) {
+                    uint8_t *buf = next_buf();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        *reinterpret_cast<float4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                            make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+                    epi_store(&J.out[0], buf, n, mrow, it.z, lane);
+                }
+                if (NOUT == 3 && (flags & OUT_BF16)) {
+                    __nv_bfloat162 y[EPI_BOX / 2];
+#pragma unroll
+                    for (int e = 0; e < EPI_BOX; e += 2) y[e / 2] = __floats2bfloat162_rn(x[e], x[e + 1]);
+                    if (flags & BF16_DIRECT) {
+                        if (row < J.M) {
+                            __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(J.cb + (size_t)row * J.N + n);
+#pragma unroll
+                            for (int e = 0; e < EPI_BOX / 2; ++e) o[e] = y[e];
+                        }
+                    } else {
+                        uint8_t *buf = next_buf();
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            *reinterpret_cast<uint4 *>(buf + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = *reinterpret_cast<uint4 *>(&y[4 * q]);
+                        epi_store(&J.out[NOUT == 3 ? 1 : 0], buf, n, mrow, it.z, lane);
                     }
-                    const size_t o = (size_t)row * N + n0 + c0;
-                    if (Pre)
-    #pragma unroll
-                        for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4 *>(Pre + o + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
-                    if (act == 1)
-    #pragma unroll
-                        for (int e = 0; e < 16; ++e) x[e] = gelu(x[e]);
-                    if (Cf)
-    #pragma unroll
-                        for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4 *>(Cf + o + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
-                    if (Cb)
-    #pragma unroll
-                        for (int e = 0; e < 16; e += 2) *reinterpret_cast<__nv_bfloat162 *>(Cb + o + e) = __floats2bfloat162_rn(x[e], x[e + 1]);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
-    if (tma_c && warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
     }
 }
 int check(cudaError_t e, const char *what);
 
-// 2-D tensor map of a K-major bf16 operand [rows, K] with boxes of BK x box_rows and the 128-byte swizzle
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn tensor_map_encoder()
 {
-    static EncodeTiledFn enc = nullptr;
-    if (!enc) {
+    static const EncodeTiledFn enc = [] {
         cudaDriverEntryPointQueryResult q;
         void *fn = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            fn && q == cudaDriverEntryPointSuccess)
-            enc = (EncodeTiledFn)fn;
-    }
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess && fn &&
+            q == cudaDriverEntryPointSuccess)
+            return (EncodeTiledFn)fn;
+        return (EncodeTiledFn) nullptr;
+    }();
     return enc;
 }
 
-int operand_map(CUtensorMap *m, const void *ptr, int rows, int K, int box_rows)
+// 2-D map of a bf16 operand of `rows` rows: K-major [rows, K] in boxes of BK x box_rows, or (mn)
+// transposed, [K, rows], in boxes of 64 rows x BK
+int operand_map(CUtensorMap *m, const void *ptr, int rows, int K, int box_rows, bool mn)
 {
     const EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return ewf_fail(EWF_ERR_CUDA, "gemm: cuTensorMapEncodeTiled unavailable");
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)ewf_umma::BK, (cuuint32_t)box_rows};
+    const cuuint64_t inner = mn ? (cuuint64_t)rows : (cuuint64_t)K;
+    const cuuint64_t dims[2] = {inner, mn ? (cuuint64_t)K : (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {inner * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)(mn ? ewf_umma::MN_ATOM : ewf_umma::BK), (cuuint32_t)(mn ? ewf_umma::BK : box_rows)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -348,59 +456,122 @@ int operand_map(CUtensorMap *m, const void *ptr, int rows, int K, int box_rows)
     return r == CUDA_SUCCESS ? EWF_OK : ewf_fail(EWF_ERR_ARG, "gemm: tensor map rejected (CUresult %d)", (int)r);
 }
 
-// tensor map of the fp32 output [M, N] for the staged epilogue: boxes of 64 columns x 32 rows
-int output_map(CUtensorMap *m, float *C, int M, int N)
+// 3-D map of an output [splits, M, N], fp32 or bf16, in boxes of 32 x 32
+int output_map(CUtensorMap *m, void *C, int M, int N, int splits, bool f32)
 {
     const EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return ewf_fail(EWF_ERR_CUDA, "gemm: cuTensorMapEncodeTiled unavailable");
-    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)N * 4};
-    const cuuint32_t box[2] = {64, 32};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint64_t e = f32 ? 4 : 2;
+    const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits};
+    const cuuint64_t strides[2] = {(cuuint64_t)N * e, (cuuint64_t)N * M * e};
+    const cuuint32_t box[3] = {EPI_BOX, EPI_BOX, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, C, dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, f32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? EWF_OK : ewf_fail(EWF_ERR_ARG, "gemm: output tensor map rejected (CUresult %d)", (int)r);
 }
 
-constexpr int EPI_STAGE_BYTES = 4 * 32 * 64 * 4;  // four epilogue warps x 32 rows x 64 fp32
-
-// The kernel's shared-memory attribute is a per-device setting: set once per device ordinal.
-template <int BN>
-int gemm_smem_attribute(int dev, int smem_max)
+// A kernel's shared-memory attribute is a per-device setting: set once per device ordinal.
+template <typename K>
+int gemm_smem_attribute(K kernel, int dev, int bytes)
 {
     static std::mutex mu;
-    static std::set<int> done;
+    static std::set<std::pair<const void *, int>> done;
     std::lock_guard<std::mutex> lock(mu);
-    if (done.count(dev)) return EWF_OK;
-    const cudaError_t e = cudaFuncSetAttribute(k_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+    const auto key = std::make_pair((const void *)kernel, dev);
+    if (done.count(key)) return EWF_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return check(e, "gemm smem attribute");
-    done.insert(dev);
+    done.insert(key);
     return EWF_OK;
 }
 
-template <int BN>
-int launch_gemm(const void *A, const void *B, const float *bias, float *Cf, void *Cb, float *pre, int M, int N, int K,
-                int act, cudaStream_t stream)
+struct Device {
+    int id = 0, sms = 1;
+};
+int this_device(Device *d)
 {
-    int dev = 0, sms = 0;
-    int st = check(cudaGetDevice(&dev), "gemm device");
+    int st = check(cudaGetDevice(&d->id), "device");
     if (st) return st;
-    if ((st = gemm_smem_attribute<BN>(dev, ewf_umma::smem_bytes(BN) + EPI_STAGE_BYTES))) return st;
-    alignas(64) CUtensorMap ma, mb, mc;
-    if ((st = operand_map(&ma, A, M, K, ewf_umma::BM))) return st;
-    if ((st = operand_map(&mb, B, N, K, BN))) return st;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int tiles = (M / ewf_umma::BM) * (N / BN);
-    const int grid = tiles < sms ? tiles : (sms > 0 ? sms : 1);  // one CTA per SM (shared memory bound)
-    // staged TMA stores for an fp32-only output when every SM has two tiles or more (fewer: per-lane
-    // stores win -- 12800 x 512 x 256, 1.3 tiles per SM: 199 against 161 TFLOP/s)
-    const int tma_c = (Cf && !Cb && !pre && tiles >= 2 * sms) ? 1 : 0;
-    memset(&mc, 0, sizeof(mc));
-    if (tma_c && (st = output_map(&mc, Cf, M, N))) return st;
-    const int smem = ewf_umma::smem_bytes(BN) + (tma_c ? EPI_STAGE_BYTES : 0);
-    k_gemm<BN><<<grid, ewf_umma::THREADS, smem, stream>>>(ma, mb, mc, tma_c, bias, Cf, (__nv_bfloat16 *)Cb, pre, M, N, K,
-                                                          act);
-    return check(cudaGetLastError(), "gemm launch");
+    return check(cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, d->id), "device");
+}
+
+// A launch that may start while the stream's previous kernel still runs (its kernel waits for it with
+// griddepcontrol.wait before it reads or writes anything).
+template <typename... P, typename... A>
+int launch_pdl(const char *what, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args)
+{
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return check(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...), what);
+}
+
+template <int BN, bool TA, bool TB, int NJ, int NOUT>
+int gemm_go(const GemmArgs<NJ, NOUT> &g, const Device &dev, cudaStream_t stream)
+{
+    const int smem = Shape<BN>::SMEM;
+    const int st = gemm_smem_attribute(k_gemm<BN, TA, TB, NJ, NOUT>, dev.id, smem);
+    if (st) return st;
+    return launch_pdl("gemm launch", k_gemm<BN, TA, TB, NJ, NOUT>, dim3(g.items < dev.sms ? g.items : dev.sms), dim3(GEMM_THREADS), smem,
+                      stream, g);
+}
+
+int gemm_tiles(int M, int N, int bn) { return ((M + ewf_umma::BM - 1) / ewf_umma::BM) * ((N + bn - 1) / bn); }
+
+struct GemmOut {
+    float *f32 = nullptr;
+    void *bf16 = nullptr;
+    float *pre = nullptr;
+    const float *bias = nullptr, *gpre = nullptr;
+    int act = 0;     // ACT_GELU, ACT_GRAD or 0
+    int splits = 1;  // f32 holds [splits, M, N]
+};
+
+// C = A . B^T (B stored [K, N] when tb).  The tile width: 256 columns once there is a tile per SM, as
+// each stage then feeds the most MMA work; below that narrower tiles, which spread the epilogue over
+// more SMs (128 x 512 x 512 runs on 8 CTAs instead of 2).
+int gemm_one(const void *A, const void *B, bool tb, const GemmOut &o, int M, int N, int K, cudaStream_t stream)
+{
+    Device dev;
+    int st = this_device(&dev);
+    if (st) return st;
+    int bn = 64;
+    if (!tb && N % 256 == 0 && gemm_tiles(M, N, 256) * o.splits >= dev.sms) bn = 256;
+    else if (!tb && gemm_tiles(M, N, 128) * o.splits >= dev.sms) bn = 128;
+    alignas(64) GemmArgs<1, 3> g;
+    memset(&g, 0, sizeof(g));
+    GemmJob<3> &J = g.job[0];
+    if ((st = operand_map(&J.a, A, M, K, ewf_umma::BM, false))) return st;
+    if ((st = operand_map(&J.b, B, N, K, bn, tb))) return st;
+    if (o.f32 && (st = output_map(&J.out[0], o.f32, M, N, o.splits, true))) return st;
+    const bool direct = o.bf16 && ((uintptr_t)o.bf16 & 15);
+    if (o.bf16 && !direct && (st = output_map(&J.out[1], o.bf16, M, N, 1, false))) return st;
+    if (o.pre && (st = output_map(&J.out[2], o.pre, M, N, 1, true))) return st;
+    J.bias = o.bias;
+    J.gpre = o.gpre;
+    J.cb = (__nv_bfloat16 *)o.bf16;
+    J.M = M;
+    J.N = N;
+    J.tiles_n = (N + bn - 1) / bn;
+    J.nk = (K + ewf_umma::BK - 1) / ewf_umma::BK;
+    J.nk_split = (J.nk + o.splits - 1) / o.splits;
+    J.flags = (o.f32 ? OUT_F32 : 0) | (o.bf16 ? OUT_BF16 : 0) | (o.pre ? OUT_PRE : 0) | o.act | (direct ? BF16_DIRECT : 0);
+    g.njobs = 1;
+    g.items = gemm_tiles(M, N, bn) * o.splits;
+    if (tb) return gemm_go<64, false, true>(g, dev, stream);
+    if (bn == 256) return gemm_go<256, false, false>(g, dev, stream);
+    if (bn == 128) return gemm_go<128, false, false>(g, dev, stream);
+    return gemm_go<64, false, false>(g, dev, stream);
 }
 
 __global__ void k_transpose(const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *__restrict__ out, int R, int Cc)
@@ -510,8 +681,13 @@ extern "C" int ewf_mlp_gemm(const void *A, const void *B, const float *bias, flo
     if (act != 0 && act != 1) return ewf_fail(EWF_ERR_ARG, "gemm: act must be 0 or 1");
     if (((uintptr_t)A | (uintptr_t)B) & 15) return ewf_fail(EWF_ERR_ARG, "gemm: A and B must be 16-byte aligned");
     if (((uintptr_t)Cf | (uintptr_t)pre) & 15 || (uintptr_t)Cb & 3) return ewf_fail(EWF_ERR_ARG, "gemm: outputs misaligned");
-    if (N % 256 == 0) return launch_gemm<256>(A, B, bias, Cf, Cb, pre, M, N, K, act, (cudaStream_t)stream);
-    return launch_gemm<128>(A, B, bias, Cf, Cb, pre, M, N, K, act, (cudaStream_t)stream);
+    GemmOut o;
+    o.f32 = Cf;
+    o.bf16 = Cb;
+    o.pre = pre;
+    o.bias = bias;
+    o.act = act == 1 ? ACT_GELU : 0;
+    return gemm_one(A, B, false, o, M, N, K, (cudaStream_t)stream);
 }
 
 extern "C" int ewf_mlp_status(void)

@@ -16,7 +16,7 @@
 // 49-51), layout type in bits 61-63 (2 = SWIZZLE_128B).
 // Instruction descriptor (32 bit, kind::f16): D format F32 (1) in bits 4-5, A and B format BF16
 // (1) in bits 7-9 and 10-12, both K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in
-// bits 24-28.
+// bits 24-28; bits 15 and 16 are set for operands stored MN-major.
 #pragma once
 #include <stdint.h>
 
@@ -35,6 +35,7 @@ constexpr int ROW_BYTES = BK * 2;
 constexpr int ATOM_BYTES = 8 * ROW_BYTES;  // 8 rows x 128 B: the swizzle atom, stride-dimension offset
 constexpr int MMA_K = 16;
 constexpr int THREADS = 192;     // warp 0: TMA producer (one lane); warp 1: MMA issuer (one lane); warps 2-5: epilogue
+constexpr int MORE_EPILOGUE = 128;  // warps 6-9: a second epilogue warp per TMEM lane quarter
 constexpr int LAYOUT_SW128 = 2;
 
 // Per tile width BN (128 or 256): bytes of a stage and of the whole pipeline; TMEM columns = 2 BN
@@ -53,6 +54,38 @@ EWF_UHD uint64_t smem_desc_sw128(uint32_t smem_addr)
     d |= (uint64_t)1 << 46;  // version
     d |= (uint64_t)LAYOUT_SW128 << 61;
     return d;
+}
+
+// An operand stored transposed, [K, rows] with the rows contiguous ("MN-major"): a k-stage is one
+// TMA box of 64 rows x BK per block of 64 rows (blocks BK * 128 = 8192 bytes apart), the box's row k
+// being k's 64 values, 128 bytes, swizzled as above.  The canonical layout's 8-k groups are then 1024
+// bytes apart (stride-dimension offset) and its 64-row atoms 8192 (leading-dimension offset); the
+// k-th MMA of a stage starts 16 k rows, 2048 k bytes, into the block.
+constexpr int MN_ATOM = 64;
+constexpr int MN_BLOCK_BYTES = BK * ROW_BYTES;
+constexpr int MN_K_STEP = MMA_K * ROW_BYTES;
+EWF_UHD uint64_t smem_desc_sw128_mn(uint32_t smem_addr)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
+    d |= (uint64_t)((MN_BLOCK_BYTES >> 4) & 0x3FFF) << 16;
+    d |= (uint64_t)((ATOM_BYTES >> 4) & 0x3FFF) << 32;
+    d |= (uint64_t)1 << 46;  // version
+    d |= (uint64_t)LAYOUT_SW128 << 61;
+    return d;
+}
+// where that layout has the 2-byte element (row mn, k) of an operand block, from the block's start
+EWF_UHD uint32_t mn_offset(int mn, int k)
+{
+    const uint32_t b = (uint32_t)(mn / MN_ATOM) * MN_BLOCK_BYTES + (uint32_t)(k / 8) * ATOM_BYTES + (uint32_t)(k % 8) * ROW_BYTES +
+                       (uint32_t)(mn % MN_ATOM) * 2;
+    return b ^ (((b >> 7) & 7) << 4);
+}
+
+EWF_UHD uint32_t instr_desc_bf16_f32(int m, int n);
+EWF_UHD uint32_t instr_desc_bf16_f32(int m, int n, bool a_mn, bool b_mn)
+{
+    return instr_desc_bf16_f32(m, n) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u);
 }
 
 EWF_UHD uint32_t instr_desc_bf16_f32(int m, int n)
@@ -81,10 +114,11 @@ EWF_UHD uint32_t mma_read_end(uint32_t start, int rows)
 // "full" completion is that slot's (g / STAGES)-th, its "empty" completion frees the slot for
 // stage g + STAGES.  Accumulators: the i-th tile of a CTA uses buffer i % 2; "acc_full" completes
 // once per tile in that buffer, "acc_empty" once per drained tile.
-EWF_UHD int ring_slot(int g) { return g % STAGES; }
-EWF_UHD uint32_t ring_full_parity(int g) { return (uint32_t)(g / STAGES) & 1u; }          // consumer of stage g
-EWF_UHD bool ring_needs_free(int g) { return g >= STAGES; }                               // producer of stage g waits?
-EWF_UHD uint32_t ring_free_parity(int g) { return (uint32_t)(g / STAGES - 1) & 1u; }     // ... for stage g - STAGES
+// (STAGES slots unless a kernel's ring has another number, `stages`)
+EWF_UHD int ring_slot(int g, int stages = STAGES) { return g % stages; }
+EWF_UHD uint32_t ring_full_parity(int g, int stages = STAGES) { return (uint32_t)(g / stages) & 1u; }  // consumer of stage g
+EWF_UHD bool ring_needs_free(int g, int stages = STAGES) { return g >= stages; }                       // producer of stage g waits?
+EWF_UHD uint32_t ring_free_parity(int g, int stages = STAGES) { return (uint32_t)(g / stages - 1) & 1u; }  // ... for stage g - stages
 EWF_UHD int acc_buf(int i) { return i & 1; }
 EWF_UHD uint32_t acc_full_parity(int i) { return (uint32_t)(i >> 1) & 1u; }              // epilogue of tile i
 EWF_UHD bool acc_needs_free(int i) { return i >= 2; }                                     // MMAs of tile i wait?
