@@ -44,13 +44,13 @@ __device__ __forceinline__ float gelu_grad(float x)
 // ---------------------------------------------------------------------------------------------
 // tcgen05 GEMM: C[M,N] = A[M,K] . B[N,K]^T on the 5th-generation tensor cores; A and B are stored either
 // K-major as written or transposed ([K, M], [K, N]: TA, TB), so gradients need no transposed copies.
-// Persistent: one CTA per SM walks the work items (job, K split, 128 x BN tile of C) of one or several
-// independent products.  Two fp32 accumulators of 128 lanes x BN columns in tensor memory, so the
-// epilogue of one item overlaps the MMAs of the next.  Warp roles, 320 threads:
-//   warp 0, one lane: TMA producer -- per k-stage the operands' boxes (128-byte swizzle, ewf_umma.h)
+// Persistent: one CTA per SM walks tiles of one product (a launch may hold two independent ones, each with
+// CTAs of its own).  Two fp32 accumulators of 128 lanes x bn columns in tensor memory, so the
+// epilogue of one tile overlaps the MMAs of the next.  Warp roles, 320 threads:
+//   warp 0: TMA producer -- per k-stage the operands' boxes (128-byte swizzle, ewf_umma.h)
 //     into the next free slot of a ring of stages, completing on that slot's "full" mbarrier; the ring
 //     runs on across items; rows and K beyond a matrix's end read as zeros;
-//   warp 1, one lane: MMA issuer -- waits for a free accumulator ("acc_empty"), then per stage for
+//   warp 1: MMA issuer -- waits for a free accumulator ("acc_empty"), then per stage for
 //     "full", issues 4 tcgen05.mma (K = 16 each) and commits them to the slot's "empty" mbarrier
 //     (freeing it for the producer); after the item's last stage commits "acc_full";
 //   warps 2-9: epilogue -- wait for "acc_full", read the accumulator with tcgen05.ld (a pair of
@@ -61,19 +61,20 @@ __device__ __forceinline__ float gelu_grad(float x)
 // What bounds it at the network's K = 512, where a tile has 8 k-stages: few rows, latency (launch, first
 // loads, epilogue); hidden layers of many rows, the GELU's erff; the output layer, the operands' way
 // from L2 and the output bytes.  With four epilogue warps storing a row per lane, and now: 128 x 512 x
-// 512 24.9 and 8.5 us, 8192 x 512 x 512 25.1 and 15.7, 8192 x 10240 x 512 140 and 93.
+// 512 24.9 and 6.8 us, 8192 x 512 x 512 25.1 and 12.8, 8192 x 10240 x 512 140 and 82.
+// 8192^3 921 and 725 (its 256-column MMAs take 0.27 of a stage's 0.29 us).
 // Every mbarrier wait is bounded (g_umma_wait_limit polls): on timeout the wait raises g_umma_err and
 // gives up (the outputs of that launch are then invalid, ewf_mlp_status reports it), and no later wait
 // of the launch waits at all.  Before the CTA frees its tensor memory and returns, the producer waits
 // (again bounded, with a fixed limit) for the last TMA loads it issued and the MMA issuer for every MMA
 // it issued, whether or not a wait gave up.  Test hook (ewf_mlp_test_hold): the MMA issuers of the
-// CTAs whose first tiles make up the first 256 columns withhold the accumulator-ready signal of one
-// of their items, so the epilogue's wait on it runs out.
+// CTAs whose first tiles lie in the first 128 x 256 of C withhold the accumulator-ready signal of one
+// of their tiles, so the epilogue's wait on it runs out.
 // ---------------------------------------------------------------------------------------------
 __device__ int g_umma_err = 0;
 constexpr int kWaitPolls = 1 << 22;
 __device__ int g_umma_wait_limit = kWaitPolls;
-__device__ int g_umma_hold = -1;  // item (CTA-local index) whose acc_full is withheld; -1: none
+__device__ int g_umma_hold = -1;  // tile (CTA-local index) whose acc_full is withheld; -1: none
 
 __device__ __forceinline__ void mbar_init(uint64_t *b, uint32_t count)
 {
@@ -88,17 +89,30 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *b, uint32_t parity)
                  : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool umma_failed() { return *(volatile int *)&g_umma_err != 0; }
-// Bounded wait; gives up at once when another wait of the launch has already given up.
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity)
+// One lane of a converged warp.  The producer's and the MMA issuer's warps run their loops whole and elect a
+// lane for the instructions themselves: as a loop of one lane under a branch, every wait cost 250 cycles
+// on a barrier that was ready and every MMA 70, a third of a microsecond per k-stage.
+__device__ __forceinline__ bool elect_one()
 {
-    const int limit = *(volatile int *)&g_umma_wait_limit;
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool umma_failed() { return *(volatile int *)&g_umma_err != 0; }
+// Bounded wait (`limit` polls: g_umma_wait_limit, which each thread reads once -- read here, it put a global
+// load's latency, 0.4 us, on every k-stage); gives up at once when another wait of the launch has.
+__device__ __noinline__ bool mbar_wait_on(uint64_t *b, uint32_t parity, int limit)
+{
     for (int i = 0; i < limit; ++i) {
         if (mbar_try_wait(b, parity)) return true;
         if ((i & 1023) == 1023 && umma_failed()) break;
     }
     atomicExch(&g_umma_err, 1);
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, int limit)
+{
+    return mbar_try_wait(b, parity) || mbar_wait_on(b, parity, limit);
 }
 // Wait for asynchronous work this thread issued itself (fixed bound: the work always completes).
 __device__ __forceinline__ void mbar_drain(uint64_t *b, uint32_t parity)
@@ -150,39 +164,44 @@ constexpr int EPI_WARPS = (GEMM_THREADS - 64) / 32;
 constexpr int EPI_BOX = 32;                                    // rows and columns of an output box
 constexpr int EPI_BUF = EPI_BOX * EPI_BOX * 4;
 
-// Shared memory of a tile width: the operand ring and the epilogue's buffers, one or two per warp.  256
-// columns: four stages and one buffer (three stages and two: 8192 x 10240 x 512 98 us instead of 93 --
+// Shared memory of a kernel: the operand ring and the epilogue's buffers, one or two per warp.  256 columns:
+// one buffer and four stages (three stages and two buffers: 8192 x 10240 x 512 98 us instead of 93 --
 // what bounds it is the operand traffic from L2, 393 KB a tile, not the epilogue's wait for a box).
+// The ring is cut into stages of the tile's own size, rows + bn rows of 128 bytes: a small tile has
+// more of them in flight.  An MMA always reads 128 rows from a stage's start; what lies beyond the tile's
+// rows belongs to lanes that are never stored.
+constexpr int MAX_STAGES = 16;
 template <int BN>
 struct Shape {
-    static constexpr int STAGES = BN == 64 ? 8 : BN == 128 ? 5 : 4;
     static constexpr int BUFS = BN == 128 ? 2 : 1;
-    static constexpr int RING = STAGES * ewf_umma::stage_bytes(BN);
+    static constexpr int RING = BN == 128 ? 160 * 1024 : 192 * 1024;
     static constexpr int SMEM = RING + EPI_WARPS * BUFS * EPI_BUF + 1024;  // + alignment slack
     static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
+    static_assert(EPI_WARPS * BUFS * EPI_BUF >= ewf_umma::a_bytes(), "an MMA on the last stage reads inside the allocation");
 };
 
 enum {
     OUT_F32 = 1, OUT_BF16 = 2, OUT_PRE = 4,  // outputs: fp32, bf16, the fp32 value before the activation
     ACT_GELU = 8,
     ACT_GRAD = 16,                           // bf16(value) * GELU'(gpre): the gradient through the activation
-    BF16_DIRECT = 32                         // the bf16 output is not 16-byte aligned: plain stores
+    BF16_DIRECT = 32,                        // the bf16 output is not 16-byte aligned: plain stores
+    TRANS_A = 64, TRANS_B = 128              // the operand is stored [K, rows]
 };
 
 // One product.  Maps of unused outputs are never read.
-template <int NOUT>
 struct GemmJob {
-    CUtensorMap a, b, out[NOUT];  // out: fp32 (and, NOUT = 3, bf16, pre), dimensions N, M, K splits
+    CUtensorMap a, b, f32, bf16, pre;
     const float *bias, *gpre;
     __nv_bfloat16 *cb;
-    int M, N, tiles_n, item0;     // the job's items start at item0
-    int nk, nk_split;             // k-stages, and of one split
+    int M, N, rows, bn;     // tile: rows (32, 64 or 128 of the accumulator's 128 lanes) x bn columns (at most BN)
+    int tiles_n, items, nk;
+    int cta0, ctas;         // its CTAs
     int flags;
 };
-template <int NJ, int NOUT>
+constexpr int MAX_JOBS = 2;
 struct GemmArgs {
-    GemmJob<NOUT> job[NJ];
-    int njobs, items;
+    GemmJob job[MAX_JOBS];
+    int njobs;
 };
 
 __device__ __forceinline__ float gelu_grad_bf16(float x, float pre)
@@ -191,31 +210,31 @@ __device__ __forceinline__ float gelu_grad_bf16(float x, float pre)
 }
 
 // Sends the warp's 32 x 32 staged values off (one lane), after the writes of every lane.
-__device__ __forceinline__ void epi_store(const CUtensorMap *map, const void *buf, int n, int m, int z, int lane)
+__device__ __forceinline__ void epi_store(const CUtensorMap *map, const void *buf, int n, int m, int lane)
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) {
-        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"((uint64_t)map),
-                     "r"(n), "r"(m), "r"(z), "r"(smem_u32(buf))
+        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"((uint64_t)map),
+                     "r"(n), "r"(m), "r"(smem_u32(buf))
                      : "memory");
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
 }
-template <int BN, bool TA, bool TB, int NJ, int NOUT>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant__ GemmArgs<NJ, NOUT> g)
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant__ GemmArgs g)
 {
     namespace U = ewf_umma;
-    constexpr int STAGE = U::stage_bytes(BN), NS = Shape<BN>::STAGES, BUFS = Shape<BN>::BUFS;
+    constexpr int BUFS = Shape<BN>::BUFS;
     constexpr int COLS = 2 * BN;  // tensor-memory columns: two accumulators
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full[NS], empty[NS], acc_full[2], acc_empty[2], mma_drain;
+    __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], mma_drain;
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
 
     if (tid == 0) {
-        for (int s = 0; s < NS; ++s) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -236,88 +255,90 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    const int limit = *(volatile int *)&g_umma_wait_limit;
     bool ok = true;
     // a dependent launch may start setting up; nothing of an earlier launch is read or written before it has completed
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    struct Item {
-        int job, m0, n0, z, kt0, kt1;
-    };
-    auto item_of = [&](int t) {
-        Item it;
-        it.job = 0;
-        while (NJ > 1 && it.job + 1 < g.njobs && t >= g.job[it.job + 1].item0) ++it.job;
-        const GemmJob<NOUT> &J = g.job[it.job];
-        t -= J.item0;
-        const int tiles = ((J.M + U::BM - 1) / U::BM) * J.tiles_n;
-        it.z = t / tiles;
-        t -= it.z * tiles;
-        it.m0 = (t / J.tiles_n) * U::BM;
-        it.n0 = (t % J.tiles_n) * BN;
-        it.kt0 = it.z * J.nk_split;
-        it.kt1 = min(it.kt0 + J.nk_split, J.nk);
-        return it;
-    };
+    const GemmJob &J = g.job[g.njobs > 1 && (int)blockIdx.x >= g.job[1].cta0 ? 1 : 0];
+    // (copied to registers: every asm volatile below would have them read again)
+    const int t0 = (int)blockIdx.x - J.cta0, bn = J.bn, rows = J.rows, items = J.items, ctas = J.ctas, tiles_n = J.tiles_n, nk = J.nk,
+              flags = J.flags, M = J.M, N = J.N;
+    const CUtensorMap *const map_a = &J.a, *const map_b = &J.b;
+    const int a_part = rows * U::ROW_BYTES, stage = a_part + bn * U::ROW_BYTES;
+    const int ns = min(MAX_STAGES, Shape<BN>::RING / stage);
+    const bool ta = flags & TRANS_A, tb = flags & TRANS_B;
 
-    if (warp == 0) {
-        if (lane == 0) {  // TMA producer: every k-stage of every item of this CTA, one ring
-            int q = 0;
-            for (int t = blockIdx.x; t < g.items && ok; t += gridDim.x) {
-                const Item it = item_of(t);
-                const GemmJob<NOUT> &J = g.job[it.job];
-                for (int kt = it.kt0; kt < it.kt1; ++kt, ++q) {
-                    const int s = U::ring_slot(q, NS);
-                    if (U::ring_needs_free(q, NS) && !mbar_wait(&empty[s], U::ring_free_parity(q, NS))) { ok = false; break; }
-                    uint8_t *As = smem + s * STAGE, *Bs = As + U::a_bytes();
-                    mbar_expect_tx(&full[s], STAGE);
-                    if (TA) {
-                        for (int r = 0; r < U::BM; r += U::MN_ATOM)
-                            tma_load_2d(As + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, &J.a, it.m0 + r, kt * U::BK, &full[s]);
+    if (warp == 0) {  // TMA producer: every k-stage of every tile of this CTA, one ring
+        int q = 0, s = 0;          // k-stages issued; slot of the next, and
+        uint32_t free_parity = 1;  // the parity its "empty" wait passes with (1: a fresh barrier)
+        for (int t = t0; t < items && ok; t += ctas) {
+            const int m0 = (t / tiles_n) * rows, n0 = (t % tiles_n) * bn;
+            for (int kt = 0; kt < nk; ++kt, ++q) {
+                if (!mbar_wait(&empty[s], free_parity, limit)) { ok = false; break; }
+                if (elect_one()) {
+                    uint8_t *As = smem + s * stage, *Bs = As + a_part;
+                    mbar_expect_tx(&full[s], (uint32_t)stage);
+                    if (ta) {
+                        for (int r = 0; r < rows; r += U::MN_ATOM)
+                            tma_load_2d(As + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, map_a, m0 + r, kt * U::BK, &full[s]);
                     } else {
-                        tma_load_2d(As, &J.a, kt * U::BK, it.m0, &full[s]);
+                        tma_load_2d(As, map_a, kt * U::BK, m0, &full[s]);
                     }
-                    if (TB) {
-                        for (int r = 0; r < BN; r += U::MN_ATOM)
-                            tma_load_2d(Bs + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, &J.b, it.n0 + r, kt * U::BK, &full[s]);
+                    if (tb) {
+                        for (int r = 0; r < bn; r += U::MN_ATOM)
+                            tma_load_2d(Bs + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, map_b, n0 + r, kt * U::BK, &full[s]);
                     } else {
-                        tma_load_2d(Bs, &J.b, kt * U::BK, it.n0, &full[s]);
+                        tma_load_2d(Bs, map_b, kt * U::BK, n0, &full[s]);
                     }
                 }
+                __syncwarp();
+                if (++s == ns) {
+                    s = 0;
+                    free_parity ^= 1;
+                }
             }
-            // the loads issued last into each slot land before the CTA's shared memory goes
-            for (int p = (q > NS ? q - NS : 0); p < q; ++p)
-                mbar_drain(&full[U::ring_slot(p, NS)], U::ring_full_parity(p, NS));
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // MMA issuer
-            const uint32_t idesc = U::instr_desc_bf16_f32(U::BM, BN, TA, TB);
-            const int hold = blockIdx.x < 256 / BN ? *(volatile int *)&g_umma_hold : -1;
-            int q = 0, i = 0;
-            for (int t = blockIdx.x; t < g.items && ok; t += gridDim.x, ++i) {
-                const Item it = item_of(t);
-                const int b = U::acc_buf(i);
-                if (U::acc_needs_free(i) && !mbar_wait(&acc_empty[b], U::acc_free_parity(i))) { ok = false; break; }
+        // the loads issued last into each slot land before the CTA's shared memory goes
+        for (int p = (q > ns ? q - ns : 0); p < q; ++p)
+            mbar_drain(&full[U::ring_slot(p, ns)], U::ring_full_parity(p, ns));
+    } else if (warp == 1) {  // MMA issuer
+        const uint32_t idesc = U::instr_desc_bf16_f32(U::BM, bn, ta, tb);
+        const bool first = (t0 / tiles_n) * rows < U::BM && (t0 % tiles_n) * bn < 256;
+        const int hold = first ? *(volatile int *)&g_umma_hold : -1;
+        // the K = 16 slices of a stage: start addresses (16-byte units) and descriptors without them
+        const uint64_t da0 = ta ? U::smem_desc_sw128_mn(0) : U::smem_desc_sw128(0), db0 = tb ? U::smem_desc_sw128_mn(0) : U::smem_desc_sw128(0);
+        const int sa = (ta ? U::MN_K_STEP : 32) >> 4, sb = (tb ? U::MN_K_STEP : 32) >> 4;
+        int s = 0, i = 0;
+        uint32_t full_parity = 0;
+        for (int t = t0; t < items && ok; t += ctas, ++i) {
+            const int b = U::acc_buf(i);
+            if (U::acc_needs_free(i) && !mbar_wait(&acc_empty[b], U::acc_free_parity(i), limit)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(b * BN);  // accumulators BN columns apart
+            for (int kt = 0; kt < nk; ++kt) {
+                if (!mbar_wait(&full[s], full_parity, limit)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * BN);
-                for (int kt = it.kt0; kt < it.kt1; ++kt, ++q) {
-                    const int s = U::ring_slot(q, NS);
-                    if (!mbar_wait(&full[s], U::ring_full_parity(q, NS))) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t a0 = smem_u32(smem + s * STAGE), b0 = a0 + U::a_bytes();
+                if (elect_one()) {
+                    const uint32_t a0 = smem_u32(smem + s * stage) >> 4, b0 = a0 + (uint32_t)(a_part >> 4);
+#pragma unroll
                     for (int j = 0; j < U::BK / U::MMA_K; ++j)
-                        umma_bf16(d, TA ? U::smem_desc_sw128_mn(a0 + U::MN_K_STEP * j) : U::smem_desc_sw128(a0 + 32 * j),
-                                  TB ? U::smem_desc_sw128_mn(b0 + U::MN_K_STEP * j) : U::smem_desc_sw128(b0 + 32 * j), idesc,
-                                  (kt > it.kt0 || j > 0) ? 1u : 0u);
+                        umma_bf16(d, da0 + a0 + (uint32_t)(sa * j), db0 + b0 + (uint32_t)(sb * j), idesc, (kt > 0 || j > 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
+                    if (kt == nk - 1 && i != hold) umma_commit(&acc_full[b]);
                 }
-                if (!ok) break;
-                if (i != hold) umma_commit(&acc_full[b]);
+                __syncwarp();
+                if (++s == ns) {
+                    s = 0;
+                    full_parity ^= 1;
+                }
             }
-            // every MMA issued completes before the tensor memory is freed
-            umma_commit(&mma_drain);
-            mbar_drain(&mma_drain, 0);
         }
+        // every MMA issued completes before the tensor memory is freed
+        if (elect_one()) umma_commit(&mma_drain);
+        __syncwarp();
+        mbar_drain(&mma_drain, 0);
     } else {  // epilogue warps 2..9: TMEM lane quarter warp % 4, half of the columns each
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         uint8_t *const bufs = smem + Shape<BN>::RING + (warp - 2) * (BUFS * EPI_BUF);
@@ -331,16 +352,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
             __syncwarp();
             return bufs + (BUFS == 2 ? (nb++ & 1) * EPI_BUF : 0);
         };
-        for (int t = blockIdx.x; t < g.items; t += gridDim.x, ++i) {
-            const Item it = item_of(t);
-            const GemmJob<NOUT> &J = g.job[it.job];
-            const int b = U::acc_buf(i), flags = J.flags;
-            const bool got = !umma_failed() && mbar_wait(&acc_full[b], U::acc_full_parity(i));
+        for (int t = t0; t < items; t += ctas, ++i) {
+            const int m0 = (t / tiles_n) * rows, n0 = (t % tiles_n) * bn;
+            const int b = U::acc_buf(i);
+            const bool got = !umma_failed() && mbar_wait(&acc_full[b], U::acc_full_parity(i), limit);
             tc_fence_after();
-            const int mrow = it.m0 + 32 * quarter, row = mrow + lane;
+            const int mrow = m0 + 32 * quarter, row = mrow + lane;
 #pragma unroll 1
-            for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += EPI_BOX) {
-                const int n = it.n0 + c0;
+            for (int c0 = half * (bn / 2); c0 < (half + 1) * (bn / 2); c0 += EPI_BOX) {
+                const int n = n0 + c0;
                 float x[EPI_BOX];
 #pragma unroll
                 for (int h = 0; h < EPI_BOX; h += 16) {
@@ -349,31 +369,32 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
 #pragma unroll
                     for (int e = 0; e < 16; ++e) x[h + e] = got ? __uint_as_float(v[e]) : __int_as_float(0x7fc00000);
                 }
-                if (c0 + EPI_BOX == (half + 1) * (BN / 2)) {  // this warp's part of the accumulator is in registers
+                if (c0 + EPI_BOX == (half + 1) * (bn / 2)) {  // this warp's part of the accumulator is in registers
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
                 }
-                if (n >= J.N) continue;  // a tile past the last column (N not a multiple of BN)
+                if (32 * quarter >= rows) continue;  // lanes past the tile's rows: what they hold is not part of C
+                if (n >= N) continue;                // columns past the last (N not a multiple of bn)
                 if (J.bias) {
 #pragma unroll
                     for (int e = 0; e < EPI_BOX; ++e) x[e] += __ldg(J.bias + n + e);
                 }
                 // staged rows: 16-byte chunk q of row r at chunk q ^ (r % 8) (fp32) or q ^ (r / 2 % 4) (bf16)
-                if (NOUT == 3 && (flags & OUT_PRE)) {
+                if ((flags & OUT_PRE)) {
                     uint8_t *buf = next_buf();
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         *reinterpret_cast<float4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
                             make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-                    epi_store(&J.out[NOUT - 1], buf, n, mrow, it.z, lane);
+                    epi_store(&J.pre, buf, n, mrow, lane);
                 }
-                if (NOUT == 3 && (flags & ACT_GELU)) {
+                if ((flags & ACT_GELU)) {
 #pragma unroll
                     for (int e = 0; e < EPI_BOX; ++e) x[e] = gelu(x[e]);
                 }
-                if (NOUT == 3 && (flags & ACT_GRAD)) {
-                    const float4 *p = reinterpret_cast<const float4 *>(J.gpre + (size_t)min(row, J.M - 1) * J.N + n);
+                if ((flags & ACT_GRAD)) {
+                    const float4 *p = reinterpret_cast<const float4 *>(J.gpre + (size_t)min(row, M - 1) * N + n);
 #pragma unroll
                     for (int e = 0; e < EPI_BOX; e += 4) {
                         const float4 pv = p[e / 4];
@@ -389,15 +410,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
                     for (int q = 0; q < 8; ++q)
                         *reinterpret_cast<float4 *>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
                             make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-                    epi_store(&J.out[0], buf, n, mrow, it.z, lane);
+                    epi_store(&J.f32, buf, n, mrow, lane);
                 }
-                if (NOUT == 3 && (flags & OUT_BF16)) {
+                if ((flags & OUT_BF16)) {
                     __nv_bfloat162 y[EPI_BOX / 2];
 #pragma unroll
                     for (int e = 0; e < EPI_BOX; e += 2) y[e / 2] = __floats2bfloat162_rn(x[e], x[e + 1]);
                     if (flags & BF16_DIRECT) {
-                        if (row < J.M) {
-                            __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(J.cb + (size_t)row * J.N + n);
+                        if (row < M) {
+                            __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(J.cb + (size_t)row * N + n);
 #pragma unroll
                             for (int e = 0; e < EPI_BOX / 2; ++e) o[e] = y[e];
                         }
@@ -406,7 +427,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                             *reinterpret_cast<uint4 *>(buf + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) = *reinterpret_cast<uint4 *>(&y[4 * q]);
-                        epi_store(&J.out[NOUT == 3 ? 1 : 0], buf, n, mrow, it.z, lane);
+                        epi_store(&J.bf16, buf, n, mrow, lane);
                     }
                 }
             }
@@ -456,17 +477,16 @@ int operand_map(CUtensorMap *m, const void *ptr, int rows, int K, int box_rows, 
     return r == CUDA_SUCCESS ? EWF_OK : ewf_fail(EWF_ERR_ARG, "gemm: tensor map rejected (CUresult %d)", (int)r);
 }
 
-// 3-D map of an output [splits, M, N], fp32 or bf16, in boxes of 32 x 32
-int output_map(CUtensorMap *m, void *C, int M, int N, int splits, bool f32)
+// map of an output [M, N], fp32 or bf16, in boxes of 32 x 32
+int output_map(CUtensorMap *m, void *C, int M, int N, bool f32)
 {
     const EncodeTiledFn enc = tensor_map_encoder();
     if (!enc) return ewf_fail(EWF_ERR_CUDA, "gemm: cuTensorMapEncodeTiled unavailable");
-    const cuuint64_t e = f32 ? 4 : 2;
-    const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits};
-    const cuuint64_t strides[2] = {(cuuint64_t)N * e, (cuuint64_t)N * M * e};
-    const cuuint32_t box[3] = {EPI_BOX, EPI_BOX, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, C, dims, strides, box, estr,
+    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
+    const cuuint64_t strides[1] = {(cuuint64_t)N * (f32 ? 4 : 2)};
+    const cuuint32_t box[2] = {EPI_BOX, EPI_BOX};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, C, dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, f32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? EWF_OK : ewf_fail(EWF_ERR_ARG, "gemm: output tensor map rejected (CUresult %d)", (int)r);
@@ -516,62 +536,102 @@ int launch_pdl(const char *what, void (*kern)(P...), dim3 grid, dim3 block, size
     return check(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...), what);
 }
 
-template <int BN, bool TA, bool TB, int NJ, int NOUT>
-int gemm_go(const GemmArgs<NJ, NOUT> &g, const Device &dev, cudaStream_t stream)
-{
-    const int smem = Shape<BN>::SMEM;
-    const int st = gemm_smem_attribute(k_gemm<BN, TA, TB, NJ, NOUT>, dev.id, smem);
-    if (st) return st;
-    return launch_pdl("gemm launch", k_gemm<BN, TA, TB, NJ, NOUT>, dim3(g.items < dev.sms ? g.items : dev.sms), dim3(GEMM_THREADS), smem,
-                      stream, g);
-}
+int gemm_tiles(int M, int N, int rows, int bn) { return ((M + rows - 1) / rows) * ((N + bn - 1) / bn); }
 
-int gemm_tiles(int M, int N, int bn) { return ((M + ewf_umma::BM - 1) / ewf_umma::BM) * ((N + bn - 1) / bn); }
-
-struct GemmOut {
+// What a product is, apart from its tiles
+struct Product {
+    const void *A = nullptr, *B = nullptr;
+    bool ta = false, tb = false;   // stored [K, M], [K, N]
+    int M = 0, N = 0, K = 0;
     float *f32 = nullptr;
     void *bf16 = nullptr;
     float *pre = nullptr;
     const float *bias = nullptr, *gpre = nullptr;
-    int act = 0;     // ACT_GELU, ACT_GRAD or 0
-    int splits = 1;  // f32 holds [splits, M, N]
+    int act = 0;                   // ACT_GELU, ACT_GRAD or 0
 };
 
-// C = A . B^T (B stored [K, N] when tb).  The tile width: 256 columns once there is a tile per SM, as
-// each stage then feeds the most MMA work; below that narrower tiles, which spread the epilogue over
-// more SMs (128 x 512 x 512 runs on 8 CTAs instead of 2).
-int gemm_one(const void *A, const void *B, bool tb, const GemmOut &o, int M, int N, int K, cudaStream_t stream)
+int make_job(GemmJob *J, const Product &p, int rows, int bn)
+{
+    int st = operand_map(&J->a, p.A, p.M, p.K, rows, p.ta);
+    if (!st) st = operand_map(&J->b, p.B, p.N, p.K, bn, p.tb);
+    if (!st && p.f32) st = output_map(&J->f32, p.f32, p.M, p.N, true);
+    const bool direct = p.bf16 && ((uintptr_t)p.bf16 & 15);
+    if (!st && p.bf16 && !direct) st = output_map(&J->bf16, p.bf16, p.M, p.N, false);
+    if (!st && p.pre) st = output_map(&J->pre, p.pre, p.M, p.N, true);
+    if (st) return st;
+    J->bias = p.bias;
+    J->gpre = p.gpre;
+    J->cb = (__nv_bfloat16 *)p.bf16;
+    J->M = p.M;
+    J->N = p.N;
+    J->rows = rows;
+    J->bn = bn;
+    J->tiles_n = (p.N + bn - 1) / bn;
+    J->items = gemm_tiles(p.M, p.N, rows, bn);
+    J->nk = (p.K + ewf_umma::BK - 1) / ewf_umma::BK;
+    J->flags = (p.f32 ? OUT_F32 : 0) | (p.bf16 ? OUT_BF16 : 0) | (p.pre ? OUT_PRE : 0) | p.act | (direct ? BF16_DIRECT : 0) |
+               (p.ta ? TRANS_A : 0) | (p.tb ? TRANS_B : 0);
+    return EWF_OK;
+}
+
+template <int BN>
+int gemm_go(const GemmArgs &g, int ctas, const Device &dev, cudaStream_t stream)
+{
+    const int st = gemm_smem_attribute(k_gemm<BN>, dev.id, Shape<BN>::SMEM);
+    if (st) return st;
+    return launch_pdl("gemm launch", k_gemm<BN>, dim3(ctas), dim3(GEMM_THREADS), Shape<BN>::SMEM, stream, g);
+}
+
+// One product.  The tile width: 256 columns once there is a tile per SM, as each stage then feeds the most
+// MMA work; below that narrower tiles and, as long as every tile still has an SM, fewer rows, which spread
+// operands and epilogue over more of them (128 x 512 x 512 runs on 32 CTAs instead of 2).
+int gemm_one(const Product &p, cudaStream_t stream)
 {
     Device dev;
     int st = this_device(&dev);
     if (st) return st;
-    int bn = 64;
-    if (!tb && N % 256 == 0 && gemm_tiles(M, N, 256) * o.splits >= dev.sms) bn = 256;
-    else if (!tb && gemm_tiles(M, N, 128) * o.splits >= dev.sms) bn = 128;
-    alignas(64) GemmArgs<1, 3> g;
+    int bn = 64, rows = ewf_umma::BM;
+    if (p.N % 256 == 0 && gemm_tiles(p.M, p.N, ewf_umma::BM, 256) >= dev.sms) bn = 256;
+    else if (gemm_tiles(p.M, p.N, ewf_umma::BM, 128) >= dev.sms) bn = 128;
+    else if (!p.ta)
+        while (rows > 32 && gemm_tiles(p.M, p.N, rows / 2, 64) <= dev.sms) rows /= 2;
+    alignas(64) GemmArgs g;
     memset(&g, 0, sizeof(g));
-    GemmJob<3> &J = g.job[0];
-    if ((st = operand_map(&J.a, A, M, K, ewf_umma::BM, false))) return st;
-    if ((st = operand_map(&J.b, B, N, K, bn, tb))) return st;
-    if (o.f32 && (st = output_map(&J.out[0], o.f32, M, N, o.splits, true))) return st;
-    const bool direct = o.bf16 && ((uintptr_t)o.bf16 & 15);
-    if (o.bf16 && !direct && (st = output_map(&J.out[1], o.bf16, M, N, 1, false))) return st;
-    if (o.pre && (st = output_map(&J.out[2], o.pre, M, N, 1, true))) return st;
-    J.bias = o.bias;
-    J.gpre = o.gpre;
-    J.cb = (__nv_bfloat16 *)o.bf16;
-    J.M = M;
-    J.N = N;
-    J.tiles_n = (N + bn - 1) / bn;
-    J.nk = (K + ewf_umma::BK - 1) / ewf_umma::BK;
-    J.nk_split = (J.nk + o.splits - 1) / o.splits;
-    J.flags = (o.f32 ? OUT_F32 : 0) | (o.bf16 ? OUT_BF16 : 0) | (o.pre ? OUT_PRE : 0) | o.act | (direct ? BF16_DIRECT : 0);
+    GemmJob &J = g.job[0];
+    if ((st = make_job(&J, p, rows, bn))) return st;
+    J.ctas = J.items < dev.sms ? J.items : dev.sms;
     g.njobs = 1;
-    g.items = gemm_tiles(M, N, bn) * o.splits;
-    if (tb) return gemm_go<64, false, true>(g, dev, stream);
-    if (bn == 256) return gemm_go<256, false, false>(g, dev, stream);
-    if (bn == 128) return gemm_go<128, false, false>(g, dev, stream);
-    return gemm_go<64, false, false>(g, dev, stream);
+    if (bn == 256) return gemm_go<256>(g, J.ctas, dev, stream);
+    if (bn == 128) return gemm_go<128>(g, J.ctas, dev, stream);
+    return gemm_go<64>(g, J.ctas, dev, stream);
+}
+
+// The two products of a layer's backward pass in one launch: dH = dY . W (its K, the layer's outputs, may be
+// far larger than its tiles are many) and gW = dY^T . H.  dH gets a CTA per tile and gW the SMs that are
+// left, so the second hides behind the first.  A dH tile takes the operands of a 64-column tile from L2
+// and multiplies stage after stage, 0.23 us each whatever its size -- its K is not split, so that its sums
+// keep their order -- so small tiles cost nothing and spread the work: 32 or 64 of the accumulator's 128 lanes
+// while CTAs for them and as many again for gW are there.  256 x 512 from K = 10240: 110 us on 4 CTAs of 128 x
+// 256 at 0.7 us a stage, now 40 with the weight gradient behind it.
+int gemm_pair(const Product &dh, const Product &gw, cudaStream_t stream)
+{
+    Device dev;
+    int st = this_device(&dev);
+    if (st) return st;
+    int rows = ewf_umma::BM;
+    while (rows > 32 && gemm_tiles(dh.M, dh.N, rows / 2, 64) <= dev.sms / 2) rows /= 2;
+    alignas(64) GemmArgs g;
+    memset(&g, 0, sizeof(g));
+    GemmJob &a = g.job[0], &b = g.job[1];
+    if ((st = make_job(&a, dh, rows, 64))) return st;
+    if ((st = make_job(&b, gw, ewf_umma::BM, gemm_tiles(gw.M, gw.N, ewf_umma::BM, 128) >= dev.sms / 2 ? 128 : 64))) return st;
+    const int left = dev.sms - a.items;
+    a.ctas = left >= dev.sms / 4 ? a.items : a.items < dev.sms ? a.items : dev.sms;
+    g.njobs = 2;
+    b.cta0 = a.ctas;
+    b.ctas = left >= dev.sms / 4 ? left : dev.sms;  // dH fills the GPU by itself: gW's CTAs follow
+    if (b.ctas > b.items) b.ctas = b.items;
+    return gemm_go<128>(g, a.ctas + b.ctas, dev, stream);
 }
 
 __global__ void k_transpose(const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *__restrict__ out, int R, int Cc)
@@ -638,6 +698,152 @@ __global__ void k_adam(float *__restrict__ w, float *__restrict__ m, float *__re
         const float we = w[e] - lr * (me / c1) / (sqrtf(ve / c2) + eps);
         w[e] = we;
         if (wb) wb[e] = __float2bfloat16_rn(we);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The training step's own forms of the kernels above: every layer's work of one kind in one launch,
+// 16-byte accesses, started while the launch before ends.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Bias gradients of every layer: a CTA sums 64 columns, a pair of columns per lane and every 32nd row per
+// warp, then the 32 warps' sums in order.  (A thread per column over all rows: 256 x 10240 20 us.)
+constexpr int BIAS_GROUP = 8;
+struct BiasJobs {
+    const __nv_bfloat16 *dy[BIAS_GROUP];
+    float *db[BIAS_GROUP];
+    int N[BIAS_GROUP], block0[BIAS_GROUP];
+    int n, M;
+};
+__global__ void __launch_bounds__(1024) k_bias_grads(const BiasJobs J)
+{
+    __shared__ float2 part[32][33];
+    pdl_wait();
+    int q = 0;
+    while (q + 1 < J.n && (int)blockIdx.x >= J.block0[q + 1]) ++q;
+    const int N = J.N[q], lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int col = ((int)blockIdx.x - J.block0[q]) * 64 + 2 * lane;
+    float2 s = make_float2(0.f, 0.f);
+    if (col < N) {
+        const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(J.dy[q] + col);
+#pragma unroll 8
+        for (int m = warp; m < J.M; m += 32) {
+            const float2 v = __bfloat1622float2(p[(size_t)m * (N / 2)]);
+            s.x += v.x;
+            s.y += v.y;
+        }
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && col < N) {
+        float2 t = part[0][lane];
+        for (int w = 1; w < 32; ++w) {
+            t.x += part[w][lane].x;
+            t.y += part[w][lane].y;
+        }
+        J.db[q][col] = t.x;
+        J.db[q][col + 1] = t.y;
+    }
+}
+
+// k_mse_grad four values at a time (n % 4 == 0, aligned), with the loss from the partial sums by the last
+// CTA to finish: done counts the CTAs and is left at zero.
+__global__ void __launch_bounds__(256) k_mse_loss(const float4 *__restrict__ y, const float4 *__restrict__ t, uint2 *__restrict__ dy,
+                                                  size_t n4, float scale, float *__restrict__ part, unsigned *__restrict__ done,
+                                                  float *__restrict__ loss)
+{
+    __shared__ float red[256];
+    __shared__ bool last;
+    pdl_wait();
+    float s = 0.f;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n4; e += (size_t)gridDim.x * blockDim.x) {
+        const float4 a = y[e], b = __ldcs(t + e);
+        const float d[4] = {a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s += d[q] * d[q];
+        __nv_bfloat162 o[2] = {__floats2bfloat162_rn(2.f * d[0] * scale, 2.f * d[1] * scale),
+                               __floats2bfloat162_rn(2.f * d[2] * scale, 2.f * d[3] * scale)};
+        dy[e] = *reinterpret_cast<uint2 *>(o);
+    }
+    auto block_sum = [&](float v) {
+        red[threadIdx.x] = v;
+        __syncthreads();
+        for (int w = 128; w > 0; w >>= 1) {
+            if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+            __syncthreads();
+        }
+    };
+    block_sum(s);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = red[0];
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    float v = 0.f;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) v += *(volatile float *)&part[b];
+    block_sum(v);
+    if (threadIdx.x == 0) {
+        *loss = red[0] * scale;
+        *done = 0u;
+    }
+}
+
+// k_adam over several tensors, four elements per thread (16-byte aligned; a tensor's tail by its last
+// threads).  Bound by memory, 28 bytes an element and 2 for the bf16 copy.
+constexpr int ADAM_GROUP = 16, ADAM_BLOCK = 256 * 4;  // elements per CTA
+struct AdamJobs {
+    float *w[ADAM_GROUP], *m[ADAM_GROUP], *v[ADAM_GROUP];
+    const float *g[ADAM_GROUP];
+    __nv_bfloat16 *wb[ADAM_GROUP];
+    unsigned n[ADAM_GROUP], block0[ADAM_GROUP];
+    float wd[ADAM_GROUP];
+    int njobs;
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ void adam_one(const AdamJobs &J, float wd, float &w, float &m, float &v, float g)
+{
+    const float ge = g + wd * w;
+    const float me = J.b1 * m + (1.f - J.b1) * ge;
+    const float ve = J.b2 * v + (1.f - J.b2) * ge * ge;
+    m = me;
+    v = ve;
+    w = w - J.lr * (me / J.c1) / (sqrtf(ve / J.c2) + J.eps);
+}
+__global__ void __launch_bounds__(256) k_adam_all(const AdamJobs J)
+{
+    pdl_wait();
+    int q = 0;
+    while (q + 1 < J.njobs && blockIdx.x >= J.block0[q + 1]) ++q;
+    const unsigned e = (blockIdx.x - J.block0[q]) * ADAM_BLOCK + threadIdx.x * 4, n = J.n[q];
+    const float wd = J.wd[q];
+    if (e + 4 <= n) {
+        float4 w = *reinterpret_cast<float4 *>(J.w[q] + e), m = *reinterpret_cast<float4 *>(J.m[q] + e),
+               v = *reinterpret_cast<float4 *>(J.v[q] + e);
+        const float4 g = *reinterpret_cast<const float4 *>(J.g[q] + e);
+        adam_one(J, wd, w.x, m.x, v.x, g.x);
+        adam_one(J, wd, w.y, m.y, v.y, g.y);
+        adam_one(J, wd, w.z, m.z, v.z, g.z);
+        adam_one(J, wd, w.w, m.w, v.w, g.w);
+        *reinterpret_cast<float4 *>(J.w[q] + e) = w;
+        *reinterpret_cast<float4 *>(J.m[q] + e) = m;
+        *reinterpret_cast<float4 *>(J.v[q] + e) = v;
+        if (J.wb[q]) {
+            __nv_bfloat162 o[2] = {__floats2bfloat162_rn(w.x, w.y), __floats2bfloat162_rn(w.z, w.w)};
+            *reinterpret_cast<uint2 *>(J.wb[q] + e) = *reinterpret_cast<uint2 *>(o);
+        }
+    } else {
+        for (unsigned k = e; k < n; ++k) {
+            adam_one(J, wd, J.w[q][k], J.m[q][k], J.v[q][k], J.g[q][k]);
+            if (J.wb[q]) J.wb[q][k] = __float2bfloat16_rn(J.w[q][k]);
+        }
     }
 }
 
@@ -739,13 +945,168 @@ extern "C" int ewf_mlp_gemm(const void *A, const void *B, const float *bias, flo
     if (act != 0 && act != 1) return ewf_fail(EWF_ERR_ARG, "gemm: act must be 0 or 1");
     if (((uintptr_t)A | (uintptr_t)B) & 15) return ewf_fail(EWF_ERR_ARG, "gemm: A and B must be 16-byte aligned");
     if (((uintptr_t)Cf | (uintptr_t)pre) & 15 || (uintptr_t)Cb & 3) return ewf_fail(EWF_ERR_ARG, "gemm: outputs misaligned");
-    GemmOut o;
-    o.f32 = Cf;
-    o.bf16 = Cb;
-    o.pre = pre;
-    o.bias = bias;
-    o.act = act == 1 ? ACT_GELU : 0;
-    return gemm_one(A, B, false, o, M, N, K, (cudaStream_t)stream);
+    Product p;
+    p.A = A;
+    p.B = B;
+    p.M = M;
+    p.N = N;
+    p.K = K;
+    p.f32 = Cf;
+    p.bf16 = Cb;
+    p.pre = pre;
+    p.bias = bias;
+    p.act = act == 1 ? ACT_GELU : 0;
+    return gemm_one(p, (cudaStream_t)stream);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The network's passes, one call each
+// ---------------------------------------------------------------------------------------------
+namespace {
+// rows: the gradients' row count has to be a multiple of 128, as ewf_mlp_gemm's
+int check_net(const char *what, int32_t n, const int32_t *sizes, int32_t M, int in_mult)
+{
+    if (n < 1 || n > 64 || !sizes || M <= 0) return ewf_fail(EWF_ERR_ARG, "%s: bad network or batch", what);
+    if (sizes[0] <= 0 || sizes[0] % in_mult) return ewf_fail(EWF_ERR_ARG, "%s: the input width must be a multiple of %d", what, in_mult);
+    for (int l = 1; l <= n; ++l)
+        if (sizes[l] <= 0 || sizes[l] % 128) return ewf_fail(EWF_ERR_ARG, "%s: layer widths must be multiples of 128 (got %d)", what, sizes[l]);
+    return EWF_OK;
+}
+bool misaligned(const void *p) { return ((uintptr_t)p & 15) != 0; }
+}  // namespace
+
+extern "C" int ewf_mlp_forward(int32_t n, const int32_t *sizes, const void *X, const void *const *W, const float *const *b,
+                               void *const *H, float *const *P, float *Y, int32_t M, void *stream)
+{
+    int st = check_net("forward", n, sizes, M, 32);
+    if (st) return st;
+    if (!X || !W || !b || !Y || (n > 1 && !H)) return ewf_fail(EWF_ERR_ARG, "forward: NULL argument");
+    for (int l = 0; l < n; ++l) {
+        const void *in = l ? H[l - 1] : X;
+        const bool last = l == n - 1;
+        Product o;
+        o.A = in;
+        o.B = W[l];
+        o.M = M;
+        o.N = sizes[l + 1];
+        o.K = sizes[l];
+        o.bias = b[l];
+        o.f32 = last ? Y : nullptr;
+        o.bf16 = last ? nullptr : H[l];
+        o.pre = last || !P ? nullptr : P[l];
+        o.act = last ? 0 : ACT_GELU;
+        if (!in || !W[l] || (!last && (!H[l] || (P && !P[l])))) return ewf_fail(EWF_ERR_ARG, "forward: NULL buffer of layer %d", l);
+        if (misaligned(in) || misaligned(W[l]) || misaligned(o.f32) || misaligned(o.bf16) || misaligned(o.pre))
+            return ewf_fail(EWF_ERR_ARG, "forward: buffers of layer %d must be 16-byte aligned", l);
+        if ((st = gemm_one(o, (cudaStream_t)stream))) return st;
+    }
+    return EWF_OK;
+}
+
+extern "C" int ewf_mlp_backward(int32_t n, const int32_t *sizes, const void *const *H, const void *const *W, const float *const *P,
+                                void *const *dY, float *const *gW, float *const *gb, int32_t M, void *stream)
+{
+    int st = check_net("backward", n, sizes, M, 128);
+    if (st) return st;
+    if (M % 128) return ewf_fail(EWF_ERR_ARG, "backward: the batch must be a multiple of 128 (got %d)", M);
+    if (!H || !W || !dY || !gW || !gb || (n > 1 && !P)) return ewf_fail(EWF_ERR_ARG, "backward: NULL argument");
+    for (int l = 0; l < n; ++l) {
+        if (!H[l] || !W[l] || !dY[l] || !gW[l] || !gb[l] || (l < n - 1 && !P[l])) return ewf_fail(EWF_ERR_ARG, "backward: NULL buffer of layer %d", l);
+        if (misaligned(H[l]) || misaligned(W[l]) || misaligned(dY[l]) || misaligned(gW[l]) || (l < n - 1 && misaligned(P[l])))
+            return ewf_fail(EWF_ERR_ARG, "backward: buffers of layer %d must be 16-byte aligned", l);
+    }
+    const cudaStream_t s = (cudaStream_t)stream;
+    for (int l = n - 1; l >= 0; --l) {
+        Product gw;  // gW[nout, nin] = dY[M, nout]^T . H[M, nin]
+        gw.A = dY[l];
+        gw.B = H[l];
+        gw.ta = gw.tb = true;
+        gw.M = sizes[l + 1];
+        gw.N = sizes[l];
+        gw.K = M;
+        gw.f32 = gW[l];
+        if (l == 0) {
+            if ((st = gemm_one(gw, s))) return st;
+            break;
+        }
+        Product dh;  // dY of the layer before: (dY[M, nout] . W[nout, nin]) GELU'(P)
+        dh.A = dY[l];
+        dh.B = W[l];
+        dh.tb = true;
+        dh.M = M;
+        dh.N = sizes[l];
+        dh.K = sizes[l + 1];
+        dh.bf16 = dY[l - 1];
+        dh.gpre = P[l - 1];
+        dh.act = ACT_GRAD;
+        if ((st = gemm_pair(dh, gw, s))) return st;
+    }
+    // every layer's bias gradient, BIAS_GROUP layers at a time
+    for (int l0 = 0; l0 < n; l0 += BIAS_GROUP) {
+        BiasJobs bj;
+        memset(&bj, 0, sizeof(bj));
+        int blocks = 0;
+        bj.n = n - l0 < BIAS_GROUP ? n - l0 : BIAS_GROUP;
+        bj.M = M;
+        for (int q = 0; q < bj.n; ++q) {
+            bj.dy[q] = (const __nv_bfloat16 *)dY[l0 + q];
+            bj.db[q] = gb[l0 + q];
+            bj.N[q] = sizes[l0 + q + 1];
+            bj.block0[q] = blocks;
+            blocks += sizes[l0 + q + 1] / 64;
+        }
+        if ((st = launch_pdl("bias_grad launch", k_bias_grads, dim3(blocks), dim3(1024), 0, s, bj))) return st;
+    }
+    return EWF_OK;
+}
+
+extern "C" int ewf_mlp_mse_loss(const float *y, const float *t, void *dy, size_t n, float scale, float *part, int32_t nblocks, void *done,
+                                float *loss, void *stream)
+{
+    if (!y || !t || !dy || !part || !done || !loss || nblocks < 1 || n == 0 || n % 4) return ewf_fail(EWF_ERR_ARG, "mse_loss: bad argument");
+    if (misaligned(y) || misaligned(t) || ((uintptr_t)dy & 7)) return ewf_fail(EWF_ERR_ARG, "mse_loss: misaligned");
+    return launch_pdl("mse_loss launch", k_mse_loss, dim3(nblocks), dim3(256), 0, (cudaStream_t)stream, (const float4 *)y, (const float4 *)t,
+                      (uint2 *)dy, n / 4, scale, part, (unsigned *)done, loss);
+}
+
+extern "C" int ewf_mlp_adam_all(int32_t count, float *const *w, float *const *m, float *const *v, const float *const *g, void *const *wb,
+                                const size_t *n, const float *wd, float lr, float b1, float b2, float eps, int32_t step, void *stream)
+{
+    if (count < 1 || !w || !m || !v || !g || !wb || !n || !wd || step < 1) return ewf_fail(EWF_ERR_ARG, "adam: bad argument");
+    for (int q = 0; q < count; ++q) {
+        if (!w[q] || !m[q] || !v[q] || !g[q]) return ewf_fail(EWF_ERR_ARG, "adam: NULL tensor %d", q);
+        if (misaligned(w[q]) || misaligned(m[q]) || misaligned(v[q]) || misaligned(g[q]) || ((uintptr_t)wb[q] & 7))
+            return ewf_fail(EWF_ERR_ARG, "adam: tensor %d must be 16-byte aligned", q);
+        if (n[q] >= (1ull << 31)) return ewf_fail(EWF_ERR_ARG, "adam: tensor %d too large", q);
+    }
+    for (int q0 = 0; q0 < count; q0 += ADAM_GROUP) {
+        AdamJobs J;
+        memset(&J, 0, sizeof(J));
+        J.njobs = count - q0 < ADAM_GROUP ? count - q0 : ADAM_GROUP;
+        unsigned blocks = 0;
+        for (int e = 0; e < J.njobs; ++e) {
+            const int q = q0 + e;
+            J.w[e] = w[q];
+            J.m[e] = m[q];
+            J.v[e] = v[q];
+            J.g[e] = g[q];
+            J.wb[e] = (__nv_bfloat16 *)wb[q];
+            J.n[e] = (unsigned)n[q];
+            J.wd[e] = wd[q];
+            J.block0[e] = blocks;
+            blocks += (unsigned)((n[q] + ADAM_BLOCK - 1) / ADAM_BLOCK);
+        }
+        J.lr = lr;
+        J.b1 = b1;
+        J.b2 = b2;
+        J.eps = eps;
+        J.c1 = 1.f - powf(b1, (float)step);
+        J.c2 = 1.f - powf(b2, (float)step);
+        if (blocks == 0) continue;
+        const int st = launch_pdl("adam launch", k_adam_all, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, J);
+        if (st) return st;
+    }
+    return EWF_OK;
 }
 
 extern "C" int ewf_mlp_status(void)

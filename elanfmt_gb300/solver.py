@@ -109,6 +109,14 @@ SIGNATURES = {
     "ewf_batch_get_l2_prefetch": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
     "ewf_mlp_gemm": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32,
                                C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
+    "ewf_mlp_forward": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                  C.c_int32, C.c_void_p]),
+    "ewf_mlp_backward": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                   C.c_int32, C.c_void_p]),
+    "ewf_mlp_mse_loss": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_float, C.c_void_p, C.c_int32, C.c_void_p,
+                                   C.c_void_p, C.c_void_p]),
+    "ewf_mlp_adam_all": (C.c_int, [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                   C.c_float, C.c_float, C.c_float, C.c_float, C.c_int32, C.c_void_p]),
     "ewf_mlp_status": (C.c_int, []),
     "ewf_sosfilt": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_int64, C.c_int64]),
     "ewf_sosfilt_device": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),

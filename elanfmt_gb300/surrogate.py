@@ -28,7 +28,7 @@ import numpy as np
 from . import fields as F
 from . import inputs as I
 from . import runs
-from .solver import Batch, _check, load_library
+from .solver import Batch, EwfError, _check, load_library
 
 IN_PAD = 128          # inputs padded to one GEMM tile
 NCOMP = 18            # 6 moment tensors x 3 velocity components
@@ -42,6 +42,11 @@ def _stream():
 
 def _p(t) -> C.c_void_p:
     return C.c_void_p(t.data_ptr())
+
+
+def _ptrs(ts):
+    """Array of the tensors' device pointers (of the call's own: tensors may be replaced between calls)."""
+    return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
 class MLP:
@@ -78,6 +83,8 @@ class MLP:
                 lst.append(torch.zeros(fan_out, device="cuda"))
         self.step_count = 0
         self._ws = {}
+        self._sizes = (C.c_int32 * len(sizes))(*sizes)
+        self._act = []   # inference: two activation buffers, for the most rows seen
 
     @property
     def nlayers(self) -> int:
@@ -91,32 +98,41 @@ class MLP:
                  "P": [t.empty(M, s[l + 1], device="cuda") for l in range(self.nlayers - 1)],
                  "Y": t.empty(M, s[-1], device="cuda"),
                  "dY": [t.empty(M, s[l + 1], dtype=t.bfloat16, device="cuda") for l in range(self.nlayers)],
-                 "dH": [t.empty(M, s[l], dtype=t.bfloat16, device="cuda") for l in range(self.nlayers)],
-                 "dYt": [t.empty(s[l + 1], M, dtype=t.bfloat16, device="cuda") for l in range(self.nlayers)],
-                 "Ht": [t.empty(s[l], M, dtype=t.bfloat16, device="cuda") for l in range(self.nlayers)],
-                 "Wt": [t.empty(s[l], s[l + 1], dtype=t.bfloat16, device="cuda") for l in range(self.nlayers)],
                  "gW": [t.empty(s[l + 1], s[l], device="cuda") for l in range(self.nlayers)],
                  "gb": [t.empty(s[l + 1], device="cuda") for l in range(self.nlayers)],
-                 "part": t.empty(1024, device="cuda")}
+                 "part": t.empty(1024, device="cuda"), "done": t.zeros(1, dtype=t.int32, device="cuda")}
             self._ws[M] = w
         return self._ws[M]
 
+    def _forward(self, X, H, P, Y, M: int) -> None:
+        """The library's forward pass of M rows: X aligned bf16 rows, H and P the hidden layers' buffers."""
+        _check(self.lib.ewf_mlp_forward(self.nlayers, self._sizes, _p(X), _ptrs(self.Wb), _ptrs(self.b), H, P, _p(Y), M,
+                                        _stream()), "ewf_mlp_forward")
+
     def forward(self, X, Y=None, keep_pre: bool = True) -> "torch.Tensor":
-        """X: bf16 [M, sizes[0]] on the GPU; returns the fp32 output [M, sizes[-1]], written into Y
-        when given (contiguous rows, e.g. a row slice of the caller's output), else into the
+        """X: bf16 [M, sizes[0]] on the GPU, M a multiple of 128; returns the fp32 output [M, sizes[-1]],
+        written into Y when given (contiguous rows, e.g. a row slice of the caller's output), else into the
         workspace.  keep_pre=False skips the pre-activations (only the backward pass reads them)."""
         M = X.shape[0]
+        if M % 128:
+            raise EwfError(-1, "ewf_mlp_forward", f"the batch must be a multiple of 128 (got {M})")
         w = self._work(M)
-        st = _stream()
         w["H"][0].copy_(X)
         Yd = w["Y"] if Y is None else Y
-        for l in range(self.nlayers):
-            last = l == self.nlayers - 1
-            _check(self.lib.ewf_mlp_gemm(_p(w["H"][l]), _p(self.Wb[l]), _p(self.b[l]),
-                                         _p(Yd) if last else None, None if last else _p(w["H"][l + 1]),
-                                         None if (last or not keep_pre) else _p(w["P"][l]), M, self.sizes[l + 1],
-                                         self.sizes[l], 0 if last else 1, st), "ewf_mlp_gemm")
+        self._forward(w["H"][0], _ptrs(w["H"][1:]), _ptrs(w["P"]) if keep_pre else None, Yd, M)
         return Yd
+
+    def _infer(self, X, Y) -> None:
+        """Forward pass of any number of rows, written to Y; hidden activations alternate between two buffers."""
+        t = self.torch
+        M = X.shape[0]
+        if not (X.dtype == t.bfloat16 and X.is_cuda and X.is_contiguous() and X.shape[1] == self.sizes[0]
+                and X.data_ptr() % 16 == 0):
+            X = t.empty(M, self.sizes[0], dtype=t.bfloat16, device="cuda").copy_(X)
+        need = M * max(self.sizes[1:-1], default=0)
+        if not self._act or self._act[0].numel() < need:
+            self._act = [t.empty(max(need, 8), dtype=t.bfloat16, device="cuda") for _ in range(2)]
+        self._forward(X, _ptrs([self._act[l & 1] for l in range(self.nlayers - 1)]), None, Y, M)
 
     def loss_grad(self, T) -> "torch.Tensor":
         """MSE against fp32 targets T; dY of the last layer into the workspace; returns the loss."""
@@ -124,41 +140,31 @@ class MLP:
         w = self._work(M)
         n = w["Y"].numel()
         nb = 1024
-        _check(self.lib.ewf_mlp_mse_grad(_p(w["Y"]), _p(T), _p(w["dY"][-1]), n, C.c_float(1.0 / n), _p(w["part"]), nb,
-                                         _stream()), "ewf_mlp_mse_grad")
-        return w["part"].sum() / n
+        if T.data_ptr() % 16:
+            _check(self.lib.ewf_mlp_mse_grad(_p(w["Y"]), _p(T), _p(w["dY"][-1]), n, C.c_float(1.0 / n), _p(w["part"]), nb,
+                                             _stream()), "ewf_mlp_mse_grad")
+            return w["part"].sum() / n
+        loss = self.torch.empty((), device="cuda")
+        _check(self.lib.ewf_mlp_mse_loss(_p(w["Y"]), _p(T), _p(w["dY"][-1]), n, C.c_float(1.0 / n), _p(w["part"]), nb,
+                                         _p(w["done"]), _p(loss), _stream()), "ewf_mlp_mse_loss")
+        return loss
 
     def backward(self, M: int) -> None:
         w = self._work(M)
-        st = _stream()
-        L = self.nlayers
-        for l in range(L - 1, -1, -1):
-            nout, nin = self.sizes[l + 1], self.sizes[l]
-            # dW = dY^T H: A = dY^T [nout, M], B = H^T [nin, M]
-            _check(self.lib.ewf_mlp_transpose(_p(w["dY"][l]), _p(w["dYt"][l]), M, nout, st), "transpose")
-            _check(self.lib.ewf_mlp_transpose(_p(w["H"][l]), _p(w["Ht"][l]), M, nin, st), "transpose")
-            _check(self.lib.ewf_mlp_gemm(_p(w["dYt"][l]), _p(w["Ht"][l]), None, _p(w["gW"][l]), None, None, nout, nin, M,
-                                         0, st), "gemm dW")
-            _check(self.lib.ewf_mlp_bias_grad(_p(w["dY"][l]), _p(w["gb"][l]), M, nout, st), "bias_grad")
-            if l > 0:
-                # dH = dY W: A = dY [M, nout], B = W^T [nin, nout]
-                _check(self.lib.ewf_mlp_transpose(_p(self.Wb[l]), _p(w["Wt"][l]), nout, nin, st), "transpose")
-                _check(self.lib.ewf_mlp_gemm(_p(w["dY"][l]), _p(w["Wt"][l]), None, None, _p(w["dH"][l]), None, M, nin,
-                                             nout, 0, st), "gemm dH")
-                _check(self.lib.ewf_mlp_gelu_grad(_p(w["dH"][l]), _p(w["P"][l - 1]), _p(w["dY"][l - 1]), w["dH"][l].numel(),
-                                                  st), "gelu_grad")
+        _check(self.lib.ewf_mlp_backward(self.nlayers, self._sizes, _ptrs(w["H"]), _ptrs(self.Wb), _ptrs(w["P"]), _ptrs(w["dY"]),
+                                         _ptrs(w["gW"]), _ptrs(w["gb"]), M, _stream()),
+               "ewf_mlp_backward")
 
     def adam(self, M: int, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0) -> None:
         w = self._work(M)
         self.step_count += 1
-        st = _stream()
-        for l in range(self.nlayers):
-            _check(self.lib.ewf_mlp_adam(_p(self.W[l]), _p(self.mW[l]), _p(self.vW[l]), _p(w["gW"][l]), _p(self.Wb[l]),
-                                         self.W[l].numel(), C.c_float(lr), C.c_float(b1), C.c_float(b2), C.c_float(eps),
-                                         self.step_count, C.c_float(wd), st), "adam W")
-            _check(self.lib.ewf_mlp_adam(_p(self.b[l]), _p(self.mb[l]), _p(self.vb[l]), _p(w["gb"][l]), None,
-                                         self.b[l].numel(), C.c_float(lr), C.c_float(b1), C.c_float(b2), C.c_float(eps),
-                                         self.step_count, C.c_float(0.0), st), "adam b")
+        L = self.nlayers
+        params = self.W + self.b
+        _check(self.lib.ewf_mlp_adam_all(2 * L, _ptrs(params), _ptrs(self.mW + self.mb), _ptrs(self.vW + self.vb),
+                                         _ptrs(w["gW"] + w["gb"]), (C.c_void_p * (2 * L))(*[t.data_ptr() for t in self.Wb]),
+                                         (C.c_size_t * (2 * L))(*[t.numel() for t in params]),
+                                         (C.c_float * (2 * L))(*([wd] * L)), C.c_float(lr), C.c_float(b1), C.c_float(b2),
+                                         C.c_float(eps), self.step_count, _stream()), "ewf_mlp_adam_all")
 
     def check_status(self) -> None:
         """Raises if a GEMM launch since the last check gave up on a bounded wait (its outputs, and
@@ -185,20 +191,11 @@ class MLP:
         return losses
 
     def predict(self, X, batch: int = 8192):
-        """Inference of X [n, sizes[0]] in batches of `batch` rows: full batches write their rows of
-        the output directly; a ragged last batch is padded to 128 rows and copied."""
-        torch = self.torch
+        """Inference of X [n, sizes[0]] in batches of `batch` rows, each written to its rows of the output."""
         n = X.shape[0]
-        out = torch.empty(n, self.sizes[-1], device="cuda")
+        out = self.torch.empty(n, self.sizes[-1], device="cuda")
         for a in range(0, n, batch):
-            xb = X[a:a + batch]
-            m = xb.shape[0]
-            if m % 128 == 0:
-                self.forward(xb, out[a:a + m], keep_pre=False)
-                continue
-            pad = torch.zeros(128 - m % 128, X.shape[1], dtype=X.dtype, device="cuda")
-            y = self.forward(torch.cat([xb, pad]), keep_pre=False)
-            out[a:a + m] = y[:m]
+            self._infer(X[a:a + batch], out[a:a + batch])
         self.check_status()
         return out
 

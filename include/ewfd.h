@@ -381,7 +381,25 @@ int ewf_batch_get_l2_prefetch(const ewf_batch *b, int32_t *planes);
  * form).  M, N multiples of 128, K a multiple of 32. */
 int ewf_mlp_gemm(const void *A, const void *B, const float *bias, float *Cf, void *Cb, float *pre, int32_t M, int32_t N,
                  int32_t K, int32_t act, void *stream);
-/* Synchronises and reports (then clears) a failed bounded wait of ewf_mlp_gemm. */
+/* The passes of a network of n layers (widths sizes[0..n]; sizes[1..n] multiples of 128), one call each;
+ * every buffer 16-byte aligned.
+ * forward: layer l is W[l] (bf16 [sizes[l+1], sizes[l]]) and b[l]; GELU between layers.  X bf16
+ * [M, sizes[0]] (sizes[0] a multiple of 32, any M >= 1); H[l], l < n - 1: the output of layer l, bf16; P[l]:
+ * its value before the activation, fp32 (P NULL: not kept); Y fp32 [M, sizes[n]].
+ * backward: H[l] the input of layer l (H[0] = X), dY[l] the gradient at the output of layer l before its
+ * activation (bf16): dY[n-1] is given, the others are written; gW[l], gb[l] fp32.  M and sizes[0] multiples of 128.
+ * mse_loss: ewf_mlp_mse_grad and, at `loss`, scale times the sum of squares; n a multiple of 4; `done` an unsigned word that
+ * is zero before the first call and after every call (calls sharing it must not overlap).
+ * adam_all: ewf_mlp_adam on `count` tensors (wb[q] may be NULL; wd[q] its weight decay). */
+int ewf_mlp_forward(int32_t n, const int32_t *sizes, const void *X, const void *const *W, const float *const *b, void *const *H,
+                    float *const *P, float *Y, int32_t M, void *stream);
+int ewf_mlp_backward(int32_t n, const int32_t *sizes, const void *const *H, const void *const *W, const float *const *P, void *const *dY,
+                     float *const *gW, float *const *gb, int32_t M, void *stream);
+int ewf_mlp_mse_loss(const float *y, const float *t, void *dy, size_t n, float scale, float *part, int32_t nblocks, void *done,
+                     float *loss, void *stream);
+int ewf_mlp_adam_all(int32_t count, float *const *w, float *const *m, float *const *v, const float *const *g, void *const *wb,
+                     const size_t *n, const float *wd, float lr, float b1, float b2, float eps, int32_t step, void *stream);
+/* Synchronises and reports (then clears) a failed bounded wait of the GEMMs. */
 int ewf_mlp_status(void);
 /* Test hook of the failure path: with tile >= 0, the MMA issuer of the first CTA of every later
  * ewf_mlp_gemm launch withholds the accumulator-ready signal of its tile number `tile` (a signal
