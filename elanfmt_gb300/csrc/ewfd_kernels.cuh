@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(split_max_threads<T>()) k_velocity(const StepA
     pdl_wait();
     if (rf.it_wr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0)
         *rf.it_wr = *rf.it_rd + 1;  // the next step's counter; this launch reads only it_rd
-    const int k0 = blockIdx.z * a.kchunk;
+    const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
     velocity_column<T, MODEL, DAMP, KAHAN, 1, false, 0, true>(a, blockIdx.x * TX + threadIdx.x,
                                                               blockIdx.y * blockDim.y + threadIdx.y, k0,
                                                               min(k0 + a.kchunk, a.nz), 0, rf);
