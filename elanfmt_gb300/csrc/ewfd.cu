@@ -550,16 +550,16 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 // Launch shape of the two-kernel step until the autotuner or a caller sets another.  A thread marches
 // kchunk planes one after the other, about a memory latency each, so a grid that does not fill the
 // GPU several times over runs faster in short chunks, and longer ones save the loads a chunk starts
-// with.  The line: one plane per chunk up to 0.5 M cells, then one more plane per 0.5 M cells, at
-// most 6 (three waves of resident warps at every size below that).  CTAs of 4 rows leave the
-// shortest tail at every size measured.  us per step of 16 planes x 8 rows and of this rule: ortho
-// 40x40x32 17.2 (4 planes) and 8.7, iso 128^3 40.0 (4 planes) and 38.9, Kahan 192^3 206.2 and 203.7.
+// with.  CTAs of 4 rows leave the shortest tail at every size measured.  us per step by planes per chunk:
+// ortho 50^3 7.0 (1) 8.2 (2); 64^3 8.7 (1) 8.4 (2) 12.3 (4); iso 80^3 13.2 (1) 11.3 (2) 11.1 (4); 96^3 15.0 (2)
+// 14.8 (4) 15.1 (6); iso 128^3 36.9 (2) 35.8 (4) 37.1 (6); Kahan 192^3 198.8 (2) 196.2 (4) 197.1 (6); ortho 256^3
+// 405.9 (4) 401.5 (6) 403.0 (8); 16 planes and 8 rows take 65 us on 40 x 40 x 32 and 63 on iso 128^3.
 // The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
 // 320x320x256 641 -> 631) and not below (128^3: 55.8 and 56.1).
 static void split_default_shape(ewf_handle *h)
 {
     const double cells = (double)h->p.nx * h->p.ny * h->p.nz;
-    if (h->p.kchunk == 0) h->kchunk = (int)std::min(6.0, std::max(1.0, std::floor(cells / 5e5 + 0.5)));
+    if (h->p.kchunk == 0) h->kchunk = cells < 2e5 ? 1 : cells < 6e5 ? 2 : cells < 1.2e7 ? 4 : 6;
     h->ty = 4;
     h->l2pf = cells >= 1.2e7 ? 3 : 0;
 }

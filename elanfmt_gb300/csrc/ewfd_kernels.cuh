@@ -472,13 +472,15 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int X, int j
 
     long long c = (long long)X + (long long)j * sxs + (long long)k0 * sys + (SOFF ? soff : 0);
     long long cm = !SEP ? c : (RC == 1) ? c - soff : (long long)i + (long long)j * a.sx + (long long)k0 * sy;
-    T vx_m = lds<COH>(a.f[0] + c - sys);  // Vx(k-1)
-    T vy_m = lds<COH>(a.f[1] + c - sys);  // Vy(k-1)
-    T vz_k = lds<COH>(a.f[2] + c);        // Vz(k)
     T wz_k = T(0);
     if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + k0);
     StressIn<T, MODEL, DAMP> nxt;
-    stress_load<T, MODEL, DAMP, RC, COH>(a, c, SEP ? cm : c, k0, nxt);
+    stress_load_mat<T, MODEL, DAMP>(a, SEP ? cm : c, k0, nxt);
+    if (SRC) pdl_wait();  // nothing above depends on an earlier launch
+    T vx_m = lds<COH>(a.f[0] + c - sys);  // Vx(k-1)
+    T vy_m = lds<COH>(a.f[1] + c - sys);  // Vy(k-1)
+    T vz_k = lds<COH>(a.f[2] + c);        // Vz(k)
+    stress_load_state<T, MODEL, DAMP, RC, COH>(a, c, nxt);
     // point sources on this column (SRC: the two-kernel step's stress kernel)
     bool src_col = false;
     T s_src = T(0);
@@ -526,15 +528,13 @@ template <typename T>
 constexpr int split_min_ctas() { return sizeof(T) == 4 ? 2 : 1; }
 
 template <typename T, int MODEL, int DAMP>
-__global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k_stress(const StepArgs<T> a,
-                                                                                        const StressSrc ss)
+__global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k_stress(const StepArgs<T> a, const StressSrc ss)
 {
     pdl_trigger();
-    pdl_wait();
     const int k0 = blockIdx.z * a.kchunk;
     stress_column<T, MODEL, DAMP, 1, false, 0, true>(a, blockIdx.x * TX + threadIdx.x,
                                                      blockIdx.y * blockDim.y + threadIdx.y, k0,
-                                                     min(k0 + a.kchunk, a.nz), 0, ss);
+                                                         min(k0 + a.kchunk, a.nz), 0, ss);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -767,11 +767,17 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
 
     long long c = (long long)X + (long long)j * sxs + (long long)k0 * sys + (SOFF ? soff : 0);
     long long cm = !SEP ? c : (RC == 1) ? c - soff : (long long)i + (long long)j * a.sx + (long long)k0 * sy;
+    VelIn<T, MODEL, DAMP, KAHAN> nxt;
+    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, SEP ? cm : c, k0, nxt);
+    if (REC && !SEP) pdl_wait();  // nothing above depends on an earlier launch
     T szz_m = lds<COH>(a.f[5] + c - sys);
     T sxz_k = lds<COH>(a.f[7] + c);
     T syz_k = lds<COH>(a.f[8] + c);
-    VelIn<T, MODEL, DAMP, KAHAN> nxt;
-    vel_load<T, MODEL, DAMP, KAHAN, RC, COH>(a, c, SEP ? cm : c, k0, nxt);
+    vel_load_state<T, MODEL, DAMP, KAHAN, RC, COH>(a, c, nxt);
+    if (KAHAN) {
+#pragma unroll
+        for (int f = 0; f < 3; ++f) nxt.cp[f] = a.comp[f][c];
+    }
     // the L2 prefetch's field for this lane (REC: the two-kernel step's velocity kernel)
     const T *pf_row = nullptr;
     if (REC && a.l2pf > 0) {
@@ -815,16 +821,17 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
 }
 
 template <typename T, int MODEL, int DAMP, bool KAHAN>
-__global__ void __launch_bounds__(split_max_threads<T>()) k_velocity(const StepArgs<T> a, const RecFuse rf)
+__global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k_velocity(const StepArgs<T> a, const RecFuse rf)
 {
     pdl_trigger();
-    pdl_wait();
-    if (rf.it_wr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0)
+    if (rf.it_wr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+        pdl_wait();
         *rf.it_wr = *rf.it_rd + 1;  // the next step's counter; this launch reads only it_rd
+    }
     const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
     velocity_column<T, MODEL, DAMP, KAHAN, 1, false, 0, true>(a, blockIdx.x * TX + threadIdx.x,
                                                               blockIdx.y * blockDim.y + threadIdx.y, k0,
-                                                              min(k0 + a.kchunk, a.nz), 0, rf);
+                                                                  min(k0 + a.kchunk, a.nz), 0, rf);
 }
 
 // ---------------------------------------------------------------------------------------------
