@@ -8,6 +8,7 @@
 #include "ewfd.h"
 #include "ewfd_internal.h"
 #include "ewfd_kernels.cuh"
+#include "ewfd_pair.cuh"
 #include "ewfd_fused.cuh"
 #include "ewfd_band.h"
 #include "ewfd_staged.h"
@@ -239,6 +240,7 @@ struct ewf_handle {
     bool pdl = true;    // two-kernel step: kernels launched as programmatic dependents (off if capture refuses)
     int l2pf = 0;       // two-kernel step: L2 prefetch distance of the velocity kernel in planes (autotuned)
     int fdiv = 0;       // StepArgs::fdiv of this handle's spacings
+    bool pair = false;       // two-kernel step, FP32: two cells per thread (ewfd_pair.cuh)
     bool src_plane1 = false;  // a fused source entry that plane 2's thread applies on plane 1
     struct Snapshots *snap = nullptr;  // queued snapshot writer (created on first use)
 };
@@ -380,6 +382,8 @@ static StepArgs<T> make_args(const ewf_handle *h, int which = -1)
     a.third = (T)1.0 / (T)3.0;
     a.fdiv = h->fdiv;
     a.l2pf = h->l2pf;
+    a.one = 1.0f;
+    a.minus_one = -1.0f;
     a.vdamp = (T)h->p.vdamp;
     a.vdamp_on = a.vdamp != T(0) ? 1 : 0;
     a.bc1 = h->p.free_surface == EWF_FS_BC1 ? 1 : 0;
@@ -562,6 +566,10 @@ static void split_default_shape(ewf_handle *h)
     if (h->p.kchunk == 0) h->kchunk = cells < 2e5 ? 1 : cells < 6e5 ? 2 : cells < 1.2e7 ? 4 : 6;
     h->ty = 4;
     h->l2pf = cells >= 1.2e7 ? 3 : 0;
+    // Two cells per thread halve the threads: from 0.6 M cells on there are enough of them.  us per step with one
+    // and two: ortho 64^3 8.4 and 8.3, iso 64^3 6.8 and 7.7; iso 96^3 14.8 and 13.6, ortho 96^3 20.1 and 19.2; iso 128^3
+    // 35.7 and 34.9, Kahan 192^3 196.1 and 189.2, ortho 256^3 401.6 and 384.1, 320x320x256 625.1 and 595.2.
+    h->pair = cells >= 6e5;
 }
 
 extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
@@ -1132,14 +1140,23 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
         rf.it_wr = it_wr;
     }
     const bool pdl = h->pdl && !ev;  // kernels timed between events run as plain launches
+    constexpr bool PAIRS = sizeof(T) == 4 && DAMP != DAMP_PERCOMP;
+    const bool pair = PAIRS && h->pair;
+    const dim3 pblk(PAIR_TX, 2 * h->ty), pgrd(grd.x, (h->p.ny + 2 * h->ty - 1) / (2 * h->ty), grd.z);
     if (ev) cudaEventRecord(ev[0], h->stream);
-    launch_on(k_stress<T, MODEL, DAMP>, grd, blk, h->stream, pdl, a, ss);
+    if constexpr (PAIRS) {
+        if (pair) launch_on(k_stress_pair<MODEL, DAMP>, pgrd, pblk, h->stream, pdl, a, ss);
+    }
+    if (!pair) launch_on(k_stress<T, MODEL, DAMP>, grd, blk, h->stream, pdl, a, ss);
     if (ev) cudaEventRecord(ev[1], h->stream);
     if (h->nsrc > 0 && ss.nsrc == 0)
         launch_on(k_inject<T>, dim3(1), dim3(32), h->stream, pdl, a, (const SrcEntry *)h->d_src, h->nsrc,
                   (const double *)h->d_stf, (int)h->nstf, (const int *)it_rd, h->p.src_order);
     if (ev) cudaEventRecord(ev[2], h->stream);
-    launch_on(k_velocity<T, MODEL, DAMP, KAHAN>, grd, blk, h->stream, pdl, a, rf);
+    if constexpr (PAIRS) {
+        if (pair) launch_on(k_velocity_pair<MODEL, DAMP, KAHAN>, pgrd, pblk, h->stream, pdl, a, rf);
+    }
+    if (!pair) launch_on(k_velocity<T, MODEL, DAMP, KAHAN>, grd, blk, h->stream, pdl, a, rf);
     if (ev) cudaEventRecord(ev[3], h->stream);
     if (!h->rec_fuse)
         launch_on(k_record<T>, dim3(1), dim3(256), h->stream, pdl, a, (const long long *)h->d_rec_off,

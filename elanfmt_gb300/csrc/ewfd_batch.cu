@@ -449,6 +449,8 @@ static int build_tables(ewf_batch *b)
         d.rdx = 1.0f / d.dx; d.rdy = 1.0f / d.dy; d.rdz = 1.0f / d.dz;
         d.c66 = (float)p.c66; d.bx = (float)p.bx; d.by = (float)p.by; d.bz = (float)p.bz;
         d.third = 1.0f / 3.0f;
+        d.one = 1.0f;
+        d.minus_one = -1.0f;
         d.fdiv = q.fdiv ? 1 : 0;
         d.bc1 = p.free_surface == EWF_FS_BC1 ? 1 : 0;
         d.smu_on = p.surface_mu > 0.0 ? 1 : 0;

@@ -59,6 +59,7 @@ struct StepArgs {
     int bc1;            // 1: BC1 after the stress update (stress_store, inject_entry); 0: none
     int smu_on;         // isotropic 1-D PML scheme: shear modulus smu instead of c66 on plane k = 1
     T smu;
+    float one, minus_one;  // 1 and -1 (ewfd_pair.cuh)
     int l2pf;           // two-kernel step: the velocity kernel asks L2 for its inputs this many planes ahead (0: off)
 };
 
