@@ -554,22 +554,30 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 // Launch shape of the two-kernel step until the autotuner or a caller sets another.  A thread marches
 // kchunk planes one after the other, about a memory latency each, so a grid that does not fill the
 // GPU several times over runs faster in short chunks, and longer ones save the loads a chunk starts
-// with.  CTAs of 4 rows leave the shortest tail at every size measured.  us per step by planes per chunk:
-// ortho 50^3 7.0 (1) 8.2 (2); 64^3 8.7 (1) 8.4 (2) 12.3 (4); iso 80^3 13.2 (1) 11.3 (2) 11.1 (4); 96^3 15.0 (2)
-// 14.8 (4) 15.1 (6); iso 128^3 36.9 (2) 35.8 (4) 37.1 (6); Kahan 192^3 198.8 (2) 196.2 (4) 197.1 (6); ortho 256^3
-// 405.9 (4) 401.5 (6) 403.0 (8); 16 planes and 8 rows take 65 us on 40 x 40 x 32 and 63 on iso 128^3.
+// with.  CTAs of 4 rows leave the shortest tail at every size measured (16 planes and 8 rows take 65 us a step on
+// 40 x 40 x 32 and 63 on iso 128^3).
+// Two cells per thread (pair) halve the threads: from 0.4 M cells on there are enough of them.
+// us per step by cells per thread and planes per chunk:
+//                 one cell                two cells
+//   iso 50^3      6.2 (1)   7.0 (2)       6.5 (1)   7.8 (2)
+//   iso 64^3      7.4 (1)   6.8 (2)       8.5 (1)   9.0 (2)
+//   ortho 64^3    8.8 (1)   8.4 (2)       8.9 (1)   9.3 (2)
+//   iso 80^3      11.3 (2)  11.1 (4)      10.4 (2)  12.5 (4)
+//   ortho 80^3    14.2 (2)  14.2 (4)      13.0 (2)  14.3 (4)
+//   iso 96^3      15.0 (2)  14.8 (4)      12.8 (2)  13.9 (3)  12.8 (4)
+//   iso 128^3     36.9 (2)  35.5 (3)      33.0 (2)  32.9 (3)  35.2 (4)
+//   iso-het 203x151x97  74.4 (2)  73.1 (3)      66.8 (2)  66.7 (3)  67.6 (4)
+//   Kahan 192^3   198.8 (2) 196.1 (4)     186.3 (4)
+//   ortho 256^3   405.9 (4) 401.6 (6)     380.2 (6)
 // The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
-// 320x320x256 641 -> 631) and not below (128^3: 55.8 and 56.1).
+// 320x320x256 641 -> 631 with one cell per thread) and not below (128^3: 55.8 and 56.1).
 static void split_default_shape(ewf_handle *h)
 {
     const double cells = (double)h->p.nx * h->p.ny * h->p.nz;
-    if (h->p.kchunk == 0) h->kchunk = cells < 2e5 ? 1 : cells < 6e5 ? 2 : cells < 1.2e7 ? 4 : 6;
+    if (h->p.kchunk == 0) h->kchunk = cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6;
     h->ty = 4;
     h->l2pf = cells >= 1.2e7 ? 3 : 0;
-    // Two cells per thread halve the threads: from 0.6 M cells on there are enough of them.  us per step with one
-    // and two: ortho 64^3 8.4 and 8.3, iso 64^3 6.8 and 7.7; iso 96^3 14.8 and 13.6, ortho 96^3 20.1 and 19.2; iso 128^3
-    // 35.7 and 34.9, Kahan 192^3 196.1 and 189.2, ortho 256^3 401.6 and 384.1, 320x320x256 625.1 and 595.2.
-    h->pair = cells >= 6e5;
+    h->pair = cells >= 4e5;
 }
 
 extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
@@ -1142,7 +1150,7 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
     const bool pdl = h->pdl && !ev;  // kernels timed between events run as plain launches
     constexpr bool PAIRS = sizeof(T) == 4 && DAMP != DAMP_PERCOMP;
     const bool pair = PAIRS && h->pair;
-    const dim3 pblk(PAIR_TX, 2 * h->ty), pgrd(grd.x, (h->p.ny + 2 * h->ty - 1) / (2 * h->ty), grd.z);
+    const dim3 pblk(PAIR_TX, pair_rows(h->ty)), pgrd(grd.x, (h->p.ny + pblk.y - 1) / pblk.y, grd.z);
     if (ev) cudaEventRecord(ev[0], h->stream);
     if constexpr (PAIRS) {
         if (pair) launch_on(k_stress_pair<MODEL, DAMP>, pgrd, pblk, h->stream, pdl, a, ss);

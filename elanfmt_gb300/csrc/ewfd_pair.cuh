@@ -139,9 +139,15 @@ __device__ __forceinline__ void stress_state2(const StepArgs<float> &a, long lon
 }
 
 // The pair (i, i+1) of row j over planes [k0, k1); soff: the state lies that far after the materials' index.
+// The orthorhombic update loads a plane ahead (PF), in 128 registers; the others have fewer loads per plane
+// and do better with 85 registers and half as many warps again (iso-het 203x151x97 72.5 -> 68.0 us a step, 96^3 15.7 ->
+// 14.4; ortho 128^3 in 85 without the prefetch 52.2 -> 54.9, 320x320x256 596 -> 603).
+template <int MODEL>
+__host__ __device__ constexpr bool pair_prefetch() { return MODEL == MODEL_ORTHO; }
 template <int MODEL, int DAMP>
 __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int j, int k0, int k1, long long soff, const StressSrc &ss)
 {
+    constexpr bool PF = pair_prefetch<MODEL>();
     if (i >= a.nx || j >= a.ny) return;
     const bool in1 = i + 1 < a.nx, row_bc = j < a.bc1_rows;
     f2 hx = 0, wxi = 0, wxy = 0, pxy = 0;
@@ -179,8 +185,12 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
     const bool g0 = !guard || i > 0;
 
     for (int k = k0; k < k1; ++k, c += a.sy, cm += a.sy) {
+        if (!PF && k > k0) {
+            stress_mat2<MODEL, DAMP>(a, cm, k, nxt);
+            stress_state2<MODEL, DAMP>(a, c, nxt);
+        }
         const StressIn2<MODEL, DAMP> q = nxt;
-        if (k + 1 < k1) {
+        if (PF && k + 1 < k1) {
             stress_mat2<MODEL, DAMP>(a, cm + a.sy, k + 1, nxt);
             stress_state2<MODEL, DAMP>(a, c + a.sy, nxt);
         }
@@ -361,11 +371,11 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
     const f2 rdx = dup(a.rdx), rdy = dup(a.rdy), rdz = dup(a.rdz);
 
     for (int k = k0; k < k1; ++k, c += a.sy, cm += a.sy) {
-        const VelIn2<MODEL, DAMP, KAHAN> q = nxt;
-        if (k + 1 < k1) {
-            vel_mat2<MODEL, DAMP, KAHAN>(a, cm + a.sy, k + 1, nxt);
-            vel_state2<MODEL, DAMP, KAHAN>(a, c + a.sy, nxt);
+        if (k > k0) {
+            vel_mat2<MODEL, DAMP, KAHAN>(a, cm, k, nxt);
+            vel_state2<MODEL, DAMP, KAHAN>(a, c, nxt);
         }
+        const VelIn2<MODEL, DAMP, KAHAN> q = nxt;
         if (pf_row && k + a.l2pf < k1) l2_prefetch_line(pf_row + (long long)(k - k0) * a.sy);
         const f2 sxx_im = pk(q.sxx_im, lo(q.sxx)), sxy_ip = pk(hi(q.sxy), q.sxy_i2), sxz_ip = pk(hi(sxz_k), q.sxz_i2);
         const f2 dSx = op.add(op.add(mul2(op.sub(q.sxx, sxx_im), rdx), mul2(op.sub(q.sxy_jp, q.sxy), rdy)), mul2(op.sub(q.sxz_p, sxz_k), rdz));
@@ -419,10 +429,11 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
 }
 
 constexpr int PAIR_TX = TX / 2;                           // pairs per row of a CTA
-constexpr int PAIR_MAX_THREADS = TX * SPLIT_MAX_TY;       // 128 registers
+constexpr int PAIR_MAX_THREADS = 256;                     // CTAs of at most 16 rows
+__host__ __device__ constexpr int pair_rows(int ty) { return 2 * ty < PAIR_MAX_THREADS / PAIR_TX ? 2 * ty : PAIR_MAX_THREADS / PAIR_TX; }
 
 template <int MODEL, int DAMP>
-__global__ void __launch_bounds__(PAIR_MAX_THREADS, 1) k_stress_pair(const StepArgs<float> a, const __grid_constant__ StressSrc ss)
+__global__ void __launch_bounds__(PAIR_MAX_THREADS, pair_prefetch<MODEL>() ? 2 : 3) k_stress_pair(const StepArgs<float> a, const __grid_constant__ StressSrc ss)
 {
     pdl_trigger();
     const int k0 = blockIdx.z * a.kchunk;
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 1) k_stress_pair(const StepA
 }
 
 template <int MODEL, int DAMP, bool KAHAN>
-__global__ void __launch_bounds__(PAIR_MAX_THREADS, 1) k_velocity_pair(const StepArgs<float> a, const RecFuse rf)
+__global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const StepArgs<float> a, const RecFuse rf)
 {
     pdl_trigger();
     if (rf.it_wr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
