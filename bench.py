@@ -343,7 +343,7 @@ def extra_batch(nt: int = 300) -> dict:
                         f"(the full workload runs 3000)", "runs": runs, "batched_runs_per_s": round(runs / batch_s, 3),
             "solo_runs_per_s": round(runs / solo_s, 3), "speedup_vs_solo": round(solo_s / batch_s, 3),
             "batch_tile_y": setting[0], "batch_l2_prefetch": setting[1],
-            "batch_launch": "own launches on parallel branches" if setting[2] else "persistent family launch",
+            "batch_launch": "on parallel branches" if setting[2] else "one after another (small ones on branches)",
             "solo": "each run alone with its own autotuned z-chunk and tile height"}
 
 
@@ -629,7 +629,7 @@ def main_batch(args):
            "batched_gcell_updates_per_s": round(cell_updates / batch_s / 1e9, 2),
            "solo_gcell_updates_per_s": round(cell_updates / solo_s / 1e9, 2),
            "kchunk_autotuned": k, "tile_y_autotuned": tile, "l2_prefetch_autotuned": l2pf,
-           "launch_autotuned": "own launches on parallel branches" if own else "persistent family launch", "dtype": "f32",
+           "launch_autotuned": "on parallel branches" if own else "one after another (small ones on branches)", "dtype": "f32",
            "data": "synthetic (seeded)",
            "config": {"workload": f"6 elementary MTs on orthorhombic {n_ortho}^3 + {args.batch_iso} isotropic models "
                                   f"96^3-224^3, {nt} steps",

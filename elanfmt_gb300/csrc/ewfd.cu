@@ -9,6 +9,7 @@
 #include "ewfd_internal.h"
 #include "ewfd_kernels.cuh"
 #include "ewfd_pair.cuh"
+#include "ewfd_step.h"
 #include "ewfd_fused.cuh"
 #include "ewfd_band.h"
 #include "ewfd_staged.h"
@@ -172,8 +173,6 @@ static bool slot_used(int model, int q)
 // ------------------------------------------------------------------------------------------
 // handle
 // ------------------------------------------------------------------------------------------
-constexpr size_t REC_TABLE_MAX = (size_t)1 << 24;  // plane offsets of the velocity kernel's receiver table (64 MB)
-
 struct ewf_handle {
     ewf_params p;
     std::string workdir;
@@ -355,9 +354,6 @@ static StepArgs<T> make_args(const ewf_handle *h, int which = -1)
     for (int q = 0; q < 6; ++q) a.w6[q] = (const T *)boxptr(h, h->w6_alloc[q]);
     a.sy = h->sy;
     a.sx = h->sx;
-    a.R = 1;
-    a.sxs = h->sx;
-    a.sys = h->sy;
     a.nx = h->p.nx;
     a.ny = h->p.ny;
     a.nz = h->p.nz;
@@ -571,13 +567,22 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 //   ortho 256^3   405.9 (4) 401.6 (6)     380.2 (6)
 // The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
 // 320x320x256 641 -> 631 with one cell per thread) and not below (128^3: 55.8 and 56.1).
+SplitShape split_shape(int nx, int ny, int nz, int R)
+{
+    const double cells = (double)nx * ny * nz * R;
+    SplitShape d = {cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6, 4, cells >= 1.2e7 ? 3 : 0, cells >= 4e5};
+    // a grid has at most 65535 CTAs along y and z
+    d.kchunk = std::max(d.kchunk, (nz + 65534) / 65535);
+    while (d.ty < 16 && ny > 65535 * d.ty) d.ty *= 2;
+    return d;
+}
 static void split_default_shape(ewf_handle *h)
 {
-    const double cells = (double)h->p.nx * h->p.ny * h->p.nz;
-    if (h->p.kchunk == 0) h->kchunk = cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6;
-    h->ty = 4;
-    h->l2pf = cells >= 1.2e7 ? 3 : 0;
-    h->pair = cells >= 4e5;
+    const SplitShape d = split_shape(h->p.nx, h->p.ny, h->p.nz);
+    if (h->p.kchunk == 0) h->kchunk = d.kchunk;
+    h->ty = d.ty;
+    h->l2pf = d.l2pf;
+    h->pair = d.pair;
 }
 
 extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
@@ -884,6 +889,88 @@ extern "C" int ewf_set_stf(ewf_handle *h, const double *stf, size_t n)
     return EWF_OK;
 }
 
+// The stress kernel's threads apply the entries when all of them lie in its cells (the injection kernel
+// covers the rest: cells on the staggered arrays' last planes, and grids too thin for BC1's plane-2
+// copy).  *plane1: a shear entry that plane 2's thread applies on plane 1.  f->src is left to the caller.
+bool make_stress_src(const std::vector<SrcEntry> &v, int nx, int ny, int nz, StressSrc *f, bool *plane1)
+{
+    *f = StressSrc{};
+    *plane1 = false;
+    if (v.empty() || nz < 3) return false;
+    f->i0 = f->j0 = f->k0 = INT32_MAX;
+    f->i1 = f->j1 = f->k1 = -1;
+    for (const SrcEntry &q : v) {
+        if (q.i >= nx || q.j >= ny || q.k >= nz) {
+            *f = StressSrc{};
+            *plane1 = false;
+            return false;
+        }
+        const int k = fused_src_plane(q.comp, q.k);
+        f->i0 = std::min(f->i0, q.i);
+        f->i1 = std::max(f->i1, q.i);
+        f->j0 = std::min(f->j0, q.j);
+        f->j1 = std::max(f->j1, q.j);
+        f->k0 = std::min(f->k0, k);
+        f->k1 = std::max(f->k1, k);
+        if (k != q.k) *plane1 = true;
+    }
+    f->nsrc = (int)v.size();
+    f->inl = f->nsrc <= SRC_INLINE ? 1 : 0;
+    if (f->inl) std::copy(v.begin(), v.end(), f->e);
+    return true;
+}
+
+// The velocity kernel's receiver tables (RecFuse), when every receiver is a velocity component on a cell
+// its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz) and the plane offsets stay below 64 MB.
+RecTables make_rec_tables(int n, const int32_t *ijkc, int nx, int ny, int nz)
+{
+    constexpr size_t MAX_OFFSETS = (size_t)1 << 24;
+    RecTables t;
+    std::vector<int> order((size_t)n);
+    for (int r = 0; r < n; ++r) {
+        const int i = ijkc[4 * r], j = ijkc[4 * r + 1], k = ijkc[4 * r + 2], c = ijkc[4 * r + 3];
+        if (c > EWF_F_VZ || i < 1 || j < 1 || k < 1 || i >= nx || j >= ny || k >= nz) t.fuse = false;
+        t.kmin = std::min(t.kmin, k);
+        t.kmax = std::max(t.kmax, k);
+        order[r] = r;
+    }
+    if (!t.fuse || n == 0) return t;
+    // entries by column (row by row), then plane; one slot of plane offsets per column
+    auto col = [&](int r) { return (size_t)ijkc[4 * r] + (size_t)ijkc[4 * r + 1] * nx; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return col(x) != col(y) ? col(x) < col(y) : ijkc[4 * x + 2] < ijkc[4 * y + 2];
+    });
+    size_t slots = 0;
+    for (int q = 0; q < n; ++q) slots += (q == 0 || col(order[q]) != col(order[q - 1]));
+    const size_t span = (size_t)(t.kmax - t.kmin + 1);
+    if (slots * (span + 1) > MAX_OFFSETS) {  // receivers all over a volume: the recording kernel
+        t.fuse = false;
+        return t;
+    }
+    const int ngx = (nx + 31) / 32;
+    t.grp.assign((size_t)ngx * ny, make_uint2(0u, 0u));
+    t.off.resize(slots * (span + 1));
+    t.ent.resize((size_t)n);
+    int slot = -1;
+    for (int q = 0; q < n; ++q) {
+        const int r = order[q], i = ijkc[4 * r], j = ijkc[4 * r + 1];
+        if (q == 0 || col(r) != col(order[q - 1])) {
+            ++slot;
+            uint2 &g = t.grp[(size_t)j * ngx + i / 32];
+            if (!g.x) g.y = (unsigned)slot;
+            g.x |= 1u << (i & 31);
+            int *o = &t.off[(size_t)slot * (span + 1)];
+            int e = q;
+            for (size_t k = 0; k <= span; ++k) {
+                while (e < n && col(order[e]) == col(r) && ijkc[4 * order[e] + 2] < t.kmin + (int)k) ++e;
+                o[k] = e;
+            }
+        }
+        t.ent[q] = make_int2(ijkc[4 * r + 3], r);
+    }
+    return t;
+}
+
 extern "C" int ewf_set_sources(ewf_handle *h, int32_t n, const int32_t *cijk, const double *coef)
 {
     if (!h || n < 0 || (n > 0 && (!cijk || !coef))) return ewf_fail(EWF_ERR_ARG, "bad source list");
@@ -909,33 +996,12 @@ extern "C" int ewf_set_sources(ewf_handle *h, int32_t n, const int32_t *cijk, co
     h->nsrc = n;
     h->src_version++;
     h->graph_dirty = true;
-    // the stress kernel's threads apply the entries when all of them lie in its cells (k_inject
-    // covers the rest: cells on the staggered arrays' last planes, and grids too thin for BC1's
-    // plane-2 copy)
     StressSrc f{};
-    bool fuse = n > 0 && h->p.nz >= 3, plane1 = false;
-    f.i0 = f.j0 = INT32_MAX;
-    f.i1 = f.j1 = f.k1 = -1;
-    f.k0 = INT32_MAX;
-    for (const SrcEntry &q : v) {
-        if (q.i >= h->p.nx || q.j >= h->p.ny || q.k >= h->p.nz) fuse = false;
-        f.i0 = std::min(f.i0, q.i);
-        f.i1 = std::max(f.i1, q.i);
-        f.j0 = std::min(f.j0, q.j);
-        f.j1 = std::max(f.j1, q.j);
-        f.k0 = std::min(f.k0, fused_src_plane(q.comp, q.k));
-        f.k1 = std::max(f.k1, fused_src_plane(q.comp, q.k));
-        if (fused_src_plane(q.comp, q.k) != q.k) plane1 = true;
-    }
-    if (fuse) {
-        f.src = h->d_src;
-        f.nsrc = n;
-        if (n <= SRC_INLINE) std::copy(v.begin(), v.end(), f.e);
-    } else {
-        f = StressSrc{};
-    }
+    bool plane1 = false;
+    const bool fuse = make_stress_src(v, h->p.nx, h->p.ny, h->p.nz, &f, &plane1);
+    if (fuse) f.src = h->d_src;
     h->src_fuse = f;
-    h->src_plane1 = fuse && plane1;
+    h->src_plane1 = plane1;
     return EWF_OK;
 }
 
@@ -1014,60 +1080,18 @@ extern "C" int ewf_set_receivers(ewf_handle *h, int32_t n, const int32_t *ijkc)
     h->d_rgrp = nullptr;
     h->d_roff = nullptr;
     h->d_rent = nullptr;
-    bool fuse = true;
-    int kmin = INT32_MAX, kmax = -1;
-    std::vector<int> order((size_t)n);
-    for (int r = 0; r < n; ++r) {
-        const int i = ijkc[4 * r], j = ijkc[4 * r + 1], k = ijkc[4 * r + 2], c = ijkc[4 * r + 3];
-        if (c > EWF_F_VZ || i < 1 || j < 1 || k < 1 || i >= h->p.nx || j >= h->p.ny || k >= h->p.nz) fuse = false;
-        kmin = std::min(kmin, k);
-        kmax = std::max(kmax, k);
-        order[r] = r;
+    const RecTables t = make_rec_tables(n, ijkc, h->p.nx, h->p.ny, h->p.nz);
+    if (t.fuse && n > 0) {
+        CK(cudaMalloc(&h->d_rgrp, t.grp.size() * sizeof(uint2)));
+        CK(cudaMalloc(&h->d_roff, t.off.size() * sizeof(int)));
+        CK(cudaMalloc(&h->d_rent, t.ent.size() * sizeof(int2)));
+        CK(cudaMemcpy(h->d_rgrp, t.grp.data(), t.grp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(h->d_roff, t.off.data(), t.off.size() * sizeof(int), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(h->d_rent, t.ent.data(), t.ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
     }
-    if (fuse && n > 0) {
-        // entries by column (row by row), then plane; one slot of plane offsets per column
-        auto col = [&](int r) { return (size_t)ijkc[4 * r] + (size_t)ijkc[4 * r + 1] * h->p.nx; };
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-            return col(x) != col(y) ? col(x) < col(y) : ijkc[4 * x + 2] < ijkc[4 * y + 2];
-        });
-        size_t slots = 0;
-        for (int q = 0; q < n; ++q) slots += (q == 0 || col(order[q]) != col(order[q - 1]));
-        const size_t span = (size_t)(kmax - kmin + 1);
-        if (slots * (span + 1) > REC_TABLE_MAX) {
-            fuse = false;  // receivers all over a volume: k_record
-        } else {
-            const int ngx = (h->p.nx + 31) / 32;
-            std::vector<uint2> grp((size_t)ngx * h->p.ny, make_uint2(0u, 0u));
-            std::vector<int> off(slots * (span + 1));
-            std::vector<int2> ent((size_t)n);
-            int slot = -1;
-            for (int q = 0; q < n; ++q) {
-                const int r = order[q], i = ijkc[4 * r], j = ijkc[4 * r + 1];
-                if (q == 0 || col(r) != col(order[q - 1])) {
-                    ++slot;
-                    uint2 &g = grp[(size_t)j * ngx + i / 32];
-                    if (!g.x) g.y = (unsigned)slot;
-                    g.x |= 1u << (i & 31);
-                    int *o = &off[(size_t)slot * (span + 1)];
-                    int e = q;
-                    for (size_t k = 0; k <= span; ++k) {
-                        while (e < n && col(order[e]) == col(r) && ijkc[4 * order[e] + 2] < kmin + (int)k) ++e;
-                        o[k] = e;
-                    }
-                }
-                ent[q] = make_int2(ijkc[4 * r + 3], r);
-            }
-            CK(cudaMalloc(&h->d_rgrp, grp.size() * sizeof(uint2)));
-            CK(cudaMalloc(&h->d_roff, off.size() * sizeof(int)));
-            CK(cudaMalloc(&h->d_rent, ent.size() * sizeof(int2)));
-            CK(cudaMemcpy(h->d_rgrp, grp.data(), grp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(h->d_roff, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(h->d_rent, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
-        }
-    }
-    h->rec_kmin = kmin;
-    h->rec_kmax = kmax;
-    h->rec_fuse = fuse;
+    h->rec_kmin = t.kmin;
+    h->rec_kmax = t.kmax;
+    h->rec_fuse = t.fuse;
     return EWF_OK;
 }
 
@@ -1099,24 +1123,6 @@ extern "C" int ewf_reset(ewf_handle *h)
 // ------------------------------------------------------------------------------------------
 // the time step
 // ------------------------------------------------------------------------------------------
-// A launch on the handle's stream; `pdl`: as a programmatic dependent of the stream's previous
-// kernel (the kernel waits for it with griddepcontrol.wait before touching any state).
-template <typename... P, typename... A>
-static void launch_on(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, A... args)
-{
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 // Planes per CTA of the two-kernel step.  A shear source entry on plane 1 is applied by the thread of
 // plane 2 (fused_src_plane), which then has to be the one that stores plane 1 too.
 static int split_kchunk(const ewf_handle *h) { return h->src_plane1 ? std::max(h->kchunk, 4) : h->kchunk; }

@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(BX *BY, band_min_ctas<BY, T>()) k_band(const F
         vz_k = ld(a.f[2] + c);
         vz_km1 = ld(a.f[2] + c - sy);
         if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + ps);
-        stress_load<T, MODEL, DAMP, 1>(a, c, c, ps, nxt);
+        stress_load<T, MODEL, DAMP>(a, c, ps, nxt);
     }
     T szz_m = T(0), szz_mm = T(0);  // szz(p-1), szz(p-2) of the own column
     // buoyancy and 3-D weight of the velocity update, loaded a plane ahead (orthorhombic model)
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(BX *BY, band_min_ctas<BY, T>()) k_band(const F
         if (compute) {
             if (in_grid) {
                 const StressIn<T, MODEL, DAMP> q = nxt;
-                if (p + 1 < nz && p + 1 <= k1) stress_load<T, MODEL, DAMP, 1>(a, c + sy, c + sy, p + 1, nxt);
+                if (p + 1 < nz && p + 1 <= k1) stress_load<T, MODEL, DAMP>(a, c + sy, p + 1, nxt);
                 const T Vxx = (q.vx_ip - q.vx) * rdx;
                 const T Vyy = (q.vy_jp - q.vy) * rdy;
                 const T Vzz = (q.vz_p - vz_k) * rdz;

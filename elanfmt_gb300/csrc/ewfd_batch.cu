@@ -2,12 +2,14 @@
 //
 // The reference runs one model and one source per process (README.md:86-102; one scenario
 // directory per run).  A batch holds several problems (models, possibly of different sizes and
-// model families) with several right-hand sides each, advanced together: per time step one
-// persistent stress launch and one velocity launch per model family, one injection launch and
-// one receiver launch for everything -- captured in a CUDA graph.
+// model families) with several right-hand sides each, advanced together: every problem's launches
+// form a chain of their own -- two per step -- and the chains of a run of steps are captured in one CUDA
+// graph, one after the other (which leaves a small model's fields in L2 for its whole run of steps) or
+// on parallel branches.
 #include "ewfd.h"
 #include "ewfd_internal.h"
 #include "ewfd_batch.cuh"
+#include "ewfd_step.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -35,9 +37,7 @@ struct Prob {
     long long sy = 0;
     size_t box = 0;
     long long base_off = 0;
-    int sxs = 0;            // state box pitches (the material box's) and size of the R boxes
-    long long sys = 0;
-    size_t sbox = 0;
+    size_t sbox = 0;        // the R state boxes (the material box's pitches)
     long long sbase_off = 0;
     void *state[9] = {};
     void *mats[12] = {};
@@ -45,21 +45,23 @@ struct Prob {
     void *w3 = nullptr;
     bool m_set[12] = {};
     bool w_set[4] = {};
-    int kchunk = 16;
+    int kchunk = 0;                         // planes per CTA (0: by size, split_shape)
+    int ty = 4;                             // CTA tile height
+    bool pair = false;                      // two cells per thread
+    StressSrc ss{};                         // sources in the stress kernel (nsrc 0: k_binject)
+    SrcEntry *d_sent = nullptr;             // its entries, right-hand side by right-hand side
+    int *d_sstart = nullptr;                // first entry of each right-hand side, R + 1
+    int group0 = 0;                         // the problem's first (problem, RHS) group of k_binject
+    int nsrc = 0;
+    RecFuse rf{};                           // receivers in the velocity kernel
+    bool rec_fuse = true;
+    uint2 *d_rgrp = nullptr;
+    int *d_roff = nullptr;
+    int2 *d_rent = nullptr;
     bool fdiv = false;                      // div_spacing verified for dx, dy, dz
     std::vector<int32_t> rec;               // n x (i,j,k,comp)
     std::vector<std::vector<BatchSrc>> src;  // per RHS
     std::vector<double> stf;
-};
-
-struct Family {
-    int model, damping;           // single-RHS problems of one (model, damping) share a launch
-    std::vector<int> probs;       // problem indices
-    BatchProb<float> *d_probs = nullptr;
-    int *d_item0 = nullptr;
-    int nitems = 0;
-    int grid_stress = 0, grid_vel = 0;
-    int ty = TY;                  // CTA tile height of the family's launches
 };
 
 float *bptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.base_off : nullptr; }
@@ -73,20 +75,16 @@ struct ewf_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<Prob> probs;
-    std::vector<Family> fams;
     BatchProb<float> *d_all = nullptr;  // every problem, indexed by problem id
     std::vector<BatchProb<float>> h_all;  // host copy of d_all
-    std::vector<int> mr;                  // problems with several RHS: launched on their own
     int nrhs_total = 0;
     // sources
     BatchSrc *d_src = nullptr;
     int *d_src_start = nullptr;
-    int ngroups = 0;
     double *d_stf = nullptr;
     int *d_stf_off = nullptr;
     int *d_order = nullptr;
     // receivers
-    int *d_rec_prob = nullptr;
     long long *d_rec_off = nullptr;
     int *d_rec_comp = nullptr;
     int nrec_total = 0;
@@ -97,27 +95,28 @@ struct ewf_batch {
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     bool dirty = true;   // device tables need a rebuild
-    int ty = TY;         // CTA tile height in rows of 32 columns (autotuned; 4, 8 or 16)
-    int l2pf = 0;        // multi-RHS velocity kernel: L2 prefetch distance of its state inputs (autotuned; 0 = off)
-    bool own = false;    // every problem gets launches of its own, on BRANCHES parallel streams (autotuned);
-                         // false: the single-RHS problems of a family share one persistent launch
-    static constexpr int BRANCHES = 4;
+    int ty = 4;          // CTA tile height (4, 8 or 16 rows of 32 columns; two-cell kernels: twice as many, 16 at most)
+    int l2pf = -1;       // the velocity kernels' L2 prefetch distance (autotuned; 0: off, -1: by size)
+    int own = -1;        // the problems' chains one after another (0), on parallel streams (1), by size (-1; autotuned)
+    bool pdl = true;     // kernels launched as programmatic dependents (off if capture refuses)
+    static constexpr int BRANCHES = 8;
     cudaStream_t branch[BRANCHES] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[BRANCHES] = {};
-    std::vector<int> branch_of;  // per entry of mr: its branch (balanced by cell-updates)
+    std::vector<int> branch_of;  // per problem: its branch (balanced by cell-updates), -1: the batch's stream
     cudaGraphExec_t gexec = nullptr;
-    int gsteps = 64;
+    int gsteps = 64;     // steps per graph (even: the step counters alternate between two locations)
     float last_ms = 0.f;
-    int sms = 152;
 };
 
 static void free_tables(ewf_batch *b)
 {
-    for (auto &f : b->fams) {
-        cudaFree(f.d_probs);
-        cudaFree(f.d_item0);
-        f.d_probs = nullptr;
-        f.d_item0 = nullptr;
+    for (auto &q : b->probs) {
+        for (void *x : {(void *)q.d_sent, (void *)q.d_sstart, (void *)q.d_rgrp, (void *)q.d_roff, (void *)q.d_rent}) cudaFree(x);
+        q.d_sent = nullptr;
+        q.d_sstart = nullptr;
+        q.d_rgrp = nullptr;
+        q.d_roff = nullptr;
+        q.d_rent = nullptr;
     }
     cudaFree(b->d_all); b->d_all = nullptr;
     cudaFree(b->d_src); b->d_src = nullptr;
@@ -125,7 +124,6 @@ static void free_tables(ewf_batch *b)
     cudaFree(b->d_stf); b->d_stf = nullptr;
     cudaFree(b->d_stf_off); b->d_stf_off = nullptr;
     cudaFree(b->d_order); b->d_order = nullptr;
-    cudaFree(b->d_rec_prob); b->d_rec_prob = nullptr;
     cudaFree(b->d_rec_off); b->d_rec_off = nullptr;
     cudaFree(b->d_rec_comp); b->d_rec_comp = nullptr;
     if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
@@ -182,7 +180,6 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
     ewf_batch *b = new (std::nothrow) ewf_batch();
     if (!b) return ewf_fail(EWF_ERR_NOMEM, "host allocation");
     cudaGetDevice(&b->device);
-    cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
     b->nt = p[0].nt;
     b->probs.resize(n);
     size_t stage = 0;
@@ -209,7 +206,7 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
         q.p = p[i];
         q.p.workdir = nullptr;
         q.R = n_rhs ? n_rhs[i] : 1;
-        q.kchunk = p[i].kchunk > 0 ? p[i].kchunk : 16;
+        q.kchunk = p[i].kchunk > 0 ? p[i].kchunk : 0;
         if (q.p.model == EWF_MODEL_ORTHO)
             q.fdiv = ewf_fdiv_verified((float)q.p.dx) && ewf_fdiv_verified((float)q.p.dy) &&
                      ewf_fdiv_verified((float)q.p.dz);
@@ -218,8 +215,6 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
         q.sy = (long long)q.sx * (q.p.ny + 3);
         q.box = (size_t)q.sy * (q.p.nz + 3);
         q.base_off = hx + (long long)q.sx + q.sy;
-        q.sxs = q.sx;
-        q.sys = q.sy;
         q.sbox = q.box * q.R;      // R boxes back to back
         q.sbase_off = q.base_off;
         q.src.resize(q.R);
@@ -247,8 +242,10 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
     }
     CKB(cudaMalloc(&b->d_stage, stage));
     b->stage_bytes = stage;
-    CKB(cudaMalloc(&b->d_it, sizeof(int)));
-    CKB(cudaMemsetAsync(b->d_it, 0, sizeof(int), b->stream));
+    // graphs of two launches per problem and step, of some 16 thousand nodes at most
+    while (b->gsteps > 2 && (long long)b->gsteps * 2 * n > 16384) b->gsteps -= 2;
+    CKB(cudaMalloc(&b->d_it, 2 * n * sizeof(int)));
+    CKB(cudaMemsetAsync(b->d_it, 0, 2 * n * sizeof(int), b->stream));
     CKB(cudaStreamSynchronize(b->stream));
 #undef CKB
     *out = b;
@@ -375,48 +372,26 @@ extern "C" int ewf_batch_set_receivers(ewf_batch *b, int32_t prob, int32_t n, co
     return EWF_OK;
 }
 
-template <typename K>
-static int persistent_grid(K kernel, int sms, int nitems, int ty)
+template <typename T>
+static int upload(T **dst, const std::vector<T> &v)
 {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TX * ty, 0);
-    return std::max(1, std::min(nitems, sms * std::max(1, per_sm)));
+    CK(cudaMalloc(dst, v.size() * sizeof(T)));
+    CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return EWF_OK;
 }
 
-template <int MODEL, int DAMP>
-static int family_grid_t(bool stress, int sms, int items, int ty)
-{
-    return stress ? persistent_grid(k_bstress<float, MODEL, DAMP>, sms, items, ty)
-                  : persistent_grid(k_bvelocity<float, MODEL, DAMP>, sms, items, ty);
-}
+// Problems below BRANCH_CELLS cells (all right-hand sides) share the GPU on parallel branches; a larger one
+// fills it, and alone keeps its fields in L2.  us per step of six problems n^3, one after another and on
+// four branches:
+//   iso    32^3 30 10   64^3 40 22   80^3 62 50   96^3 76 88     128^3 198 222   160^3 432 441
+//   ortho  32^3 30 11   64^3 50 30   80^3 75 76   96^3 104 122   128^3 296 287   160^3 571 565
+// As many branches as hold BRANCH_SHARE cells between them, which L2 still keeps.  us per step on 2, 4 and
+// 8 branches:
+//   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
+//   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
+constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
 
-template <bool STRESS>
-static int family_grid(const Family &f, int sms, int items)
-{
-    if (f.model == EWF_MODEL_ISO) return family_grid_t<MODEL_ISO, DAMP_PML1D>(STRESS, sms, items, f.ty);
-    if (f.damping == EWF_DAMP_W3D) return family_grid_t<MODEL_ORTHO, DAMP_W3D>(STRESS, sms, items, f.ty);
-    return family_grid_t<MODEL_ORTHO, DAMP_SEP>(STRESS, sms, items, f.ty);
-}
-
-template <int MODEL, int DAMP>
-static void launch_family_t(const Family &f, bool stress, cudaStream_t s)
-{
-    if (stress)
-        k_bstress<float, MODEL, DAMP><<<f.grid_stress, dim3(TX, f.ty), 0, s>>>(f.d_probs, f.d_item0, (int)f.probs.size(),
-                                                                               f.nitems);
-    else
-        k_bvelocity<float, MODEL, DAMP><<<f.grid_vel, dim3(TX, f.ty), 0, s>>>(f.d_probs, f.d_item0, (int)f.probs.size(),
-                                                                              f.nitems);
-}
-
-static void launch_family(const Family &f, bool stress, cudaStream_t s)
-{
-    if (f.model == EWF_MODEL_ISO) launch_family_t<MODEL_ISO, DAMP_PML1D>(f, stress, s);
-    else if (f.damping == EWF_DAMP_W3D) launch_family_t<MODEL_ORTHO, DAMP_W3D>(f, stress, s);
-    else launch_family_t<MODEL_ORTHO, DAMP_SEP>(f, stress, s);
-}
-
-// Rebuilds the device tables (problem descriptors, work lists, sources, receivers, traces).
+// Rebuilds the device tables (problem descriptors, sources, receivers, traces).
 static int build_tables(ewf_batch *b)
 {
     CK(cudaStreamSynchronize(b->stream));
@@ -435,14 +410,13 @@ static int build_tables(ewf_batch *b)
         d.w3 = bptr(q, q.w3);
         d.sy = q.sy;
         d.sx = q.sx;
-        d.R = 1;
-        d.sxs = q.sx;
-        d.sys = q.sy;
         bp.rhs_stride = (long long)q.box;
-        bp.R = q.R;
         d.nx = p.nx; d.ny = p.ny; d.nz = p.nz;
         d.bc1_rows = std::min(p.ny, std::min(p.nx, p.ny + std::max(0, p.over_y)));
-        d.kchunk = q.kchunk;
+        const SplitShape shape = split_shape(p.nx, p.ny, p.nz, q.R);
+        q.ty = std::max(b->ty, shape.ty);
+        q.pair = shape.pair || q.R > 1;
+        d.kchunk = q.kchunk > 0 ? q.kchunk : shape.kchunk;
         d.dt = (float)p.dt;
         d.rdt = 1.0f / d.dt;
         d.dx = (float)p.dx; d.dy = (float)p.dy; d.dz = (float)p.dz;
@@ -455,69 +429,28 @@ static int build_tables(ewf_batch *b)
         d.bc1 = p.free_surface == EWF_FS_BC1 ? 1 : 0;
         d.smu_on = p.surface_mu > 0.0 ? 1 : 0;
         d.smu = (float)p.surface_mu;
-        d.l2pf = (q.R > 1 || b->own) ? b->l2pf : 0;
-        bp.tiles_x = (p.nx + TX - 1) / TX;
-        bp.tiles_y = (p.ny + b->ty - 1) / b->ty;
-        bp.chunks = (p.nz + q.kchunk - 1) / q.kchunk;
+        d.l2pf = b->l2pf >= 0 ? b->l2pf : shape.l2pf;
     }
-    // families (single-RHS problems sharing one persistent launch) and their work lists;
-    // problems with several RHS get their own launches (k_stress_mr / k_velocity_mr)
-    b->fams.clear();
-    b->mr.clear();
-    std::map<std::pair<int, int>, int> fam_of;
-    for (int i = 0; i < n; ++i) {
-        if (b->probs[i].R > 1 || b->own) {
-            b->mr.push_back(i);
-            continue;
-        }
-        const auto key = std::make_pair(b->probs[i].p.model, b->probs[i].p.damping);
-        if (!fam_of.count(key)) {
-            fam_of[key] = (int)b->fams.size();
-            b->fams.push_back(Family{key.first, key.second});
-            b->fams.back().ty = b->ty;
-        }
-        b->fams[fam_of[key]].probs.push_back(i);
-    }
-    // branches of the own launches: largest problems first, each to the least loaded branch
-    b->branch_of.assign(b->mr.size(), 0);
-    {
-        std::vector<int> idx(b->mr.size());
-        for (size_t e = 0; e < idx.size(); ++e) idx[e] = (int)e;
-        auto work = [&](int e) {
-            const Prob &q = b->probs[b->mr[e]];
+    // branches: largest problems first, each to the least loaded branch
+    b->branch_of.assign(n, -1);
+    if (b->own != 0 && n > 1) {
+        std::vector<int> idx(n);
+        for (int i = 0; i < n; ++i) idx[i] = i;
+        auto work = [&](int i) {
+            const Prob &q = b->probs[i];
             return (double)q.p.nx * q.p.ny * q.p.nz * q.R;
         };
         std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return work(x) > work(y); });
+        idx.erase(std::remove_if(idx.begin(), idx.end(), [&](int i) { return b->own < 0 && work(i) >= BRANCH_CELLS; }), idx.end());
+        const int branches = idx.empty() ? 1 : (int)std::max(2.0, std::min((double)ewf_batch::BRANCHES, BRANCH_SHARE / work(idx[0])));
         double load[ewf_batch::BRANCHES] = {};
-        for (int e : idx) {
-            const int k = (int)(std::min_element(load, load + ewf_batch::BRANCHES) - load);
-            b->branch_of[e] = k;
-            load[k] += work(e);
+        for (int i : idx) {
+            const int k = (int)(std::min_element(load, load + branches) - load);
+            b->branch_of[i] = k;
+            load[k] += work(i);
         }
-    }
-    for (auto &f : b->fams) {
-        std::vector<BatchProb<float>> v;
-        std::vector<int> item0;
-        int items = 0;
-        for (int i : f.probs) {
-            BatchProb<float> d = all[i];
-            d.item0 = items;
-            item0.push_back(items);
-            items += d.tiles_x * d.tiles_y * d.chunks * d.R;
-            v.push_back(d);
-        }
-        f.nitems = items;
-        CK(cudaMalloc(&f.d_probs, v.size() * sizeof(BatchProb<float>)));
-        CK(cudaMemcpy(f.d_probs, v.data(), v.size() * sizeof(BatchProb<float>), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&f.d_item0, item0.size() * sizeof(int)));
-        CK(cudaMemcpy(f.d_item0, item0.data(), item0.size() * sizeof(int), cudaMemcpyHostToDevice));
-        f.grid_stress = family_grid<true>(f, b->sms, items);
-        f.grid_vel = family_grid<false>(f, b->sms, items);
     }
     CK(cudaMalloc(&b->d_all, n * sizeof(BatchProb<float>)));
-    for (int i = 0; i < n; ++i) all[i].item0 = 0;
-    b->h_all = all;
-    CK(cudaMemcpy(b->d_all, all.data(), n * sizeof(BatchProb<float>), cudaMemcpyHostToDevice));
     // sources grouped by (problem, rhs)
     std::vector<BatchSrc> src;
     std::vector<int> start;
@@ -525,17 +458,37 @@ static int build_tables(ewf_batch *b)
     std::vector<int> stf_off(n), order(n);
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
+        q.group0 = (int)start.size();
+        const int first = (int)src.size();
+        std::vector<SrcEntry> ent;
+        std::vector<int> from;
         for (int r = 0; r < q.R; ++r) {
             start.push_back((int)src.size());
-            for (auto &e : q.src[r]) src.push_back(e);
+            from.push_back((int)ent.size());
+            for (auto &e : q.src[r]) {
+                src.push_back(e);
+                ent.push_back(SrcEntry{e.comp, e.i, e.j, e.k, e.coef});
+            }
             if (!q.src[r].empty() && q.stf.empty()) return ewf_fail(EWF_ERR_STATE, "problem %d has sources but no Src", i);
+        }
+        q.nsrc = (int)src.size() - first;
+        bool plane1 = false;
+        if (make_stress_src(ent, q.p.nx, q.p.ny, q.p.nz, &q.ss, &plane1)) {
+            from.push_back((int)ent.size());
+            if (int st = upload(&q.d_sent, ent)) return st;
+            if (int st = upload(&q.d_sstart, from)) return st;
+            q.ss.src = q.d_sent;
+            if (q.R > 1) q.ss.inl = 0;
+            // plane 2's thread applies a shear entry on plane 1, so it has to store that plane too
+            if (plane1) all[i].a.kchunk = std::max(all[i].a.kchunk, 4);
         }
         stf_off[i] = i * b->nt;
         if (!q.stf.empty()) std::copy(q.stf.begin(), q.stf.end(), stf.begin() + (size_t)i * b->nt);
         order[i] = q.p.src_order;
     }
     start.push_back((int)src.size());
-    b->ngroups = (int)start.size() - 1;
+    b->h_all = all;
+    CK(cudaMemcpy(b->d_all, all.data(), n * sizeof(BatchProb<float>), cudaMemcpyHostToDevice));
     if (!src.empty()) {
         CK(cudaMalloc(&b->d_src, src.size() * sizeof(BatchSrc)));
         CK(cudaMemcpy(b->d_src, src.data(), src.size() * sizeof(BatchSrc), cudaMemcpyHostToDevice));
@@ -574,9 +527,29 @@ static int build_tables(ewf_batch *b)
         }
     }
     b->nrec_total = nrec;
+    for (int i = 0; i < n; ++i) {
+        Prob &q = b->probs[i];
+        q.ss.stf = b->d_stf + (size_t)i * b->nt;
+        q.ss.nstf = b->nt;
+        q.ss.order = q.p.src_order;
+        const RecTables t = make_rec_tables((int)q.rec.size() / 4, q.rec.data(), q.p.nx, q.p.ny, q.p.nz);
+        q.rec_fuse = t.fuse;
+        q.rf = RecFuse{};
+        if (t.fuse && !t.ent.empty()) {
+            if (int st = upload(&q.d_rgrp, t.grp)) return st;
+            if (int st = upload(&q.d_roff, t.off)) return st;
+            if (int st = upload(&q.d_rent, t.ent)) return st;
+            q.rf.grp = q.d_rgrp;
+            q.rf.off = q.d_roff;
+            q.rf.ent = q.d_rent;
+            q.rf.ngx = (q.p.nx + 31) / 32;
+            q.rf.kmin = t.kmin;
+            q.rf.kmax = t.kmax;
+            q.rf.traces = b->d_traces + (size_t)b->rec_base[i] * b->nt;
+            q.rf.trace_len = b->nt;
+        }
+    }
     if (nrec) {
-        CK(cudaMalloc(&b->d_rec_prob, nrec * sizeof(int)));
-        CK(cudaMemcpy(b->d_rec_prob, rp.data(), nrec * sizeof(int), cudaMemcpyHostToDevice));
         CK(cudaMalloc(&b->d_rec_comp, nrec * sizeof(int)));
         CK(cudaMemcpy(b->d_rec_comp, rc.data(), nrec * sizeof(int), cudaMemcpyHostToDevice));
         CK(cudaMalloc(&b->d_rec_off, nrec * sizeof(long long)));
@@ -586,58 +559,92 @@ static int build_tables(ewf_batch *b)
     return EWF_OK;
 }
 
+// One step of problem i on a stream; `parity` = the step number's: its counter is at d_it[2 i + parity], the
+// next step's at d_it[2 i + 1 - parity].
 template <int MODEL, int DAMP>
-static void launch_mr_t(const BatchProb<float> &p, int ty, bool stress, cudaStream_t s)
+static void problem_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
 {
-    const dim3 grd(p.tiles_x * p.R, p.tiles_y, p.chunks);
-    if (stress)
-        k_stress_mr<float, MODEL, DAMP><<<grd, dim3(TX, ty), 0, s>>>(p.a, p.R, p.rhs_stride);
-    else
-        k_velocity_mr<float, MODEL, DAMP><<<grd, dim3(TX, ty), 0, s>>>(p.a, p.R, p.rhs_stride);
+    const Prob &q = b->probs[i];
+    const StepArgs<float> &a = b->h_all[i].a;
+    int *const it_rd = b->d_it + 2 * i + parity, *const it_wr = b->d_it + 2 * i + 1 - parity;
+    StressSrc ss = q.ss;
+    ss.it_ptr = it_rd;
+    RecFuse rf = q.rf;
+    rf.it_rd = it_rd;
+    if (q.rec_fuse) rf.it_wr = it_wr;
+    const int rows = q.pair ? pair_rows(q.ty) : q.ty, tiles_x = (q.p.nx + TX - 1) / TX;
+    const dim3 blk(q.pair ? PAIR_TX : TX, rows), grd(tiles_x * q.R, (q.p.ny + rows - 1) / rows, (q.p.nz + a.kchunk - 1) / a.kchunk);
+    const long long stride = b->h_all[i].rhs_stride, nr = (long long)q.rec.size() / 4;
+    if (q.R > 1) launch_on(k_stress_pair_mr<MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, q.R, stride, ss, (const int *)q.d_sstart);
+    else if (q.pair) launch_on(k_stress_pair<MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
+    else launch_on(k_stress<float, MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
+    if (q.nsrc > 0 && ss.nsrc == 0)
+        k_binject<float><<<(q.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, q.group0, q.R, b->d_stf, b->d_stf_off, b->d_order,
+                                                        b->nt, it_rd);
+    if (q.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP>, grd, blk, s, b->pdl, a, q.R, stride, rf, nr * b->nt);
+    else if (q.pair) launch_on(k_velocity_pair<MODEL, DAMP, false>, grd, blk, s, b->pdl, a, rf);
+    else launch_on(k_velocity<float, MODEL, DAMP, false>, grd, blk, s, b->pdl, a, rf);
+    if (!q.rec_fuse) {
+        const int rows_ = (int)nr * q.R;
+        k_brecord<float><<<std::min((rows_ + 255) / 256, 1024), 256, 0, s>>>(a, b->d_rec_off, b->d_rec_comp, b->rec_base[i], rows_, b->d_traces,
+                                                                            b->nt, it_rd);
+        k_advance<<<1, 1, 0, s>>>(it_rd, it_wr);
+    }
 }
 
-static void launch_mr(const ewf_batch *b, int i, bool stress, cudaStream_t s)
+// `steps` steps of every problem from step parity `parity` on, chain by chain: the branches' problems on
+// streams forked from the batch's and joined, then the others on the batch's stream.
+static void batch_steps(ewf_batch *b, int steps, int parity)
 {
-    const ewf_params &q = b->probs[i].p;
-    const BatchProb<float> &p = b->h_all[i];
-    if (q.model == EWF_MODEL_ISO) launch_mr_t<MODEL_ISO, DAMP_PML1D>(p, b->ty, stress, s);
-    else if (q.damping == EWF_DAMP_W3D) launch_mr_t<MODEL_ORTHO, DAMP_W3D>(p, b->ty, stress, s);
-    else launch_mr_t<MODEL_ORTHO, DAMP_SEP>(p, b->ty, stress, s);
-}
-
-static void batch_step(ewf_batch *b, cudaEvent_t *ev)
-{
-    cudaStream_t s = b->stream;
-    if (ev) cudaEventRecord(ev[0], s);
-    // the own launches of one phase: on one stream, or forked over the branch streams and joined
-    auto own_phase = [&](bool stress) {
-        if (!b->own || b->mr.size() < 2) {
-            for (int i : b->mr) launch_mr(b, i, stress, s);
-            return;
-        }
-        cudaEventRecord(b->fork_ev, s);
-        for (auto &x : b->branch) cudaStreamWaitEvent(x, b->fork_ev, 0);
-        for (size_t e = 0; e < b->mr.size(); ++e) launch_mr(b, b->mr[e], stress, b->branch[b->branch_of[e]]);
-        for (int k = 0; k < ewf_batch::BRANCHES; ++k) {
-            cudaEventRecord(b->join_ev[k], b->branch[k]);
-            cudaStreamWaitEvent(s, b->join_ev[k], 0);
+    auto chain = [&](size_t i, cudaStream_t s) {
+        const ewf_params &p = b->probs[i].p;
+        for (int k = 0; k < steps; ++k) {
+            const int par = (parity + k) & 1;
+            // nothing of another problem's to overlap with: a chain's first launch is a plain one
+            if (p.model == EWF_MODEL_ISO) problem_step_t<MODEL_ISO, DAMP_PML1D>(b, (int)i, par, k == 0, s);
+            else if (p.damping == EWF_DAMP_W3D) problem_step_t<MODEL_ORTHO, DAMP_W3D>(b, (int)i, par, k == 0, s);
+            else problem_step_t<MODEL_ORTHO, DAMP_SEP>(b, (int)i, par, k == 0, s);
         }
     };
-    own_phase(true);
-    for (auto &f : b->fams) launch_family(f, true, s);
-    if (ev) cudaEventRecord(ev[1], s);
-    if (b->d_src)
-        k_binject<float><<<(b->ngroups + 127) / 128, 128, 0, s>>>(b->d_all, b->d_src, b->d_src_start, b->ngroups, b->d_stf,
-                                                                  b->d_stf_off, b->d_order, b->nt, b->d_it);
-    if (ev) cudaEventRecord(ev[2], s);
-    own_phase(false);
-    for (auto &f : b->fams) launch_family(f, false, s);
-    if (ev) cudaEventRecord(ev[3], s);
-    if (b->nrec_total)
-        k_brecord<float><<<std::min((b->nrec_total + 255) / 256, 1024), 256, 0, s>>>(b->d_all, b->d_rec_prob, b->d_rec_off,
-                                                                                   b->d_rec_comp, b->nrec_total, b->d_traces, b->nt, b->d_it);
-    k_advance<<<1, 1, 0, s>>>(b->d_it);
-    if (ev) cudaEventRecord(ev[4], s);
+    bool used[ewf_batch::BRANCHES] = {};
+    for (int k : b->branch_of)
+        if (k >= 0) used[k] = true;
+    bool forked = false;
+    for (int k = 0; k < ewf_batch::BRANCHES; ++k) {
+        if (!used[k]) continue;
+        if (!forked) cudaEventRecord(b->fork_ev, b->stream);
+        forked = true;
+        cudaStreamWaitEvent(b->branch[k], b->fork_ev, 0);
+    }
+    for (size_t i = 0; i < b->probs.size(); ++i)
+        if (b->branch_of[i] >= 0) chain(i, b->branch[b->branch_of[i]]);
+    for (int k = 0; k < ewf_batch::BRANCHES; ++k) {
+        if (!used[k]) continue;
+        cudaEventRecord(b->join_ev[k], b->branch[k]);
+        cudaStreamWaitEvent(b->stream, b->join_ev[k], 0);
+    }
+    for (size_t i = 0; i < b->probs.size(); ++i)
+        if (b->branch_of[i] < 0) chain(i, b->stream);
+}
+
+static int batch_graph(ewf_batch *b)
+{
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    batch_steps(b, b->gsteps, 0);
+    const cudaError_t le = cudaGetLastError();
+    const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
+    if (le != cudaSuccess || ce != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return ewf_fail(EWF_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(le != cudaSuccess ? le : ce));
+    }
+    const cudaError_t ie = cudaGraphInstantiate(&b->gexec, g, 0);
+    cudaGraphDestroy(g);
+    if (ie != cudaSuccess) {
+        b->gexec = nullptr;
+        return ewf_fail(EWF_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(ie));
+    }
+    return EWF_OK;
 }
 
 static int batch_ready(ewf_batch *b)
@@ -660,7 +667,7 @@ extern "C" int ewf_batch_reset(ewf_batch *b)
     for (auto &q : b->probs)
         for (auto &x : q.state) CK(cudaMemsetAsync(x, 0, q.sbox * 4, b->stream));
     if (b->d_traces) CK(cudaMemsetAsync(b->d_traces, 0, (size_t)b->nrec_total * b->nt * sizeof(double), b->stream));
-    CK(cudaMemsetAsync(b->d_it, 0, sizeof(int), b->stream));
+    CK(cudaMemsetAsync(b->d_it, 0, 2 * b->probs.size() * sizeof(int), b->stream));
     CK(cudaStreamSynchronize(b->stream));
     b->it = 0;
     return EWF_OK;
@@ -672,29 +679,28 @@ extern "C" int ewf_batch_run(ewf_batch *b, int32_t nsteps)
     int st = batch_ready(b);
     if (st) return st;
     if (b->it + nsteps > b->nt) return ewf_fail(EWF_ERR_ARG, "step %d + %d exceeds nt = %d", b->it, nsteps, b->nt);
-    const bool use_graph = b->gsteps > 0 && nsteps >= b->gsteps;
+    // the graph starts from an even step
+    const int odd = b->it & 1;
+    const bool use_graph = nsteps >= b->gsteps + odd;
     if (use_graph && !b->gexec) {
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        for (int s = 0; s < b->gsteps; ++s) batch_step(b, nullptr);
-        const cudaError_t le = cudaGetLastError();
-        const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
-        if (le != cudaSuccess || ce != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            return ewf_fail(EWF_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(le != cudaSuccess ? le : ce));
+        st = batch_graph(b);
+        if (st && b->pdl) {  // a driver that cannot capture dependent launches: plain ones
+            cudaGetLastError();
+            b->pdl = false;
+            st = batch_graph(b);
         }
-        const cudaError_t ie = cudaGraphInstantiate(&b->gexec, g, 0);
-        cudaGraphDestroy(g);
-        if (ie != cudaSuccess) {
-            b->gexec = nullptr;
-            return ewf_fail(EWF_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(ie));
-        }
+        if (st) return st;
     }
     CK(cudaEventRecord(b->ev0, b->stream));
     int done = 0;
-    if (use_graph)
+    if (use_graph) {
+        if (odd) {
+            batch_steps(b, 1, 1);
+            done = 1;
+        }
         for (; done + b->gsteps <= nsteps; done += b->gsteps) CK(cudaGraphLaunch(b->gexec, b->stream));
-    for (; done < nsteps; ++done) batch_step(b, nullptr);
+    }
+    if (done < nsteps) batch_steps(b, nsteps - done, (b->it + done) & 1);
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev1, b->stream));
     CK(cudaStreamSynchronize(b->stream));
@@ -751,65 +757,59 @@ extern "C" int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int3
 extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_out)
 {
     if (!b || nsteps < 1) return ewf_fail(EWF_ERR_ARG, "bad argument");
-    static const int cand[] = {8, 12, 16, 24, 32, 48, 64};
-    static const int ty_cand[] = {4, 8, 16};
-    float best = 1e30f;
-    int best_k = 16, best_ty = b->ty;
-    bool best_own = b->own;
-    cudaEvent_t ev[5];
-    for (auto &e : ev) CK(cudaEventCreate(&e));
-    for (int own = 0; own < 2; ++own)
-    for (int ty : ty_cand)
-    for (int kc : cand) {
-        for (auto &q : b->probs) q.kchunk = std::max(4, std::min(kc, q.p.nz));
+    // planes per CTA: what the batch was created with or the rule by size (0), or one number for all
+    static const int cand[] = {0, 8, 12, 16, 24, 32};
+    static const int ty_cand[] = {4, 8};
+    static const int pf_cand[] = {0, 2, 3, 4};
+    const int steps = std::min(nsteps, b->nt - 1);
+    std::vector<int> given;
+    for (auto &q : b->probs) given.push_back(q.kchunk);
+    int best_k = 0, best_ty = b->ty, best_pf = -1;
+    int best_own = b->own;
+    auto apply = [&](int kc, int ty, int own, int pf) {
+        for (size_t i = 0; i < given.size(); ++i) b->probs[i].kchunk = kc ? std::max(4, std::min(kc, b->probs[i].p.nz)) : given[i];
         b->ty = ty;
-        b->own = own != 0;
+        b->own = own;
+        b->l2pf = pf;
         b->dirty = true;
+    };
+    auto time = [&](float *ms) {
         int st = batch_ready(b);
-        if (st) { for (auto &e : ev) cudaEventDestroy(e); return st; }
-        st = ewf_batch_reset(b);
-        if (st) { for (auto &e : ev) cudaEventDestroy(e); return st; }
-        batch_step(b, nullptr);  // warm
+        if (!st) st = ewf_batch_reset(b);
+        if (st) return st;
+        batch_steps(b, 1, 0);  // warm
         CK(cudaEventRecord(b->ev0, b->stream));
-        for (int s = 1; s < std::min(nsteps + 1, b->nt); ++s) batch_step(b, nullptr);
+        if (steps > 0) batch_steps(b, steps, 1);
         CK(cudaEventRecord(b->ev1, b->stream));
         CK(cudaStreamSynchronize(b->stream));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
-        if (ms < best) { best = ms; best_k = kc; best_ty = ty; best_own = own != 0; }
-    }
-    for (auto &q : b->probs) q.kchunk = std::max(4, std::min(best_k, q.p.nz));
-    b->ty = best_ty;
-    b->own = best_own;
-    b->dirty = true;
-    if (int st = batch_ready(b)) { for (auto &e : ev) cudaEventDestroy(e); return st; }
-    // then the multi-RHS velocity kernel's L2 prefetch distance at that setting
-    int best_pf = 0;
-    if (!b->mr.empty()) {
-        static const int pf_cand[] = {0, 2, 3, 4};
-        float best_pf_ms = 1e30f;
-        for (int pf : pf_cand) {
-            b->l2pf = pf;
-            b->dirty = true;
-            int st = batch_ready(b);
-            if (!st) st = ewf_batch_reset(b);
-            if (st) { for (auto &e : ev) cudaEventDestroy(e); return st; }
-            batch_step(b, nullptr);  // warm
-            CK(cudaEventRecord(b->ev0, b->stream));
-            for (int s = 1; s < std::min(nsteps + 1, b->nt); ++s) batch_step(b, nullptr);
-            CK(cudaEventRecord(b->ev1, b->stream));
-            CK(cudaStreamSynchronize(b->stream));
-            float ms = 0.f;
-            CK(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
-            if (ms < best_pf_ms) { best_pf_ms = ms; best_pf = pf; }
+        CK(cudaEventElapsedTime(ms, b->ev0, b->ev1));
+        return (int)EWF_OK;
+    };
+    float best = 1e30f, ms = 0.f;
+    for (int own = -1; own < 2; ++own)
+        for (int ty : ty_cand)
+            for (int kc : cand) {
+                apply(kc, ty, own, -1);
+                if (int st = time(&ms)) return st;
+                if (ms < best) {
+                    best = ms;
+                    best_k = kc;
+                    best_ty = ty;
+                    best_own = own;
+                }
+            }
+    for (int pf : pf_cand) {  // then the velocity kernels' L2 prefetch distance at that setting
+        apply(best_k, best_ty, best_own, pf);
+        if (int st = time(&ms)) return st;
+        if (ms < best) {
+            best = ms;
+            best_pf = pf;
         }
     }
-    for (auto &e : ev) cudaEventDestroy(e);
-    b->l2pf = best_pf;
-    b->dirty = true;
-    int st = batch_ready(b);
-    if (st) return st;
-    if (kchunk_out) *kchunk_out = best_k;
+    apply(best_k, best_ty, best_own, best_pf);
+    if (int st = batch_ready(b)) return st;
+    // the rule by size gives every problem its own chunk; 8 is the nearest of the candidates
+    if (kchunk_out) *kchunk_out = best_k ? best_k : 8;
     return ewf_batch_reset(b);
 }
 
@@ -826,7 +826,7 @@ extern "C" int ewf_batch_set_launch(ewf_batch *b, int32_t own)
 {
     if (!b) return ewf_fail(EWF_ERR_ARG, "NULL batch");
     if (own != 0 && own != 1) return ewf_fail(EWF_ERR_ARG, "own must be 0 or 1 (got %d)", own);
-    b->own = own != 0;
+    b->own = own;
     b->dirty = true;
     return EWF_OK;
 }
@@ -834,7 +834,7 @@ extern "C" int ewf_batch_set_launch(ewf_batch *b, int32_t own)
 extern "C" int ewf_batch_get_launch(const ewf_batch *b, int32_t *own)
 {
     if (!b || !own) return ewf_fail(EWF_ERR_ARG, "NULL argument");
-    *own = b->own ? 1 : 0;
+    *own = b->own > 0 ? 1 : 0;
     return EWF_OK;
 }
 

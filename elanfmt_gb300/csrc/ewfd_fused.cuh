@@ -24,7 +24,6 @@ namespace ewf {
 constexpr int FX = 32;                      // tile width (one warp per row)
 constexpr int FY = 8;                       // tile height
 constexpr int NHALO = 2 * FX + 2 * FY;      // halo positions per plane
-constexpr int MAXSRC = 64;                  // point sources per run (checked on the host)
 
 template <typename T>
 struct FusedArgs {
@@ -221,7 +220,7 @@ __global__ void __launch_bounds__(FX * FY, 3) k_step(const FusedArgs<T> fa)
         vy_m = ld(a.f[1] + c - sy);
         vz_k = ld(a.f[2] + c);
         if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + ps);
-        stress_load<T, MODEL, DAMP, 1>(a, c, c, ps, nxt);
+        stress_load<T, MODEL, DAMP>(a, c, ps, nxt);
     }
     T szz_m = T(0), szz_mm = T(0);   // szz(p-1), szz(p-2) of the own column
     __syncthreads();                  // s_src ready
@@ -262,7 +261,7 @@ __global__ void __launch_bounds__(FX * FY, 3) k_step(const FusedArgs<T> fa)
         if (compute) {
             if (in_grid) {
                 const StressIn<T, MODEL, DAMP> q = nxt;
-                if (p + 1 < nz && p + 1 <= k1) stress_load<T, MODEL, DAMP, 1>(a, c + sy, c + sy, p + 1, nxt);
+                if (p + 1 < nz && p + 1 <= k1) stress_load<T, MODEL, DAMP>(a, c + sy, p + 1, nxt);
                 const T Vxx = (q.vx_ip - q.vx) * rdx;
                 const T Vyy = (q.vy_jp - q.vy) * rdy;
                 const T Vzz = (q.vz_p - vz_k) * rdz;

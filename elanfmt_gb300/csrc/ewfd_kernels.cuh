@@ -43,9 +43,6 @@ struct StepArgs {
     const T *w6[6];   // per-component weights of Vx/sxx, Vy/syy, Vz/szz, sxy, sxz, syz (box layout)
     long long sy;     // plane pitch of materials / damping, elements
     int sx;           // row pitch of materials / damping, elements
-    int R;            // right-hand sides interleaved along x in the state arrays (1: one source)
-    int sxs;          // state row pitch (R * sx)
-    long long sys;    // state plane pitch
     int nx, ny, nz;
     int bc1_rows;     // rows j < bc1_rows get the szz / sxz free-surface rule (OK4:279-281)
     int kchunk;       // planes per CTA
@@ -76,10 +73,12 @@ struct SrcEntry {
 // test per plane.  The entries travel in the kernel's parameters (e) when there are few: read from
 // memory, a plane's pass over six of them was a chain of loads that outlasted the rest of a small
 // grid's launch.
+constexpr int MAXSRC = 64;     // point sources per run (checked on the host)
 constexpr int SRC_INLINE = 8;  // the 6 entries of a moment tensor, and room for a pressure source
 struct StressSrc {
     SrcEntry e[SRC_INLINE];
-    const SrcEntry *src;  // more than SRC_INLINE entries: all of them, in device memory
+    const SrcEntry *src;  // all of them in device memory
+    int inl;              // 1: e holds them
     int nsrc;             // 0: none (k_inject applies the sources, if any); every entry has i < nx, j < ny, k < nz
     const double *stf;
     int nstf;
@@ -117,7 +116,7 @@ struct RecFuse {
 __host__ __device__ __forceinline__ int fused_src_plane(int comp, int k) { return (k == 1 && (comp == 7 || comp == 8)) ? 2 : k; }
 
 template <typename T>
-__device__ __forceinline__ void inject_entry(const StepArgs<T> &a, const SrcEntry &q, T s, int order);
+__device__ __forceinline__ void inject_entry(const StepArgs<T> &a, const SrcEntry &q, T s, int order, long long soff = 0);
 
 template <typename T>
 __device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
@@ -281,27 +280,26 @@ struct StressIn {
     T pw[DAMP == DAMP_PERCOMP ? 6 : 1];  // per-component weights at the cell
 };
 
-// State part of a cell's stress inputs (c: state index, x stride R).
-template <typename T, int MODEL, int DAMP, int RC, int COH = 0>
+// State part of a cell's stress inputs (c: the cell's index).
+template <typename T, int MODEL, int DAMP, int COH = 0>
 __device__ __forceinline__ void stress_load_state(const StepArgs<T> &a, long long c, StressIn<T, MODEL, DAMP> &q)
 {
-    const int R = RC ? RC : a.R;
-    const int sx = (RC == 1) ? a.sx : a.sxs;
-    const long long sy = (RC == 1) ? a.sy : a.sys;
+    const int sx = a.sx;
+    const long long sy = a.sy;
     q.vx = lds<COH>(a.f[0] + c);
-    q.vx_ip = lds<COH>(a.f[0] + c + R);
+    q.vx_ip = lds<COH>(a.f[0] + c + 1);
     q.vx_jm = lds<COH>(a.f[0] + c - sx);
     q.vy = lds<COH>(a.f[1] + c);
     q.vy_jp = lds<COH>(a.f[1] + c + sx);
-    q.vy_im = lds<COH>(a.f[1] + c - R);
+    q.vy_im = lds<COH>(a.f[1] + c - 1);
     q.vz_p = lds<COH>(a.f[2] + c + sy);
-    q.vz_im = lds<COH>(a.f[2] + c - R);
+    q.vz_im = lds<COH>(a.f[2] + c - 1);
     q.vz_jm = lds<COH>(a.f[2] + c - sx);
 #pragma unroll
     for (int f = 0; f < 6; ++f) q.s[f] = a.f[3 + f][c];
 }
 
-// Material part (moduli, damping) of a cell's stress inputs (cm: material index, plane k).
+// Material part (moduli, damping) of a cell's stress inputs (cm: the cell's index, plane k).
 template <typename T, int MODEL, int DAMP>
 __device__ __forceinline__ void stress_load_mat(const StepArgs<T> &a, long long cm, int k, StressIn<T, MODEL, DAMP> &q)
 {
@@ -326,13 +324,12 @@ __device__ __forceinline__ void stress_load_mat(const StepArgs<T> &a, long long 
         q.w = (DAMP == DAMP_W3D) ? ld(a.w3 + cm) : ld(a.w1[2] + k);
     }
 }
-// c: state index (x stride R), cm: material index of the same cell
-template <typename T, int MODEL, int DAMP, int RC, int COH = 0>
-__device__ __forceinline__ void stress_load(const StepArgs<T> &a, long long c, long long cm, int k,
+template <typename T, int MODEL, int DAMP, int COH = 0>
+__device__ __forceinline__ void stress_load(const StepArgs<T> &a, long long c, int k,
                                             StressIn<T, MODEL, DAMP> &q)
 {
-    stress_load_state<T, MODEL, DAMP, RC, COH>(a, c, q);
-    stress_load_mat<T, MODEL, DAMP>(a, cm, k, q);
+    stress_load_state<T, MODEL, DAMP, COH>(a, c, q);
+    stress_load_mat<T, MODEL, DAMP>(a, c, k, q);
 }
 
 // damping factors constant along a column
@@ -427,12 +424,12 @@ __device__ __forceinline__ void stress_math(const StepArgs<T> &a, const StressIn
     }
 }
 
-// Stores the new stresses of cell c (plane k; sys: state plane pitch), with BC1 (when a.bc1):
+// Stores the new stresses of cell c (plane k; sy: plane pitch), with BC1 (when a.bc1):
 // szz = 0 on plane 0 and, from the freshly updated plane 2, sxz / syz on plane 1 (OK4:279-282).
 // BC1OWN: plane 1's shear cells that BC1 rewrites are stored by plane 2's thread alone, so planes 1
 // and 2 may belong to different CTAs (chunks of one or two planes).
 template <typename T, bool BC1OWN = false>
-__device__ __forceinline__ void stress_store(const StepArgs<T> &a, long long c, long long sys, int k, int i, int j,
+__device__ __forceinline__ void stress_store(const StepArgs<T> &a, long long c, long long sy, int k, int i, int j,
                                              bool row_bc, const T (&o)[6], bool w_xy, bool w_xz, bool w_yz)
 {
     if (BC1OWN && k == 1 && a.bc1) {
@@ -446,42 +443,33 @@ __device__ __forceinline__ void stress_store(const StepArgs<T> &a, long long c, 
     if (w_xz) a.f[7][c] = o[4];
     if (w_yz) a.f[8][c] = o[5];
     if (k == 2 && a.bc1) {
-        if (i > 0 && row_bc) a.f[7][c - sys] = a.third * o[4];
-        if (j > 0) a.f[8][c - sys] = a.third * o[5];
+        if (i > 0 && row_bc) a.f[7][c - sy] = a.third * o[4];
+        if (j > 0) a.f[8][c - sy] = a.third * o[5];
     }
 }
 
 // L2 prefetch of one 128-byte line (a hint: no completion to wait for, no register written).
 __device__ __forceinline__ void l2_prefetch_line(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// The column (X = i*R + r, j) over planes [k0, k1): X runs over the cells of every RHS.
-// RC: R known at compile time (1: one RHS, state and materials share one index; 0: a.R).
-// SOFF (with RC = 1): the state lives soff elements after the materials' index (one of several
-// right-hand sides in separate boxes of the same geometry).  COH: coherent state loads (lds).
-template <typename T, int MODEL, int DAMP, int RC, bool SOFF = false, int COH = 0, bool SRC = false>
-__device__ __forceinline__ void stress_column(const StepArgs<T> &a, int X, int j, int k0, int k1, long long soff = 0,
-                                              const StressSrc &ss = StressSrc{})
+// The column (i, j) over planes [k0, k1).  COH: coherent state loads (lds).
+template <typename T, int MODEL, int DAMP, int COH = 0, bool SRC = false>
+__device__ __forceinline__ void stress_column(const StepArgs<T> &a, int i, int j, int k0, int k1, const StressSrc &ss = StressSrc{})
 {
-    constexpr bool SEP = (RC != 1) || SOFF;  // separate state and material indices
-    const int R = RC ? RC : a.R;
-    const int i = (RC == 1) ? X : X / R;
     if (i >= a.nx || j >= a.ny) return;
-    const int sxs = (RC == 1) ? a.sx : a.sxs;
-    const long long sys = (RC == 1) ? a.sy : a.sys, sy = a.sy;
+    const long long sy = a.sy;
     const ColDamp<T> cd = col_damp<T, DAMP>(a, i, j);
     const bool row_bc = (j < a.bc1_rows);
 
-    long long c = (long long)X + (long long)j * sxs + (long long)k0 * sys + (SOFF ? soff : 0);
-    long long cm = !SEP ? c : (RC == 1) ? c - soff : (long long)i + (long long)j * a.sx + (long long)k0 * sy;
+    long long c = (long long)i + (long long)j * a.sx + (long long)k0 * sy;
     T wz_k = T(0);
     if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + k0);
     StressIn<T, MODEL, DAMP> nxt;
-    stress_load_mat<T, MODEL, DAMP>(a, SEP ? cm : c, k0, nxt);
+    stress_load_mat<T, MODEL, DAMP>(a, c, k0, nxt);
     if (SRC) pdl_wait();  // nothing above depends on an earlier launch
-    T vx_m = lds<COH>(a.f[0] + c - sys);  // Vx(k-1)
-    T vy_m = lds<COH>(a.f[1] + c - sys);  // Vy(k-1)
+    T vx_m = lds<COH>(a.f[0] + c - sy);  // Vx(k-1)
+    T vy_m = lds<COH>(a.f[1] + c - sy);  // Vy(k-1)
     T vz_k = lds<COH>(a.f[2] + c);        // Vz(k)
-    stress_load_state<T, MODEL, DAMP, RC, COH>(a, c, nxt);
+    stress_load_state<T, MODEL, DAMP, COH>(a, c, nxt);
     // point sources on this column (SRC: the two-kernel step's stress kernel)
     bool src_col = false;
     T s_src = T(0);
@@ -491,16 +479,15 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int X, int j
         if (src_col) s_src = (T)ss.stf[it];
     }
 
-    for (int k = k0; k < k1; ++k, c += sys) {
-        if (SEP && k > k0) cm += sy;
+    for (int k = k0; k < k1; ++k, c += sy) {
         const StressIn<T, MODEL, DAMP> q = nxt;
-        if (k + 1 < k1) stress_load<T, MODEL, DAMP, RC, COH>(a, c + sys, SEP ? cm + sy : c + sys, k + 1, nxt);
+        if (k + 1 < k1) stress_load<T, MODEL, DAMP, COH>(a, c + sy, k + 1, nxt);
         T o[6];
         bool w_xy, w_xz, w_yz;
         stress_math<T, MODEL, DAMP>(a, q, cd, i, j, k, vx_m, vy_m, vz_k, wz_k, o, w_xy, w_xz, w_yz);
-        stress_store<T, SRC>(a, c, sys, k, i, j, row_bc, o, w_xy, w_xz, w_yz);
+        stress_store<T, SRC>(a, c, sy, k, i, j, row_bc, o, w_xy, w_xz, w_yz);
         if (SRC && src_col && k >= ss.k0 && k <= ss.k1) {
-            if (ss.nsrc <= SRC_INLINE) {
+            if (ss.inl) {
 #pragma unroll
                 for (int e = 0; e < SRC_INLINE; ++e)
                     if (e < ss.nsrc && ss.e[e].i == i && ss.e[e].j == j && fused_src_plane(ss.e[e].comp, ss.e[e].k) == k)
@@ -533,9 +520,7 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
 {
     pdl_trigger();
     const int k0 = blockIdx.z * a.kchunk;
-    stress_column<T, MODEL, DAMP, 1, false, 0, true>(a, blockIdx.x * TX + threadIdx.x,
-                                                     blockIdx.y * blockDim.y + threadIdx.y, k0,
-                                                         min(k0 + a.kchunk, a.nz), 0, ss);
+    stress_column<T, MODEL, DAMP, 0, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz), ss);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -545,9 +530,9 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
 // refreshes the copy.  order 1 is "BC1, then inject" (ANISO:533-535).
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void inject_entry(const StepArgs<T> &a, const SrcEntry &q, T s, int order)
+__device__ __forceinline__ void inject_entry(const StepArgs<T> &a, const SrcEntry &q, T s, int order, long long soff)
 {
-    const long long c = (long long)q.i * a.R + (long long)q.j * a.sxs + (long long)q.k * a.sys;
+    const long long c = soff + (long long)q.i + (long long)q.j * a.sx + (long long)q.k * a.sy;
     T *f = a.f[q.comp];
     if (order == 0) {
         const bool row_bc = a.bc1 && q.j < a.bc1_rows;
@@ -555,7 +540,7 @@ __device__ __forceinline__ void inject_entry(const StepArgs<T> &a, const SrcEntr
         const bool yz_bc = a.bc1 && (q.comp == 8) && q.j > 0 && q.j < a.ny && q.i < a.nx;
         if ((q.comp == 5 && q.k == 0 && row_bc) || ((xz_bc || yz_bc) && q.k == 1)) return;
         f[c] = f[c] + (T)q.coef * s;
-        if ((xz_bc || yz_bc) && q.k == 2) f[c - a.sys] = a.third * f[c];
+        if ((xz_bc || yz_bc) && q.k == 2) f[c - a.sy] = a.third * f[c];
     } else {
         f[c] = f[c] + (T)q.coef * s;
     }
@@ -591,37 +576,36 @@ struct VelIn {
     T cp[KAHAN ? 3 : 1];
 };
 
-// The stresses around a cell that its velocity update reads (c: state index, x stride R).
-template <typename T, int MODEL, int DAMP, bool KAHAN, int RC, int COH = 0>
+// The stresses around a cell that its velocity update reads (c: the cell's index).
+template <typename T, int MODEL, int DAMP, bool KAHAN, int COH = 0>
 __device__ __forceinline__ void vel_load_sigma(const StepArgs<T> &a, long long c, VelIn<T, MODEL, DAMP, KAHAN> &q)
 {
-    const int R = RC ? RC : a.R;
-    const int sx = (RC == 1) ? a.sx : a.sxs;
-    const long long sy = (RC == 1) ? a.sy : a.sys;
+    const int sx = a.sx;
+    const long long sy = a.sy;
     q.sxx = lds<COH>(a.f[3] + c);
-    q.sxx_im = lds<COH>(a.f[3] + c - R);
+    q.sxx_im = lds<COH>(a.f[3] + c - 1);
     q.syy = lds<COH>(a.f[4] + c);
     q.syy_jm = lds<COH>(a.f[4] + c - sx);
     q.szz = lds<COH>(a.f[5] + c);
     q.sxy = lds<COH>(a.f[6] + c);
     q.sxy_jp = lds<COH>(a.f[6] + c + sx);
-    q.sxy_ip = lds<COH>(a.f[6] + c + R);
+    q.sxy_ip = lds<COH>(a.f[6] + c + 1);
     q.sxz_p = lds<COH>(a.f[7] + c + sy);
-    q.sxz_ip = lds<COH>(a.f[7] + c + R);
+    q.sxz_ip = lds<COH>(a.f[7] + c + 1);
     q.syz_p = lds<COH>(a.f[8] + c + sy);
     q.syz_jp = lds<COH>(a.f[8] + c + sx);
 }
 
 // State part of a cell's velocity inputs: the stresses around the cell and the old velocities.
-template <typename T, int MODEL, int DAMP, bool KAHAN, int RC, int COH = 0>
+template <typename T, int MODEL, int DAMP, bool KAHAN, int COH = 0>
 __device__ __forceinline__ void vel_load_state(const StepArgs<T> &a, long long c, VelIn<T, MODEL, DAMP, KAHAN> &q)
 {
-    vel_load_sigma<T, MODEL, DAMP, KAHAN, RC, COH>(a, c, q);
+    vel_load_sigma<T, MODEL, DAMP, KAHAN, COH>(a, c, q);
 #pragma unroll
     for (int f = 0; f < 3; ++f) q.v[f] = a.f[f][c];
 }
 
-// Material part (buoyancy, damping) of a cell's velocity inputs (cm: material index, plane k).
+// Material part (buoyancy, damping) of a cell's velocity inputs (cm: the cell's index, plane k).
 template <typename T, int MODEL, int DAMP, bool KAHAN>
 __device__ __forceinline__ void vel_load_mat(const StepArgs<T> &a, long long cm, int k, VelIn<T, MODEL, DAMP, KAHAN> &q)
 {
@@ -636,12 +620,12 @@ __device__ __forceinline__ void vel_load_mat(const StepArgs<T> &a, long long cm,
         q.w = (DAMP == DAMP_W3D) ? ld(a.w3 + cm) : ld(a.w1[2] + k);
     }
 }
-template <typename T, int MODEL, int DAMP, bool KAHAN, int RC, int COH = 0>
-__device__ __forceinline__ void vel_load(const StepArgs<T> &a, long long c, long long cm, int k,
+template <typename T, int MODEL, int DAMP, bool KAHAN, int COH = 0>
+__device__ __forceinline__ void vel_load(const StepArgs<T> &a, long long c, int k,
                                          VelIn<T, MODEL, DAMP, KAHAN> &q)
 {
-    vel_load_state<T, MODEL, DAMP, KAHAN, RC, COH>(a, c, q);
-    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, cm, k, q);
+    vel_load_state<T, MODEL, DAMP, KAHAN, COH>(a, c, q);
+    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, c, k, q);
     if (KAHAN) {
 #pragma unroll
         for (int f = 0; f < 3; ++f) q.cp[f] = a.comp[f][c];
@@ -751,30 +735,24 @@ __device__ __forceinline__ const T *vel_prefetch_field(const StepArgs<T> &a, int
     return nullptr;
 }
 
-template <typename T, int MODEL, int DAMP, bool KAHAN, int RC, bool SOFF = false, int COH = 0, bool REC = false>
-__device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int j, int kc0, int kc1, long long soff = 0,
-                                                const RecFuse &rf = RecFuse{})
+template <typename T, int MODEL, int DAMP, bool KAHAN, int COH = 0, bool REC = false>
+__device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int i, int j, int kc0, int kc1, const RecFuse &rf = RecFuse{})
 {
-    constexpr bool SEP = (RC != 1) || SOFF;  // separate state and material indices (see stress_column)
-    const int R = RC ? RC : a.R;
-    const int i = (RC == 1) ? X : X / R;
     if (i < 1 || j < 1 || i >= a.nx || j >= a.ny) return;
     const int k0 = max(1, kc0);
     const int k1 = kc1;
     if (k0 >= k1) return;
-    const int sxs = (RC == 1) ? a.sx : a.sxs;
-    const long long sys = (RC == 1) ? a.sy : a.sys, sy = a.sy;
+    const long long sy = a.sy;
     const VelDamp<T> vd = vel_damp<T, DAMP>(a, i, j);
 
-    long long c = (long long)X + (long long)j * sxs + (long long)k0 * sys + (SOFF ? soff : 0);
-    long long cm = !SEP ? c : (RC == 1) ? c - soff : (long long)i + (long long)j * a.sx + (long long)k0 * sy;
+    long long c = (long long)i + (long long)j * a.sx + (long long)k0 * sy;
     VelIn<T, MODEL, DAMP, KAHAN> nxt;
-    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, SEP ? cm : c, k0, nxt);
-    if (REC && !SEP) pdl_wait();  // nothing above depends on an earlier launch
-    T szz_m = lds<COH>(a.f[5] + c - sys);
+    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, c, k0, nxt);
+    if (REC) pdl_wait();  // nothing above depends on an earlier launch
+    T szz_m = lds<COH>(a.f[5] + c - sy);
     T sxz_k = lds<COH>(a.f[7] + c);
     T syz_k = lds<COH>(a.f[8] + c);
-    vel_load_state<T, MODEL, DAMP, KAHAN, RC, COH>(a, c, nxt);
+    vel_load_state<T, MODEL, DAMP, KAHAN, COH>(a, c, nxt);
     if (KAHAN) {
 #pragma unroll
         for (int f = 0; f < 3; ++f) nxt.cp[f] = a.comp[f][c];
@@ -782,8 +760,8 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
     // the L2 prefetch's field for this lane (REC: the two-kernel step's velocity kernel)
     const T *pf_row = nullptr;
     if (REC && a.l2pf > 0) {
-        pf_row = vel_prefetch_field<T, MODEL, DAMP, KAHAN, SOFF>(a, (int)threadIdx.x);
-        if (pf_row) pf_row += c - (long long)threadIdx.x + (long long)a.l2pf * sys;
+        pf_row = vel_prefetch_field<T, MODEL, DAMP, KAHAN>(a, (int)threadIdx.x);
+        if (pf_row) pf_row += c - (long long)threadIdx.x + (long long)a.l2pf * sy;
     }
     // receivers on this column (REC: the two-kernel step's velocity kernel)
     int slot = -1, r_it = 0;
@@ -795,11 +773,10 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int X, int
         }
     }
 
-    for (int k = k0; k < k1; ++k, c += sys) {
-        if (SEP && k > k0) cm += sy;
+    for (int k = k0; k < k1; ++k, c += sy) {
         VelIn<T, MODEL, DAMP, KAHAN> q = nxt;
-        if (k + 1 < k1) vel_load<T, MODEL, DAMP, KAHAN, RC, COH>(a, c + sys, SEP ? cm + sy : c + sys, k + 1, nxt);
-        if (REC && pf_row && k + a.l2pf < k1) l2_prefetch_line(pf_row + (long long)(k - k0) * sys);
+        if (k + 1 < k1) vel_load<T, MODEL, DAMP, KAHAN, COH>(a, c + sy, k + 1, nxt);
+        if (REC && pf_row && k + a.l2pf < k1) l2_prefetch_line(pf_row + (long long)(k - k0) * sy);
         T v[3], cp[3] = {KAHAN ? q.cp[0] : T(0), KAHAN ? q.cp[1] : T(0), KAHAN ? q.cp[2] : T(0)};
         vel_math<T, MODEL, DAMP, KAHAN>(a, q, vd, szz_m, sxz_k, syz_k, v, cp);
         vel_store<T, KAHAN>(a, c, k, i, j, v, cp);
@@ -830,9 +807,8 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
         *rf.it_wr = *rf.it_rd + 1;  // the next step's counter; this launch reads only it_rd
     }
     const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
-    velocity_column<T, MODEL, DAMP, KAHAN, 1, false, 0, true>(a, blockIdx.x * TX + threadIdx.x,
-                                                              blockIdx.y * blockDim.y + threadIdx.y, k0,
-                                                                  min(k0 + a.kchunk, a.nz), 0, rf);
+    velocity_column<T, MODEL, DAMP, KAHAN, 0, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
+                                                    min(k0 + a.kchunk, a.nz), rf);
 }
 
 // ---------------------------------------------------------------------------------------------

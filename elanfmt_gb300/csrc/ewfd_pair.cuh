@@ -138,14 +138,16 @@ __device__ __forceinline__ void stress_state2(const StepArgs<float> &a, long lon
     for (int f = 0; f < 6; ++f) q.s[f] = ld2<false>(a.f[3 + f] + c);
 }
 
-// The pair (i, i+1) of row j over planes [k0, k1); soff: the state lies that far after the materials' index.
+// The pair (i, i+1) of row j over planes [k0, k1).  soff, start, r: right-hand side r of several -- its state
+// lies soff elements after the materials' index, its sources are entries start[r] .. start[r+1] - 1.
 // The orthorhombic update loads a plane ahead (PF), in 128 registers; the others have fewer loads per plane
 // and do better with 85 registers and half as many warps again (iso-het 203x151x97 72.5 -> 68.0 us a step, 96^3 15.7 ->
 // 14.4; ortho 128^3 in 85 without the prefetch 52.2 -> 54.9, 320x320x256 596 -> 603).
 template <int MODEL>
 __host__ __device__ constexpr bool pair_prefetch() { return MODEL == MODEL_ORTHO; }
 template <int MODEL, int DAMP>
-__device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int j, int k0, int k1, long long soff, const StressSrc &ss)
+__device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int j, int k0, int k1, long long soff, const StressSrc &ss,
+                                            const int *start = nullptr, int r = 0)
 {
     constexpr bool PF = pair_prefetch<MODEL>();
     if (i >= a.nx || j >= a.ny) return;
@@ -174,10 +176,15 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
     stress_state2<MODEL, DAMP>(a, c, nxt);
     bool src_col = false;
     float s_src = 0.f;
+    int e0 = 0, e1 = ss.nsrc;
     if (ss.nsrc > 0 && i + 1 >= ss.i0 && i <= ss.i1 && j >= ss.j0 && j <= ss.j1 && k0 <= ss.k1 && k1 > ss.k0) {
         const int it = *ss.it_ptr;
         src_col = it >= 0 && it < ss.nstf;
         if (src_col) s_src = (float)ss.stf[it];
+        if (start) {
+            e0 = start[r];
+            e1 = start[r + 1];
+        }
     }
     const PairOps op = {dup(a.one), dup(a.minus_one)};
     const f2 dt = dup(a.dt), rdx = dup(a.rdx), rdy = dup(a.rdy), rdz = dup(a.rdz);
@@ -246,13 +253,10 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
             if (j > 0) st2(a.f[8] + c - a.sy, mul2(dup(a.third), o[5]), true, in1);
         }
         if (src_col && k >= ss.k0 && k <= ss.k1) {
-            StepArgs<float> b = a;
-            if (soff)
-                for (auto &f : b.f) f += soff;
-            for (int e = 0; e < ss.nsrc; ++e) {
-                const SrcEntry q_e = ss.nsrc <= SRC_INLINE ? ss.e[e] : ss.src[e];
+            for (int e = e0; e < e1; ++e) {
+                const SrcEntry q_e = ss.inl ? ss.e[e] : ss.src[e];
                 if ((q_e.i == i || (q_e.i == i + 1 && in1)) && q_e.j == j && fused_src_plane(q_e.comp, q_e.k) == k)
-                    inject_entry(b, q_e, s_src, ss.order);
+                    inject_entry(a, q_e, s_src, ss.order, soff);
             }
         }
         wz_k = q.w;
@@ -326,7 +330,8 @@ __device__ __forceinline__ f2 vel_update2(const StepArgs<float> &a, const PairOp
 }
 
 template <int MODEL, int DAMP, bool KAHAN>
-__device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, int j, int kc0, int k1, long long soff, const RecFuse &rf)
+__device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, int j, int kc0, int k1, long long soff, const RecFuse &rf,
+                                              double *traces)
 {
     const int k0 = max(1, kc0);
     if (j < 1 || i >= a.nx || j >= a.ny || k0 >= k1) return;
@@ -418,7 +423,7 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
                     const f2 nv = re.x == 0 ? v[0] : re.x == 1 ? v[1] : v[2], ov = re.x == 0 ? q.v[0] : re.x == 1 ? q.v[1] : q.v[2];
                     const bool upd = h ? (re.x == 0 ? m1[0] : re.x == 1 ? m1[1] : m1[2]) : (re.x == 0 ? m0[0] : re.x == 1 ? m0[1] : m0[2]);
                     const f2 val = upd ? nv : ov;
-                    rf.traces[(long long)re.y * rf.trace_len + r_it] = (double)(h ? hi(val) : lo(val));
+                    traces[(long long)re.y * rf.trace_len + r_it] = (double)(h ? hi(val) : lo(val));
                 }
             }
         }
@@ -450,7 +455,37 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const Ste
     }
     const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
     velocity_pair<MODEL, DAMP, KAHAN>(a, blockIdx.x * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
-                                      min(k0 + a.kchunk, a.nz), 0, rf);
+                                      min(k0 + a.kchunk, a.nz), 0, rf, rf.traces);
+}
+
+// Several right-hand sides of one model, their state boxes rhs_stride elements apart: the index of the
+// right-hand side is the fastest part of blockIdx.x, so the CTAs of a tile are dispatched together and read
+// its material planes from HBM once (the others' reads hit L2).  start: their source entries in ss.src;
+// trace_stride: elements between their trace blocks.  A batch of 6 right-hand sides on ortho 128^3 and 6 isotropic
+// models of 96^3 to 160^3: 503 us a step, 640 with one cell per thread and separate injection and receiver launches
+// for all problems; its fields and materials move in 425 us at the copy bandwidth.
+template <int MODEL, int DAMP>
+__global__ void __launch_bounds__(PAIR_MAX_THREADS, pair_prefetch<MODEL>() ? 2 : 3)
+    k_stress_pair_mr(const StepArgs<float> a, int R, long long rhs_stride, const __grid_constant__ StressSrc ss, const int *start)
+{
+    pdl_trigger();
+    const int r = blockIdx.x % R, k0 = blockIdx.z * a.kchunk;
+    stress_pair<MODEL, DAMP>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz),
+                             (long long)r * rhs_stride, ss, start, r);
+}
+
+template <int MODEL, int DAMP>
+__global__ void __launch_bounds__(PAIR_MAX_THREADS, 3)
+    k_velocity_pair_mr(const StepArgs<float> a, int R, long long rhs_stride, const RecFuse rf, long long trace_stride)
+{
+    pdl_trigger();
+    if (rf.it_wr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+        pdl_wait();
+        *rf.it_wr = *rf.it_rd + 1;
+    }
+    const int r = blockIdx.x % R, k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
+    velocity_pair<MODEL, DAMP, false>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
+                                      min(k0 + a.kchunk, a.nz), (long long)r * rhs_stride, rf, rf.traces + r * trace_stride);
 }
 
 }  // namespace ewf

@@ -1,0 +1,47 @@
+// ewfd_step.h -- host side of the two-kernel step shared by the solver and the batch (ewfd.cu).
+#pragma once
+#include <limits.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <vector>
+
+#include "ewfd_kernels.cuh"
+
+// Sources for the stress kernel (false: the injection kernel applies them)
+bool make_stress_src(const std::vector<ewf::SrcEntry> &v, int nx, int ny, int nz, ewf::StressSrc *f, bool *plane1);
+
+// Receivers for the velocity kernel (fuse false: the recording kernel samples them)
+struct RecTables {
+    bool fuse = true;
+    int kmin = INT32_MAX, kmax = -1;
+    std::vector<uint2> grp;
+    std::vector<int> off;
+    std::vector<int2> ent;
+};
+RecTables make_rec_tables(int n, const int32_t *ijkc, int nx, int ny, int nz);
+
+// Launch shape by the cells a launch updates (R right-hand sides)
+struct SplitShape {
+    int kchunk, ty, l2pf;
+    bool pair;
+};
+SplitShape split_shape(int nx, int ny, int nz, int R = 1);
+
+// A launch on a stream; `pdl`: as a programmatic dependent of the stream's previous
+// kernel (the kernel waits for it with griddepcontrol.wait before touching any state).
+template <typename... P, typename... A>
+inline void launch_on(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, A... args)
+{
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}

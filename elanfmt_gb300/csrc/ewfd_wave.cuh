@@ -227,10 +227,10 @@ __global__ void __launch_bounds__(WAVE_THREADS, MINB) k_wave(const StepArgs<T> a
         int k0, k1;
         if (!vel) {
             wave_stress_planes(w, a.nz, s, k0, k1);
-            stress_column<T, MODEL, DAMP, 1, false, true>(a, X, j, k0, k1);
+            stress_column<T, MODEL, DAMP, true>(a, X, j, k0, k1);
         } else {
             wave_velocity_planes(w, a.nz, s, k0, k1);
-            velocity_column<T, MODEL, DAMP, KAHAN, 1, false, true>(a, X, j, k0, k1);
+            velocity_column<T, MODEL, DAMP, KAHAN, true>(a, X, j, k0, k1);
         }
         mbar_arrive(&s_empty[b]);
     }

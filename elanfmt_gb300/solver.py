@@ -495,7 +495,8 @@ class Batch:
         return k.value
 
     def set_tile(self, tile_y: int) -> None:
-        """CTA tile height of the batch's launches (4, 8 or 16 rows of 32 columns)."""
+        """CTA tile height of the batch's launches (4, 8 or 16 rows of 32 columns; twice as many, 16 at
+        most, with two cells per thread)."""
         _check(self._lib.ewf_batch_set_tile(self._h, int(tile_y)), "ewf_batch_set_tile")
 
     def tile(self) -> int:
@@ -504,8 +505,8 @@ class Batch:
         return ty.value
 
     def set_launch(self, own: int) -> None:
-        """Single-RHS problems: 0 = one persistent launch per model family, 1 = launches of their own
-        on parallel branches (results do not depend on it)."""
+        """0 = one problem's run of steps after another's, 1 = on parallel branches; by default the small
+        problems on branches, then the others (results do not depend on it)."""
         _check(self._lib.ewf_batch_set_launch(self._h, int(own)), "ewf_batch_set_launch")
 
     def launch(self) -> int:
@@ -514,7 +515,7 @@ class Batch:
         return v.value
 
     def set_l2_prefetch(self, planes: int) -> None:
-        """Multi-RHS problems: L2 prefetch distance of their velocity kernel (0 = off; results do not depend on it)."""
+        """L2 prefetch distance of the velocity kernels (0 = off; results do not depend on it)."""
         _check(self._lib.ewf_batch_set_l2_prefetch(self._h, int(planes)), "ewf_batch_set_l2_prefetch")
 
     def l2_prefetch(self) -> int:

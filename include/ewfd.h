@@ -329,10 +329,10 @@ int ewf_restore(ewf_handle *h, const char *path);
  * Batched solver (no counterpart in the reference, which runs one model and one source per
  * process): n problems -- models of any size and family -- each with n_rhs[i] right-hand sides
  * (independent source sets sharing the problem's model, e.g. the 6 elementary moment tensors of
- * a moment-tensor inversion), advanced together.  Per time step one persistent launch per model
- * family for each of the stress and velocity phases (materials read once per cell for all the
- * problem's RHS), one injection and one receiver launch, replayed from a CUDA graph.  FP32;
- * every problem runs the same nt; state starts at zero.
+ * a moment-tensor inversion), advanced together.  Per time step and problem one stress and one
+ * velocity launch for all its RHS (materials read from HBM once), with sources and receivers inside
+ * where the solver's own step has them there, replayed from a CUDA graph.  FP32; every problem runs the
+ * same nt; state starts at zero.
  * ------------------------------------------------------------------------------------------- */
 typedef struct ewf_batch ewf_batch;
 int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n_rhs, ewf_batch **out);
@@ -352,20 +352,19 @@ int ewf_batch_last_run_ms(const ewf_batch *b, double *ms);
 int ewf_batch_get_seismograms(ewf_batch *b, int32_t prob, int32_t rhs, double *out, size_t n);
 int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int32_t field, void *host, size_t n, int32_t dtype_bytes);
 /* the autotuner over the whole batch: launch form, z-chunk and CTA tile height, then the
- * multi-RHS velocity kernel's L2 prefetch distance (leaves the batch reset) */
+ * velocity kernels' L2 prefetch distance (leaves the batch reset) */
 int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk);
-/* CTA tile height of every launch of the batch, in rows of 32 columns: 4, 8 (default) or 16;
- * results do not depend on it */
+/* CTA tile height of every launch of the batch, in rows of 32 columns: 4 (default), 8 or 16
+ * (kernels with two cells per thread take twice as many rows, 16 at most); results do not depend on it */
 int ewf_batch_set_tile(ewf_batch *b, int32_t tile_y);
 int ewf_batch_get_tile(const ewf_batch *b, int32_t *tile_y);
-/* Problems with several RHS: their velocity kernel asks L2 for the state lines `planes` planes
- * ahead (0..8; 0 = off, the default; ewf_batch_autotune picks it).  A hint: results do not
- * depend on it. */
+/* The velocity kernels ask L2 for their state lines `planes` planes ahead (0..8; 0 = off; by
+ * default large problems do; ewf_batch_autotune picks it).  A hint: results do not depend on it. */
 int ewf_batch_set_l2_prefetch(ewf_batch *b, int32_t planes);
-/* Launch form of the single-RHS problems: 0 (default) -- those of one model family share one
- * persistent launch per phase; 1 -- every problem gets launches of its own, spread over four
- * parallel branches (streams of the captured graph) balanced by cell-updates.  Problems with
- * several RHS always have their own launches.  Results do not depend on it. */
+/* Launch form: 0 -- one problem's run of steps after another's; 1 -- spread over up to eight parallel
+ * branches (streams of the captured graph) balanced by cell-updates.  By default (reported as 0) the
+ * problems too small to fill the GPU run on branches, then the others one after another.  Results do
+ * not depend on it. */
 int ewf_batch_set_launch(ewf_batch *b, int32_t own);
 int ewf_batch_get_launch(const ewf_batch *b, int32_t *own);
 int ewf_batch_get_l2_prefetch(const ewf_batch *b, int32_t *planes);
