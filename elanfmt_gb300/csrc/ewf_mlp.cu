@@ -46,8 +46,8 @@ __device__ __forceinline__ float gelu_grad(float x)
 // K-major as written or transposed ([K, M], [K, N]: TA, TB), so gradients need no transposed copies.
 // Persistent: one CTA per SM walks tiles of one product (a launch may hold two independent ones, each with
 // CTAs of its own).  Two fp32 accumulators of 128 lanes x bn columns in tensor memory, so the
-// epilogue of one tile overlaps the MMAs of the next.  Warp roles, 320 threads:
-//   warp 0: TMA producer -- per k-stage the operands' boxes (128-byte swizzle, ewf_umma.h)
+// epilogue of one tile overlaps the MMAs of the next.  Warp roles, 352 threads:
+//   warps 0 and 10: TMA producers -- per k-stage the boxes of A and of B (128-byte swizzle, ewf_umma.h)
 //     into the next free slot of a ring of stages, completing on that slot's "full" mbarrier; the ring
 //     runs on across items; rows and K beyond a matrix's end read as zeros;
 //   warp 1: MMA issuer -- waits for a free accumulator ("acc_empty"), then per stage for
@@ -62,7 +62,14 @@ __device__ __forceinline__ float gelu_grad(float x)
 // loads, epilogue); hidden layers of many rows, the GELU's erff; the output layer, the operands' way
 // from L2 and the output bytes.  With four epilogue warps storing a row per lane, and now: 128 x 512 x
 // 512 24.9 and 6.8 us, 8192 x 512 x 512 25.1 and 12.8, 8192 x 10240 x 512 140 and 82.
-// 8192^3 921 and 725 (its 256-column MMAs take 0.27 of a stage's 0.29 us).
+// 8192^3 921 and 712 (its 256-column MMAs take 0.27 of a stage's 0.29 us).
+// Narrow tiles with a long K are bound by the MMA issuer's chain per k-stage, measured alone with 64 columns:
+// four MMAs take 192 cycles, with their commit 218, a wait on a barrier that is ready +130, a commit of the
+// accumulator under a condition in the loop +50: 399 in all, as they were.  With the warp's index made uniform by
+// a shuffle (addresses and descriptors then stay in uniform registers) those are 192, 195, +80 and +57;
+// asking for the next slot while this one's MMAs go out and committing the accumulator after the loop takes the
+// last two off the chain.  Gradients of 256 x 512 from 10240 outputs 52 -> 40.5 us, of 1024 x 512 from
+// 18432 93 -> 79 (there a 128 x 64 tile's operands come at 54 bytes a cycle, what an SM gets from L2).
 // Every mbarrier wait is bounded (g_umma_wait_limit polls): on timeout the wait raises g_umma_err and
 // gives up (the outputs of that launch are then invalid, ewf_mlp_status reports it), and no later wait
 // of the launch waits at all.  Before the CTA frees its tensor memory and returns, the producer waits
@@ -84,6 +91,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *b, uint32_t parity)
 {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(smem_u32(b)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+// Whether the barrier's phase is over already, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t *b, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok)
                  : "r"(smem_u32(b)), "r"(parity)
                  : "memory");
@@ -159,8 +176,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
 }
 
 // tcgen05.fence::before pairs with the mbarrier arrive that releases an accumulator
-constexpr int GEMM_THREADS = ewf_umma::THREADS + ewf_umma::MORE_EPILOGUE;
-constexpr int EPI_WARPS = (GEMM_THREADS - 64) / 32;
+constexpr int GEMM_THREADS = ewf_umma::THREADS + ewf_umma::MORE_EPILOGUE + 32;
+constexpr int EPI_WARPS = (GEMM_THREADS - 96) / 32;
 constexpr int EPI_BOX = 32;                                    // rows and columns of an output box
 constexpr int EPI_BUF = EPI_BOX * EPI_BOX * 4;
 
@@ -230,12 +247,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], mma_drain;
     __shared__ uint32_t s_tmem;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform to the compiler too: the roles' loops run on uniform registers
     uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
 
     if (tid == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) {
-            mbar_init(&full[s], 1);
+            mbar_init(&full[s], 2);
             mbar_init(&empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -270,34 +288,35 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
     const int ns = min(MAX_STAGES, Shape<BN>::RING / stage);
     const bool ta = flags & TRANS_A, tb = flags & TRANS_B;
 
-    if (warp == 0) {  // TMA producer: every k-stage of every tile of this CTA, one ring
+    if (warp == 0 || warp == 10) {  // TMA producers of the one and the other operand: every k-stage of every tile of this CTA, one ring
+        const bool is_b = warp != 0;
+        const bool tr = is_b ? tb : ta;
+        const int ext = is_b ? bn : rows, boxes = tr ? (ext + U::MN_ATOM - 1) / U::MN_ATOM : 1;
+        const CUtensorMap *const map = is_b ? map_b : map_a;
+        const uint32_t bytes = (uint32_t)(ext * U::ROW_BYTES);
+        uint8_t *const base = smem + (is_b ? a_part : 0);
         int q = 0, s = 0;          // k-stages issued; slot of the next, and
         uint32_t free_parity = 1;  // the parity its "empty" wait passes with (1: a fresh barrier)
+        bool ready = true;         // that wait has passed already
         for (int t = t0; t < items && ok; t += ctas) {
-            const int m0 = (t / tiles_n) * rows, n0 = (t % tiles_n) * bn;
+            const int r0 = is_b ? (t % tiles_n) * bn : (t / tiles_n) * rows;
             for (int kt = 0; kt < nk; ++kt, ++q) {
-                if (!mbar_wait(&empty[s], free_parity, limit)) { ok = false; break; }
+                if (!ready && !mbar_wait(&empty[s], free_parity, limit)) { ok = false; break; }
+                const int s1 = s + 1 == ns ? 0 : s + 1;
+                const uint32_t p1 = s1 ? free_parity : free_parity ^ 1;
+                ready = mbar_test(&empty[s1], p1);
                 if (elect_one()) {
-                    uint8_t *As = smem + s * stage, *Bs = As + a_part;
-                    mbar_expect_tx(&full[s], (uint32_t)stage);
-                    if (ta) {
-                        for (int r = 0; r < rows; r += U::MN_ATOM)
-                            tma_load_2d(As + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, map_a, m0 + r, kt * U::BK, &full[s]);
+                    uint8_t *dst = base + s * stage;
+                    mbar_expect_tx(&full[s], bytes);
+                    if (tr) {
+                        for (int r = 0; r < boxes; ++r) tma_load_2d(dst + r * U::MN_BLOCK_BYTES, map, r0 + r * U::MN_ATOM, kt * U::BK, &full[s]);
                     } else {
-                        tma_load_2d(As, map_a, kt * U::BK, m0, &full[s]);
-                    }
-                    if (tb) {
-                        for (int r = 0; r < bn; r += U::MN_ATOM)
-                            tma_load_2d(Bs + (r / U::MN_ATOM) * U::MN_BLOCK_BYTES, map_b, n0 + r, kt * U::BK, &full[s]);
-                    } else {
-                        tma_load_2d(Bs, map_b, kt * U::BK, n0, &full[s]);
+                        tma_load_2d(dst, map, kt * U::BK, r0, &full[s]);
                     }
                 }
                 __syncwarp();
-                if (++s == ns) {
-                    s = 0;
-                    free_parity ^= 1;
-                }
+                s = s1;
+                free_parity = p1;
             }
         }
         // the loads issued last into each slot land before the CTA's shared memory goes
@@ -312,28 +331,31 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
         const int sa = (ta ? U::MN_K_STEP : 32) >> 4, sb = (tb ? U::MN_K_STEP : 32) >> 4;
         int s = 0, i = 0;
         uint32_t full_parity = 0;
+        bool ready = false;  // the wait for slot s has passed already
         for (int t = t0; t < items && ok; t += ctas, ++i) {
             const int b = U::acc_buf(i);
             if (U::acc_needs_free(i) && !mbar_wait(&acc_empty[b], U::acc_free_parity(i), limit)) { ok = false; break; }
             tc_fence_after();
             const uint32_t d = tmem + (uint32_t)(b * BN);  // accumulators BN columns apart
             for (int kt = 0; kt < nk; ++kt) {
-                if (!mbar_wait(&full[s], full_parity, limit)) { ok = false; break; }
+                if (!ready && !mbar_wait(&full[s], full_parity, limit)) { ok = false; break; }
                 tc_fence_after();
+                const int s1 = s + 1 == ns ? 0 : s + 1;
+                const uint32_t p1 = s1 ? full_parity : full_parity ^ 1;
+                ready = mbar_test(&full[s1], p1);
                 if (elect_one()) {
                     const uint32_t a0 = smem_u32(smem + s * stage) >> 4, b0 = a0 + (uint32_t)(a_part >> 4);
 #pragma unroll
                     for (int j = 0; j < U::BK / U::MMA_K; ++j)
                         umma_bf16(d, da0 + a0 + (uint32_t)(sa * j), db0 + b0 + (uint32_t)(sb * j), idesc, (kt > 0 || j > 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
-                    if (kt == nk - 1 && i != hold) umma_commit(&acc_full[b]);
                 }
                 __syncwarp();
-                if (++s == ns) {
-                    s = 0;
-                    full_parity ^= 1;
-                }
+                s = s1;
+                full_parity = p1;
             }
+            if (ok && i != hold && elect_one()) umma_commit(&acc_full[b]);
+            __syncwarp();
         }
         // every MMA issued completes before the tensor memory is freed
         if (elect_one()) umma_commit(&mma_drain);
@@ -608,11 +630,11 @@ int gemm_one(const Product &p, cudaStream_t stream)
 
 // The two products of a layer's backward pass in one launch: dH = dY . W (its K, the layer's outputs, may be
 // far larger than its tiles are many) and gW = dY^T . H.  dH gets a CTA per tile and gW the SMs that are
-// left, so the second hides behind the first.  A dH tile takes the operands of a 64-column tile from L2
-// and multiplies stage after stage, 0.23 us each whatever its size -- its K is not split, so that its sums
-// keep their order -- so small tiles cost nothing and spread the work: 32 or 64 of the accumulator's 128 lanes
-// while CTAs for them and as many again for gW are there.  256 x 512 from K = 10240: 110 us on 4 CTAs of 128 x
-// 256 at 0.7 us a stage, now 40 with the weight gradient behind it.
+// left, so the second hides behind the first.  A dH tile multiplies stage after stage, 0.16 us each up to 64 rows
+// and 0.24 with 128 -- its K is not split, so that its sums keep their order -- so small tiles spread the
+// work: 32 or 64 of the accumulator's 128 lanes while CTAs for them and as many again for gW are there.
+// 256 x 512 from K = 10240: 110 us on 4 CTAs of 128 x 256 at 0.7 us a stage, now 28 with the weight gradient
+// behind it.
 int gemm_pair(const Product &dh, const Product &gw, cudaStream_t stream)
 {
     Device dev;

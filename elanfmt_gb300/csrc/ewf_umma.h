@@ -35,7 +35,7 @@ constexpr int ROW_BYTES = BK * 2;
 constexpr int ATOM_BYTES = 8 * ROW_BYTES;  // 8 rows x 128 B: the swizzle atom, stride-dimension offset
 constexpr int MMA_K = 16;
 constexpr int THREADS = 192;     // warp 0: TMA producer (one lane); warp 1: MMA issuer (one lane); warps 2-5: epilogue
-constexpr int MORE_EPILOGUE = 128;  // warps 6-9: a second epilogue warp per TMEM lane quarter
+constexpr int MORE_EPILOGUE = 128;  // warps 6-9: a second epilogue warp per TMEM lane quarter (warp 10: the producer of B)
 constexpr int LAYOUT_SW128 = 2;
 
 // Per tile width BN (128 or 256): bytes of a stage and of the whole pipeline; TMEM columns = 2 BN
