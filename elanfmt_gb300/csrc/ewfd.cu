@@ -230,7 +230,7 @@ struct ewf_handle {
     int it = 0;
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
-    cudaGraphExec_t gexec = nullptr;
+    cudaGraphExec_t gexec = nullptr, gexec_short = nullptr;  // of gsteps and of SHORT_GRAPH steps
     int gsteps = 0;
     bool graph_dirty = true;
     float last_ms = 0.f;
@@ -473,6 +473,7 @@ extern "C" void ewf_destroy(ewf_handle *h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     snapshots_close(h);  // finishes the queued snapshot files first
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
+    if (h->gexec_short) cudaGraphExecDestroy(h->gexec_short);
     for (auto &x : h->f_alloc) cudaFree(x);
     for (auto &x : h->g_alloc) cudaFree(x);
     for (auto &x : h->comp_alloc) cudaFree(x);
@@ -1471,29 +1472,48 @@ static int inputs_ready(const ewf_handle *h)
 // The two-kernel step keeps its step counter in two alternating device locations (d_it[it & 1]).
 static bool split_form(const ewf_handle *h) { return !h->fused && !h->wave; }
 
-static int build_graph(ewf_handle *h, step_fn fn)
+// What a long graph leaves of a run, and runs shorter than one: in graphs of SHORT_GRAPH steps where the
+// host would not keep up with launches one by one (the rest is fewer than SHORT_GRAPH).  us per step of a 60-step
+// run of ortho 40 x 40 x 32: 6.8 launched one by one, 6.2 in graphs of 4, 5.9 of 8 and of 16 steps, 5.7 of 60; its first
+// run, the graph's making included, 542, 473, 467, 512 and 702 us in all.  A grid of SHORT_CELLS cells takes
+// 8 us a step, more than its two launches.
+static int short_graph(const ewf_handle *h)
 {
-    if (h->gexec) {
-        cudaGraphExecDestroy(h->gexec);
-        h->gexec = nullptr;
-    }
+    const bool small = (double)h->p.nx * h->p.ny * h->p.nz < SHORT_CELLS;
+    return small && split_form(h) && h->p.graph_steps == 0 ? SHORT_GRAPH : 0;
+}
+
+static int build_graph(ewf_handle *h, step_fn fn, int steps, cudaGraphExec_t *exec)
+{
+    if (*exec) cudaGraphExecDestroy(*exec);
+    *exec = nullptr;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < h->gsteps; ++s) fn(h, nullptr, (h->dbuf || split_form(h)) ? (s & 1) : 0);
+    for (int s = 0; s < steps; ++s) fn(h, nullptr, (h->dbuf || split_form(h)) ? (s & 1) : 0);
     const cudaError_t le = cudaGetLastError();
     const cudaError_t ce = cudaStreamEndCapture(h->stream, &g);
     if (le != cudaSuccess || ce != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return ewf_fail(EWF_ERR_CUDA, "graph capture: %s", cudaGetErrorString(le != cudaSuccess ? le : ce));
     }
-    const cudaError_t ie = cudaGraphInstantiate(&h->gexec, g, 0);
+    const cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) {
-        h->gexec = nullptr;
+        *exec = nullptr;
         return ewf_fail(EWF_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ie));
     }
-    h->graph_dirty = false;
     return EWF_OK;
+}
+static int ready_graph(ewf_handle *h, step_fn fn, int steps, cudaGraphExec_t *exec)
+{
+    if (*exec) return EWF_OK;
+    int st = build_graph(h, fn, steps, exec);
+    if (st && h->pdl) {  // a driver that cannot capture dependent launches: plain ones
+        cudaGetLastError();
+        h->pdl = false;
+        st = build_graph(h, fn, steps, exec);
+    }
+    return st;
 }
 
 extern "C" int ewf_run(ewf_handle *h, int32_t nsteps)
@@ -1512,33 +1532,33 @@ extern "C" int ewf_run(ewf_handle *h, int32_t nsteps)
     // graph starts at parity 0
     const bool alt = h->dbuf || split_form(h);
     int parity = h->dbuf ? h->flip : (split_form(h) ? (h->it & 1) : 0);
-    const bool use_graph = h->gsteps > 0 && nsteps >= h->gsteps + parity;
-    bool graph = use_graph;
-    if (graph && (h->graph_dirty || !h->gexec)) {
-        st = build_graph(h, fn);
-        if (st && h->pdl) {  // a driver that cannot capture dependent launches: plain ones
-            cudaGetLastError();
-            h->pdl = false;
-            st = build_graph(h, fn);
+    // graphs start from parity 0: a direct step first if there is need
+    const int rest = nsteps - parity, brief = short_graph(h);
+    const int nlong = h->gsteps > 0 ? std::max(0, rest) / h->gsteps : 0, nshort = brief > 0 ? std::max(0, rest - nlong * h->gsteps) / brief : 0;
+    if (h->graph_dirty) {
+        for (cudaGraphExec_t *x : {&h->gexec, &h->gexec_short}) {
+            if (*x) cudaGraphExecDestroy(*x);
+            *x = nullptr;
         }
-        if (st) return st;
+        h->graph_dirty = false;
     }
+    if (nlong && (st = ready_graph(h, fn, h->gsteps, &h->gexec))) return st;
+    if (nshort && (st = ready_graph(h, fn, brief, &h->gexec_short))) return st;
     CK(cudaEventRecord(h->ev0, h->stream));
     int done = 0;
-    if (graph && parity) {  // the graph starts from parity 0: one direct step first
+    if ((nlong || nshort) && parity) {
         fn(h, nullptr, parity);
         parity = 0;
         ++done;
     }
-    if (graph) {
-        for (; done + h->gsteps <= nsteps; done += h->gsteps) {
-            CK(cudaGraphLaunch(h->gexec, h->stream));
-            if (h->p.nout > 0 && ((h->it + done) / h->p.nout) != ((h->it + done + h->gsteps) / h->p.nout)) {
-                printf("it=%05d > ", h->it + done + h->gsteps);
-                fflush(stdout);
-            }
+    for (int q = 0; q < nlong; ++q, done += h->gsteps) {
+        CK(cudaGraphLaunch(h->gexec, h->stream));
+        if (h->p.nout > 0 && ((h->it + done) / h->p.nout) != ((h->it + done + h->gsteps) / h->p.nout)) {
+            printf("it=%05d > ", h->it + done + h->gsteps);
+            fflush(stdout);
         }
     }
+    for (int q = 0; q < nshort; ++q, done += brief) CK(cudaGraphLaunch(h->gexec_short, h->stream));
     for (; done < nsteps; ++done) {
         fn(h, nullptr, parity);
         if (alt) parity ^= 1;

@@ -103,7 +103,7 @@ struct ewf_batch {
     cudaStream_t branch[BRANCHES] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[BRANCHES] = {};
     std::vector<int> branch_of;  // per problem: its branch (balanced by cell-updates), -1: the batch's stream
-    cudaGraphExec_t gexec = nullptr;
+    cudaGraphExec_t gexec = nullptr, gexec_short = nullptr;  // of gsteps and of SHORT_GRAPH steps
     int gsteps = 64;     // steps per graph (even: the step counters alternate between two locations)
     float last_ms = 0.f;
 };
@@ -126,7 +126,10 @@ static void free_tables(ewf_batch *b)
     cudaFree(b->d_order); b->d_order = nullptr;
     cudaFree(b->d_rec_off); b->d_rec_off = nullptr;
     cudaFree(b->d_rec_comp); b->d_rec_comp = nullptr;
-    if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
+    for (cudaGraphExec_t *x : {&b->gexec, &b->gexec_short}) {
+        if (*x) cudaGraphExecDestroy(*x);
+        *x = nullptr;
+    }
 }
 
 extern "C" void ewf_batch_destroy(ewf_batch *b)
@@ -627,24 +630,45 @@ static void batch_steps(ewf_batch *b, int steps, int parity)
         if (b->branch_of[i] < 0) chain(i, b->stream);
 }
 
-static int batch_graph(ewf_batch *b)
+static int batch_graph(ewf_batch *b, int steps, cudaGraphExec_t *exec)
 {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    batch_steps(b, b->gsteps, 0);
+    batch_steps(b, steps, 0);
     const cudaError_t le = cudaGetLastError();
     const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
     if (le != cudaSuccess || ce != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return ewf_fail(EWF_ERR_CUDA, "batch graph capture: %s", cudaGetErrorString(le != cudaSuccess ? le : ce));
     }
-    const cudaError_t ie = cudaGraphInstantiate(&b->gexec, g, 0);
+    const cudaError_t ie = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) {
-        b->gexec = nullptr;
+        *exec = nullptr;
         return ewf_fail(EWF_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(ie));
     }
     return EWF_OK;
+}
+
+static int ready_graph(ewf_batch *b, int steps, cudaGraphExec_t *exec)
+{
+    if (*exec) return EWF_OK;
+    int st = batch_graph(b, steps, exec);
+    if (st && b->pdl) {  // a driver that cannot capture dependent launches: plain ones
+        cudaGetLastError();
+        b->pdl = false;
+        st = batch_graph(b, steps, exec);
+    }
+    return st;
+}
+
+// The steps a long graph leaves over go in graphs of SHORT_GRAPH steps where the problems are small on average
+// (SHORT_CELLS): launched one by one, a step of n problems takes the host some 5 n us.
+static int short_graph(const ewf_batch *b)
+{
+    double cells = 0;
+    for (auto &q : b->probs) cells += (double)q.p.nx * q.p.ny * q.p.nz * q.R;
+    return cells < SHORT_CELLS * b->probs.size() && SHORT_GRAPH < b->gsteps ? SHORT_GRAPH : 0;
 }
 
 static int batch_ready(ewf_batch *b)
@@ -679,27 +703,19 @@ extern "C" int ewf_batch_run(ewf_batch *b, int32_t nsteps)
     int st = batch_ready(b);
     if (st) return st;
     if (b->it + nsteps > b->nt) return ewf_fail(EWF_ERR_ARG, "step %d + %d exceeds nt = %d", b->it, nsteps, b->nt);
-    // the graph starts from an even step
-    const int odd = b->it & 1;
-    const bool use_graph = nsteps >= b->gsteps + odd;
-    if (use_graph && !b->gexec) {
-        st = batch_graph(b);
-        if (st && b->pdl) {  // a driver that cannot capture dependent launches: plain ones
-            cudaGetLastError();
-            b->pdl = false;
-            st = batch_graph(b);
-        }
-        if (st) return st;
-    }
+    // graphs start from an even step
+    const int odd = b->it & 1, rest = std::max(0, nsteps - odd), brief = short_graph(b);
+    const int nlong = rest / b->gsteps, nshort = brief > 0 ? (rest - nlong * b->gsteps) / brief : 0;
+    if (nlong && (st = ready_graph(b, b->gsteps, &b->gexec))) return st;
+    if (nshort && (st = ready_graph(b, brief, &b->gexec_short))) return st;
     CK(cudaEventRecord(b->ev0, b->stream));
     int done = 0;
-    if (use_graph) {
-        if (odd) {
-            batch_steps(b, 1, 1);
-            done = 1;
-        }
-        for (; done + b->gsteps <= nsteps; done += b->gsteps) CK(cudaGraphLaunch(b->gexec, b->stream));
+    if ((nlong || nshort) && odd) {
+        batch_steps(b, 1, 1);
+        done = 1;
     }
+    for (int q = 0; q < nlong; ++q, done += b->gsteps) CK(cudaGraphLaunch(b->gexec, b->stream));
+    for (int q = 0; q < nshort; ++q, done += brief) CK(cudaGraphLaunch(b->gexec_short, b->stream));
     if (done < nsteps) batch_steps(b, nsteps - done, (b->it + done) & 1);
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev1, b->stream));

@@ -21,6 +21,11 @@ struct RecTables {
 };
 RecTables make_rec_tables(int n, const int32_t *ijkc, int nx, int ny, int nz);
 
+// Graphs of a few steps for small grids: the steps a long graph leaves over (even), and up to how many
+// cells (on average, in a batch) the host's launches are what a step takes
+constexpr int SHORT_GRAPH = 8;
+constexpr double SHORT_CELLS = 4e5;
+
 // Launch shape by the cells a launch updates (R right-hand sides)
 struct SplitShape {
     int kchunk, ty, l2pf;

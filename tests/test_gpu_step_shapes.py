@@ -72,3 +72,16 @@ def test_fp64_division(cuda_device, spacing):
     m.dx, m.dy, m.dz = spacing
     m.dt = m.dt * min(spacing) / 12.0
     _check(m, 24, precision=F.PREC_F64)
+
+
+@pytest.mark.parametrize("splits", [(7, 1, 8, 9, 25), (64 + 8 + 3, 16, 9), (1, 8, 64 + 16)])  # odd and even starts, graphs of 64 and of 8
+@pytest.mark.parametrize("precision", [F.PREC_F32, F.PREC_F64])
+def test_runs_in_graphs_and_single_steps(cuda_device, splits, precision):
+    m = I.random_small(F.MODEL_ORTHO, 26, 19, 12, nt=sum(splits), seed=9, damping=F.DAMP_SEPARABLE)
+    ref = O.run(m, m.nt, precision=precision)
+    with Solver.from_model(m, precision=precision) as s:
+        for n in splits:
+            s.run(n)
+        np.testing.assert_array_equal(s.seismograms(), ref.traces)
+        for q in F.STATE:
+            np.testing.assert_array_equal(s.field(q, ref.f[q].dtype), ref.f[q], err_msg=F.STATE_NAMES[q])
