@@ -389,7 +389,7 @@ static int upload(T **dst, const std::vector<T> &v)
 //   iso    32^3 30 10   64^3 40 22   80^3 62 50   96^3 76 88     128^3 198 222   160^3 432 441
 //   ortho  32^3 30 11   64^3 50 30   80^3 75 76   96^3 104 122   128^3 296 287   160^3 571 565
 // As many branches as hold BRANCH_SHARE cells between them, which L2 still keeps.  us per step on 2, 4 and
-// 8 branches:
+// 8 branches (these and the above with chunks by each problem's own size):
 //   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
 //   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
 constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
@@ -400,6 +400,27 @@ static int build_tables(ewf_batch *b)
     CK(cudaStreamSynchronize(b->stream));
     free_tables(b);
     const int n = (int)b->probs.size();
+    // branches: largest problems first, each to the least loaded branch
+    b->branch_of.assign(n, -1);
+    int share = 1;  // problems that run at the same time
+    if (b->own != 0 && n > 1) {
+        std::vector<int> idx(n);
+        for (int i = 0; i < n; ++i) idx[i] = i;
+        auto work = [&](int i) {
+            const Prob &q = b->probs[i];
+            return (double)q.p.nx * q.p.ny * q.p.nz * q.R;
+        };
+        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return work(x) > work(y); });
+        idx.erase(std::remove_if(idx.begin(), idx.end(), [&](int i) { return b->own < 0 && work(i) >= BRANCH_CELLS; }), idx.end());
+        const int branches = idx.empty() ? 1 : (int)std::max(2.0, std::min((double)ewf_batch::BRANCHES, BRANCH_SHARE / work(idx[0])));
+        share = std::min(branches, std::max(1, (int)idx.size()));
+        double load[ewf_batch::BRANCHES] = {};
+        for (int i : idx) {
+            const int k = (int)(std::min_element(load, load + branches) - load);
+            b->branch_of[i] = k;
+            load[k] += work(i);
+        }
+    }
     std::vector<BatchProb<float>> all(n);
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
@@ -419,7 +440,10 @@ static int build_tables(ewf_batch *b)
         const SplitShape shape = split_shape(p.nx, p.ny, p.nz, q.R);
         q.ty = std::max(b->ty, shape.ty);
         q.pair = shape.pair || q.R > 1;
-        d.kchunk = q.kchunk > 0 ? q.kchunk : shape.kchunk;
+        // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
+        // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
+        // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
+        d.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, q.R * (b->branch_of[i] >= 0 ? share : 1)).kchunk;
         d.dt = (float)p.dt;
         d.rdt = 1.0f / d.dt;
         d.dx = (float)p.dx; d.dy = (float)p.dy; d.dz = (float)p.dz;
@@ -433,25 +457,6 @@ static int build_tables(ewf_batch *b)
         d.smu_on = p.surface_mu > 0.0 ? 1 : 0;
         d.smu = (float)p.surface_mu;
         d.l2pf = b->l2pf >= 0 ? b->l2pf : shape.l2pf;
-    }
-    // branches: largest problems first, each to the least loaded branch
-    b->branch_of.assign(n, -1);
-    if (b->own != 0 && n > 1) {
-        std::vector<int> idx(n);
-        for (int i = 0; i < n; ++i) idx[i] = i;
-        auto work = [&](int i) {
-            const Prob &q = b->probs[i];
-            return (double)q.p.nx * q.p.ny * q.p.nz * q.R;
-        };
-        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return work(x) > work(y); });
-        idx.erase(std::remove_if(idx.begin(), idx.end(), [&](int i) { return b->own < 0 && work(i) >= BRANCH_CELLS; }), idx.end());
-        const int branches = idx.empty() ? 1 : (int)std::max(2.0, std::min((double)ewf_batch::BRANCHES, BRANCH_SHARE / work(idx[0])));
-        double load[ewf_batch::BRANCHES] = {};
-        for (int i : idx) {
-            const int k = (int)(std::min_element(load, load + branches) - load);
-            b->branch_of[i] = k;
-            load[k] += work(i);
-        }
     }
     CK(cudaMalloc(&b->d_all, n * sizeof(BatchProb<float>)));
     // sources grouped by (problem, rhs)
