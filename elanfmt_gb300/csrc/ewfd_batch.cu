@@ -693,10 +693,12 @@ static int batch_ready(ewf_batch *b)
 extern "C" int ewf_batch_reset(ewf_batch *b)
 {
     if (!b) return ewf_fail(EWF_ERR_ARG, "NULL batch");
+    std::vector<ZeroBuf> z;
     for (auto &q : b->probs)
-        for (auto &x : q.state) CK(cudaMemsetAsync(x, 0, q.sbox * 4, b->stream));
-    if (b->d_traces) CK(cudaMemsetAsync(b->d_traces, 0, (size_t)b->nrec_total * b->nt * sizeof(double), b->stream));
-    CK(cudaMemsetAsync(b->d_it, 0, 2 * b->probs.size() * sizeof(int), b->stream));
+        for (auto &x : q.state) z.push_back({x, q.sbox * 4});
+    if (b->d_traces) z.push_back({b->d_traces, (size_t)b->nrec_total * b->nt * sizeof(double)});
+    z.push_back({b->d_it, 2 * b->probs.size() * sizeof(int)});
+    if (int st = zero_buffers(z, b->stream)) return st;
     CK(cudaStreamSynchronize(b->stream));
     b->it = 0;
     return EWF_OK;

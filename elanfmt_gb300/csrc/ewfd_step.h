@@ -33,6 +33,13 @@ struct SplitShape {
 };
 SplitShape split_shape(int nx, int ny, int nz, int R = 1);
 
+// Buffers (16-byte aligned) set to zero in stream order, ZERO_GROUP of them per launch
+struct ZeroBuf {
+    void *p;
+    size_t bytes;
+};
+int zero_buffers(const std::vector<ZeroBuf> &v, cudaStream_t stream);
+
 // A launch on a stream; `pdl`: as a programmatic dependent of the stream's previous
 // kernel (the kernel waits for it with griddepcontrol.wait before touching any state).
 template <typename... P, typename... A>
