@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
                 if (n >= N) continue;                // columns past the last (N not a multiple of bn)
                 if (J.bias) {
 #pragma unroll
-                    for (int e = 0; e < EPI_BOX; ++e) x[e] += __ldg(J.bias + n + e);
+                    for (int e = 0; e < EPI_BOX; ++e) x[e] += J.bias[n + e];
                 }
                 // staged rows: 16-byte chunk q of row r at chunk q ^ (r % 8) (fp32) or q ^ (r / 2 % 4) (bf16)
                 if ((flags & OUT_PRE)) {
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(1024) k_bias_grads(const BiasJobs J)
 
 // k_mse_grad four values at a time (n % 4 == 0, aligned), with the loss from the partial sums by the last
 // CTA to finish: done counts the CTAs and is left at zero.
-__global__ void __launch_bounds__(256) k_mse_loss(const float4 *__restrict__ y, const float4 *__restrict__ t, uint2 *__restrict__ dy,
+__global__ void __launch_bounds__(256) k_mse_loss(const float4 *y, const float4 *t, uint2 *dy,
                                                   size_t n4, float scale, float *__restrict__ part, unsigned *__restrict__ done,
                                                   float *__restrict__ loss)
 {

@@ -130,16 +130,15 @@ __device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// State loads.  COH = 0: the read-only path (the field is not written during the launch).
-// COH = 1: a plain coherent load, for the wavefront step, where other CTAs of the same launch
-// write the fields (ordered by its release/acquire flags).  COH = 2: a load cached in L2 only
-// (ld.global.cg), for the sweep step's reads of values other CTAs wrote: no L1 line can hold
-// an older copy.
+// State loads.  COH = 0: the read-only path, in launches that start when the one before has ended and do not
+// write the field.  COH = 1: a plain load, where other CTAs of the same launch write the fields (the
+// wavefront step, ordered by its release/acquire flags) and after pdl_wait: the compiler may move a read-only
+// load across it, and the read-only path need not see what the previous launch wrote while this one
+// was already there.
 template <int COH, typename T>
 __device__ __forceinline__ T lds(const T *p)
 {
-    if constexpr (COH == 2) return __ldcg(p);
-    else if constexpr (COH == 1) return *p;
+    if constexpr (COH == 1) return *p;
     else return __ldg(p);
 }
 
@@ -520,7 +519,7 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
 {
     pdl_trigger();
     const int k0 = blockIdx.z * a.kchunk;
-    stress_column<T, MODEL, DAMP, 0, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz), ss);
+    stress_column<T, MODEL, DAMP, 1, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz), ss);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -807,7 +806,7 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
         *rf.it_wr = *rf.it_rd + 1;  // the next step's counter; this launch reads only it_rd
     }
     const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
-    velocity_column<T, MODEL, DAMP, KAHAN, 0, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
+    velocity_column<T, MODEL, DAMP, KAHAN, 1, true>(a, blockIdx.x * TX + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
                                                     min(k0 + a.kchunk, a.nz), rf);
 }
 

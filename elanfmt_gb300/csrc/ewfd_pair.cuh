@@ -46,6 +46,7 @@ struct PairOps {
 };
 __device__ __forceinline__ f2 neg2(f2 a) { return a ^ 0x8000000080000000ull; }
 
+// NC: the read-only path, for what no launch writes; the state is read plainly (lds)
 template <bool NC = true>
 __device__ __forceinline__ f2 ld2(const float *p)
 {
@@ -125,15 +126,15 @@ __device__ __forceinline__ void stress_mat2(const StepArgs<float> &a, long long 
 template <int MODEL, int DAMP>
 __device__ __forceinline__ void stress_state2(const StepArgs<float> &a, long long c, StressIn2<MODEL, DAMP> &q)
 {
-    q.vx = ld2(a.f[0] + c);
-    q.vx_i2 = ld(a.f[0] + c + 2);
-    q.vx_jm = ld2(a.f[0] + c - a.sx);
-    q.vy = ld2(a.f[1] + c);
-    q.vy_jp = ld2(a.f[1] + c + a.sx);
-    q.vy_im = ld(a.f[1] + c - 1);
-    q.vz_p = ld2(a.f[2] + c + a.sy);
-    q.vz_im = ld(a.f[2] + c - 1);
-    q.vz_jm = ld2(a.f[2] + c - a.sx);
+    q.vx = ld2<false>(a.f[0] + c);
+    q.vx_i2 = a.f[0][c + 2];
+    q.vx_jm = ld2<false>(a.f[0] + c - a.sx);
+    q.vy = ld2<false>(a.f[1] + c);
+    q.vy_jp = ld2<false>(a.f[1] + c + a.sx);
+    q.vy_im = a.f[1][c - 1];
+    q.vz_p = ld2<false>(a.f[2] + c + a.sy);
+    q.vz_im = a.f[2][c - 1];
+    q.vz_jm = ld2<false>(a.f[2] + c - a.sx);
 #pragma unroll
     for (int f = 0; f < 6; ++f) q.s[f] = ld2<false>(a.f[3 + f] + c);
 }
@@ -172,7 +173,7 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
     StressIn2<MODEL, DAMP> nxt;
     stress_mat2<MODEL, DAMP>(a, cm, k0, nxt);
     pdl_wait();  // nothing above depends on an earlier launch
-    f2 vx_m = ld2(a.f[0] + c - a.sy), vy_m = ld2(a.f[1] + c - a.sy), vz_k = ld2(a.f[2] + c);
+    f2 vx_m = ld2<false>(a.f[0] + c - a.sy), vy_m = ld2<false>(a.f[1] + c - a.sy), vz_k = ld2<false>(a.f[2] + c);
     stress_state2<MODEL, DAMP>(a, c, nxt);
     bool src_col = false;
     float s_src = 0.f;
@@ -291,18 +292,18 @@ __device__ __forceinline__ void vel_mat2(const StepArgs<float> &a, long long cm,
 template <int MODEL, int DAMP, bool KAHAN>
 __device__ __forceinline__ void vel_state2(const StepArgs<float> &a, long long c, VelIn2<MODEL, DAMP, KAHAN> &q)
 {
-    q.sxx = ld2(a.f[3] + c);
-    q.sxx_im = ld(a.f[3] + c - 1);
-    q.syy = ld2(a.f[4] + c);
-    q.syy_jm = ld2(a.f[4] + c - a.sx);
-    q.szz = ld2(a.f[5] + c);
-    q.sxy = ld2(a.f[6] + c);
-    q.sxy_jp = ld2(a.f[6] + c + a.sx);
-    q.sxy_i2 = ld(a.f[6] + c + 2);
-    q.sxz_p = ld2(a.f[7] + c + a.sy);
-    q.sxz_i2 = ld(a.f[7] + c + 2);
-    q.syz_p = ld2(a.f[8] + c + a.sy);
-    q.syz_jp = ld2(a.f[8] + c + a.sx);
+    q.sxx = ld2<false>(a.f[3] + c);
+    q.sxx_im = a.f[3][c - 1];
+    q.syy = ld2<false>(a.f[4] + c);
+    q.syy_jm = ld2<false>(a.f[4] + c - a.sx);
+    q.szz = ld2<false>(a.f[5] + c);
+    q.sxy = ld2<false>(a.f[6] + c);
+    q.sxy_jp = ld2<false>(a.f[6] + c + a.sx);
+    q.sxy_i2 = a.f[6][c + 2];
+    q.sxz_p = ld2<false>(a.f[7] + c + a.sy);
+    q.sxz_i2 = a.f[7][c + 2];
+    q.syz_p = ld2<false>(a.f[8] + c + a.sy);
+    q.syz_jp = ld2<false>(a.f[8] + c + a.sx);
 #pragma unroll
     for (int f = 0; f < 3; ++f) q.v[f] = ld2<false>(a.f[f] + c);
     if (KAHAN) {
@@ -350,7 +351,7 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
     VelIn2<MODEL, DAMP, KAHAN> nxt;
     vel_mat2<MODEL, DAMP, KAHAN>(a, cm, k0, nxt);
     pdl_wait();  // nothing above depends on an earlier launch
-    f2 szz_m = ld2(a.f[5] + c - a.sy), sxz_k = ld2(a.f[7] + c), syz_k = ld2(a.f[8] + c);
+    f2 szz_m = ld2<false>(a.f[5] + c - a.sy), sxz_k = ld2<false>(a.f[7] + c), syz_k = ld2<false>(a.f[8] + c);
     vel_state2<MODEL, DAMP, KAHAN>(a, c, nxt);
     // L2 prefetch: lane l of a row's 16 asks for the row's line of input field l
     const float *pf_row = nullptr;
