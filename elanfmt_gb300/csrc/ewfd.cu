@@ -240,6 +240,7 @@ struct ewf_handle {
     int l2pf = 0;       // two-kernel step: L2 prefetch distance of the velocity kernel in planes (autotuned)
     int fdiv = 0;       // StepArgs::fdiv of this handle's spacings
     bool pair = false;       // two-kernel step, FP32: two cells per thread (ewfd_pair.cuh)
+    bool stream_l2 = false;  // those kernels: materials and new velocities first to leave L2
     bool src_plane1 = false;  // a fused source entry that plane 2's thread applies on plane 1
     struct Snapshots *snap = nullptr;  // queued snapshot writer (created on first use)
 };
@@ -595,10 +596,17 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 //   ortho 256^3   405.9 (4) 401.6 (6)     380.2 (6)
 // The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
 // 320x320x256 641 -> 631 with one cell per thread) and not below (128^3: 55.8 and 56.1).
+// stream: the state's nine fields (36 bytes a cell) are read and written by both kernels, the moduli and
+// buoyancies (up to 48 bytes) once a step.  Where the fields by themselves about fit the 129 MB L2, what
+// is read once, and the new velocities, are marked to leave it first.  us per step without and with:
+//   ortho 80^3 12.9 13.3   96^3 17.9 18.0   112^3 36.8 30.6   128^3 49.7 42.3   144^3 75.3 71.3   192^3 162.3 160.7
+//   iso 128^3 33.1 30.2    144^3 55.1 53.5  176^3 99.9 99.4   192^3 123.0 122.9  iso-het 203x151x97 66.6 63.0
+//   ortho 256^3 380.5 384.1   320x320x256 590 597   Kahan 192^3 186.7 187.3
+// (Marking the old velocities or the stresses as well gains nothing more.)
 SplitShape split_shape(int nx, int ny, int nz, int R)
 {
     const double cells = (double)nx * ny * nz * R;
-    SplitShape d = {cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6, 4, cells >= 1.2e7 ? 3 : 0, cells >= 4e5};
+    SplitShape d = {cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6, 4, cells >= 1.2e7 ? 3 : 0, cells >= 4e5, cells >= 1e6 && cells < 6e6};
     // a grid has at most 65535 CTAs along y and z
     d.kchunk = std::max(d.kchunk, (nz + 65534) / 65535);
     while (d.ty < 16 && ny > 65535 * d.ty) d.ty *= 2;
@@ -611,6 +619,7 @@ static void split_default_shape(ewf_handle *h)
     h->ty = d.ty;
     h->l2pf = d.l2pf;
     h->pair = d.pair;
+    h->stream_l2 = d.stream;
 }
 
 extern "C" int ewf_create(const ewf_params *p, ewf_handle **out)
@@ -1190,7 +1199,7 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
     const dim3 pblk(PAIR_TX, pair_rows(h->ty)), pgrd(grd.x, (h->p.ny + pblk.y - 1) / pblk.y, grd.z);
     if (ev) cudaEventRecord(ev[0], h->stream);
     if constexpr (PAIRS) {
-        if (pair) launch_on(k_stress_pair<MODEL, DAMP>, pgrd, pblk, h->stream, pdl, a, ss);
+        if (pair) launch_on(h->stream_l2 ? k_stress_pair<MODEL, DAMP, true> : k_stress_pair<MODEL, DAMP, false>, pgrd, pblk, h->stream, pdl, a, ss);
     }
     if (!pair) launch_on(k_stress<T, MODEL, DAMP>, grd, blk, h->stream, pdl, a, ss);
     if (ev) cudaEventRecord(ev[1], h->stream);
@@ -1199,7 +1208,7 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
                   (const double *)h->d_stf, (int)h->nstf, (const int *)it_rd, h->p.src_order);
     if (ev) cudaEventRecord(ev[2], h->stream);
     if constexpr (PAIRS) {
-        if (pair) launch_on(k_velocity_pair<MODEL, DAMP, KAHAN>, pgrd, pblk, h->stream, pdl, a, rf);
+        if (pair) launch_on(h->stream_l2 ? k_velocity_pair<MODEL, DAMP, KAHAN, true> : k_velocity_pair<MODEL, DAMP, KAHAN, false>, pgrd, pblk, h->stream, pdl, a, rf);
     }
     if (!pair) launch_on(k_velocity<T, MODEL, DAMP, KAHAN>, grd, blk, h->stream, pdl, a, rf);
     if (ev) cudaEventRecord(ev[3], h->stream);

@@ -48,6 +48,7 @@ struct Prob {
     int kchunk = 0;                         // planes per CTA (0: by size, split_shape)
     int ty = 4;                             // CTA tile height
     bool pair = false;                      // two cells per thread
+    bool stream_l2 = false;                 // its kernels: materials and new velocities first to leave L2
     StressSrc ss{};                         // sources in the stress kernel (nsrc 0: k_binject)
     SrcEntry *d_sent = nullptr;             // its entries, right-hand side by right-hand side
     int *d_sstart = nullptr;                // first entry of each right-hand side, R + 1
@@ -440,6 +441,7 @@ static int build_tables(ewf_batch *b)
         const SplitShape shape = split_shape(p.nx, p.ny, p.nz, q.R);
         q.ty = std::max(b->ty, shape.ty);
         q.pair = shape.pair || q.R > 1;
+        q.stream_l2 = shape.stream;
         // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
         // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
         // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
@@ -569,7 +571,7 @@ static int build_tables(ewf_batch *b)
 
 // One step of problem i on a stream; `parity` = the step number's: its counter is at d_it[2 i + parity], the
 // next step's at d_it[2 i + 1 - parity].
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 static void problem_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
 {
     const Prob &q = b->probs[i];
@@ -583,14 +585,14 @@ static void problem_step_t(ewf_batch *b, int i, int parity, bool first, cudaStre
     const int rows = q.pair ? pair_rows(q.ty) : q.ty, tiles_x = (q.p.nx + TX - 1) / TX;
     const dim3 blk(q.pair ? PAIR_TX : TX, rows), grd(tiles_x * q.R, (q.p.ny + rows - 1) / rows, (q.p.nz + a.kchunk - 1) / a.kchunk);
     const long long stride = b->h_all[i].rhs_stride, nr = (long long)q.rec.size() / 4;
-    if (q.R > 1) launch_on(k_stress_pair_mr<MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, q.R, stride, ss, (const int *)q.d_sstart);
-    else if (q.pair) launch_on(k_stress_pair<MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
+    if (q.R > 1) launch_on(k_stress_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, q.R, stride, ss, (const int *)q.d_sstart);
+    else if (q.pair) launch_on(k_stress_pair<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, ss);
     else launch_on(k_stress<float, MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
     if (q.nsrc > 0 && ss.nsrc == 0)
         k_binject<float><<<(q.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, q.group0, q.R, b->d_stf, b->d_stf_off, b->d_order,
                                                         b->nt, it_rd);
-    if (q.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP>, grd, blk, s, b->pdl, a, q.R, stride, rf, nr * b->nt);
-    else if (q.pair) launch_on(k_velocity_pair<MODEL, DAMP, false>, grd, blk, s, b->pdl, a, rf);
+    if (q.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl, a, q.R, stride, rf, nr * b->nt);
+    else if (q.pair) launch_on(k_velocity_pair<MODEL, DAMP, false, ST>, grd, blk, s, b->pdl, a, rf);
     else launch_on(k_velocity<float, MODEL, DAMP, false>, grd, blk, s, b->pdl, a, rf);
     if (!q.rec_fuse) {
         const int rows_ = (int)nr * q.R;
@@ -598,6 +600,13 @@ static void problem_step_t(ewf_batch *b, int i, int parity, bool first, cudaStre
                                                                             b->nt, it_rd);
         k_advance<<<1, 1, 0, s>>>(it_rd, it_wr);
     }
+}
+
+template <int MODEL, int DAMP>
+static void problem_step(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
+{
+    if (b->probs[i].stream_l2) problem_step_t<MODEL, DAMP, true>(b, i, parity, first, s);
+    else problem_step_t<MODEL, DAMP, false>(b, i, parity, first, s);
 }
 
 // `steps` steps of every problem from step parity `parity` on, chain by chain: the branches' problems on
@@ -609,9 +618,9 @@ static void batch_steps(ewf_batch *b, int steps, int parity)
         for (int k = 0; k < steps; ++k) {
             const int par = (parity + k) & 1;
             // nothing of another problem's to overlap with: a chain's first launch is a plain one
-            if (p.model == EWF_MODEL_ISO) problem_step_t<MODEL_ISO, DAMP_PML1D>(b, (int)i, par, k == 0, s);
-            else if (p.damping == EWF_DAMP_W3D) problem_step_t<MODEL_ORTHO, DAMP_W3D>(b, (int)i, par, k == 0, s);
-            else problem_step_t<MODEL_ORTHO, DAMP_SEP>(b, (int)i, par, k == 0, s);
+            if (p.model == EWF_MODEL_ISO) problem_step<MODEL_ISO, DAMP_PML1D>(b, (int)i, par, k == 0, s);
+            else if (p.damping == EWF_DAMP_W3D) problem_step<MODEL_ORTHO, DAMP_W3D>(b, (int)i, par, k == 0, s);
+            else problem_step<MODEL_ORTHO, DAMP_SEP>(b, (int)i, par, k == 0, s);
         }
     };
     bool used[ewf_batch::BRANCHES] = {};

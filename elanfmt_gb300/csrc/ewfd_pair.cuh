@@ -52,10 +52,18 @@ __device__ __forceinline__ f2 ld2(const float *p)
 {
     return NC ? __ldg(reinterpret_cast<const f2 *>(p)) : *reinterpret_cast<const f2 *>(p);
 }
+// ST: a line that the step does not need again soon, the first to leave L2 (split_shape).
+template <bool ST>
+__device__ __forceinline__ f2 ldm(const float *p)
+{
+    return ST ? __ldcs(reinterpret_cast<const f2 *>(p)) : ld2(p);
+}
+template <bool ST = false>
 __device__ __forceinline__ void st2(float *p, f2 v, bool m0, bool m1)
 {
     if (m0 && m1) {
-        *reinterpret_cast<f2 *>(p) = v;
+        if (ST) __stcs(reinterpret_cast<f2 *>(p), v);
+        else *reinterpret_cast<f2 *>(p) = v;
     } else {
         if (m0) p[0] = lo(v);
         if (m1) p[1] = hi(v);
@@ -102,24 +110,24 @@ struct StressIn2 {
     float w;
 };
 
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 __device__ __forceinline__ void stress_mat2(const StepArgs<float> &a, long long cm, int k, StressIn2<MODEL, DAMP> &q)
 {
     if (MODEL == MODEL_ISO) {
-        q.c[0] = ld2(a.m[0] + cm);
-        q.c[1] = ld2(a.m[1] + cm);
+        q.c[0] = ldm<ST>(a.m[0] + cm);
+        q.c[1] = ldm<ST>(a.m[1] + cm);
         q.w = ld(a.w1[2] + k + 1);
     } else {
         if (MODEL == MODEL_ISOHET) {
-            q.c[0] = ld2(a.m[0] + cm);
-            q.c[1] = ld2(a.m[3] + cm);
+            q.c[0] = ldm<ST>(a.m[0] + cm);
+            q.c[1] = ldm<ST>(a.m[3] + cm);
 #pragma unroll
-            for (int f = 0; f < 3; ++f) q.c[2 + f] = ld2(a.m[6 + f] + cm);
+            for (int f = 0; f < 3; ++f) q.c[2 + f] = ldm<ST>(a.m[6 + f] + cm);
         } else {
 #pragma unroll
-            for (int f = 0; f < 9; ++f) q.c[f] = ld2(a.m[f] + cm);
+            for (int f = 0; f < 9; ++f) q.c[f] = ldm<ST>(a.m[f] + cm);
         }
-        if (DAMP == DAMP_W3D) q.w3 = ld2(a.w3 + cm);
+        if (DAMP == DAMP_W3D) q.w3 = ldm<ST>(a.w3 + cm);
         else q.w = ld(a.w1[2] + k);
     }
 }
@@ -146,7 +154,7 @@ __device__ __forceinline__ void stress_state2(const StepArgs<float> &a, long lon
 // 14.4; ortho 128^3 in 85 without the prefetch 52.2 -> 54.9, 320x320x256 596 -> 603).
 template <int MODEL>
 __host__ __device__ constexpr bool pair_prefetch() { return MODEL == MODEL_ORTHO; }
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int j, int k0, int k1, long long soff, const StressSrc &ss,
                                             const int *start = nullptr, int r = 0)
 {
@@ -171,7 +179,7 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
     float wz_k = 0.f;
     if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + k0);
     StressIn2<MODEL, DAMP> nxt;
-    stress_mat2<MODEL, DAMP>(a, cm, k0, nxt);
+    stress_mat2<MODEL, DAMP, ST>(a, cm, k0, nxt);
     pdl_wait();  // nothing above depends on an earlier launch
     f2 vx_m = ld2<false>(a.f[0] + c - a.sy), vy_m = ld2<false>(a.f[1] + c - a.sy), vz_k = ld2<false>(a.f[2] + c);
     stress_state2<MODEL, DAMP>(a, c, nxt);
@@ -194,12 +202,12 @@ __device__ __forceinline__ void stress_pair(const StepArgs<float> &a, int i, int
 
     for (int k = k0; k < k1; ++k, c += a.sy, cm += a.sy) {
         if (!PF && k > k0) {
-            stress_mat2<MODEL, DAMP>(a, cm, k, nxt);
+            stress_mat2<MODEL, DAMP, ST>(a, cm, k, nxt);
             stress_state2<MODEL, DAMP>(a, c, nxt);
         }
         const StressIn2<MODEL, DAMP> q = nxt;
         if (PF && k + 1 < k1) {
-            stress_mat2<MODEL, DAMP>(a, cm + a.sy, k + 1, nxt);
+            stress_mat2<MODEL, DAMP, ST>(a, cm + a.sy, k + 1, nxt);
             stress_state2<MODEL, DAMP>(a, c + a.sy, nxt);
         }
         const f2 vx_ip = pk(hi(q.vx), q.vx_i2), vy_im = pk(q.vy_im, lo(q.vy)), vz_im = pk(q.vz_im, lo(vz_k));
@@ -277,15 +285,15 @@ struct VelIn2 {
     float w;
     f2 cp[KAHAN ? 3 : 1];
 };
-template <int MODEL, int DAMP, bool KAHAN>
+template <int MODEL, int DAMP, bool KAHAN, bool ST>
 __device__ __forceinline__ void vel_mat2(const StepArgs<float> &a, long long cm, int k, VelIn2<MODEL, DAMP, KAHAN> &q)
 {
     if (MODEL == MODEL_ISO) {
         q.w = ld(a.w1[2] + k - 1);
     } else {
 #pragma unroll
-        for (int f = 0; f < 3; ++f) q.b[f] = ld2(a.m[9 + f] + cm);
-        if (DAMP == DAMP_W3D) q.w3 = ld2(a.w3 + cm);
+        for (int f = 0; f < 3; ++f) q.b[f] = ldm<ST>(a.m[9 + f] + cm);
+        if (DAMP == DAMP_W3D) q.w3 = ldm<ST>(a.w3 + cm);
         else q.w = ld(a.w1[2] + k);
     }
 }
@@ -330,7 +338,7 @@ __device__ __forceinline__ f2 vel_update2(const StepArgs<float> &a, const PairOp
     return t;
 }
 
-template <int MODEL, int DAMP, bool KAHAN>
+template <int MODEL, int DAMP, bool KAHAN, bool ST>
 __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, int j, int kc0, int k1, long long soff, const RecFuse &rf,
                                               double *traces)
 {
@@ -349,7 +357,7 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
     long long cm = (long long)i + (long long)j * a.sx + (long long)k0 * a.sy;
     long long c = cm + soff;
     VelIn2<MODEL, DAMP, KAHAN> nxt;
-    vel_mat2<MODEL, DAMP, KAHAN>(a, cm, k0, nxt);
+    vel_mat2<MODEL, DAMP, KAHAN, ST>(a, cm, k0, nxt);
     pdl_wait();  // nothing above depends on an earlier launch
     f2 szz_m = ld2<false>(a.f[5] + c - a.sy), sxz_k = ld2<false>(a.f[7] + c), syz_k = ld2<false>(a.f[8] + c);
     vel_state2<MODEL, DAMP, KAHAN>(a, c, nxt);
@@ -378,7 +386,7 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
 
     for (int k = k0; k < k1; ++k, c += a.sy, cm += a.sy) {
         if (k > k0) {
-            vel_mat2<MODEL, DAMP, KAHAN>(a, cm, k, nxt);
+            vel_mat2<MODEL, DAMP, KAHAN, ST>(a, cm, k, nxt);
             vel_state2<MODEL, DAMP, KAHAN>(a, c, nxt);
         }
         const VelIn2<MODEL, DAMP, KAHAN> q = nxt;
@@ -410,7 +418,7 @@ __device__ __forceinline__ void velocity_pair(const StepArgs<float> &a, int i, i
         const bool m0[3] = {in0 && jn && kn, in0 && l0 && kn, in0 && l0 && jn}, m1[3] = {in1 && jn && kn, l1 && kn, l1 && jn};
 #pragma unroll
         for (int f = 0; f < 3; ++f) {
-            st2(a.f[f] + c, v[f], m0[f], m1[f]);
+            st2<ST>(a.f[f] + c, v[f], m0[f], m1[f]);
             if (KAHAN) st2(a.comp[f] + c, cp[f], m0[f], m1[f]);
         }
         if ((slot0 >= 0 || slot1 >= 0) && k >= rf.kmin && k <= rf.kmax) {
@@ -438,15 +446,15 @@ constexpr int PAIR_TX = TX / 2;                           // pairs per row of a 
 constexpr int PAIR_MAX_THREADS = 256;                     // CTAs of at most 16 rows
 __host__ __device__ constexpr int pair_rows(int ty) { return 2 * ty < PAIR_MAX_THREADS / PAIR_TX ? 2 * ty : PAIR_MAX_THREADS / PAIR_TX; }
 
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 __global__ void __launch_bounds__(PAIR_MAX_THREADS, pair_prefetch<MODEL>() ? 2 : 3) k_stress_pair(const StepArgs<float> a, const __grid_constant__ StressSrc ss)
 {
     pdl_trigger();
     const int k0 = blockIdx.z * a.kchunk;
-    stress_pair<MODEL, DAMP>(a, blockIdx.x * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz), 0, ss);
+    stress_pair<MODEL, DAMP, ST>(a, blockIdx.x * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz), 0, ss);
 }
 
-template <int MODEL, int DAMP, bool KAHAN>
+template <int MODEL, int DAMP, bool KAHAN, bool ST>
 __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const StepArgs<float> a, const RecFuse rf)
 {
     pdl_trigger();
@@ -455,7 +463,7 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const Ste
         *rf.it_wr = *rf.it_rd + 1;
     }
     const int k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
-    velocity_pair<MODEL, DAMP, KAHAN>(a, blockIdx.x * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
+    velocity_pair<MODEL, DAMP, KAHAN, ST>(a, blockIdx.x * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
                                       min(k0 + a.kchunk, a.nz), 0, rf, rf.traces);
 }
 
@@ -465,17 +473,17 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const Ste
 // trace_stride: elements between their trace blocks.  A batch of 6 right-hand sides on ortho 128^3 and 6 isotropic
 // models of 96^3 to 160^3: 503 us a step, 640 with one cell per thread and separate injection and receiver launches
 // for all problems; its fields and materials move in 425 us at the copy bandwidth.
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 __global__ void __launch_bounds__(PAIR_MAX_THREADS, pair_prefetch<MODEL>() ? 2 : 3)
     k_stress_pair_mr(const StepArgs<float> a, int R, long long rhs_stride, const __grid_constant__ StressSrc ss, const int *start)
 {
     pdl_trigger();
     const int r = blockIdx.x % R, k0 = blockIdx.z * a.kchunk;
-    stress_pair<MODEL, DAMP>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz),
+    stress_pair<MODEL, DAMP, ST>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, min(k0 + a.kchunk, a.nz),
                              (long long)r * rhs_stride, ss, start, r);
 }
 
-template <int MODEL, int DAMP>
+template <int MODEL, int DAMP, bool ST>
 __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3)
     k_velocity_pair_mr(const StepArgs<float> a, int R, long long rhs_stride, const RecFuse rf, long long trace_stride)
 {
@@ -485,7 +493,7 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3)
         *rf.it_wr = *rf.it_rd + 1;
     }
     const int r = blockIdx.x % R, k0 = ((int)gridDim.z - 1 - (int)blockIdx.z) * a.kchunk;
-    velocity_pair<MODEL, DAMP, false>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
+    velocity_pair<MODEL, DAMP, false, ST>(a, (blockIdx.x / R) * TX + 2 * threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0,
                                       min(k0 + a.kchunk, a.nz), (long long)r * rhs_stride, rf, rf.traces + r * trace_stride);
 }
 

@@ -30,6 +30,7 @@ constexpr double SHORT_CELLS = 4e5;
 struct SplitShape {
     int kchunk, ty, l2pf;
     bool pair;
+    bool stream;
 };
 SplitShape split_shape(int nx, int ny, int nz, int R = 1);
 
