@@ -1,7 +1,7 @@
 """Cache of the autotuner's choices (JSON), so a workload is timed once per GPU model.
 
 The library's autotuner (`ewf_autotune`, `ewf_batch_autotune`) times the step for z-chunks of
-4..64 planes and, for the two-kernel step, CTA tile heights of 4, 8 and 16 rows.  The best
+up to 32 planes and, for the two-kernel step, CTA tile heights of 4, 8 and 16 rows.  The best
 setting depends on the GPU, the scheme (model, damping, precision, step form) and the grid, not
 on the inputs' values, so it is stored under that key (the wavefront form's lag is re-tuned by
 `ewf_autotune` when a handle needs it):

@@ -123,8 +123,9 @@ typedef struct ewf_params {
     int32_t src_order;    /* ewf_src_order */
     int32_t over_y;       /* legacy OVERY: BC1 rows are j < min(nx, ny + over_y) (OK4:279-281) */
     int32_t nout;         /* progress line every nout steps (OK4:502-504); 0 = quiet */
-    int32_t kchunk;       /* planes per CTA of the z-marching kernels; 0 = autotuned/default */
-    int32_t graph_steps;  /* steps captured per CUDA graph; 0 = default, <0 = no graph */
+    int32_t kchunk;       /* planes per CTA of the z-marching kernels, from 4; 0 = autotuned/default (by size) */
+    int32_t graph_steps;  /* steps captured per CUDA graph; 0 = default (64; what is left of a run in graphs of 8 on
+                             small grids), <0 = no graph */
     int32_t check_finite; /* 1: ewf_run checks the receiver traces for NaN/Inf */
     int32_t fused;        /* ewf_step_form: 0 (default) two kernels; 1 one-pass kernel; 2 wavefront */
     double dx, dy, dz, dt; /* pa1[0..3] (OK4:404) */
@@ -215,7 +216,8 @@ int ewf_launches_per_step(const ewf_handle *h, int32_t *n);
 int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk);
 
 /* Two-kernel step (fused = EWF_STEP_SPLIT): the height of a CTA's tile in rows of 32 columns
- * (a power of two, 1..16 in FP32, 1..8 in FP64; default 8), set by ewf_autotune together with the
+ * (a power of two, 1..16 in FP32, 1..8 in FP64; default 4; with two cells per
+ * thread a tile has twice as many rows, 16 at most), set by ewf_autotune together with the
  * z-chunk; results do not depend on it.  ewf_set_tile: EWF_ERR_STATE for the other step forms. */
 int ewf_set_tile(ewf_handle *h, int32_t tile_y);
 int ewf_get_tile(const ewf_handle *h, int32_t *tile_y);
@@ -315,7 +317,7 @@ int ewf_pack_field_noalloc(void *dst, int32_t dst_dtype_bytes, int32_t sx, int64
  * (src/FastWaveED_GPU3D_v1_DC_Earthquake_FULL_OK4_final/vizme_FastBiotED_GPU3D_OK_2024_final.m
  * :551-558, 579-582, 604-607).  sos: nsec rows of (b0 b1 b2 a0 a1 a2) as MATLAB and scipy lay
  * them out; each section is the direct form II transposed recursion from zero state.
- * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (one thread per trace,
+ * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (a section of a trace per lane,
  * on `stream`), with the same bits. */
 #define EWF_SOS_MAX_SECTIONS 16
 int ewf_sosfilt(const double *sos, int32_t nsec, double *x, int64_t ntr, int64_t n);
