@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <set>
@@ -210,7 +211,7 @@ struct GemmJob {
     CUtensorMap a, b, f32, bf16, pre;
     const float *bias, *gpre;
     __nv_bfloat16 *cb;
-    int M, N, rows, bn;     // tile: rows (32, 64 or 128 of the accumulator's 128 lanes) x bn columns (at most BN)
+    int M, N, rows, bn;     // tile: rows (32 to 128 of the accumulator's 128 lanes) x bn columns (at most BN)
     int tiles_n, items, nk;
     int cta0, ctas;         // its CTAs
     int flags;
@@ -635,18 +636,35 @@ int gemm_one(const Product &p, cudaStream_t stream)
 // work: 32 or 64 of the accumulator's 128 lanes while CTAs for them and as many again for gW are there.
 // 256 x 512 from K = 10240: 110 us on 4 CTAs of 128 x 256 at 0.7 us a stage, now 28 with the weight gradient
 // behind it.
+// How the SMs are shared: the tile height that has the slower of the two done first, by the measured time of a
+// k-stage.  1024 x 512 from K = 18432 beside 18432 x 512: 64 tiles of 128 rows take 69 us and the other 88
+// SMs 33, 88 of 96 rows about 60 (a backward pass of these layers 79.6 -> 71.7).
+float stage_us(int rows, int bn) { return std::max(0.16f, (float)(rows + bn) * ewf_umma::ROW_BYTES / 104e3f); }
 int gemm_pair(const Product &dh, const Product &gw, cudaStream_t stream)
 {
     Device dev;
     int st = this_device(&dev);
     if (st) return st;
+    const int bn = gemm_tiles(gw.M, gw.N, ewf_umma::BM, 128) >= dev.sms / 2 ? 128 : 64, gw_items = gemm_tiles(gw.M, gw.N, ewf_umma::BM, bn);
+    const int nk_dh = (dh.K + ewf_umma::BK - 1) / ewf_umma::BK, nk_gw = (gw.K + ewf_umma::BK - 1) / ewf_umma::BK;
     int rows = ewf_umma::BM;
-    while (rows > 32 && gemm_tiles(dh.M, dh.N, rows / 2, 64) <= dev.sms / 2) rows /= 2;
+    float best = 1e30f;
+    for (int r = 32; r <= ewf_umma::BM; r += 32) {
+        const int tiles = gemm_tiles(dh.M, dh.N, r, 64), left = dev.sms - tiles;
+        if (left < dev.sms / 4 && r < ewf_umma::BM) continue;
+        const float t_dh = (float)((tiles + dev.sms - 1) / dev.sms) * nk_dh * stage_us(r, 64),
+                    t_gw = (float)((gw_items + std::max(left, 1) - 1) / std::max(left, 1)) * (nk_gw * stage_us(ewf_umma::BM, bn) + 1.f);
+        const float t = std::max(t_dh, t_gw);
+        if (t < best) {
+            best = t;
+            rows = r;
+        }
+    }
     alignas(64) GemmArgs g;
     memset(&g, 0, sizeof(g));
     GemmJob &a = g.job[0], &b = g.job[1];
     if ((st = make_job(&a, dh, rows, 64))) return st;
-    if ((st = make_job(&b, gw, ewf_umma::BM, gemm_tiles(gw.M, gw.N, ewf_umma::BM, 128) >= dev.sms / 2 ? 128 : 64))) return st;
+    if ((st = make_job(&b, gw, ewf_umma::BM, bn))) return st;
     const int left = dev.sms - a.items;
     a.ctas = left >= dev.sms / 4 ? a.items : a.items < dev.sms ? a.items : dev.sms;
     g.njobs = 2;
