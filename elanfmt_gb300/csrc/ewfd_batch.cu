@@ -2,10 +2,10 @@
 //
 // The reference runs one model and one source per process (README.md:86-102; one scenario
 // directory per run).  A batch holds several problems (models, possibly of different sizes and
-// model families) with several right-hand sides each, advanced together: every problem's launches
-// form a chain of their own -- two per step -- and the chains of a run of steps are captured in one CUDA
-// graph, one after the other (which leaves a small model's fields in L2 for its whole run of steps) or
-// on parallel branches.
+// model families) with several right-hand sides each, advanced together: the launches of a right-hand
+// side, or of all of a large model's, form a chain of their own -- two per step -- and the chains of a run
+// of steps are captured in one CUDA graph, one after the other (which leaves a model's fields in L2 for
+// its whole run of steps) or on parallel branches.
 #include "ewfd.h"
 #include "ewfd_internal.h"
 #include "ewfd_batch.cuh"
@@ -46,14 +46,9 @@ struct Prob {
     bool m_set[12] = {};
     bool w_set[4] = {};
     int kchunk = 0;                         // planes per CTA (0: by size, split_shape)
-    int ty = 4;                             // CTA tile height
-    bool pair = false;                      // two cells per thread
-    bool stream_l2 = false;                 // its kernels: materials and new velocities first to leave L2
-    StressSrc ss{};                         // sources in the stress kernel (nsrc 0: k_binject)
-    SrcEntry *d_sent = nullptr;             // its entries, right-hand side by right-hand side
+    SrcEntry *d_sent = nullptr;             // source entries, right-hand side by right-hand side
     int *d_sstart = nullptr;                // first entry of each right-hand side, R + 1
     int group0 = 0;                         // the problem's first (problem, RHS) group of k_binject
-    int nsrc = 0;
     RecFuse rf{};                           // receivers in the velocity kernel
     bool rec_fuse = true;
     uint2 *d_rgrp = nullptr;
@@ -65,7 +60,30 @@ struct Prob {
     std::vector<double> stf;
 };
 
+// What one sequence of launches advances: right-hand sides [r0, r0 + R) of a problem
+struct Chain {
+    int prob = 0, r0 = 0, R = 1;
+    int branch = -1;          // its branch (balanced by cell-updates), -1: the batch's stream
+    int ty = 4;               // CTA tile height
+    bool pair = false;        // two cells per thread
+    bool stream_l2 = false;   // its kernels: materials and new velocities first to leave L2
+    StepArgs<float> a;        // of right-hand side r0
+    StressSrc ss{};           // sources in the stress kernel (nsrc 0: k_binject)
+    int nsrc = 0;
+    RecFuse rf{};
+    double work = 0;          // cells
+};
+
 float *bptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.base_off : nullptr; }
+// Right-hand sides of a model between these many cells run apart, each its own chain: by itself one keeps its
+// fields in L2 from step to step.  On larger grids they share launches, and the materials' way from HBM; on
+// smaller ones a step of many chains is bound by their launches, about 1 us each.  us per step of 2, 3 and 6
+// right-hand sides of ortho n^3 in shared launches and apart:
+//   64^3 13 17 33 and 10 14 31        96^3 35 56 116 and 34 52 103      112^3 66 101 198 and 61 91 182
+//   128^3 92 136 260 and 84 126 251   144^3 142 206 396 and 142 213 426   160^3 182 265 513 and 186 278 556
+// and of 6 with a small isotropic model: 30^3 11.4 and 14.5, 40^3 16.1 and 17.9, 50^3 28.1 and 23.6, 64^3 40.3 and 30.7.
+constexpr double APART_FROM = 1e5, APART_TO = 2.5e6;
+
 float *sptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.sbase_off : nullptr; }
 
 }  // namespace
@@ -76,6 +94,7 @@ struct ewf_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<Prob> probs;
+    std::vector<Chain> chains;          // the same list for the batch's life: each has its step counters
     BatchProb<float> *d_all = nullptr;  // every problem, indexed by problem id
     std::vector<BatchProb<float>> h_all;  // host copy of d_all
     int nrhs_total = 0;
@@ -103,7 +122,6 @@ struct ewf_batch {
     static constexpr int BRANCHES = 8;
     cudaStream_t branch[BRANCHES] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[BRANCHES] = {};
-    std::vector<int> branch_of;  // per problem: its branch (balanced by cell-updates), -1: the batch's stream
     cudaGraphExec_t gexec = nullptr, gexec_short = nullptr;  // of gsteps and of SHORT_GRAPH steps
     int gsteps = 64;     // steps per graph (even: the step counters alternate between two locations)
     float last_ms = 0.f;
@@ -246,10 +264,25 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
     }
     CKB(cudaMalloc(&b->d_stage, stage));
     b->stage_bytes = stage;
-    // graphs of two launches per problem and step, of some 16 thousand nodes at most
-    while (b->gsteps > 2 && (long long)b->gsteps * 2 * n > 16384) b->gsteps -= 2;
-    CKB(cudaMalloc(&b->d_it, 2 * n * sizeof(int)));
-    CKB(cudaMemsetAsync(b->d_it, 0, 2 * n * sizeof(int), b->stream));
+    for (int i = 0; i < n; ++i) {
+        const Prob &q = b->probs[i];
+        const double cells = (double)q.p.nx * q.p.ny * q.p.nz;
+        Chain c;
+        c.prob = i;
+        if (cells >= APART_FROM && cells < APART_TO) {
+            c.work = cells;
+            for (c.r0 = 0; c.r0 < q.R; ++c.r0) b->chains.push_back(c);
+        } else {
+            c.R = q.R;
+            c.work = cells * q.R;
+            b->chains.push_back(c);
+        }
+    }
+    // graphs of two launches per chain and step, of some 16 thousand nodes at most
+    const size_t nch = b->chains.size();
+    while (b->gsteps > 2 && b->gsteps * 2 * nch > 16384) b->gsteps -= 2;
+    CKB(cudaMalloc(&b->d_it, 2 * nch * sizeof(int)));
+    CKB(cudaMemsetAsync(b->d_it, 0, 2 * nch * sizeof(int), b->stream));
     CKB(cudaStreamSynchronize(b->stream));
 #undef CKB
     *out = b;
@@ -384,12 +417,12 @@ static int upload(T **dst, const std::vector<T> &v)
     return EWF_OK;
 }
 
-// Problems below BRANCH_CELLS cells (all right-hand sides) share the GPU on parallel branches; a larger one
+// Chains below BRANCH_CELLS cells share the GPU on parallel branches; a larger one
 // fills it, and alone keeps its fields in L2.  us per step of six problems n^3, one after another and on
 // four branches:
 //   iso    32^3 30 10   64^3 40 22   80^3 62 50   96^3 76 88     128^3 198 222   160^3 432 441
 //   ortho  32^3 30 11   64^3 50 30   80^3 75 76   96^3 104 122   128^3 296 287   160^3 571 565
-// As many branches as hold BRANCH_SHARE cells between them, which L2 still keeps.  us per step on 2, 4 and
+// As many branches (two at least) as hold BRANCH_SHARE cells between them, which L2 still keeps.  us per step on 2, 4 and
 // 8 branches (these and the above with chunks by each problem's own size):
 //   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
 //   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
@@ -401,25 +434,25 @@ static int build_tables(ewf_batch *b)
     CK(cudaStreamSynchronize(b->stream));
     free_tables(b);
     const int n = (int)b->probs.size();
-    // branches: largest problems first, each to the least loaded branch
-    b->branch_of.assign(n, -1);
-    int share = 1;  // problems that run at the same time
-    if (b->own != 0 && n > 1) {
-        std::vector<int> idx(n);
-        for (int i = 0; i < n; ++i) idx[i] = i;
-        auto work = [&](int i) {
-            const Prob &q = b->probs[i];
-            return (double)q.p.nx * q.p.ny * q.p.nz * q.R;
-        };
-        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return work(x) > work(y); });
-        idx.erase(std::remove_if(idx.begin(), idx.end(), [&](int i) { return b->own < 0 && work(i) >= BRANCH_CELLS; }), idx.end());
-        const int branches = idx.empty() ? 1 : (int)std::max(2.0, std::min((double)ewf_batch::BRANCHES, BRANCH_SHARE / work(idx[0])));
-        share = std::min(branches, std::max(1, (int)idx.size()));
+    // branches: largest chains first, each to the least loaded branch
+    int share = 1;  // chains that run at the same time
+    for (auto &c : b->chains) c.branch = -1;
+    if (b->own != 0 && b->chains.size() > 1) {
+        std::vector<Chain *> idx;
+        for (auto &c : b->chains)
+            if (b->own > 0 || c.work < BRANCH_CELLS) idx.push_back(&c);
+        std::stable_sort(idx.begin(), idx.end(), [](const Chain *x, const Chain *y) { return x->work > y->work; });
+        int branches = std::min(2, (int)idx.size());
+        double held = 0;
+        for (int k = 0; k < (int)idx.size() && k < ewf_batch::BRANCHES; ++k) {
+            held += idx[k]->work;
+            if (held <= BRANCH_SHARE) branches = std::max(branches, k + 1);
+        }
+        share = std::max(1, branches);
         double load[ewf_batch::BRANCHES] = {};
-        for (int i : idx) {
-            const int k = (int)(std::min_element(load, load + branches) - load);
-            b->branch_of[i] = k;
-            load[k] += work(i);
+        for (Chain *c : idx) {
+            c->branch = (int)(std::min_element(load, load + branches) - load);
+            load[c->branch] += c->work;
         }
     }
     std::vector<BatchProb<float>> all(n);
@@ -438,14 +471,6 @@ static int build_tables(ewf_batch *b)
         bp.rhs_stride = (long long)q.box;
         d.nx = p.nx; d.ny = p.ny; d.nz = p.nz;
         d.bc1_rows = std::min(p.ny, std::min(p.nx, p.ny + std::max(0, p.over_y)));
-        const SplitShape shape = split_shape(p.nx, p.ny, p.nz, q.R);
-        q.ty = std::max(b->ty, shape.ty);
-        q.pair = shape.pair || q.R > 1;
-        q.stream_l2 = shape.stream;
-        // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
-        // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
-        // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
-        d.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, q.R * (b->branch_of[i] >= 0 ? share : 1)).kchunk;
         d.dt = (float)p.dt;
         d.rdt = 1.0f / d.dt;
         d.dx = (float)p.dx; d.dy = (float)p.dy; d.dz = (float)p.dz;
@@ -458,7 +483,6 @@ static int build_tables(ewf_batch *b)
         d.bc1 = p.free_surface == EWF_FS_BC1 ? 1 : 0;
         d.smu_on = p.surface_mu > 0.0 ? 1 : 0;
         d.smu = (float)p.surface_mu;
-        d.l2pf = b->l2pf >= 0 ? b->l2pf : shape.l2pf;
     }
     CK(cudaMalloc(&b->d_all, n * sizeof(BatchProb<float>)));
     // sources grouped by (problem, rhs)
@@ -469,7 +493,6 @@ static int build_tables(ewf_batch *b)
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
         q.group0 = (int)start.size();
-        const int first = (int)src.size();
         std::vector<SrcEntry> ent;
         std::vector<int> from;
         for (int r = 0; r < q.R; ++r) {
@@ -481,16 +504,10 @@ static int build_tables(ewf_batch *b)
             }
             if (!q.src[r].empty() && q.stf.empty()) return ewf_fail(EWF_ERR_STATE, "problem %d has sources but no Src", i);
         }
-        q.nsrc = (int)src.size() - first;
-        bool plane1 = false;
-        if (make_stress_src(ent, q.p.nx, q.p.ny, q.p.nz, &q.ss, &plane1)) {
-            from.push_back((int)ent.size());
+        from.push_back((int)ent.size());
+        if (!ent.empty()) {
             if (int st = upload(&q.d_sent, ent)) return st;
             if (int st = upload(&q.d_sstart, from)) return st;
-            q.ss.src = q.d_sent;
-            if (q.R > 1) q.ss.inl = 0;
-            // plane 2's thread applies a shear entry on plane 1, so it has to store that plane too
-            if (plane1) all[i].a.kchunk = std::max(all[i].a.kchunk, 4);
         }
         stf_off[i] = i * b->nt;
         if (!q.stf.empty()) std::copy(q.stf.begin(), q.stf.end(), stf.begin() + (size_t)i * b->nt);
@@ -539,9 +556,6 @@ static int build_tables(ewf_batch *b)
     b->nrec_total = nrec;
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
-        q.ss.stf = b->d_stf + (size_t)i * b->nt;
-        q.ss.nstf = b->nt;
-        q.ss.order = q.p.src_order;
         const RecTables t = make_rec_tables((int)q.rec.size() / 4, q.rec.data(), q.p.nx, q.p.ny, q.p.nz);
         q.rec_fuse = t.fuse;
         q.rf = RecFuse{};
@@ -559,6 +573,41 @@ static int build_tables(ewf_batch *b)
             q.rf.trace_len = b->nt;
         }
     }
+    for (auto &c : b->chains) {
+        const Prob &q = b->probs[c.prob];
+        const ewf_params &p = q.p;
+        const SplitShape shape = split_shape(p.nx, p.ny, p.nz, c.R);
+        c.ty = std::max(b->ty, shape.ty);
+        c.pair = shape.pair || c.R > 1;
+        c.stream_l2 = shape.stream;
+        c.a = all[c.prob].a;
+        for (auto &f : c.a.f) f += c.r0 * (long long)q.box;
+        c.a.l2pf = b->l2pf >= 0 ? b->l2pf : shape.l2pf;
+        // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
+        // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
+        // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
+        c.a.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, c.R * (c.branch >= 0 ? share : 1)).kchunk;
+        std::vector<SrcEntry> ent;
+        int before = 0;
+        for (int r = 0; r < c.r0 + c.R; ++r) {
+            if (r < c.r0) before += (int)q.src[r].size();
+            else
+                for (auto &e : q.src[r]) ent.push_back(SrcEntry{e.comp, e.i, e.j, e.k, e.coef});
+        }
+        c.nsrc = (int)ent.size();
+        bool plane1 = false;
+        if (make_stress_src(ent, p.nx, p.ny, p.nz, &c.ss, &plane1)) {
+            c.ss.src = q.d_sent + before;
+            if (c.R > 1) c.ss.inl = 0;
+            // plane 2's thread applies a shear entry on plane 1, so it has to store that plane too
+            if (plane1) c.a.kchunk = std::max(c.a.kchunk, 4);
+        }
+        c.ss.stf = b->d_stf + (size_t)c.prob * b->nt;
+        c.ss.nstf = b->nt;
+        c.ss.order = p.src_order;
+        c.rf = q.rf;
+        if (c.rf.grp) c.rf.traces += (size_t)c.r0 * (q.rec.size() / 4) * b->nt;
+    }
     if (nrec) {
         CK(cudaMalloc(&b->d_rec_comp, nrec * sizeof(int)));
         CK(cudaMemcpy(b->d_rec_comp, rc.data(), nrec * sizeof(int), cudaMemcpyHostToDevice));
@@ -569,63 +618,65 @@ static int build_tables(ewf_batch *b)
     return EWF_OK;
 }
 
-// One step of problem i on a stream; `parity` = the step number's: its counter is at d_it[2 i + parity], the
+// One step of chain i on a stream; `parity` = the step number's: its counter is at d_it[2 i + parity], the
 // next step's at d_it[2 i + 1 - parity].
 template <int MODEL, int DAMP, bool ST>
-static void problem_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
+static void chain_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
 {
-    const Prob &q = b->probs[i];
-    const StepArgs<float> &a = b->h_all[i].a;
+    const Chain &c = b->chains[i];
+    const Prob &q = b->probs[c.prob];
+    const StepArgs<float> &a = c.a;
     int *const it_rd = b->d_it + 2 * i + parity, *const it_wr = b->d_it + 2 * i + 1 - parity;
-    StressSrc ss = q.ss;
+    StressSrc ss = c.ss;
     ss.it_ptr = it_rd;
-    RecFuse rf = q.rf;
+    RecFuse rf = c.rf;
     rf.it_rd = it_rd;
     if (q.rec_fuse) rf.it_wr = it_wr;
-    const int rows = q.pair ? pair_rows(q.ty) : q.ty, tiles_x = (q.p.nx + TX - 1) / TX;
-    const dim3 blk(q.pair ? PAIR_TX : TX, rows), grd(tiles_x * q.R, (q.p.ny + rows - 1) / rows, (q.p.nz + a.kchunk - 1) / a.kchunk);
-    const long long stride = b->h_all[i].rhs_stride, nr = (long long)q.rec.size() / 4;
-    if (q.R > 1) launch_on(k_stress_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, q.R, stride, ss, (const int *)q.d_sstart);
-    else if (q.pair) launch_on(k_stress_pair<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, ss);
+    const int rows = c.pair ? pair_rows(c.ty) : c.ty, tiles_x = (q.p.nx + TX - 1) / TX;
+    const dim3 blk(c.pair ? PAIR_TX : TX, rows), grd(tiles_x * c.R, (q.p.ny + rows - 1) / rows, (q.p.nz + a.kchunk - 1) / a.kchunk);
+    const long long stride = (long long)q.box, nr = (long long)q.rec.size() / 4;
+    // (a problem with several right-hand sides in one launch has all of them: r0 = 0)
+    if (c.R > 1) launch_on(k_stress_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, c.R, stride, ss, (const int *)q.d_sstart);
+    else if (c.pair) launch_on(k_stress_pair<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, ss);
     else launch_on(k_stress<float, MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
-    if (q.nsrc > 0 && ss.nsrc == 0)
-        k_binject<float><<<(q.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, q.group0, q.R, b->d_stf, b->d_stf_off, b->d_order,
-                                                        b->nt, it_rd);
-    if (q.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl, a, q.R, stride, rf, nr * b->nt);
-    else if (q.pair) launch_on(k_velocity_pair<MODEL, DAMP, false, ST>, grd, blk, s, b->pdl, a, rf);
+    if (c.nsrc > 0 && ss.nsrc == 0)
+        k_binject<float><<<(c.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, q.group0 + c.r0, c.R, b->d_stf, b->d_stf_off,
+                                                        b->d_order, b->nt, it_rd);
+    if (c.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl, a, c.R, stride, rf, nr * b->nt);
+    else if (c.pair) launch_on(k_velocity_pair<MODEL, DAMP, false, ST>, grd, blk, s, b->pdl, a, rf);
     else launch_on(k_velocity<float, MODEL, DAMP, false>, grd, blk, s, b->pdl, a, rf);
     if (!q.rec_fuse) {
-        const int rows_ = (int)nr * q.R;
-        k_brecord<float><<<std::min((rows_ + 255) / 256, 1024), 256, 0, s>>>(a, b->d_rec_off, b->d_rec_comp, b->rec_base[i], rows_, b->d_traces,
-                                                                            b->nt, it_rd);
+        const int nrow = (int)nr * c.R;
+        k_brecord<float><<<std::min((nrow + 255) / 256, 1024), 256, 0, s>>>(b->h_all[c.prob].a, b->d_rec_off, b->d_rec_comp,
+                                                                            b->rec_base[c.prob] + c.r0 * (int)nr, nrow, b->d_traces, b->nt, it_rd);
         k_advance<<<1, 1, 0, s>>>(it_rd, it_wr);
     }
 }
 
 template <int MODEL, int DAMP>
-static void problem_step(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
+static void chain_step(ewf_batch *b, int i, int parity, bool first, cudaStream_t s)
 {
-    if (b->probs[i].stream_l2) problem_step_t<MODEL, DAMP, true>(b, i, parity, first, s);
-    else problem_step_t<MODEL, DAMP, false>(b, i, parity, first, s);
+    if (b->chains[i].stream_l2) chain_step_t<MODEL, DAMP, true>(b, i, parity, first, s);
+    else chain_step_t<MODEL, DAMP, false>(b, i, parity, first, s);
 }
 
-// `steps` steps of every problem from step parity `parity` on, chain by chain: the branches' problems on
+// `steps` steps of every chain from step parity `parity` on, one chain after the other: the branches' on
 // streams forked from the batch's and joined, then the others on the batch's stream.
 static void batch_steps(ewf_batch *b, int steps, int parity)
 {
     auto chain = [&](size_t i, cudaStream_t s) {
-        const ewf_params &p = b->probs[i].p;
+        const ewf_params &p = b->probs[b->chains[i].prob].p;
         for (int k = 0; k < steps; ++k) {
             const int par = (parity + k) & 1;
-            // nothing of another problem's to overlap with: a chain's first launch is a plain one
-            if (p.model == EWF_MODEL_ISO) problem_step<MODEL_ISO, DAMP_PML1D>(b, (int)i, par, k == 0, s);
-            else if (p.damping == EWF_DAMP_W3D) problem_step<MODEL_ORTHO, DAMP_W3D>(b, (int)i, par, k == 0, s);
-            else problem_step<MODEL_ORTHO, DAMP_SEP>(b, (int)i, par, k == 0, s);
+            // nothing of another chain's to overlap with: a chain's first launch is a plain one
+            if (p.model == EWF_MODEL_ISO) chain_step<MODEL_ISO, DAMP_PML1D>(b, (int)i, par, k == 0, s);
+            else if (p.damping == EWF_DAMP_W3D) chain_step<MODEL_ORTHO, DAMP_W3D>(b, (int)i, par, k == 0, s);
+            else chain_step<MODEL_ORTHO, DAMP_SEP>(b, (int)i, par, k == 0, s);
         }
     };
     bool used[ewf_batch::BRANCHES] = {};
-    for (int k : b->branch_of)
-        if (k >= 0) used[k] = true;
+    for (const Chain &c : b->chains)
+        if (c.branch >= 0) used[c.branch] = true;
     bool forked = false;
     for (int k = 0; k < ewf_batch::BRANCHES; ++k) {
         if (!used[k]) continue;
@@ -633,15 +684,15 @@ static void batch_steps(ewf_batch *b, int steps, int parity)
         forked = true;
         cudaStreamWaitEvent(b->branch[k], b->fork_ev, 0);
     }
-    for (size_t i = 0; i < b->probs.size(); ++i)
-        if (b->branch_of[i] >= 0) chain(i, b->branch[b->branch_of[i]]);
+    for (size_t i = 0; i < b->chains.size(); ++i)
+        if (b->chains[i].branch >= 0) chain(i, b->branch[b->chains[i].branch]);
     for (int k = 0; k < ewf_batch::BRANCHES; ++k) {
         if (!used[k]) continue;
         cudaEventRecord(b->join_ev[k], b->branch[k]);
         cudaStreamWaitEvent(b->stream, b->join_ev[k], 0);
     }
-    for (size_t i = 0; i < b->probs.size(); ++i)
-        if (b->branch_of[i] < 0) chain(i, b->stream);
+    for (size_t i = 0; i < b->chains.size(); ++i)
+        if (b->chains[i].branch < 0) chain(i, b->stream);
 }
 
 static int batch_graph(ewf_batch *b, int steps, cudaGraphExec_t *exec)
@@ -676,13 +727,13 @@ static int ready_graph(ewf_batch *b, int steps, cudaGraphExec_t *exec)
     return st;
 }
 
-// The steps a long graph leaves over go in graphs of SHORT_GRAPH steps where the problems are small on average
-// (SHORT_CELLS): launched one by one, a step of n problems takes the host some 5 n us.
+// The steps a long graph leaves over go in graphs of SHORT_GRAPH steps where the chains are small on average
+// (SHORT_CELLS): launched one by one, a step of n chains takes the host some 5 n us.
 static int short_graph(const ewf_batch *b)
 {
     double cells = 0;
-    for (auto &q : b->probs) cells += (double)q.p.nx * q.p.ny * q.p.nz * q.R;
-    return cells < SHORT_CELLS * b->probs.size() && SHORT_GRAPH < b->gsteps ? SHORT_GRAPH : 0;
+    for (auto &c : b->chains) cells += c.work;
+    return cells < SHORT_CELLS * b->chains.size() && SHORT_GRAPH < b->gsteps ? SHORT_GRAPH : 0;
 }
 
 static int batch_ready(ewf_batch *b)
@@ -706,7 +757,7 @@ extern "C" int ewf_batch_reset(ewf_batch *b)
     for (auto &q : b->probs)
         for (auto &x : q.state) z.push_back({x, q.sbox * 4});
     if (b->d_traces) z.push_back({b->d_traces, (size_t)b->nrec_total * b->nt * sizeof(double)});
-    z.push_back({b->d_it, 2 * b->probs.size() * sizeof(int)});
+    z.push_back({b->d_it, 2 * b->chains.size() * sizeof(int)});
     if (int st = zero_buffers(z, b->stream)) return st;
     CK(cudaStreamSynchronize(b->stream));
     b->it = 0;

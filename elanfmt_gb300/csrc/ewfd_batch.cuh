@@ -3,9 +3,10 @@
 //
 // A problem is one model (grid, materials, damping) with R right-hand sides (source sets); its R
 // state sets are separate boxes (rhs_stride elements apart) sharing the material arrays.  Problems do
-// not depend on one another, so each runs its own chain of the solver's launches (k_stress / k_velocity
-// or their two-cell forms, with sources, receivers and step counter inside); with several right-hand sides
-// k_stress_pair_mr / k_velocity_pair_mr, whose CTAs of a tile read its material planes from HBM once.
+// not depend on one another, nor do right-hand sides, so each chain -- a right-hand side, or all of a
+// large model -- runs the solver's launches by itself (k_stress / k_velocity or their two-cell forms, with
+// sources, receivers and step counter inside); k_stress_pair_mr / k_velocity_pair_mr advance several
+// right-hand sides, their CTAs of a tile reading its material planes from HBM once.
 // Here: the problem descriptor, and the separate injection and recording kernels for the entries
 // those launches do not take (sources outside the stress cells, receivers of other fields or cells).
 #pragma once

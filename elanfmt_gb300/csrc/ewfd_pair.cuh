@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(PAIR_MAX_THREADS, 3) k_velocity_pair(const Ste
 // right-hand side is the fastest part of blockIdx.x, so the CTAs of a tile are dispatched together and read
 // its material planes from HBM once (the others' reads hit L2).  start: their source entries in ss.src;
 // trace_stride: elements between their trace blocks.  A batch of 6 right-hand sides on ortho 128^3 and 6 isotropic
-// models of 96^3 to 160^3: 503 us a step, 640 with one cell per thread and separate injection and receiver launches
+// models of 96^3 to 160^3 with these: 493 us a step, 640 with one cell per thread and separate injection and receiver launches
 // for all problems; its fields and materials move in 425 us at the copy bandwidth.
 template <int MODEL, int DAMP, bool ST>
 __global__ void __launch_bounds__(PAIR_MAX_THREADS, pair_prefetch<MODEL>() ? 2 : 3)

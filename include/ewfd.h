@@ -331,9 +331,9 @@ int ewf_restore(ewf_handle *h, const char *path);
  * Batched solver (no counterpart in the reference, which runs one model and one source per
  * process): n problems -- models of any size and family -- each with n_rhs[i] right-hand sides
  * (independent source sets sharing the problem's model, e.g. the 6 elementary moment tensors of
- * a moment-tensor inversion), advanced together.  Per time step and problem one stress and one
- * velocity launch for all its RHS (materials read from HBM once), with sources and receivers inside
- * where the solver's own step has them there, replayed from a CUDA graph.  FP32; every problem runs the
+ * a moment-tensor inversion), advanced together.  Per time step one stress and one velocity launch for
+ * an RHS or, on large and very small models, for all of a problem's (materials read from HBM once), with
+ * sources and receivers inside where the solver's own step has them there, replayed from a CUDA graph.  FP32; every problem runs the
  * same nt; state starts at zero.
  * ------------------------------------------------------------------------------------------- */
 typedef struct ewf_batch ewf_batch;
@@ -365,7 +365,7 @@ int ewf_batch_get_tile(const ewf_batch *b, int32_t *tile_y);
 int ewf_batch_set_l2_prefetch(ewf_batch *b, int32_t planes);
 /* Launch form: 0 -- one problem's run of steps after another's; 1 -- spread over up to eight parallel
  * branches (streams of the captured graph) balanced by cell-updates.  By default (reported as 0) the
- * problems too small to fill the GPU run on branches, then the others one after another.  Results do
+ * chains of launches too small to fill the GPU run on branches, then the others one after another.  Results do
  * not depend on it. */
 int ewf_batch_set_launch(ewf_batch *b, int32_t own);
 int ewf_batch_get_launch(const ewf_batch *b, int32_t *own);

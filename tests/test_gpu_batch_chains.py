@@ -53,3 +53,21 @@ def test_chains(cuda_device, own, outside, stress_rec):
                 np.testing.assert_array_equal(b.seismograms(p, r), ref.traces, err_msg=f"problem {p} rhs {r}")
                 for q in F.STATE:
                     np.testing.assert_array_equal(b.field(p, r, q), ref.f[q], err_msg=f"problem {p} rhs {r} {F.STATE_NAMES[q]}")
+
+
+@pytest.mark.parametrize("model,damping", [(F.MODEL_ISO, None), (F.MODEL_ORTHO, F.DAMP_SEPARABLE), (F.MODEL_ORTHO, F.DAMP_W3D)])
+@pytest.mark.parametrize("outside,stress_rec", [(False, False), (True, True)])
+def test_shared_launches(cuda_device, model, damping, outside, stress_rec):
+    """A model large enough for its right-hand sides to share launches."""
+    nt, shape = 9, (139, 137, 133)
+    assert np.prod(shape) >= 2.5e6
+    m, rhs = _problem(model, shape, nt, 4, 8, outside, stress_rec, **({} if damping is None else {"damping": damping}))
+    with Batch([(m, rhs)]) as b:
+        for n in (3, 6):
+            b.run(n)
+        for r, (ent, coef) in enumerate(rhs):
+            m.sources, m.source_coef = ent, coef
+            ref = O.run(m, nt)
+            np.testing.assert_array_equal(b.seismograms(0, r), ref.traces, err_msg=f"rhs {r}")
+            for q in F.STATE:
+                np.testing.assert_array_equal(b.field(0, r, q), ref.f[q], err_msg=f"rhs {r} {F.STATE_NAMES[q]}")
