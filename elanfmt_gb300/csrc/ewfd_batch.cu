@@ -426,6 +426,8 @@ static int upload(T **dst, const std::vector<T> &v)
 // 8 branches (these and the above with chunks by each problem's own size):
 //   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
 //   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
+// Many tiny models are bound by their launches, 0.35 us each on eight branches: 50, 200 of 16^3 38, 139 us a step,
+// of 24^3 40, 147, 100 of 40^3 142 (one launch per phase over all of them: 28, 52, 35, 112, 237).
 constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
 
 // Rebuilds the device tables (problem descriptors, sources, receivers, traces).
