@@ -72,6 +72,10 @@ struct Chain {
     int nsrc = 0;
     RecFuse rf{};
     double work = 0;          // cells
+    std::vector<int> many;    // the chains of tiny problems it stands for (k_stress_many), and for each step parity
+    ManyProb *d_many[2] = {nullptr, nullptr};  // their arguments,
+    int2 *d_map = nullptr;    // and the problem of each CTA
+    int blocks = 0;
 };
 
 float *bptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.base_off : nullptr; }
@@ -94,7 +98,7 @@ struct ewf_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<Prob> probs;
-    std::vector<Chain> chains;          // the same list for the batch's life: each has its step counters
+    std::vector<Chain> chains;
     BatchProb<float> *d_all = nullptr;  // every problem, indexed by problem id
     std::vector<BatchProb<float>> h_all;  // host copy of d_all
     int nrhs_total = 0;
@@ -137,6 +141,9 @@ static void free_tables(ewf_batch *b)
         q.d_roff = nullptr;
         q.d_rent = nullptr;
     }
+    for (auto &c : b->chains)
+        for (void *x : {(void *)c.d_many[0], (void *)c.d_many[1], (void *)c.d_map}) cudaFree(x);
+    b->chains.clear();
     cudaFree(b->d_all); b->d_all = nullptr;
     cudaFree(b->d_src); b->d_src = nullptr;
     cudaFree(b->d_src_start); b->d_src_start = nullptr;
@@ -264,22 +271,8 @@ extern "C" int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n
     }
     CKB(cudaMalloc(&b->d_stage, stage));
     b->stage_bytes = stage;
-    for (int i = 0; i < n; ++i) {
-        const Prob &q = b->probs[i];
-        const double cells = (double)q.p.nx * q.p.ny * q.p.nz;
-        Chain c;
-        c.prob = i;
-        if (cells >= APART_FROM && cells < APART_TO) {
-            c.work = cells;
-            for (c.r0 = 0; c.r0 < q.R; ++c.r0) b->chains.push_back(c);
-        } else {
-            c.R = q.R;
-            c.work = cells * q.R;
-            b->chains.push_back(c);
-        }
-    }
     // graphs of two launches per chain and step, of some 16 thousand nodes at most
-    const size_t nch = b->chains.size();
+    const size_t nch = b->nrhs_total;  // chains, at most
     while (b->gsteps > 2 && b->gsteps * 2 * nch > 16384) b->gsteps -= 2;
     CKB(cudaMalloc(&b->d_it, 2 * nch * sizeof(int)));
     CKB(cudaMemsetAsync(b->d_it, 0, 2 * nch * sizeof(int), b->stream));
@@ -426,9 +419,13 @@ static int upload(T **dst, const std::vector<T> &v)
 // 8 branches (these and the above with chunks by each problem's own size):
 //   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
 //   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
-// Many tiny models are bound by their launches, 0.35 us each on eight branches: 50, 200 of 16^3 38, 139 us a step,
-// of 24^3 40, 147, 100 of 40^3 142 (one launch per phase over all of them: 28, 52, 35, 112, 237).
 constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
+// MANY_MIN or more problems of one scheme below MANY_CELLS cells share two launches a step (k_stress_many): chains of
+// their own are bound by their launches, 0.35 us each on eight branches.  us per step of chains and of shared
+// launches: 50 iso 16^3 38 and 15, 200 139 and 50; 24 iso 24^3 17.5 and 15, 50 40 and 24, 200 147 and 110.
+constexpr double MANY_CELLS = 2e4;
+constexpr int MANY_MIN = 16;
+static int scheme(const ewf_params &p) { return p.model == EWF_MODEL_ISO ? 0 : p.damping == EWF_DAMP_W3D ? 1 : 2; }
 
 // Rebuilds the device tables (problem descriptors, sources, receivers, traces).
 static int build_tables(ewf_batch *b)
@@ -436,27 +433,6 @@ static int build_tables(ewf_batch *b)
     CK(cudaStreamSynchronize(b->stream));
     free_tables(b);
     const int n = (int)b->probs.size();
-    // branches: largest chains first, each to the least loaded branch
-    int share = 1;  // chains that run at the same time
-    for (auto &c : b->chains) c.branch = -1;
-    if (b->own != 0 && b->chains.size() > 1) {
-        std::vector<Chain *> idx;
-        for (auto &c : b->chains)
-            if (b->own > 0 || c.work < BRANCH_CELLS) idx.push_back(&c);
-        std::stable_sort(idx.begin(), idx.end(), [](const Chain *x, const Chain *y) { return x->work > y->work; });
-        int branches = std::min(2, (int)idx.size());
-        double held = 0;
-        for (int k = 0; k < (int)idx.size() && k < ewf_batch::BRANCHES; ++k) {
-            held += idx[k]->work;
-            if (held <= BRANCH_SHARE) branches = std::max(branches, k + 1);
-        }
-        share = std::max(1, branches);
-        double load[ewf_batch::BRANCHES] = {};
-        for (Chain *c : idx) {
-            c->branch = (int)(std::min_element(load, load + branches) - load);
-            load[c->branch] += c->work;
-        }
-    }
     std::vector<BatchProb<float>> all(n);
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
@@ -575,7 +551,75 @@ static int build_tables(ewf_batch *b)
             q.rf.trace_len = b->nt;
         }
     }
-    for (auto &c : b->chains) {
+    // the chains, and which of them are tiny problems whose launches take sources and receivers
+    auto fuses = [&](const Chain &c, std::vector<SrcEntry> *ent, int *before, StressSrc *f, bool *plane1) {
+        const Prob &q = b->probs[c.prob];
+        *before = 0;
+        for (int r = 0; r < c.r0 + c.R; ++r) {
+            if (r < c.r0) *before += (int)q.src[r].size();
+            else
+                for (auto &e : q.src[r]) ent->push_back(SrcEntry{e.comp, e.i, e.j, e.k, e.coef});
+        }
+        return make_stress_src(*ent, q.p.nx, q.p.ny, q.p.nz, f, plane1);
+    };
+    std::vector<Chain> singles;
+    std::vector<int> tiny[3];
+    for (int i = 0; i < n; ++i) {
+        const Prob &q = b->probs[i];
+        const double cells = (double)q.p.nx * q.p.ny * q.p.nz;
+        Chain c;
+        c.prob = i;
+        if (cells >= APART_FROM && cells < APART_TO) {
+            c.work = cells;
+            for (c.r0 = 0; c.r0 < q.R; ++c.r0) singles.push_back(c);
+            continue;
+        }
+        c.R = q.R;
+        c.work = cells * q.R;
+        std::vector<SrcEntry> ent;
+        int before;
+        bool plane1;
+        StressSrc f;
+        if (cells < MANY_CELLS && q.R == 1 && q.rec_fuse && (fuses(c, &ent, &before, &f, &plane1) || ent.empty()))
+            tiny[scheme(q.p)].push_back((int)singles.size());
+        singles.push_back(c);
+    }
+    std::vector<char> grouped(singles.size(), 0);
+    for (auto &list : tiny) {
+        if ((int)list.size() < MANY_MIN) continue;
+        Chain c;
+        c.prob = singles[list[0]].prob;
+        c.many = list;
+        for (int q : list) {
+            c.work += singles[q].work;
+            grouped[q] = 1;
+        }
+        b->chains.push_back(c);
+    }
+    for (size_t q = 0; q < singles.size(); ++q)
+        if (!grouped[q]) b->chains.push_back(singles[q]);
+    // branches: largest chains first, each to the least loaded branch
+    int share = 1;  // chains that run at the same time
+    for (auto &c : b->chains) c.branch = -1;
+    if (b->own != 0 && b->chains.size() > 1) {
+        std::vector<Chain *> idx;
+        for (auto &c : b->chains)
+            if (b->own > 0 || c.work < BRANCH_CELLS) idx.push_back(&c);
+        std::stable_sort(idx.begin(), idx.end(), [](const Chain *x, const Chain *y) { return x->work > y->work; });
+        int branches = std::min(2, (int)idx.size());
+        double held = 0;
+        for (int k = 0; k < (int)idx.size() && k < ewf_batch::BRANCHES; ++k) {
+            held += idx[k]->work;
+            if (held <= BRANCH_SHARE) branches = std::max(branches, k + 1);
+        }
+        share = std::max(1, branches);
+        double load[ewf_batch::BRANCHES] = {};
+        for (Chain *c : idx) {
+            c->branch = (int)(std::min_element(load, load + branches) - load);
+            load[c->branch] += c->work;
+        }
+    }
+    auto prepare = [&](Chain &c, double together) {
         const Prob &q = b->probs[c.prob];
         const ewf_params &p = q.p;
         const SplitShape shape = split_shape(p.nx, p.ny, p.nz, c.R);
@@ -588,17 +632,13 @@ static int build_tables(ewf_batch *b)
         // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
         // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
         // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
-        c.a.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, c.R * (c.branch >= 0 ? share : 1)).kchunk;
+        c.a.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
         std::vector<SrcEntry> ent;
         int before = 0;
-        for (int r = 0; r < c.r0 + c.R; ++r) {
-            if (r < c.r0) before += (int)q.src[r].size();
-            else
-                for (auto &e : q.src[r]) ent.push_back(SrcEntry{e.comp, e.i, e.j, e.k, e.coef});
-        }
-        c.nsrc = (int)ent.size();
         bool plane1 = false;
-        if (make_stress_src(ent, p.nx, p.ny, p.nz, &c.ss, &plane1)) {
+        const bool fused = fuses(c, &ent, &before, &c.ss, &plane1);
+        c.nsrc = (int)ent.size();
+        if (fused) {
             c.ss.src = q.d_sent + before;
             if (c.R > 1) c.ss.inl = 0;
             // plane 2's thread applies a shear entry on plane 1, so it has to store that plane too
@@ -609,7 +649,42 @@ static int build_tables(ewf_batch *b)
         c.ss.order = p.src_order;
         c.rf = q.rf;
         if (c.rf.grp) c.rf.traces += (size_t)c.r0 * (q.rec.size() / 4) * b->nt;
+    };
+    for (auto &c : b->chains) {
+        if (c.many.empty()) {
+            prepare(c, c.branch >= 0 ? share : 1);
+            continue;
+        }
+        std::vector<ManyProb> mp[2];
+        std::vector<int2> map;
+        const int at = (int)(&c - b->chains.data());
+        for (int q : c.many) {
+            Chain &o = singles[q];
+            prepare(o, c.work / o.work);
+            ManyProb m;
+            m.a = o.a;
+            m.ss = o.ss;
+            m.rf = o.rf;
+            const ewf_params &p = b->probs[o.prob].p;
+            m.ntx = (p.nx + TX - 1) / TX;
+            m.nty = (p.ny + b->ty - 1) / b->ty;
+            const int ctas = m.ntx * m.nty * ((p.nz + o.a.kchunk - 1) / o.a.kchunk);
+            for (int k = 0; k < ctas; ++k) map.push_back(make_int2((int)mp[0].size(), k));
+            for (int par = 0; par < 2; ++par) {
+                m.ss.it_ptr = b->d_it + 2 * at + par;
+                m.rf.it_rd = b->d_it + 2 * at + par;
+                m.rf.it_wr = nullptr;
+                mp[par].push_back(m);
+            }
+        }
+        c.blocks = (int)map.size();
+        for (int par = 0; par < 2; ++par)
+            if (int st = upload(&c.d_many[par], mp[par])) return st;
+        if (int st = upload(&c.d_map, map)) return st;
     }
+    // every chain's counters at the batch's step
+    const std::vector<int> its(2 * b->chains.size(), b->it);
+    CK(cudaMemcpy(b->d_it, its.data(), its.size() * sizeof(int), cudaMemcpyHostToDevice));
     if (nrec) {
         CK(cudaMalloc(&b->d_rec_comp, nrec * sizeof(int)));
         CK(cudaMemcpy(b->d_rec_comp, rc.data(), nrec * sizeof(int), cudaMemcpyHostToDevice));
@@ -629,6 +704,13 @@ static void chain_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream
     const Prob &q = b->probs[c.prob];
     const StepArgs<float> &a = c.a;
     int *const it_rd = b->d_it + 2 * i + parity, *const it_wr = b->d_it + 2 * i + 1 - parity;
+    if (!c.many.empty()) {
+        launch_on(k_stress_many<MODEL, DAMP>, dim3(c.blocks), dim3(TX, b->ty), s, b->pdl && !first, (const ManyProb *)c.d_many[parity],
+                  (const int2 *)c.d_map);
+        launch_on(k_velocity_many<MODEL, DAMP>, dim3(c.blocks), dim3(TX, b->ty), s, b->pdl, (const ManyProb *)c.d_many[parity],
+                  (const int2 *)c.d_map, (const int *)it_rd, it_wr);
+        return;
+    }
     StressSrc ss = c.ss;
     ss.it_ptr = it_rd;
     RecFuse rf = c.rf;
@@ -759,7 +841,7 @@ extern "C" int ewf_batch_reset(ewf_batch *b)
     for (auto &q : b->probs)
         for (auto &x : q.state) z.push_back({x, q.sbox * 4});
     if (b->d_traces) z.push_back({b->d_traces, (size_t)b->nrec_total * b->nt * sizeof(double)});
-    z.push_back({b->d_it, 2 * b->chains.size() * sizeof(int)});
+    z.push_back({b->d_it, 2 * (size_t)b->nrhs_total * sizeof(int)});
     if (int st = zero_buffers(z, b->stream)) return st;
     CK(cudaStreamSynchronize(b->stream));
     b->it = 0;

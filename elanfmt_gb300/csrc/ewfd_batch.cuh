@@ -44,6 +44,41 @@ __global__ void k_binject(const BatchProb<T> *__restrict__ probs, const BatchSrc
     }
 }
 
+// Tiny problems of one scheme in one launch (separate ones would be bound by the launch rate): a CTA looks up its problem and its place in it (map: problem,
+// CTA of the problem) and runs the one-cell update with that problem's arguments, sources and receivers.
+struct ManyProb {
+    StepArgs<float> a;
+    StressSrc ss;
+    RecFuse rf;
+    int ntx, nty;
+};
+template <int MODEL, int DAMP>
+__global__ void __launch_bounds__(split_max_threads<float>(), split_min_ctas<float>()) k_stress_many(const ManyProb *__restrict__ probs,
+                                                                                                    const int2 *__restrict__ map)
+{
+    pdl_trigger();
+    const int2 m = map[blockIdx.x];
+    const ManyProb &p = probs[m.x];
+    const int t = m.y / p.ntx, k0 = (t / p.nty) * p.a.kchunk;
+    stress_column<float, MODEL, DAMP, 1, true>(p.a, (m.y % p.ntx) * TX + threadIdx.x, (t % p.nty) * blockDim.y + threadIdx.y, k0,
+                                               min(k0 + p.a.kchunk, p.a.nz), p.ss);
+}
+template <int MODEL, int DAMP>
+__global__ void __launch_bounds__(split_max_threads<float>(), split_min_ctas<float>())
+    k_velocity_many(const ManyProb *__restrict__ probs, const int2 *__restrict__ map, const int *it_rd, int *it_wr)
+{
+    pdl_trigger();
+    if (blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+        pdl_wait();
+        *it_wr = *it_rd + 1;
+    }
+    const int2 m = map[blockIdx.x];
+    const ManyProb &p = probs[m.x];
+    const int t = m.y / p.ntx, k0 = (t / p.nty) * p.a.kchunk;
+    velocity_column<float, MODEL, DAMP, false, 1, true>(p.a, (m.y % p.ntx) * TX + threadIdx.x, (t % p.nty) * blockDim.y + threadIdx.y, k0,
+                                                        min(k0 + p.a.kchunk, p.a.nz), p.rf);
+}
+
 // Receiver gather of one problem, all its right-hand sides: rows [row0, row0 + nrow) of the traces.
 template <typename T>
 __global__ void k_brecord(const StepArgs<T> a, const long long *__restrict__ rec_off, const int *__restrict__ rec_comp, int row0,

@@ -71,3 +71,29 @@ def test_shared_launches(cuda_device, model, damping, outside, stress_rec):
             np.testing.assert_array_equal(b.seismograms(0, r), ref.traces, err_msg=f"rhs {r}")
             for q in F.STATE:
                 np.testing.assert_array_equal(b.field(0, r, q), ref.f[q], err_msg=f"rhs {r} {F.STATE_NAMES[q]}")
+
+
+@pytest.mark.parametrize("own", [0, 1])
+def test_many_tiny_problems(cuda_device, own):
+    """Problems small and many enough for one launch over all of a scheme's, among others that are not."""
+    nt = 80
+    rng = np.random.default_rng(12)
+    probs = []
+    for q in range(46):
+        shape = tuple(int(v) for v in rng.integers(7, 35, 2)) + (int(rng.integers(4, 14)),)
+        model, kw = ((F.MODEL_ISO, {}), (F.MODEL_ORTHO, {"damping": F.DAMP_SEPARABLE}))[q % 2] if q < 44 else (F.MODEL_ORTHO, {"damping": F.DAMP_W3D})
+        if q % 6 == 0:
+            kw = {**kw, "src_order": F.SRC_AFTER_BC1}
+        # 0: seven entries and two near the surface; some with a source or a receiver for the separate kernels
+        probs.append(_problem(model, shape, nt, 1 if q % 12 else 2, 20 + q, q in (3, 4), q in (4, 7), **kw))
+    with Batch(probs) as b:
+        b.set_launch(own)
+        for n in (1, 2, 67, 10):
+            b.run(n)
+        for p, (m, rhs) in enumerate(probs):
+            for r, (ent, coef) in enumerate(rhs):
+                m.sources, m.source_coef = ent, coef
+                ref = O.run(m, nt)
+                np.testing.assert_array_equal(b.seismograms(p, r), ref.traces, err_msg=f"problem {p} rhs {r}")
+                for q in F.STATE:
+                    np.testing.assert_array_equal(b.field(p, r, q), ref.f[q], err_msg=f"problem {p} rhs {r} {F.STATE_NAMES[q]}")
