@@ -72,14 +72,15 @@ def cubin_path(model: str, variant: str) -> str:
 
 
 def build_ref_cubins(force: bool = False) -> list[str]:
-    """Compile the reference kernels into oracle/_ref/ (no-op where the reference is absent)."""
+    """Compile the reference kernels whose sources are there into oracle/_ref/ (no-op where the reference is absent)."""
     nv = _nvcc()
-    if not nv or not os.path.isdir(REFERENCE_ROOT):
+    present = {model: os.path.join(REFERENCE_ROOT, rel) for model, rel in REF_SOURCES.items()}
+    present = {model: src for model, src in present.items() if os.path.isfile(src)}
+    if not nv or not present:
         return []
     os.makedirs(REF_OUT, exist_ok=True)
     cmds, outs = [], []
-    for model, rel in REF_SOURCES.items():
-        src = os.path.join(REFERENCE_ROOT, rel)
+    for model, src in present.items():
         for variant, fmad in (("stock", "true"), ("exact", "false")):
             out = cubin_path(model, variant)
             outs.append(out)
