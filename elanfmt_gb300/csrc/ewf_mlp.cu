@@ -117,20 +117,19 @@ __device__ __forceinline__ bool elect_one()
     return p != 0;
 }
 __device__ __forceinline__ bool umma_failed() { return *(volatile int *)&g_umma_err != 0; }
-// Bounded wait (`limit` polls: g_umma_wait_limit, which each thread reads once -- read here, it put a global
-// load's latency, 0.4 us, on every k-stage); gives up at once when another wait of the launch has.
+__device__ __forceinline__ bool warp_all(bool x) { return __all_sync(0xffffffffu, x) != 0; }
+// Bounded wait of a whole warp, one answer for all its lanes (warp_wait; `limit` polls: g_umma_wait_limit, which each
+// warp reads once -- read here, it put a global load's latency, 0.4 us, on every k-stage); gives up at once when another
+// wait of the launch has.
 __device__ __noinline__ bool mbar_wait_on(uint64_t *b, uint32_t parity, int limit)
 {
-    for (int i = 0; i < limit; ++i) {
-        if (mbar_try_wait(b, parity)) return true;
-        if ((i & 1023) == 1023 && umma_failed()) break;
-    }
+    if (ewf_umma::warp_wait(limit, [&] { return mbar_try_wait(b, parity); }, umma_failed, warp_all)) return true;
     atomicExch(&g_umma_err, 1);
     return false;
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, int limit)
 {
-    return mbar_try_wait(b, parity) || mbar_wait_on(b, parity, limit);
+    return warp_all(mbar_try_wait(b, parity)) || mbar_wait_on(b, parity, limit);
 }
 // Wait for asynchronous work this thread issued itself (fixed bound: the work always completes).
 __device__ __forceinline__ void mbar_drain(uint64_t *b, uint32_t parity)
@@ -274,8 +273,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const int limit = *(volatile int *)&g_umma_wait_limit;
-    bool ok = true;
+    const int limit = __shfl_sync(0xffffffffu, *(volatile int *)&g_umma_wait_limit, 0);
+    bool ok = true;  // the same in every lane of a warp, as all that the roles' loops go by
     // a dependent launch may start setting up; nothing of an earlier launch is read or written before it has completed
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -303,9 +302,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
             const int r0 = is_b ? (t % tiles_n) * bn : (t / tiles_n) * rows;
             for (int kt = 0; kt < nk; ++kt, ++q) {
                 if (!ready && !mbar_wait(&empty[s], free_parity, limit)) { ok = false; break; }
-                const int s1 = s + 1 == ns ? 0 : s + 1;
-                const uint32_t p1 = s1 ? free_parity : free_parity ^ 1;
-                ready = mbar_test(&empty[s1], p1);
+                int s1;
+                uint32_t p1;
+                U::ring_next(s, free_parity, ns, &s1, &p1);
+                const bool next = mbar_test(&empty[s1], p1);
                 if (elect_one()) {
                     uint8_t *dst = base + s * stage;
                     mbar_expect_tx(&full[s], bytes);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
                         tma_load_2d(dst, map, kt * U::BK, r0, &full[s]);
                     }
                 }
-                __syncwarp();
+                ready = warp_all(next);
                 s = s1;
                 free_parity = p1;
             }
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
     } else if (warp == 1) {  // MMA issuer
         const uint32_t idesc = U::instr_desc_bf16_f32(U::BM, bn, ta, tb);
         const bool first = (t0 / tiles_n) * rows < U::BM && (t0 % tiles_n) * bn < 256;
-        const int hold = first ? *(volatile int *)&g_umma_hold : -1;
+        const int hold = __shfl_sync(0xffffffffu, first ? *(volatile int *)&g_umma_hold : -1, 0);
         // the K = 16 slices of a stage: start addresses (16-byte units) and descriptors without them
         const uint64_t da0 = ta ? U::smem_desc_sw128_mn(0) : U::smem_desc_sw128(0), db0 = tb ? U::smem_desc_sw128_mn(0) : U::smem_desc_sw128(0);
         const int sa = (ta ? U::MN_K_STEP : 32) >> 4, sb = (tb ? U::MN_K_STEP : 32) >> 4;
@@ -341,9 +341,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
             for (int kt = 0; kt < nk; ++kt) {
                 if (!ready && !mbar_wait(&full[s], full_parity, limit)) { ok = false; break; }
                 tc_fence_after();
-                const int s1 = s + 1 == ns ? 0 : s + 1;
-                const uint32_t p1 = s1 ? full_parity : full_parity ^ 1;
-                ready = mbar_test(&full[s1], p1);
+                int s1;
+                uint32_t p1;
+                U::ring_next(s, full_parity, ns, &s1, &p1);
+                const bool next = mbar_test(&full[s1], p1);
                 if (elect_one()) {
                     const uint32_t a0 = smem_u32(smem + s * stage) >> 4, b0 = a0 + (uint32_t)(a_part >> 4);
 #pragma unroll
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
                         umma_bf16(d, da0 + a0 + (uint32_t)(sa * j), db0 + b0 + (uint32_t)(sb * j), idesc, (kt > 0 || j > 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
                 }
-                __syncwarp();
+                ready = warp_all(next);
                 s = s1;
                 full_parity = p1;
             }
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(const __grid_constant_
         for (int t = t0; t < items; t += ctas, ++i) {
             const int m0 = (t / tiles_n) * rows, n0 = (t % tiles_n) * bn;
             const int b = U::acc_buf(i);
-            const bool got = !umma_failed() && mbar_wait(&acc_full[b], U::acc_full_parity(i), limit);
+            const bool got = warp_all(!umma_failed()) && mbar_wait(&acc_full[b], U::acc_full_parity(i), limit);
             tc_fence_after();
             const int mrow = m0 + 32 * quarter, row = mrow + lane;
 #pragma unroll 1

@@ -119,9 +119,29 @@ EWF_UHD int ring_slot(int g, int stages = STAGES) { return g % stages; }
 EWF_UHD uint32_t ring_full_parity(int g, int stages = STAGES) { return (uint32_t)(g / stages) & 1u; }  // consumer of stage g
 EWF_UHD bool ring_needs_free(int g, int stages = STAGES) { return g >= stages; }                       // producer of stage g waits?
 EWF_UHD uint32_t ring_free_parity(int g, int stages = STAGES) { return (uint32_t)(g / stages - 1) & 1u; }  // ... for stage g - stages
+// The slot after `s` in a ring of ns, and the parity of its wait (it toggles each time round).
+EWF_UHD void ring_next(int s, uint32_t parity, int ns, int *s1, uint32_t *p1)
+{
+    *s1 = s + 1 == ns ? 0 : s + 1;
+    *p1 = *s1 ? parity : parity ^ 1u;
+}
 EWF_UHD int acc_buf(int i) { return i & 1; }
 EWF_UHD uint32_t acc_full_parity(int i) { return (uint32_t)(i >> 1) & 1u; }              // epilogue of tile i
 EWF_UHD bool acc_needs_free(int i) { return i >= 2; }                                     // MMAs of tile i wait?
 EWF_UHD uint32_t acc_free_parity(int i) { return (uint32_t)((i >> 1) - 1) & 1u; }        // ... for tile i - 2
+
+// A warp's wait of at most `limit` polls.  Each lane polls for itself and nothing says that two lanes of a poll
+// see the same, so the warp decides together -- vote(x): whether x holds in every lane.  Lanes that each went by their
+// own poll could part as the limit ends, some leaving the role's loop and the others waiting for them there
+// (elect.sync, __syncwarp) for good.
+template <class Poll, class Failed, class Vote>
+EWF_UHD bool warp_wait(int limit, Poll poll, Failed failed, Vote vote)
+{
+    for (int i = 0; i < limit; ++i) {
+        if (vote(poll())) return true;
+        if ((i & 1023) == 1023 && !vote(!failed())) return false;
+    }
+    return false;
+}
 
 }  // namespace ewf_umma
