@@ -1,9 +1,9 @@
 // ewf_umma.h -- operand layout and descriptors of the surrogate's tcgen05 (UMMA) GEMM
-// (host and device code; the host side is exercised by tests/test_umma_layout_cpu.py).
+// (host and device code; the host side is exercised by tests/test_umma_*_cpu.py).
 //
-// One CTA computes a BM x BN tile of C = A . B^T with A [M, K] and B [N, K] both K-major bf16.
-// A k-stage of BK = 64 elements (128 bytes of every operand row) is brought into shared memory
-// by one 2-D TMA copy per operand with the 128-byte swizzle: row r of a stage tile occupies bytes
+// One CTA computes tiles of C = A . B^T, up to BM rows each, from bf16 operands that are stored K-major, A [M, K]
+// and B [N, K], or transposed (below).  Of a K-major operand a k-stage of BK = 64 elements (128 bytes of every operand row) is brought into shared memory
+// by one 2-D TMA copy with the 128-byte swizzle: row r of a stage tile occupies bytes
 // [r * 128, r * 128 + 128) and its 16-byte chunk c sits at chunk c ^ (r % 8).  That is the
 // tensor core's canonical K-major SWIZZLE_128B layout: 8-row atoms of 1024 bytes, one after the
 // other (stride-dimension offset 1024 B), and the k-th MMA of a stage (K = 16, 32 bytes of each
@@ -30,11 +30,11 @@ namespace ewf_umma {
 
 constexpr int BM = 128;          // rows of A per CTA tile (TMEM lanes of the accumulator)
 constexpr int BK = 64;           // K per pipeline stage: 128 bytes per operand row
-constexpr int STAGES = 4;
+constexpr int STAGES = 4;        // slots of the ring of 128-row tiles 256 columns wide; narrower tiles have more
 constexpr int ROW_BYTES = BK * 2;
 constexpr int ATOM_BYTES = 8 * ROW_BYTES;  // 8 rows x 128 B: the swizzle atom, stride-dimension offset
 constexpr int MMA_K = 16;
-constexpr int THREADS = 192;     // warp 0: TMA producer (one lane); warp 1: MMA issuer (one lane); warps 2-5: epilogue
+constexpr int THREADS = 192;     // warp 0: TMA producer of A; warp 1: MMA issuer; warps 2-5: epilogue
 constexpr int MORE_EPILOGUE = 128;  // warps 6-9: a second epilogue warp per TMEM lane quarter (warp 10: the producer of B)
 constexpr int LAYOUT_SW128 = 2;
 
@@ -110,11 +110,12 @@ EWF_UHD uint32_t mma_read_end(uint32_t start, int rows)
 // Phase bookkeeping of the GEMM's mbarriers.  An mbarrier wait with parity P returns once the
 // barrier's current phase has a parity other than P, i.e. once the latest completed phase has
 // parity P; a fresh barrier (phase 0 running) therefore lets a parity-1 wait through at once.
-// Stage ring: the g-th k-stage of a CTA (counted across its tiles) uses slot g % STAGES; its
-// "full" completion is that slot's (g / STAGES)-th, its "empty" completion frees the slot for
-// stage g + STAGES.  Accumulators: the i-th tile of a CTA uses buffer i % 2; "acc_full" completes
+// Stage ring of `stages` slots: the g-th k-stage of a CTA (counted across its tiles) uses slot g % stages; its
+// "full" completion is that slot's (g / stages)-th, its "empty" completion frees the slot for
+// stage g + stages.  Accumulators: the i-th tile of a CTA uses buffer i % 2; "acc_full" completes
 // once per tile in that buffer, "acc_empty" once per drained tile.
-// (STAGES slots unless a kernel's ring has another number, `stages`)
+// The kernel's roles keep a slot and a parity and move on with ring_next; ring_slot and ring_full_parity serve its
+// last waits, and ring_needs_free and ring_free_parity the host model of a single producer.
 EWF_UHD int ring_slot(int g, int stages = STAGES) { return g % stages; }
 EWF_UHD uint32_t ring_full_parity(int g, int stages = STAGES) { return (uint32_t)(g / stages) & 1u; }  // consumer of stage g
 EWF_UHD bool ring_needs_free(int g, int stages = STAGES) { return g >= stages; }                       // producer of stage g waits?

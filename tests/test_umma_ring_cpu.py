@@ -1,5 +1,7 @@
 """The tcgen05 GEMM's waits, host builds of the header that the kernel uses (ewf_umma.h):
-  * umma_warp_wait.cpp: a bounded wait has one answer for all lanes of a warp."""
+  * umma_warp_wait.cpp: a bounded wait has one answer for all lanes of a warp;
+  * umma_ring_sim.cpp: the ring of stages and the accumulators between the producers, the MMA issuer and the epilogue's
+    warps under random interleavings -- no deadlock, nothing refilled, overwritten or read too early."""
 import os
 import shutil
 import subprocess
@@ -18,3 +20,7 @@ def _run(tmp_path, name):
 
 def test_a_wait_has_one_answer_per_warp(tmp_path):
     _run(tmp_path, "umma_warp_wait")
+
+
+def test_ring_protocol(tmp_path):
+    _run(tmp_path, "umma_ring_sim")
