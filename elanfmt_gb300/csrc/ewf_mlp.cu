@@ -131,11 +131,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, int limi
 {
     return warp_all(mbar_try_wait(b, parity)) || mbar_wait_on(b, parity, limit);
 }
-// Wait for asynchronous work this thread issued itself (fixed bound: the work always completes).
 __device__ __forceinline__ void mbar_drain(uint64_t *b, uint32_t parity)
 {
-    for (int i = 0; i < kWaitPolls; ++i)
-        if (mbar_try_wait(b, parity)) return;
+    ewf_umma::bounded_drain([&] { return mbar_test(b, parity); });
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *b, uint32_t bytes)
 {

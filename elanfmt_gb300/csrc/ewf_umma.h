@@ -145,4 +145,15 @@ EWF_UHD bool warp_wait(int limit, Poll poll, Failed failed, Vote vote)
     return false;
 }
 
+// The last wait for copies or MMAs that a role issued itself, before the CTA's memory goes: they land within
+// microseconds, and the polls (which do not suspend the thread) take milliseconds.  A copy's barrier need not complete:
+// where the other operand's producer gave up first, its arrival never comes.
+constexpr int DRAIN_POLLS = 1 << 18;
+template <class Poll>
+EWF_UHD void bounded_drain(Poll poll, int polls = DRAIN_POLLS)
+{
+    for (int i = 0; i < polls; ++i)
+        if (poll()) return;
+}
+
 }  // namespace ewf_umma

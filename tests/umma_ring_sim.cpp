@@ -6,7 +6,9 @@
 // still expects; a wait with parity P passes when n % 2 != P.
 // Checked: the run ends; a slot is refilled only after the stage before in it was consumed; the issuer reads a stage
 // exactly when both operands have landed, and writes an accumulator only after it was drained; an
-// epilogue warp reads a tile exactly when its MMAs are complete.
+// epilogue warp reads a tile exactly when its MMAs are complete.  In half of the runs waits give up at random, as when
+// a limit runs out (the flag they raise makes later ones give up): the roles then still end, each after
+// its own copies and MMAs, within the polls of bounded_drain.
 // Prints "ok <runs>" or the first failure.
 #include <cstdio>
 #include <deque>
@@ -41,9 +43,11 @@ struct Bar {
 };
 
 constexpr int WARPS = 8;
+constexpr int POLLS = 3000;  // of a drain (in the kernel DRAIN_POLLS)
 
 struct Sim {
     int tiles, nk, ns;
+    bool failing, err = false;
     std::mt19937 rng;
     std::vector<Bar> full, empty;
     Bar acc_full[2], acc_empty[2];
@@ -56,7 +60,8 @@ struct Sim {
     struct Producer {
         int op, q = 0, s = 0;
         uint32_t parity = 1;
-        bool ready = true, done = false;
+        bool ready = true, done = false, drained = false;
+        int at = -1, polls = 0;  // the stage whose copy it drains, and the polls so far
     } prod[2];
     struct Issuer {
         int i = 0, kt = 0, s = 0, g = 0;
@@ -65,7 +70,14 @@ struct Sim {
     } mma;
     int epi[WARPS] = {};
 
-    Sim(int tiles_, int nk_, int ns_, unsigned seed) : tiles(tiles_), nk(nk_), ns(ns_), rng(seed), full(ns_), empty(ns_), consumed(ns_, 0)
+    // a wait that has not passed: whether it gives up
+    bool gives_up()
+    {
+        if (failing && (err || rng() % 40 == 0)) err = true;
+        return err;
+    }
+
+    Sim(int tiles_, int nk_, int ns_, bool failing_, unsigned seed) : tiles(tiles_), nk(nk_), ns(ns_), failing(failing_), rng(seed), full(ns_), empty(ns_), consumed(ns_, 0)
     {
         for (auto &b : full) b.need = 2;
         for (auto &b : acc_empty) b.need = WARPS;
@@ -78,8 +90,11 @@ struct Sim {
 
     bool produce(Producer &p)
     {
-        if (p.done) return false;
-        if (!p.ready && !empty[p.s].pass(p.parity)) return false;
+        if (p.done) return last_copies(p);
+        if (!p.ready && !empty[p.s].pass(p.parity)) {
+            p.done = gives_up();
+            return p.done;
+        }
         int s1;
         uint32_t p1;
         ring_next(p.s, p.parity, ns, &s1, &p1);
@@ -93,17 +108,40 @@ struct Sim {
         if (++p.q == tiles * nk) p.done = true;
         return true;
     }
+    // the kernel's loop over the last ns stages, bounded_drain on each, a poll at a time
+    bool last_copies(Producer &p)
+    {
+        if (p.drained) return false;
+        if (p.at < 0) p.at = p.q > ns ? p.q - ns : 0;
+        if (p.at == p.q) {
+            p.drained = true;
+            for (const auto &c : flying)
+                if (c.first == p.op) bad = "a producer ends before its copies landed";
+            return true;
+        }
+        if (full[ring_slot(p.at, ns)].pass(ring_full_parity(p.at, ns)) || ++p.polls == POLLS) {
+            ++p.at;
+            p.polls = 0;
+        }
+        return true;
+    }
     bool issue()
     {
         Issuer &m = mma;
         if (m.done) return false;
         if (!m.open) {
             const int b = acc_buf(m.i);
-            if (acc_needs_free(m.i) && !acc_empty[b].pass(acc_free_parity(m.i))) return false;
-            if (drained[b] != m.i / 2) bad = "an accumulator is written before it was drained";
+            if (acc_needs_free(m.i) && !acc_empty[b].pass(acc_free_parity(m.i))) {
+                m.done = gives_up();
+                return m.done;
+            }
+            if (!err && drained[b] != m.i / 2) bad = "an accumulator is written before it was drained";
             m.open = true;
         }
-        if (!m.ready && !full[m.s].pass(m.parity)) return false;
+        if (!m.ready && !full[m.s].pass(m.parity)) {
+            m.done = gives_up();
+            return m.done;
+        }
         int s1;
         uint32_t p1;
         ring_next(m.s, m.parity, ns, &s1, &p1);
@@ -126,8 +164,10 @@ struct Sim {
     bool drain(int w)
     {
         const int i = epi[w], b = acc_buf(i);
-        if (i == tiles || !acc_full[b].pass(acc_full_parity(i))) return false;
-        if (computed[b] != i / 2 + 1) bad = "an accumulator is read before its MMAs completed";
+        if (i == tiles) return false;
+        const bool got = acc_full[b].pass(acc_full_parity(i));
+        if (!got && !gives_up()) return false;
+        if (!err && computed[b] != i / 2 + 1) bad = "an accumulator is read before its MMAs completed";
         ++epi[w];
         const int before = acc_empty[b].n;
         acc_empty[b].arrive();
@@ -162,7 +202,7 @@ struct Sim {
     {
         for (int w = 0; w < WARPS; ++w)
             if (epi[w] != tiles) return false;
-        return prod[0].done && prod[1].done && mma.done && flying.empty() && commits.empty();
+        return prod[0].drained && prod[1].drained && mma.done && flying.empty() && commits.empty();
     }
     const char *run()
     {
@@ -184,10 +224,12 @@ int main()
 {
     int runs = 0;
     unsigned seed = 1;
+    for (int rep = 0; rep < 2; ++rep)
     for (int ns = 4; ns <= 16; ++ns)
         for (int tiles = 1; tiles <= 5; ++tiles)
             for (int nk : {1, 2, 3, 4, 5, 8, 15, 16, 17, 33}) {
-                const char *e = Sim(tiles, nk, ns, seed++).run();
+                const bool failing = seed & 1;
+                const char *e = Sim(tiles, nk, ns, failing, seed++).run();
                 if (e) {
                     printf("FAIL %s: slots %d tiles %d nk %d seed %u\n", e, ns, tiles, nk, seed - 1);
                     return 1;
