@@ -10,6 +10,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "ewfd.h"
 #include "ewfd_internal.h"
 
@@ -39,8 +42,8 @@ int make_sos(const double *sos, int32_t nsec, Sos *out)
     return EWF_OK;
 }
 
-// one trace in place (the host path)
-void filter_trace(const Sos &q, double *x, int64_t n)
+// one trace in place: the host path, and a device thread of k_sosfilt_trace
+__host__ __device__ inline void filter_trace(const Sos &q, double *x, int64_t n)
 {
     double s1[MAXSEC], s2[MAXSEC];
     for (int s = 0; s < q.n; ++s) s1[s] = s2[s] = 0.0;
@@ -163,9 +166,34 @@ __global__ void __launch_bounds__(64) k_sosfilt(const Sos q, double *__restrict_
     }
 }
 
+// A thread per trace: its latency is that of all the sections' instructions in a row, but every lane of a warp issues for
+// a trace of its own, whatever the number of sections.
+__global__ void __launch_bounds__(64) k_sosfilt_trace(const Sos q, double *x, int64_t ntr, int64_t n)
+{
+    const int64_t tr = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tr < ntr) filter_trace(q, x + tr * n, n);
+}
+
+// Which of the two is faster, by their measured times: a pair of warps takes 0.21 us per sample alone and 0.095 (one
+// section 0.14) times the pairs per SM when there are many, over the samples and two phases per section; a thread
+// 0.2 us and 0.315 per section, and 0.15 and 1.8e-5 times the traces per section when there are many.  ms by pairs and by threads:
+//   192 x 4000, 4 sections 0.86 and 5.9     4864 x 2000, 5 sections 2.1 and 3.7     9728 x 1000, 9 sections 3.8 and 3.0
+//   20000 x 1000: 4 sections 1.7 and 2.1, 5 sections 3.4 and 2.6     40000 x 500, 8 sections 4.1 and 3.4     1e6 x 16, 4 sections 4.5 and 1.1
+bool trace_per_thread(int nsec, int lanes, double ntr, double n)
+{
+    const double pairs = ntr * lanes / 32, len = U * (std::ceil(n / U) + 2 * nsec);
+    const double by_pairs = len * std::max(0.212, (lanes == 1 ? 0.14 : 0.095) * pairs / 152);
+    const double by_threads = n * std::max(0.2 + 0.315 * nsec, nsec * (0.15 + 1.78e-5 * ntr));
+    return by_threads < by_pairs;
+}
+
 template <int G>
 void launch_sosfilt(const Sos &q, double *x, int64_t ntr, int64_t n, cudaStream_t stream)
 {
+    if (trace_per_thread(q.n, G, (double)ntr, (double)n)) {
+        k_sosfilt_trace<<<(unsigned)((ntr + 63) / 64), 64, 0, stream>>>(q, x, ntr, n);
+        return;
+    }
     k_sosfilt<G><<<(unsigned)((ntr * G + 31) / 32), 64, 0, stream>>>(q, x, ntr, n);
 }
 

@@ -14,7 +14,7 @@ samples of a trace into a zero signal of 150000 samples and runs `sosfilt(sos, s
   into the first section, and sections are ordered by increasing pole radius, so the poles
   nearest the unit circle are applied last.
 * The recursion itself runs in libewfd.so (`ewf_sosfilt` on host arrays, `ewf_sosfilt_device` on
-  device arrays, the sections of a trace on lanes of a warp pair): direct form II transposed sections from zero state.
+  device arrays, the sections of a trace on lanes of a warp pair or, with many traces, a thread per trace): direct form II transposed sections from zero state.
 
 The driver's comparison against frequency-wavenumber synthetics (Zhu's third-party `fk`, which
 the reference does not ship) is not reproduced: parity of that overlay is unpinned.

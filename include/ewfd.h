@@ -317,7 +317,7 @@ int ewf_pack_field_noalloc(void *dst, int32_t dst_dtype_bytes, int32_t sx, int64
  * (src/FastWaveED_GPU3D_v1_DC_Earthquake_FULL_OK4_final/vizme_FastBiotED_GPU3D_OK_2024_final.m
  * :551-558, 579-582, 604-607).  sos: nsec rows of (b0 b1 b2 a0 a1 a2) as MATLAB and scipy lay
  * them out; each section is the direct form II transposed recursion from zero state.
- * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (a section of a trace per lane,
+ * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (a section of a trace per lane, or a trace per thread when there are many,
  * on `stream`), with the same bits. */
 #define EWF_SOS_MAX_SECTIONS 16
 int ewf_sosfilt(const double *sos, int32_t nsec, double *x, int64_t ntr, int64_t n);
