@@ -958,11 +958,20 @@ bool make_stress_src(const std::vector<SrcEntry> &v, int nx, int ny, int nz, Str
 }
 
 // The velocity kernel's receiver tables (RecFuse), when every receiver is a velocity component on a cell
-// its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz) and the plane offsets stay below 64 MB.
+// its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz), there are few of them and the plane offsets stay below 64 MB.
+// With many, what counts is their scattered trace samples, and the recording kernel, whose tables are the list
+// itself, is as fast or faster.  us a step and ms to set them, sampled by the velocity kernel and by k_record:
+//   iso 40 x 40 x 32, 1521 receivers 6.6 0.6, 7.4 0.6     128^3, 4096 on a plane 32.3 1.1, 34.1 1.0     128^3, 16129 43.9 1.4, 44.4 1.1
+//   300 x 300 x 64, two planes: 11250 115.2 2.0, 112.6 1.3     45000 162.5 4.8, 156.1 1.5     178802 332.9 14.9, 314.0 2.3
 RecTables make_rec_tables(int n, const int32_t *ijkc, int nx, int ny, int nz)
 {
     constexpr size_t MAX_OFFSETS = (size_t)1 << 24;
+    constexpr int FUSE_MAX = 8192;
     RecTables t;
+    if (n > FUSE_MAX) {
+        t.fuse = false;
+        return t;
+    }
     std::vector<int> order((size_t)n);
     for (int r = 0; r < n; ++r) {
         const int i = ijkc[4 * r], j = ijkc[4 * r + 1], k = ijkc[4 * r + 2], c = ijkc[4 * r + 3];
@@ -1213,7 +1222,8 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
     if (!pair) launch_on(k_velocity<T, MODEL, DAMP, KAHAN>, grd, blk, h->stream, pdl, a, rf);
     if (ev) cudaEventRecord(ev[3], h->stream);
     if (!h->rec_fuse)
-        launch_on(k_record<T>, dim3(1), dim3(256), h->stream, pdl, a, (const long long *)h->d_rec_off,
+        // (several CTAs: the counter's two locations differ here.  420 x 420 x 110 with 351122 receivers 1946 us a step with one, 760)
+        launch_on(k_record<T>, dim3(std::max(1, std::min((h->nrec + 255) / 256, 1024))), dim3(256), h->stream, pdl, a, (const long long *)h->d_rec_off,
                   (const int *)h->d_rec_comp, h->nrec, h->d_traces, (int)h->p.nt, (const int *)it_rd, it_wr);
     if (ev) cudaEventRecord(ev[4], h->stream);
 }

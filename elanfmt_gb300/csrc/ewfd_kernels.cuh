@@ -816,6 +816,7 @@ __global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k
 // it_rd + 1: the same location for the one-pass and wavefront forms, the other of the two
 // parity locations for the two-kernel step).
 // ---------------------------------------------------------------------------------------------
+// (more than one CTA only where it_wr is another location than it_rd)
 template <typename T>
 __global__ void k_record(const StepArgs<T> a, const long long *__restrict__ rec_off, const int *__restrict__ rec_comp,
                          int nrec, double *__restrict__ traces, int trace_len, const int *it_rd, int *it_wr)
@@ -824,10 +825,10 @@ __global__ void k_record(const StepArgs<T> a, const long long *__restrict__ rec_
     pdl_wait();
     const int it = *it_rd;
     if (it >= 0 && it < trace_len)
-        for (int r = threadIdx.x; r < nrec; r += blockDim.x)
+        for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrec; r += gridDim.x * blockDim.x)
             traces[(long long)r * trace_len + it] = (double)a.f[rec_comp[r]][rec_off[r]];
     __syncthreads();
-    if (threadIdx.x == 0) *it_wr = it + 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *it_wr = it + 1;
 }
 
 // ---------------------------------------------------------------------------------------------
