@@ -1035,6 +1035,9 @@ extern "C" int ewf_set_sources(ewf_handle *h, int32_t n, const int32_t *cijk, co
     if (n > h->nsrc || !h->d_src) {
         cudaFree(h->d_src);
         h->d_src = nullptr;
+        h->nsrc = 0;  // no sources, should the allocation fail
+        h->src_fuse = StressSrc{};
+        h->graph_dirty = true;
         if (n > 0) CK(cudaMalloc(&h->d_src, (size_t)n * sizeof(SrcEntry)));
     }
     if (n > 0) CK(cudaMemcpy(h->d_src, v.data(), (size_t)n * sizeof(SrcEntry), cudaMemcpyHostToDevice));
@@ -1084,6 +1087,57 @@ extern "C" int ewf_set_moment_tensor(ewf_handle *h, const double mt[6], int32_t 
     return ewf_set_sources(h, n, cijk, coef);
 }
 
+// No receivers: nothing that a step reads points at freed memory, whatever fails after it.
+static void drop_receivers(ewf_handle *h)
+{
+    for (void *x : {(void *)h->d_rec_off, (void *)h->d_rec_comp, (void *)h->d_traces, (void *)h->d_rgrp, (void *)h->d_roff, (void *)h->d_rent})
+        cudaFree(x);
+    h->d_rec_off = nullptr;
+    h->d_rec_comp = nullptr;
+    h->d_traces = nullptr;
+    h->d_rgrp = nullptr;
+    h->d_roff = nullptr;
+    h->d_rent = nullptr;
+    h->nrec = 0;
+    h->h_rec.clear();
+    h->rec_kmin = INT32_MAX;
+    h->rec_kmax = -1;
+    h->rec_fuse = true;
+    h->graph_dirty = true;
+}
+
+template <typename T>
+static int upload(T **dst, const std::vector<T> &v)
+{
+    CK(cudaMalloc(dst, v.size() * sizeof(T)));
+    CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    return EWF_OK;
+}
+
+static int place_receivers(ewf_handle *h, int n, const int32_t *ijkc, const std::vector<long long> &off, const std::vector<int> &comp)
+{
+    int st = upload(&h->d_rec_off, off);
+    if (!st) st = upload(&h->d_rec_comp, comp);
+    if (st) return st;
+    CK(cudaMalloc(&h->d_traces, (size_t)n * h->p.nt * sizeof(double)));
+    CK(cudaMemset(h->d_traces, 0, (size_t)n * h->p.nt * sizeof(double)));
+    // the two-kernel step's velocity kernel samples the receivers itself when every one is a
+    // velocity component on a cell its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz)
+    const RecTables t = make_rec_tables(n, ijkc, h->p.nx, h->p.ny, h->p.nz);
+    if (t.fuse) {
+        st = upload(&h->d_rgrp, t.grp);
+        if (!st) st = upload(&h->d_roff, t.off);
+        if (!st) st = upload(&h->d_rent, t.ent);
+        if (st) return st;
+    }
+    h->nrec = n;
+    h->h_rec.assign(ijkc, ijkc + 4 * (size_t)n);
+    h->rec_kmin = t.kmin;
+    h->rec_kmax = t.kmax;
+    h->rec_fuse = t.fuse;
+    return EWF_OK;
+}
+
 extern "C" int ewf_set_receivers(ewf_handle *h, int32_t n, const int32_t *ijkc)
 {
     if (!h || n < 0 || (n > 0 && !ijkc)) return ewf_fail(EWF_ERR_ARG, "bad receiver list");
@@ -1100,45 +1154,13 @@ extern "C" int ewf_set_receivers(ewf_handle *h, int32_t n, const int32_t *ijkc)
         comp[r] = c;
     }
     CK(cudaStreamSynchronize(h->stream));
-    cudaFree(h->d_rec_off);
-    cudaFree(h->d_rec_comp);
-    cudaFree(h->d_traces);
-    h->d_rec_off = nullptr;
-    h->d_rec_comp = nullptr;
-    h->d_traces = nullptr;
-    h->nrec = 0;
-    if (n > 0) {
-        CK(cudaMalloc(&h->d_rec_off, (size_t)n * sizeof(long long)));
-        CK(cudaMalloc(&h->d_rec_comp, (size_t)n * sizeof(int)));
-        CK(cudaMalloc(&h->d_traces, (size_t)n * h->p.nt * sizeof(double)));
-        CK(cudaMemcpy(h->d_rec_off, off.data(), (size_t)n * sizeof(long long), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->d_rec_comp, comp.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMemset(h->d_traces, 0, (size_t)n * h->p.nt * sizeof(double)));
+    drop_receivers(h);
+    const int st = n > 0 ? place_receivers(h, n, ijkc, off, comp) : EWF_OK;
+    if (st) {
+        cudaGetLastError();  // a failed allocation is reported here and not by the next run
+        drop_receivers(h);
     }
-    h->nrec = n;
-    h->h_rec.assign(ijkc, ijkc + 4 * (size_t)n);
-    h->graph_dirty = true;
-    // the two-kernel step's velocity kernel samples the receivers itself when every one is a
-    // velocity component on a cell its threads visit (1 <= i < nx, 1 <= j < ny, 1 <= k < nz)
-    cudaFree(h->d_rgrp);
-    cudaFree(h->d_roff);
-    cudaFree(h->d_rent);
-    h->d_rgrp = nullptr;
-    h->d_roff = nullptr;
-    h->d_rent = nullptr;
-    const RecTables t = make_rec_tables(n, ijkc, h->p.nx, h->p.ny, h->p.nz);
-    if (t.fuse && n > 0) {
-        CK(cudaMalloc(&h->d_rgrp, t.grp.size() * sizeof(uint2)));
-        CK(cudaMalloc(&h->d_roff, t.off.size() * sizeof(int)));
-        CK(cudaMalloc(&h->d_rent, t.ent.size() * sizeof(int2)));
-        CK(cudaMemcpy(h->d_rgrp, t.grp.data(), t.grp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->d_roff, t.off.data(), t.off.size() * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(h->d_rent, t.ent.data(), t.ent.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    }
-    h->rec_kmin = t.kmin;
-    h->rec_kmax = t.kmax;
-    h->rec_fuse = t.fuse;
-    return EWF_OK;
+    return st;
 }
 
 extern "C" int ewf_receiver_count(const ewf_handle *h, int32_t *n)
