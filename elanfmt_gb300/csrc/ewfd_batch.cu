@@ -46,18 +46,46 @@ struct Prob {
     bool m_set[12] = {};
     bool w_set[4] = {};
     int kchunk = 0;                         // planes per CTA (0: by size, split_shape)
-    SrcEntry *d_sent = nullptr;             // source entries, right-hand side by right-hand side
-    int *d_sstart = nullptr;                // first entry of each right-hand side, R + 1
+    const SrcEntry *d_sent = nullptr;       // source entries, right-hand side by right-hand side
+    const int *d_sstart = nullptr;          // first entry of each right-hand side, R + 1
     int group0 = 0;                         // the problem's first (problem, RHS) group of k_binject
     RecFuse rf{};                           // receivers in the velocity kernel
     bool rec_fuse = true;
-    uint2 *d_rgrp = nullptr;
-    int *d_roff = nullptr;
-    int2 *d_rent = nullptr;
     bool fdiv = false;                      // div_spacing verified for dx, dy, dz
     std::vector<int32_t> rec;               // n x (i,j,k,comp)
     std::vector<std::vector<BatchSrc>> src;  // per RHS
     std::vector<double> stf;
+};
+
+// Tables for the device, gathered on the host: one allocation and one copy for all of them (one each took the host
+// 42 us a problem: 8 ms for 200 problems of 16^3, which take 45 us a step).
+struct Tables {
+    std::vector<unsigned char> h;
+    unsigned char *d = nullptr;
+    template <typename T>
+    size_t add(const std::vector<T> &v)  // its place, for at()
+    {
+        const size_t at = (h.size() + 255) / 256 * 256;
+        h.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) memcpy(h.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+    int send()
+    {
+        if (h.empty()) return EWF_OK;
+        CK(cudaMalloc(&d, h.size()));
+        CK(cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice));
+        h = std::vector<unsigned char>();
+        return EWF_OK;
+    }
+    template <typename T>
+    const T *at(size_t place) const { return reinterpret_cast<const T *>(d + place); }
+    void free()
+    {
+        cudaFree(d);
+        d = nullptr;
+        h.clear();
+    }
 };
 
 // What one sequence of launches advances: right-hand sides [r0, r0 + R) of a problem
@@ -73,8 +101,8 @@ struct Chain {
     RecFuse rf{};
     double work = 0;          // cells
     std::vector<int> many;    // the chains of tiny problems it stands for (k_stress_many), and for each step parity
-    ManyProb *d_many[2] = {nullptr, nullptr};  // their arguments,
-    int2 *d_map = nullptr;    // and the problem of each CTA
+    const ManyProb *d_many[2] = {nullptr, nullptr};  // their arguments,
+    const int2 *d_map = nullptr;  // and the problem of each CTA
     int blocks = 0;
 };
 
@@ -99,18 +127,19 @@ struct ewf_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<Prob> probs;
     std::vector<Chain> chains;
-    BatchProb<float> *d_all = nullptr;  // every problem, indexed by problem id
+    Tables tables, many_tables;          // what the pointers below and those of the problems and chains point into
+    const BatchProb<float> *d_all = nullptr;  // every problem, indexed by problem id
     std::vector<BatchProb<float>> h_all;  // host copy of d_all
     int nrhs_total = 0;
     // sources
-    BatchSrc *d_src = nullptr;
-    int *d_src_start = nullptr;
-    double *d_stf = nullptr;
-    int *d_stf_off = nullptr;
-    int *d_order = nullptr;
+    const BatchSrc *d_src = nullptr;
+    const int *d_src_start = nullptr;
+    const double *d_stf = nullptr;
+    const int *d_stf_off = nullptr;
+    const int *d_order = nullptr;
     // receivers
-    long long *d_rec_off = nullptr;
-    int *d_rec_comp = nullptr;
+    const long long *d_rec_off = nullptr;
+    const int *d_rec_comp = nullptr;
     int nrec_total = 0;
     std::vector<int> rec_base;  // per problem: first trace row
     double *d_traces = nullptr;
@@ -133,25 +162,9 @@ struct ewf_batch {
 
 static void free_tables(ewf_batch *b)
 {
-    for (auto &q : b->probs) {
-        for (void *x : {(void *)q.d_sent, (void *)q.d_sstart, (void *)q.d_rgrp, (void *)q.d_roff, (void *)q.d_rent}) cudaFree(x);
-        q.d_sent = nullptr;
-        q.d_sstart = nullptr;
-        q.d_rgrp = nullptr;
-        q.d_roff = nullptr;
-        q.d_rent = nullptr;
-    }
-    for (auto &c : b->chains)
-        for (void *x : {(void *)c.d_many[0], (void *)c.d_many[1], (void *)c.d_map}) cudaFree(x);
     b->chains.clear();
-    cudaFree(b->d_all); b->d_all = nullptr;
-    cudaFree(b->d_src); b->d_src = nullptr;
-    cudaFree(b->d_src_start); b->d_src_start = nullptr;
-    cudaFree(b->d_stf); b->d_stf = nullptr;
-    cudaFree(b->d_stf_off); b->d_stf_off = nullptr;
-    cudaFree(b->d_order); b->d_order = nullptr;
-    cudaFree(b->d_rec_off); b->d_rec_off = nullptr;
-    cudaFree(b->d_rec_comp); b->d_rec_comp = nullptr;
+    b->tables.free();
+    b->many_tables.free();
     for (cudaGraphExec_t *x : {&b->gexec, &b->gexec_short}) {
         if (*x) cudaGraphExecDestroy(*x);
         *x = nullptr;
@@ -402,14 +415,6 @@ extern "C" int ewf_batch_set_receivers(ewf_batch *b, int32_t prob, int32_t n, co
     return EWF_OK;
 }
 
-template <typename T>
-static int upload(T **dst, const std::vector<T> &v)
-{
-    CK(cudaMalloc(dst, v.size() * sizeof(T)));
-    CK(cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-    return EWF_OK;
-}
-
 // Chains below BRANCH_CELLS cells share the GPU on parallel branches; a larger one
 // fills it, and alone keeps its fields in L2.  us per step of six problems n^3, one after another and on
 // four branches:
@@ -462,7 +467,12 @@ static int build_tables(ewf_batch *b)
         d.smu_on = p.surface_mu > 0.0 ? 1 : 0;
         d.smu = (float)p.surface_mu;
     }
-    CK(cudaMalloc(&b->d_all, n * sizeof(BatchProb<float>)));
+    Tables &tab = b->tables;
+    struct Places {
+        size_t ent, from, grp, off, rent;
+    };
+    std::vector<Places> at(n);
+    const size_t at_all = tab.add(all);
     // sources grouped by (problem, rhs)
     std::vector<BatchSrc> src;
     std::vector<int> start;
@@ -483,46 +493,31 @@ static int build_tables(ewf_batch *b)
             if (!q.src[r].empty() && q.stf.empty()) return ewf_fail(EWF_ERR_STATE, "problem %d has sources but no Src", i);
         }
         from.push_back((int)ent.size());
-        if (!ent.empty()) {
-            if (int st = upload(&q.d_sent, ent)) return st;
-            if (int st = upload(&q.d_sstart, from)) return st;
-        }
+        at[i].ent = tab.add(ent);
+        at[i].from = tab.add(from);
         stf_off[i] = i * b->nt;
         if (!q.stf.empty()) std::copy(q.stf.begin(), q.stf.end(), stf.begin() + (size_t)i * b->nt);
         order[i] = q.p.src_order;
     }
     start.push_back((int)src.size());
     b->h_all = all;
-    CK(cudaMemcpy(b->d_all, all.data(), n * sizeof(BatchProb<float>), cudaMemcpyHostToDevice));
-    if (!src.empty()) {
-        CK(cudaMalloc(&b->d_src, src.size() * sizeof(BatchSrc)));
-        CK(cudaMemcpy(b->d_src, src.data(), src.size() * sizeof(BatchSrc), cudaMemcpyHostToDevice));
-    }
-    CK(cudaMalloc(&b->d_src_start, start.size() * sizeof(int)));
-    CK(cudaMemcpy(b->d_src_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&b->d_stf, stf.size() * sizeof(double)));
-    CK(cudaMemcpy(b->d_stf, stf.data(), stf.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&b->d_stf_off, n * sizeof(int)));
-    CK(cudaMemcpy(b->d_stf_off, stf_off.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&b->d_order, n * sizeof(int)));
-    CK(cudaMemcpy(b->d_order, order.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    const size_t at_src = tab.add(src), at_start = tab.add(start), at_stf = tab.add(stf), at_stf_off = tab.add(stf_off), at_order = tab.add(order);
     // receivers: per problem, RHS-major
-    std::vector<int> rp, rc;
+    std::vector<int> rc;
     std::vector<long long> ro;
     b->rec_base.assign(n, 0);
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
-        b->rec_base[i] = (int)rp.size();
+        b->rec_base[i] = (int)rc.size();
         const int nr = (int)q.rec.size() / 4;
         for (int r = 0; r < q.R; ++r)
             for (int e = 0; e < nr; ++e) {
-                rp.push_back(i);
                 rc.push_back(q.rec[4 * e + 3]);
                 ro.push_back((long long)q.rec[4 * e] + (long long)q.rec[4 * e + 1] * q.sx +
                              (long long)q.rec[4 * e + 2] * q.sy + (long long)r * (long long)q.box);
             }
     }
-    const int nrec = (int)rp.size();
+    const int nrec = (int)rc.size();
     if (nrec != b->nrec_total || !b->d_traces) {
         cudaFree(b->d_traces);
         b->d_traces = nullptr;
@@ -532,23 +527,40 @@ static int build_tables(ewf_batch *b)
         }
     }
     b->nrec_total = nrec;
+    const size_t at_rec_off = tab.add(ro), at_rec_comp = tab.add(rc);
     for (int i = 0; i < n; ++i) {
         Prob &q = b->probs[i];
         const RecTables t = make_rec_tables((int)q.rec.size() / 4, q.rec.data(), q.p.nx, q.p.ny, q.p.nz);
         q.rec_fuse = t.fuse;
         q.rf = RecFuse{};
+        at[i].grp = tab.add(t.grp);
+        at[i].off = tab.add(t.off);
+        at[i].rent = tab.add(t.ent);
         if (t.fuse && !t.ent.empty()) {
-            if (int st = upload(&q.d_rgrp, t.grp)) return st;
-            if (int st = upload(&q.d_roff, t.off)) return st;
-            if (int st = upload(&q.d_rent, t.ent)) return st;
-            q.rf.grp = q.d_rgrp;
-            q.rf.off = q.d_roff;
-            q.rf.ent = q.d_rent;
             q.rf.ngx = (q.p.nx + 31) / 32;
             q.rf.kmin = t.kmin;
             q.rf.kmax = t.kmax;
             q.rf.traces = b->d_traces + (size_t)b->rec_base[i] * b->nt;
             q.rf.trace_len = b->nt;
+        }
+    }
+    if (int st = tab.send()) return st;
+    b->d_all = tab.at<BatchProb<float>>(at_all);
+    b->d_src = tab.at<BatchSrc>(at_src);
+    b->d_src_start = tab.at<int>(at_start);
+    b->d_stf = tab.at<double>(at_stf);
+    b->d_stf_off = tab.at<int>(at_stf_off);
+    b->d_order = tab.at<int>(at_order);
+    b->d_rec_off = tab.at<long long>(at_rec_off);
+    b->d_rec_comp = tab.at<int>(at_rec_comp);
+    for (int i = 0; i < n; ++i) {
+        Prob &q = b->probs[i];
+        q.d_sent = tab.at<SrcEntry>(at[i].ent);
+        q.d_sstart = tab.at<int>(at[i].from);
+        if (q.rf.traces) {
+            q.rf.grp = tab.at<uint2>(at[i].grp);
+            q.rf.off = tab.at<int>(at[i].off);
+            q.rf.ent = tab.at<int2>(at[i].rent);
         }
     }
     // the chains, and which of them are tiny problems whose launches take sources and receivers
@@ -650,6 +662,11 @@ static int build_tables(ewf_batch *b)
         c.rf = q.rf;
         if (c.rf.grp) c.rf.traces += (size_t)c.r0 * (q.rec.size() / 4) * b->nt;
     };
+    struct ManyPlaces {
+        Chain *c;
+        size_t many[2], map;
+    };
+    std::vector<ManyPlaces> many_at;
     for (auto &c : b->chains) {
         if (c.many.empty()) {
             prepare(c, c.branch >= 0 ? share : 1);
@@ -678,19 +695,16 @@ static int build_tables(ewf_batch *b)
             }
         }
         c.blocks = (int)map.size();
-        for (int par = 0; par < 2; ++par)
-            if (int st = upload(&c.d_many[par], mp[par])) return st;
-        if (int st = upload(&c.d_map, map)) return st;
+        many_at.push_back({&c, {b->many_tables.add(mp[0]), b->many_tables.add(mp[1])}, b->many_tables.add(map)});
+    }
+    if (int st = b->many_tables.send()) return st;
+    for (auto &m : many_at) {
+        for (int par = 0; par < 2; ++par) m.c->d_many[par] = b->many_tables.at<ManyProb>(m.many[par]);
+        m.c->d_map = b->many_tables.at<int2>(m.map);
     }
     // every chain's counters at the batch's step
     const std::vector<int> its(2 * b->chains.size(), b->it);
     CK(cudaMemcpy(b->d_it, its.data(), its.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (nrec) {
-        CK(cudaMalloc(&b->d_rec_comp, nrec * sizeof(int)));
-        CK(cudaMemcpy(b->d_rec_comp, rc.data(), nrec * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&b->d_rec_off, nrec * sizeof(long long)));
-        CK(cudaMemcpy(b->d_rec_off, ro.data(), nrec * sizeof(long long), cudaMemcpyHostToDevice));
-    }
     b->dirty = false;
     return EWF_OK;
 }
