@@ -157,12 +157,14 @@ struct ewf_batch {
     cudaEvent_t fork_ev = nullptr, join_ev[BRANCHES] = {};
     cudaGraphExec_t gexec = nullptr, gexec_short = nullptr;  // of gsteps and of SHORT_GRAPH steps
     int gsteps = 64;     // steps per graph (even: the step counters alternate between two locations)
+    long long ran = 0;   // steps run since the tables were made
     float last_ms = 0.f;
 };
 
 static void free_tables(ewf_batch *b)
 {
     b->chains.clear();
+    b->ran = 0;
     b->tables.free();
     b->many_tables.free();
     for (cudaGraphExec_t *x : {&b->gexec, &b->gexec_short}) {
@@ -825,13 +827,24 @@ static int ready_graph(ewf_batch *b, int steps, cudaGraphExec_t *exec)
     return st;
 }
 
-// The steps a long graph leaves over go in graphs of SHORT_GRAPH steps where the chains are small on average
-// (SHORT_CELLS): launched one by one, a step of n chains takes the host some 5 n us.
-static int short_graph(const ewf_batch *b)
+// Steps go in graphs of SHORT_GRAPH steps where the chains are small on average (SHORT_CELLS): launched one by one, a
+// step of n chains takes the host some 5 n us.  Larger chains hide that.
+static double chain_cells(const ewf_batch *b)
 {
     double cells = 0;
     for (auto &c : b->chains) cells += c.work;
-    return cells < SHORT_CELLS * b->chains.size() && SHORT_GRAPH < b->gsteps ? SHORT_GRAPH : 0;
+    return cells / std::max<size_t>(1, b->chains.size());
+}
+static int short_graph(const ewf_batch *b) { return chain_cells(b) < SHORT_CELLS ? std::min(SHORT_GRAPH, b->gsteps) : 0; }
+// A graph of gsteps steps leaves fewer gaps, but takes the host as long to make as launching its steps would (2.6 us
+// a launch), so one is made once the batch has run, or is about to run, steps that take four times as long,
+// at least 256 and at most 768 of them (a step of a chain: 0.9 us, or 6e4 cells a us).  us per step in graphs of 8 (*: launches) and of 64, and ms of the first
+// 64 steps that way: 64 rhs of iso 50^3 134.5 129.0, 11.2 29.8     100 iso 40^3 143.4 135.2, 14.2 45     100 ortho 32^3 99.8 90.7, 11.9 46
+//   12 iso 72^3 80.1 76.3, 5.9 9.5     12 rhs of iso 50^3 26.2 25.0, 2.4 5.4     12 rhs of ortho 100^3* 288 278, 18.2 22
+static long long long_from(const ewf_batch *b)
+{
+    const double step_us = std::max(0.9, chain_cells(b) / 6e4);
+    return (long long)std::min(768.0, std::max(256.0, 4 * 2.6 * 2 * b->gsteps / step_us));
 }
 
 static int batch_ready(ewf_batch *b)
@@ -870,7 +883,7 @@ extern "C" int ewf_batch_run(ewf_batch *b, int32_t nsteps)
     if (b->it + nsteps > b->nt) return ewf_fail(EWF_ERR_ARG, "step %d + %d exceeds nt = %d", b->it, nsteps, b->nt);
     // graphs start from an even step
     const int odd = b->it & 1, rest = std::max(0, nsteps - odd), brief = short_graph(b);
-    const int nlong = rest / b->gsteps, nshort = brief > 0 ? (rest - nlong * b->gsteps) / brief : 0;
+    const int nlong = b->gexec || b->ran + nsteps >= long_from(b) ? rest / b->gsteps : 0, nshort = brief > 0 ? (rest - nlong * b->gsteps) / brief : 0;
     if (nlong && (st = ready_graph(b, b->gsteps, &b->gexec))) return st;
     if (nshort && (st = ready_graph(b, brief, &b->gexec_short))) return st;
     CK(cudaEventRecord(b->ev0, b->stream));
@@ -881,12 +894,16 @@ extern "C" int ewf_batch_run(ewf_batch *b, int32_t nsteps)
     }
     for (int q = 0; q < nlong; ++q, done += b->gsteps) CK(cudaGraphLaunch(b->gexec, b->stream));
     for (int q = 0; q < nshort; ++q, done += brief) CK(cudaGraphLaunch(b->gexec_short, b->stream));
-    if (done < nsteps) batch_steps(b, nsteps - done, (b->it + done) & 1);
+    for (int n = 0; done < nsteps; done += n) {
+        n = std::min(nsteps - done, b->gsteps);
+        batch_steps(b, n, (b->it + done) & 1);
+    }
     CK(cudaGetLastError());
     CK(cudaEventRecord(b->ev1, b->stream));
     CK(cudaStreamSynchronize(b->stream));
     CK(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
     b->it += nsteps;
+    b->ran += nsteps;
     return EWF_OK;
 }
 

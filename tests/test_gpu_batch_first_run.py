@@ -36,3 +36,31 @@ def test_tables_of_many_problems(cuda_device):
             first.append(_seconds(lambda: b.run(1)))
             again.append(_seconds(lambda: b.run(1)))
     assert min(first) - min(again) < 4e-3, (first, again)
+
+
+def test_first_steps_of_many_chains(cuda_device):
+    """The first 64 steps of 100 chains against the next: 40 ms when a graph of all 64 was made for them, 5 of 8."""
+    with Batch(_many(40, 100)) as b:
+        first, again = [], []
+        for _ in range(3):
+            b.set_tile(4)
+            b.reset()
+            first.append(_seconds(lambda: b.run(64)))
+            b.reset()
+            again.append(_seconds(lambda: b.run(64)))
+    assert min(first) - min(again) < 15e-3, (first, again)
+
+
+def test_graphs_of_both_lengths(cuda_device):
+    """Runs before and after the longer graph is made, from odd and even steps: one trajectory."""
+    nt = 1000
+    probs = _many(20, 3, nt) + _many(9, 12, nt)
+    with Batch(probs) as b:
+        b.run(nt)
+        ref = [b.seismograms(p, 0) for p in range(len(probs))]
+        b.reset()
+        for n in (3, 64, 8, 7, 600, 1, 150, 167):
+            b.run(n)
+        for p, r in enumerate(ref):
+            np.testing.assert_array_equal(b.seismograms(p, 0), r)
+            assert np.abs(r).max() > 0
