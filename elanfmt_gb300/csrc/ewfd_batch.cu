@@ -104,6 +104,9 @@ struct Chain {
     const ManyProb *d_many[2] = {nullptr, nullptr};  // their arguments,
     const int2 *d_map = nullptr;  // and the problem of each CTA
     int blocks = 0;
+    const int *d_groups = nullptr;  // the (problem, RHS) groups of theirs that k_binject applies,
+    const int2 *d_rows = nullptr;   // the receivers (row, problem) that k_brecord_many samples
+    int groups = 0, rows = 0;
 };
 
 float *bptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.base_off : nullptr; }
@@ -427,11 +430,17 @@ extern "C" int ewf_batch_set_receivers(ewf_batch *b, int32_t prob, int32_t n, co
 //   12 iso 24^3 29 16 11    6 iso 40^3 17 14 12     8 iso 50^3 29 24 25    8 iso 64^3 32 28 39
 //   8 ortho 64^3 40 40 54   8 iso 72^3 52 61 82     8 iso 80^3 50 74 91    6 ortho 80^3 64 76 85
 constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
-// MANY_MIN or more problems of one scheme below MANY_CELLS cells share two launches a step (k_stress_many): chains of
-// their own are bound by their launches, 0.35 us each on eight branches.  us per step of chains and of shared
-// launches: 50 iso 16^3 38 and 15, 200 139 and 50; 24 iso 24^3 17.5 and 15, 50 40 and 24, 200 147 and 110.
-constexpr double MANY_CELLS = 2e4;
-constexpr int MANY_MIN = 16;
+// MANY_MIN or more problems of one scheme below MANY_CELLS cells share two launches a step (k_stress_many), and one more each for
+// sources and receivers that those do not take: more chains than there are branches wait for one another's launches.  A few of
+// the largest run better as chains, so those up to MANY_CELLS_2 have to be MANY_MIN_2, and fit L2 together where the model has
+// twelve material arrays (MANY_ORTHO cells).  us per step of chains and of shared launches by number of problems:
+//   iso 12^3  8 5.7 8.2   16 11.1 8.2   100 71 19       iso 16^3  8 5.5 7.7   15 10.7 8.0   50 36 13.6   200 134 45
+//   iso 24^3  8 5.8 8.0   15 11.2 9.3   50 38 22   200 143 103      iso 28^3  8 6.4 11.8   16 12.6 14.1   50 43 28   200 159 144
+//   iso 27^3  9 11.0 12.2   12 11.8 10.6     iso 32^3  16 13.2 14.9   50 44.5 42.9   200 165 178
+//   ortho 24^3  9 10.9 11.4   15 11.9 11.0   50 40 30     ortho 28^3  33 30.8 27.3   100 84 93     ortho 32^3  100 91 120
+// and of problems with a stress receiver each: iso 16^3  15 17.4 9.6   50 60 15.8   200 253 48     iso 28^3  50 74 31   200 277 147.
+constexpr double MANY_CELLS = 2e4, MANY_CELLS_2 = 2.8e4, MANY_ORTHO = 1.2e6;
+constexpr int MANY_MIN = 12, MANY_MIN_2 = 32;
 static int scheme(const ewf_params &p) { return p.model == EWF_MODEL_ISO ? 0 : p.damping == EWF_DAMP_W3D ? 1 : 2; }
 
 // Rebuilds the device tables (problem descriptors, sources, receivers, traces).
@@ -577,7 +586,7 @@ static int build_tables(ewf_batch *b)
         return make_stress_src(*ent, q.p.nx, q.p.ny, q.p.nz, f, plane1);
     };
     std::vector<Chain> singles;
-    std::vector<int> tiny[3];
+    std::vector<int> tiny[3][2];  // by scheme, up to MANY_CELLS and above
     for (int i = 0; i < n; ++i) {
         const Prob &q = b->probs[i];
         const double cells = (double)q.p.nx * q.p.ny * q.p.nz;
@@ -590,17 +599,17 @@ static int build_tables(ewf_batch *b)
         }
         c.R = q.R;
         c.work = cells * q.R;
-        std::vector<SrcEntry> ent;
-        int before;
-        bool plane1;
-        StressSrc f;
-        if (cells < MANY_CELLS && q.R == 1 && q.rec_fuse && (fuses(c, &ent, &before, &f, &plane1) || ent.empty()))
-            tiny[scheme(q.p)].push_back((int)singles.size());
+        if (cells < MANY_CELLS_2 && q.R == 1) tiny[scheme(q.p)][cells < MANY_CELLS ? 0 : 1].push_back((int)singles.size());
         singles.push_back(c);
     }
     std::vector<char> grouped(singles.size(), 0);
-    for (auto &list : tiny) {
-        if ((int)list.size() < MANY_MIN) continue;
+    for (auto &t : tiny) {
+        std::vector<int> list;
+        double cells = 0;
+        for (int q : t[1]) cells += singles[q].work;
+        if (t[0].size() + t[1].size() >= MANY_MIN_2 && (&t == &tiny[0] || cells <= MANY_ORTHO)) list = t[1];
+        if (t[0].size() + list.size() >= MANY_MIN) list.insert(list.begin(), t[0].begin(), t[0].end());
+        if (list.empty()) continue;
         Chain c;
         c.prob = singles[list[0]].prob;
         c.many = list;
@@ -666,7 +675,7 @@ static int build_tables(ewf_batch *b)
     };
     struct ManyPlaces {
         Chain *c;
-        size_t many[2], map;
+        size_t many[2], map, groups, rows;
     };
     std::vector<ManyPlaces> many_at;
     for (auto &c : b->chains) {
@@ -675,11 +684,16 @@ static int build_tables(ewf_batch *b)
             continue;
         }
         std::vector<ManyProb> mp[2];
-        std::vector<int2> map;
+        std::vector<int2> map, rows;
+        std::vector<int> groups;
         const int at = (int)(&c - b->chains.data());
         for (int q : c.many) {
             Chain &o = singles[q];
             prepare(o, c.work / o.work);
+            const Prob &pr = b->probs[o.prob];
+            if (o.nsrc > 0 && o.ss.nsrc == 0) groups.push_back(pr.group0);
+            if (!pr.rec_fuse)
+                for (int e = 0; e < (int)pr.rec.size() / 4; ++e) rows.push_back(make_int2(b->rec_base[o.prob] + e, o.prob));
             ManyProb m;
             m.a = o.a;
             m.ss = o.ss;
@@ -697,12 +711,16 @@ static int build_tables(ewf_batch *b)
             }
         }
         c.blocks = (int)map.size();
-        many_at.push_back({&c, {b->many_tables.add(mp[0]), b->many_tables.add(mp[1])}, b->many_tables.add(map)});
+        c.groups = (int)groups.size();
+        c.rows = (int)rows.size();
+        many_at.push_back({&c, {b->many_tables.add(mp[0]), b->many_tables.add(mp[1])}, b->many_tables.add(map), b->many_tables.add(groups), b->many_tables.add(rows)});
     }
     if (int st = b->many_tables.send()) return st;
     for (auto &m : many_at) {
         for (int par = 0; par < 2; ++par) m.c->d_many[par] = b->many_tables.at<ManyProb>(m.many[par]);
         m.c->d_map = b->many_tables.at<int2>(m.map);
+        m.c->d_groups = b->many_tables.at<int>(m.groups);
+        m.c->d_rows = b->many_tables.at<int2>(m.rows);
     }
     // every chain's counters at the batch's step
     const std::vector<int> its(2 * b->chains.size(), b->it);
@@ -723,8 +741,14 @@ static void chain_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream
     if (!c.many.empty()) {
         launch_on(k_stress_many<MODEL, DAMP>, dim3(c.blocks), dim3(TX, b->ty), s, b->pdl && !first, (const ManyProb *)c.d_many[parity],
                   (const int2 *)c.d_map);
+        if (c.groups)
+            k_binject<float><<<(c.groups + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, c.d_groups, 0, c.groups, b->d_stf, b->d_stf_off,
+                                                                 b->d_order, b->nt, it_rd);
         launch_on(k_velocity_many<MODEL, DAMP>, dim3(c.blocks), dim3(TX, b->ty), s, b->pdl, (const ManyProb *)c.d_many[parity],
                   (const int2 *)c.d_map, (const int *)it_rd, it_wr);
+        if (c.rows)
+            k_brecord_many<float><<<std::min((c.rows + 255) / 256, 1024), 256, 0, s>>>(b->d_all, c.d_rows, c.rows, b->d_rec_off, b->d_rec_comp,
+                                                                                       b->d_traces, b->nt, it_rd);
         return;
     }
     StressSrc ss = c.ss;
@@ -740,7 +764,7 @@ static void chain_step_t(ewf_batch *b, int i, int parity, bool first, cudaStream
     else if (c.pair) launch_on(k_stress_pair<MODEL, DAMP, ST>, grd, blk, s, b->pdl && !first, a, ss);
     else launch_on(k_stress<float, MODEL, DAMP>, grd, blk, s, b->pdl && !first, a, ss);
     if (c.nsrc > 0 && ss.nsrc == 0)
-        k_binject<float><<<(c.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, q.group0 + c.r0, c.R, b->d_stf, b->d_stf_off,
+        k_binject<float><<<(c.R + 31) / 32, 32, 0, s>>>(b->d_all, b->d_src, b->d_src_start, nullptr, q.group0 + c.r0, c.R, b->d_stf, b->d_stf_off,
                                                         b->d_order, b->nt, it_rd);
     if (c.R > 1) launch_on(k_velocity_pair_mr<MODEL, DAMP, ST>, grd, blk, s, b->pdl, a, c.R, stride, rf, nr * b->nt);
     else if (c.pair) launch_on(k_velocity_pair<MODEL, DAMP, false, ST>, grd, blk, s, b->pdl, a, rf);

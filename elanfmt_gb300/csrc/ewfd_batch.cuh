@@ -20,7 +20,8 @@ struct BatchProb {
     long long rhs_stride;                 // elements between the state boxes of consecutive RHS
 };
 
-// Point injection: one thread per (problem, RHS), entries in order, as k_inject.
+// Point injection: one thread per (problem, RHS), entries in order, as k_inject.  `list`: which of them (else `groups` from
+// group0 on).
 struct BatchSrc {
     int prob, rhs, comp, i, j, k;
     double coef;
@@ -28,12 +29,13 @@ struct BatchSrc {
 
 template <typename T>
 __global__ void k_binject(const BatchProb<T> *__restrict__ probs, const BatchSrc *__restrict__ src,
-                          const int *__restrict__ src_start, int group0, int groups, const double *__restrict__ stf,
+                          const int *__restrict__ src_start, const int *__restrict__ list, int group0, int groups, const double *__restrict__ stf,
                           const int *__restrict__ stf_off, const int *__restrict__ order, int nstf,
                           const int *__restrict__ it_ptr)
 {
-    const int g = group0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= group0 + groups) return;
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= groups) return;
+    const int g = list ? list[n] : group0 + n;
     const int it = *it_ptr;
     if (it < 0 || it >= nstf) return;
     for (int e = src_start[g]; e < src_start[g + 1]; ++e) {
@@ -88,6 +90,20 @@ __global__ void k_brecord(const StepArgs<T> a, const long long *__restrict__ rec
     if (it >= 0 && it < nt)
         for (int r = row0 + blockIdx.x * blockDim.x + threadIdx.x; r < row0 + nrow; r += gridDim.x * blockDim.x)
             traces[(long long)r * nt + it] = (double)a.f[rec_comp[r]][rec_off[r]];
+}
+
+// The same for rows of several problems: (row, problem) each.
+template <typename T>
+__global__ void k_brecord_many(const BatchProb<T> *__restrict__ probs, const int2 *__restrict__ rows, int nrow,
+                               const long long *__restrict__ rec_off, const int *__restrict__ rec_comp, double *__restrict__ traces, int nt,
+                               const int *it_rd)
+{
+    const int it = *it_rd;
+    if (it >= 0 && it < nt)
+        for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nrow; n += gridDim.x * blockDim.x) {
+            const int r = rows[n].x;
+            traces[(long long)r * nt + it] = (double)probs[rows[n].y].a.f[rec_comp[r]][rec_off[r]];
+        }
 }
 
 __global__ void k_advance(const int *it_rd, int *it_wr) { *it_wr = *it_rd + 1; }

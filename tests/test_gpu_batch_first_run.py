@@ -11,11 +11,11 @@ from elanfmt_gb300.solver import Batch
 pytestmark = pytest.mark.gpu
 
 
-def _many(n, count, nt=200):
+def _many(n, count, nt=200, extra=()):
     probs = []
     for q in range(count):
         m = I.random_small(F.MODEL_ISO, n, n, n, nt=nt, seed=q % 4)
-        m.receivers = np.array([(n // 2, n // 2, 1, c) for c in range(3)], np.int32)
+        m.receivers = np.array([(n // 2, n // 2, 1, c) for c in range(3)] + list(extra), np.int32)
         probs.append((m, [(m.sources, m.source_coef)]))
     return probs
 
@@ -64,3 +64,18 @@ def test_graphs_of_both_lengths(cuda_device):
         for p, r in enumerate(ref):
             np.testing.assert_array_equal(b.seismograms(p, 0), r)
             assert np.abs(r).max() > 0
+
+
+def test_tiny_problems_with_a_stress_receiver_share_launches(cuda_device):
+    """50 problems whose receivers the velocity kernel does not take, against 50 whose receivers it does: 4.4 times
+    the time as chains of five launches, 1.2 in shared ones."""
+    times = []
+    for extra in ((), ((3, 4, 1, F.F_SXY),)):
+        with Batch(_many(16, 50, 200, extra)) as b:
+            b.run(64)
+            best = 1e9
+            for _ in range(3):
+                b.reset()
+                best = min(best, b.run(128))
+        times.append(best)
+    assert times[1] < 2 * times[0], times
