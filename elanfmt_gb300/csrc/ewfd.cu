@@ -615,7 +615,8 @@ SplitShape split_shape(int nx, int ny, int nz, int R)
 static void split_default_shape(ewf_handle *h)
 {
     const SplitShape d = split_shape(h->p.nx, h->p.ny, h->p.nz);
-    if (h->p.kchunk == 0) h->kchunk = d.kchunk;
+    // 4, the shortest chunk that can be asked for, stands for the shorter ones of the rule too
+    if (h->p.kchunk == 0 || h->p.kchunk == 4) h->kchunk = h->p.kchunk ? std::min(h->p.kchunk, d.kchunk) : d.kchunk;
     h->ty = d.ty;
     h->l2pf = d.l2pf;
     h->pair = d.pair;
@@ -1717,7 +1718,7 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
     if (!h || nsteps < 1) return ewf_fail(EWF_ERR_ARG, "bad argument");
     int st = inputs_ready(h);
     if (st) return st;
-    static const int cand[] = {1, 2, 3, 4, 6, 8, 12, 16, 32};
+    static const int cand[] = {4, 6, 8, 12, 16, 32};
     const int steps = std::min(nsteps, h->p.nt - 1);
     if (steps < 1) return ewf_fail(EWF_ERR_ARG, "nt too small to tune");
     if (h->nsrc > 0 && h->nstf < (size_t)steps + 1) return ewf_fail(EWF_ERR_STATE, "source time function too short");
@@ -1761,10 +1762,11 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
         if (!split && ty != h->ty) continue;
         if (ty > (h->esz == 4 ? SPLIT_MAX_TY : TY)) continue;
         for (int kc : cand) {
-            if (kc > h->p.nz) continue;
-            if (h->wave && (kc < 4 || kc > 16)) continue;
+            if (kc > h->p.nz && kc != cand[0]) continue;
+            if (h->wave && kc > 16) continue;
             for (int vi = 0; vi < nvar; ++vi) {
-                h->kchunk = kc;
+                // 4 as for a handle made with it (split_default_shape): the setting returned is the one that was timed
+                h->kchunk = split && kc == 4 ? std::min(4, split_shape(h->p.nx, h->p.ny, h->p.nz).kchunk) : std::max(4, std::min(kc, h->p.nz));
                 h->ty = ty;
                 if (h->wave) {
                     h->wave_lag_pct = lag_pct[vi];
@@ -1803,7 +1805,6 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
         h->l2pf = best_pf;
     }
     h->graph_dirty = true;
-    // what ewf_params.kchunk takes: shorter chunks are this handle's own (and the default's for such grids)
     if (kchunk) *kchunk = std::max(4, best_k);
     return ewf_reset(h);
 }

@@ -152,8 +152,8 @@ struct ewf_batch {
     size_t stage_bytes = 0;
     bool dirty = true;   // device tables need a rebuild
     int ty = 4;          // CTA tile height (4, 8 or 16 rows of 32 columns; two-cell kernels: twice as many, 16 at most)
-    int l2pf = -1;       // the velocity kernels' L2 prefetch distance (autotuned; 0: off, -1: by size)
-    int own = -1;        // the problems' chains one after another (0), on parallel streams (1), by size (-1; autotuned)
+    int l2pf = 0;        // the velocity kernels' L2 prefetch distance (autotuned; 0: by size)
+    int own = 0;         // the problems' chains on parallel streams: those that do not fill the GPU (0), all (1) (autotuned)
     bool pdl = true;     // kernels launched as programmatic dependents (off if capture refuses)
     static constexpr int BRANCHES = 8;
     cudaStream_t branch[BRANCHES] = {};
@@ -441,6 +441,9 @@ constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
 // and of problems with a stress receiver each: iso 16^3  15 17.4 9.6   50 60 15.8   200 253 48     iso 28^3  50 74 31   200 277 147.
 constexpr double MANY_CELLS = 2e4, MANY_CELLS_2 = 2.8e4, MANY_ORTHO = 1.2e6;
 constexpr int MANY_MIN = 12, MANY_MIN_2 = 32;
+// A chunk that is asked for up to this many planes is the most that the rule by size may take, which takes no more than
+// 6 by itself: 8 asks for the rule, and stands for it where the autotuner chose it.
+constexpr int KCHUNK_BY_SIZE = 8;
 static int scheme(const ewf_params &p) { return p.model == EWF_MODEL_ISO ? 0 : p.damping == EWF_DAMP_W3D ? 1 : 2; }
 
 // Rebuilds the device tables (problem descriptors, sources, receivers, traces).
@@ -624,10 +627,10 @@ static int build_tables(ewf_batch *b)
     // branches: largest chains first, each to the least loaded branch
     int share = 1;  // chains that run at the same time
     for (auto &c : b->chains) c.branch = -1;
-    if (b->own != 0 && b->chains.size() > 1) {
+    if (b->chains.size() > 1) {
         std::vector<Chain *> idx;
         for (auto &c : b->chains)
-            if (b->own > 0 || c.work < BRANCH_CELLS) idx.push_back(&c);
+            if (b->own || c.work < BRANCH_CELLS) idx.push_back(&c);
         std::stable_sort(idx.begin(), idx.end(), [](const Chain *x, const Chain *y) { return x->work > y->work; });
         int branches = std::min(2, (int)idx.size());
         double held = 0;
@@ -651,11 +654,12 @@ static int build_tables(ewf_batch *b)
         c.stream_l2 = shape.stream;
         c.a = all[c.prob].a;
         for (auto &f : c.a.f) f += c.r0 * (long long)q.box;
-        c.a.l2pf = b->l2pf >= 0 ? b->l2pf : shape.l2pf;
+        c.a.l2pf = b->l2pf ? b->l2pf : shape.l2pf;
         // Chunks as long as for one problem of all the cells that run at the same time.  us per step with chunks by
         // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
         // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
-        c.a.kchunk = q.kchunk > 0 ? q.kchunk : split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
+        c.a.kchunk = split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
+        if (q.kchunk > 0) c.a.kchunk = q.kchunk <= KCHUNK_BY_SIZE ? std::min(q.kchunk, c.a.kchunk) : q.kchunk;
         std::vector<SrcEntry> ent;
         int before = 0;
         bool plane1 = false;
@@ -979,17 +983,15 @@ extern "C" int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int3
 extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_out)
 {
     if (!b || nsteps < 1) return ewf_fail(EWF_ERR_ARG, "bad argument");
-    // planes per CTA: what the batch was created with or the rule by size (0), or one number for all
-    static const int cand[] = {0, 8, 12, 16, 24, 32};
+    // planes per CTA: the rule by size, or one number for all problems
+    static const int cand[] = {KCHUNK_BY_SIZE, 12, 16, 24, 32};
     static const int ty_cand[] = {4, 8};
     static const int pf_cand[] = {0, 2, 3, 4};
     const int steps = std::min(nsteps, b->nt - 1);
-    std::vector<int> given;
-    for (auto &q : b->probs) given.push_back(q.kchunk);
-    int best_k = 0, best_ty = b->ty, best_pf = -1;
+    int best_k = KCHUNK_BY_SIZE, best_ty = b->ty, best_pf = 0;
     int best_own = b->own;
     auto apply = [&](int kc, int ty, int own, int pf) {
-        for (size_t i = 0; i < given.size(); ++i) b->probs[i].kchunk = kc ? std::max(4, std::min(kc, b->probs[i].p.nz)) : given[i];
+        for (auto &q : b->probs) q.kchunk = kc;
         b->ty = ty;
         b->own = own;
         b->l2pf = pf;
@@ -1008,10 +1010,10 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
         return (int)EWF_OK;
     };
     float best = 1e30f, ms = 0.f;
-    for (int own = -1; own < 2; ++own)
+    for (int own = 0; own < 2; ++own)
         for (int ty : ty_cand)
             for (int kc : cand) {
-                apply(kc, ty, own, -1);
+                apply(kc, ty, own, 0);
                 if (int st = time(&ms)) return st;
                 if (ms < best) {
                     best = ms;
@@ -1030,8 +1032,7 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
     }
     apply(best_k, best_ty, best_own, best_pf);
     if (int st = batch_ready(b)) return st;
-    // the rule by size gives every problem its own chunk; 8 is the nearest of the candidates
-    if (kchunk_out) *kchunk_out = best_k ? best_k : 8;
+    if (kchunk_out) *kchunk_out = best_k;
     return ewf_batch_reset(b);
 }
 
@@ -1056,7 +1057,7 @@ extern "C" int ewf_batch_set_launch(ewf_batch *b, int32_t own)
 extern "C" int ewf_batch_get_launch(const ewf_batch *b, int32_t *own)
 {
     if (!b || !own) return ewf_fail(EWF_ERR_ARG, "NULL argument");
-    *own = b->own > 0 ? 1 : 0;
+    *own = b->own;
     return EWF_OK;
 }
 

@@ -505,8 +505,8 @@ class Batch:
         return ty.value
 
     def set_launch(self, own: int) -> None:
-        """0 = one problem's run of steps after another's, 1 = on parallel branches; by default the small
-        problems on branches, then the others (results do not depend on it)."""
+        """0 (default) = the small problems on parallel branches, then the others one after another; 1 = all of
+        them on branches (results do not depend on it)."""
         _check(self._lib.ewf_batch_set_launch(self._h, int(own)), "ewf_batch_set_launch")
 
     def launch(self) -> int:
@@ -515,7 +515,7 @@ class Batch:
         return v.value
 
     def set_l2_prefetch(self, planes: int) -> None:
-        """L2 prefetch distance of the velocity kernels (0 = off; results do not depend on it)."""
+        """L2 prefetch distance of the velocity kernels (0 = by size, the default; results do not depend on it)."""
         _check(self._lib.ewf_batch_set_l2_prefetch(self._h, int(planes)), "ewf_batch_set_l2_prefetch")
 
     def l2_prefetch(self) -> int:

@@ -31,12 +31,15 @@ def cache_path() -> str:
                                                               "kchunk.json")
 
 
+# part of every key: settings found with other kernels are looked for again
+KERNELS = 2
+
 FORM_NAMES = {F.STEP_SPLIT: "split", F.STEP_FUSED: "fused", F.STEP_WAVE: "wave"}
 
 
 def key(device_name: str, m, precision: int, form: int) -> str:
     return (f"{device_name}|model{m.model}|damp{m.damping}|prec{precision}|{FORM_NAMES[int(form)]}|"
-            f"{m.nx}x{m.ny}x{m.nz}")
+            f"{m.nx}x{m.ny}x{m.nz}|k{KERNELS}")
 
 
 def load(path: str | None = None) -> dict:

@@ -123,7 +123,8 @@ typedef struct ewf_params {
     int32_t src_order;    /* ewf_src_order */
     int32_t over_y;       /* legacy OVERY: BC1 rows are j < min(nx, ny + over_y) (OK4:279-281) */
     int32_t nout;         /* progress line every nout steps (OK4:502-504); 0 = quiet */
-    int32_t kchunk;       /* planes per CTA of the z-marching kernels, from 4; 0 = autotuned/default (by size) */
+    int32_t kchunk;       /* planes per CTA of the z-marching kernels, from 4; 0 = by size.  Two-kernel step: with 4 (in a
+                             batch, up to 8) the rule by size may take fewer */
     int32_t graph_steps;  /* steps captured per CUDA graph; 0 = default (64; what is left of a run in graphs of 8 on
                              small grids), <0 = no graph */
     int32_t check_finite; /* 1: ewf_run checks the receiver traces for NaN/Inf */
@@ -210,7 +211,7 @@ int ewf_time_kernels(ewf_handle *h, int32_t nsteps, double out_ms[4]);
 int ewf_launches_per_step(const ewf_handle *h, int32_t *n);
 
 /* Autotuner: times `nsteps` steps for each z-chunk candidate (planes per CTA) with CUDA events,
- * keeps the fastest (returned in *kchunk, may be NULL) and resets the state.  The two-kernel step
+ * keeps the fastest (returned in *kchunk, may be NULL: a handle made with it has the same one) and resets the state.  The two-kernel step
  * also tunes its tile height (4, 8, 16 rows; ewf_get_tile) and then its L2 prefetch distance
  * (0, 2, 3, 4 planes; ewf_get_l2_prefetch), the wavefront step its lag (all kept in the handle). */
 int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk);
@@ -255,7 +256,7 @@ int ewf_staged_test_hold(int32_t plane, int32_t polls);
 int ewf_set_dependent_launch(ewf_handle *h, int32_t on);
 int ewf_get_dependent_launch(const ewf_handle *h, int32_t *on);
 /* Two-kernel step: the velocity kernel asks L2 for the input lines of the plane `planes` ahead
- * (0..8; 0 = off, the default; ewf_autotune picks it).  A hint: results do not depend on it. */
+ * (0..8; 0 = off; by default 3 from 12 M cells on, else off; ewf_autotune picks it).  A hint: results do not depend on it. */
 int ewf_set_l2_prefetch(ewf_handle *h, int32_t planes);
 int ewf_get_l2_prefetch(const ewf_handle *h, int32_t *planes);
 
@@ -354,19 +355,19 @@ int ewf_batch_last_run_ms(const ewf_batch *b, double *ms);
 int ewf_batch_get_seismograms(ewf_batch *b, int32_t prob, int32_t rhs, double *out, size_t n);
 int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int32_t field, void *host, size_t n, int32_t dtype_bytes);
 /* the autotuner over the whole batch: launch form, z-chunk and CTA tile height, then the
- * velocity kernels' L2 prefetch distance (leaves the batch reset) */
+ * velocity kernels' L2 prefetch distance (leaves the batch reset).  A batch made with *kchunk and set to what
+ * the getters below return has the same setting. */
 int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk);
 /* CTA tile height of every launch of the batch, in rows of 32 columns: 4 (default), 8 or 16
  * (kernels with two cells per thread take twice as many rows, 16 at most); results do not depend on it */
 int ewf_batch_set_tile(ewf_batch *b, int32_t tile_y);
 int ewf_batch_get_tile(const ewf_batch *b, int32_t *tile_y);
-/* The velocity kernels ask L2 for their state lines `planes` planes ahead (0..8; 0 = off; by
- * default large problems do; ewf_batch_autotune picks it).  A hint: results do not depend on it. */
+/* The velocity kernels ask L2 for their state lines `planes` planes ahead (0..8; 0, the default: launches of
+ * 12 M cells or more 3, others none; ewf_batch_autotune picks it).  A hint: results do not depend on it. */
 int ewf_batch_set_l2_prefetch(ewf_batch *b, int32_t planes);
-/* Launch form: 0 -- one problem's run of steps after another's; 1 -- spread over up to eight parallel
- * branches (streams of the captured graph) balanced by cell-updates.  By default (reported as 0) the
- * chains of launches too small to fill the GPU run on branches, then the others one after another.  Results do
- * not depend on it. */
+/* Launch form: 0 (default) -- the chains of launches too small to fill the GPU on up to eight parallel branches
+ * (streams of the captured graph) balanced by cell-updates, then the others one after another; 1 -- all of them
+ * on branches.  Results do not depend on it. */
 int ewf_batch_set_launch(ewf_batch *b, int32_t own);
 int ewf_batch_get_launch(const ewf_batch *b, int32_t *own);
 int ewf_batch_get_l2_prefetch(const ewf_batch *b, int32_t *planes);
