@@ -1688,8 +1688,9 @@ extern "C" int ewf_time_kernels(ewf_handle *h, int32_t nsteps, double out_ms[4])
     return EWF_OK;
 }
 
-// Device time of `steps` steps from a reset state (one untimed step first); -1 when the current
-// settings cannot run.
+// Device time per step over `steps` steps from a reset state (some untimed ones first); -1 when the current
+// settings cannot run.  Small grids are timed in the graphs that they run in: the host does not keep up with their
+// launches one by one, and every setting would take what it takes.
 static int time_setting(ewf_handle *h, int steps, float *ms)
 {
     int st = ewf_reset(h);
@@ -1699,6 +1700,23 @@ static int time_setting(ewf_handle *h, int steps, float *ms)
         return EWF_OK;
     }
     const step_fn fn = pick_step(h);
+    const int brief = std::min(short_graph(h), steps & ~1);
+    if (brief > 0) {
+        h->graph_dirty = true;  // no graph of another setting stays
+        cudaGraphExec_t exec = nullptr;
+        if ((st = ready_graph(h, fn, brief, &exec))) return st;
+        const int n = std::max(1, steps / brief);
+        cudaError_t e = cudaGraphLaunch(exec, h->stream);  // warm
+        if (e == cudaSuccess) e = cudaEventRecord(h->ev0, h->stream);
+        for (int q = 0; q < n && e == cudaSuccess; ++q) e = cudaGraphLaunch(exec, h->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(h->ev1, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        cudaGraphExecDestroy(exec);
+        CK(e);
+        CK(cudaEventElapsedTime(ms, h->ev0, h->ev1));
+        *ms /= n * brief;
+        return step_check(h);
+    }
     fn(h, nullptr, h->flip);  // warm (step 0 after the reset)
     if (h->dbuf) h->flip ^= 1;
     CK(cudaEventRecord(h->ev0, h->stream));
@@ -1710,6 +1728,7 @@ static int time_setting(ewf_handle *h, int steps, float *ms)
     CK(cudaStreamSynchronize(h->stream));
     if ((st = step_check(h))) return st;
     CK(cudaEventElapsedTime(ms, h->ev0, h->ev1));
+    *ms /= steps;
     return EWF_OK;
 }
 
@@ -1758,6 +1777,22 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
     // two-kernel step: z-chunk x tile height (rows of 32 columns per CTA)
     const bool split = !h->wave && !h->fused;
     static const int ty_cand[] = {4, 8, 16};
+    // the rule's own setting is timed twice, and another one has to be faster by more than those two differ
+    const SplitShape by_size = split_shape(h->p.nx, h->p.ny, h->p.nz);
+    float margin = 0.f;
+    if (split) {
+        h->kchunk = by_size.kchunk;
+        h->ty = std::min(by_size.ty, h->esz == 4 ? SPLIT_MAX_TY : TY);
+        h->l2pf = by_size.l2pf;
+        float t[2] = {};
+        for (float &ms : t)
+            if ((st = time_setting(h, steps, &ms))) return st;
+        margin = std::max(0.01f * std::min(t[0], t[1]), std::fabs(t[0] - t[1]));
+        best = std::min(t[0], t[1]) - margin;
+        best_k = h->kchunk;
+        best_ty = h->ty;
+    }
+    const int rule_k = best_k, rule_ty = best_ty;
     for (int ty : ty_cand) {
         if (!split && ty != h->ty) continue;
         if (ty > (h->esz == 4 ? SPLIT_MAX_TY : TY)) continue;
@@ -1787,13 +1822,11 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
     h->ty = best_ty;
     h->wave_lag_pct = best_lag;
     if (split) {  // then the velocity kernel's L2 prefetch distance at that setting
-        int best_pf = 0;
-        h->l2pf = 0;
-        float base = 0.f;
-        if ((st = time_setting(h, steps, &base))) return st;
-        best = base;
-        static const int pf_cand[] = {2, 3, 4};
+        int best_pf = by_size.l2pf;
+        if (best_k != rule_k || best_ty != rule_ty) best -= margin;  // (`best` was timed with the rule's distance)
+        static const int pf_cand[] = {0, 2, 3, 4};
         for (int pf : pf_cand) {
+            if (pf == by_size.l2pf) continue;
             h->l2pf = pf;
             float ms = 0.f;
             if ((st = time_setting(h, steps, &ms))) return st;
