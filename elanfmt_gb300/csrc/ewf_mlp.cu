@@ -1005,7 +1005,7 @@ namespace {
 // rows: the gradients' row count has to be a multiple of 128, as ewf_mlp_gemm's
 int check_net(const char *what, int32_t n, const int32_t *sizes, int32_t M, int in_mult)
 {
-    if (n < 1 || n > 64 || !sizes || M <= 0) return ewf_fail(EWF_ERR_ARG, "%s: bad network or batch", what);
+    if (n < 1 || !sizes || M <= 0) return ewf_fail(EWF_ERR_ARG, "%s: bad network or batch", what);
     if (sizes[0] <= 0 || sizes[0] % in_mult) return ewf_fail(EWF_ERR_ARG, "%s: the input width must be a multiple of %d", what, in_mult);
     for (int l = 1; l <= n; ++l)
         if (sizes[l] <= 0 || sizes[l] % 128) return ewf_fail(EWF_ERR_ARG, "%s: layer widths must be multiples of 128 (got %d)", what, sizes[l]);
