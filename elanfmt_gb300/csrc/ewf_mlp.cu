@@ -1114,17 +1114,24 @@ extern "C" int ewf_mlp_adam_all(int32_t count, float *const *w, float *const *m,
     if (count < 1 || !w || !m || !v || !g || !wb || !n || !wd || step < 1) return ewf_fail(EWF_ERR_ARG, "adam: bad argument");
     for (int q = 0; q < count; ++q) {
         if (!w[q] || !m[q] || !v[q] || !g[q]) return ewf_fail(EWF_ERR_ARG, "adam: NULL tensor %d", q);
-        if (misaligned(w[q]) || misaligned(m[q]) || misaligned(v[q]) || misaligned(g[q]) || ((uintptr_t)wb[q] & 7))
-            return ewf_fail(EWF_ERR_ARG, "adam: tensor %d must be 16-byte aligned", q);
-        if (n[q] >= (1ull << 31)) return ewf_fail(EWF_ERR_ARG, "adam: tensor %d too large", q);
     }
-    for (int q0 = 0; q0 < count; q0 += ADAM_GROUP) {
+    // tensors off 16 bytes (parameters that are views into one buffer), or of 2^31 elements and more, by the kernel of one element a thread
+    auto alone = [&](int q) {
+        return misaligned(w[q]) || misaligned(m[q]) || misaligned(v[q]) || misaligned(g[q]) || ((uintptr_t)wb[q] & 7) || n[q] >= (1ull << 31);
+    };
+    for (int q0 = 0; q0 < count;) {
+        if (alone(q0)) {
+            const int st = n[q0] ? ewf_mlp_adam(w[q0], m[q0], v[q0], g[q0], wb[q0], n[q0], lr, b1, b2, eps, step, wd[q0], stream) : EWF_OK;
+            if (st) return st;
+            ++q0;
+            continue;
+        }
         AdamJobs J;
         memset(&J, 0, sizeof(J));
-        J.njobs = count - q0 < ADAM_GROUP ? count - q0 : ADAM_GROUP;
         unsigned blocks = 0;
-        for (int e = 0; e < J.njobs; ++e) {
-            const int q = q0 + e;
+        int q = q0;
+        for (; q < count && J.njobs < ADAM_GROUP && !alone(q); ++q) {
+            const int e = J.njobs++;
             J.w[e] = w[q];
             J.m[e] = m[q];
             J.v[e] = v[q];
@@ -1141,6 +1148,7 @@ extern "C" int ewf_mlp_adam_all(int32_t count, float *const *w, float *const *m,
         J.eps = eps;
         J.c1 = 1.f - powf(b1, (float)step);
         J.c2 = 1.f - powf(b2, (float)step);
+        q0 = q;
         if (blocks == 0) continue;
         const int st = launch_pdl("adam launch", k_adam_all, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, J);
         if (st) return st;

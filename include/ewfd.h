@@ -384,7 +384,7 @@ int ewf_batch_get_l2_prefetch(const ewf_batch *b, int32_t *planes);
 int ewf_mlp_gemm(const void *A, const void *B, const float *bias, float *Cf, void *Cb, float *pre, int32_t M, int32_t N,
                  int32_t K, int32_t act, void *stream);
 /* The passes of a network of n layers (widths sizes[0..n]; sizes[1..n] multiples of 128), one call each;
- * every buffer 16-byte aligned.
+ * every buffer 16-byte aligned (adam_all takes any).
  * forward: layer l is W[l] (bf16 [sizes[l+1], sizes[l]]) and b[l]; GELU between layers.  X bf16
  * [M, sizes[0]] (sizes[0] a multiple of 32, any M >= 1); H[l], l < n - 1: the output of layer l, bf16; P[l]:
  * its value before the activation, fp32 (P NULL: not kept); Y fp32 [M, sizes[n]].
