@@ -84,7 +84,7 @@ class MLP:
         self.step_count = 0
         self._ws = {}
         self._sizes = (C.c_int32 * len(sizes))(*sizes)
-        self._act = []   # inference: two activation buffers, for the most rows seen
+        self._act = {}   # inference: two activation buffers per batch size in GEMM tiles (passes of different sizes may overlap)
 
     @property
     def nlayers(self) -> int:
@@ -129,10 +129,12 @@ class MLP:
         if not (X.dtype == t.bfloat16 and X.is_cuda and X.is_contiguous() and X.shape[1] == self.sizes[0]
                 and X.data_ptr() % 16 == 0):
             X = t.empty(M, self.sizes[0], dtype=t.bfloat16, device="cuda").copy_(X)
-        need = M * max(self.sizes[1:-1], default=0)
-        if not self._act or self._act[0].numel() < need:
-            self._act = [t.empty(max(need, 8), dtype=t.bfloat16, device="cuda") for _ in range(2)]
-        self._forward(X, _ptrs([self._act[l & 1] for l in range(self.nlayers - 1)]), None, Y, M)
+        rows = -(-M // 128) * 128
+        act = self._act.get(rows)
+        if act is None:
+            act = self._act[rows] = [t.empty(max(rows * max(self.sizes[1:-1], default=0), 8), dtype=t.bfloat16, device="cuda")
+                                     for _ in range(2)]
+        self._forward(X, _ptrs([act[l & 1] for l in range(self.nlayers - 1)]), None, Y, M)
 
     def loss_grad(self, T) -> "torch.Tensor":
         """MSE against fp32 targets T; dY of the last layer into the workspace; returns the loss."""
