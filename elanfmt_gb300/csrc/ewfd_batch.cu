@@ -607,13 +607,7 @@ static int build_tables(ewf_batch *b)
         singles.push_back(c);
     }
     std::vector<char> grouped(singles.size(), 0);
-    for (auto &t : tiny) {
-        std::vector<int> list;
-        double cells = 0;
-        for (int q : t[1]) cells += singles[q].work;
-        if (t[0].size() + t[1].size() >= MANY_MIN_2 && (&t == &tiny[0] || cells <= MANY_ORTHO)) list = t[1];
-        if (t[0].size() + list.size() >= MANY_MIN) list.insert(list.begin(), t[0].begin(), t[0].end());
-        if (list.empty()) continue;
+    auto share_launches = [&](const std::vector<int> &list) {
         Chain c;
         c.prob = singles[list[0]].prob;
         c.many = list;
@@ -622,7 +616,18 @@ static int build_tables(ewf_batch *b)
             grouped[q] = 1;
         }
         b->chains.push_back(c);
+    };
+    for (auto &t : tiny) {
+        std::vector<int> list;
+        double cells = 0;
+        for (int q : t[1]) cells += singles[q].work;
+        if (t[0].size() + t[1].size() >= MANY_MIN_2 && (&t == &tiny[0] || cells <= MANY_ORTHO)) list = t[1];
+        if (t[0].size() + list.size() >= MANY_MIN) list.insert(list.begin(), t[0].begin(), t[0].end());
+        if (!list.empty()) share_launches(list);
     }
+    // their list of CTAs also takes a model of more rows than a grid of 65535 CTAs of 16
+    for (int q = 0; q < (int)singles.size(); ++q)
+        if (singles[q].R == 1 && b->probs[singles[q].prob].p.ny > 65535 * 16) share_launches({q});
     for (size_t q = 0; q < singles.size(); ++q)
         if (!grouped[q]) b->chains.push_back(singles[q]);
     // branches: largest chains first, each to the least loaded branch
@@ -661,6 +666,7 @@ static int build_tables(ewf_batch *b)
         // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
         c.a.kchunk = split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
         if (q.kchunk > 0) c.a.kchunk = q.kchunk <= KCHUNK_BY_SIZE ? std::min(q.kchunk, c.a.kchunk) : q.kchunk;
+        c.a.kchunk = std::max(c.a.kchunk, (p.nz + 65534) / 65535);  // a grid has at most 65535 CTAs along z
         std::vector<SrcEntry> ent;
         int before = 0;
         bool plane1 = false;
