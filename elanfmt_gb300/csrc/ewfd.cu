@@ -593,9 +593,18 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 //   iso 128^3     36.9 (2)  35.5 (3)      33.0 (2)  32.9 (3)  35.2 (4)
 //   iso-het 203x151x97  74.4 (2)  73.1 (3)      66.8 (2)  66.7 (3)  67.6 (4)
 //   Kahan 192^3   198.8 (2) 196.1 (4)     186.3 (4)
-//   ortho 256^3   405.9 (4) 401.6 (6)     380.2 (6)
-// The velocity kernel's L2 prefetch pays once its inputs come from HBM (ortho 256^3 406.5 -> 400.1,
-// 320x320x256 641 -> 631 with one cell per thread) and not below (128^3: 55.8 and 56.1).
+// and with two cells per thread and the velocity kernel's L2 prefetch off, 2 and 3 planes ahead:
+//                      3 planes              4                     6
+//   ortho 192^3        161.2 161.0 161.3     161.1 160.8 162.9     163.6 162.2 164.3
+//   iso 192^3          124.0 122.0 124.1     123.3 121.2 122.4     127.3 124.9 125.8
+//   ortho 230^3        297.7 295.8 297.8     295.0 293.6 295.2     297.9 295.6 297.2
+//   ortho 256^3        373.5 371.9 373.6     375.5 374.8 377.0     376.7 374.6 376.2
+//   iso 256^3          287.8 282.1 287.9     289.1 284.3 286.2     288.9 283.6 284.0
+//   ortho 320x320x256  579.7 575.6 579.9     578.3 577.0 581.5     583.4 580.2 581.8
+//   ortho 400x400x300  1103.3 1097.9 1103.4  1102.5 1099.6 1104.8  1110.8 1107.8 1112.5
+// and for right-hand sides in one launch, 3 planes with the prefetch 2 ahead and 6 with 3: 2 of iso 192^3 238.2 242.1, 3 of iso 160^3
+// 215.6 215.9, 6 of ortho 160^3 522.7 517.6, 16 of iso 136^3 789.3 782.5.
+// The prefetch pays once the velocity kernel's inputs come from HBM, and not below (128^3: 55.8 and 56.1).
 // stream: the state's nine fields (36 bytes a cell) are read and written by both kernels, the moduli and
 // buoyancies (up to 48 bytes) once a step.  Where the fields by themselves about fit the 129 MB L2, what
 // is read once, and the new velocities, are marked to leave it first.  us per step without and with:
@@ -606,7 +615,7 @@ static int band_rows(int onepass) { return onepass == EWF_ONEPASS_BAND4 ? 4 : (o
 SplitShape split_shape(int nx, int ny, int nz, int R)
 {
     const double cells = (double)nx * ny * nz * R;
-    SplitShape d = {cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 ? 3 : cells < 1.2e7 ? 4 : 6, 4, cells >= 1.2e7 ? 3 : 0, cells >= 4e5, cells >= 1e6 && cells < 6e6};
+    SplitShape d = {cells < 2e5 ? 1 : cells < 1e6 ? 2 : cells < 6e6 || (cells >= 1.5e7 && R < 4) ? 3 : cells < 1.5e7 ? 4 : 6, 4, cells < 1.2e7 ? 0 : R < 4 ? 2 : 3, cells >= 4e5, cells >= 1e6 && cells < 6e6};
     // a grid has at most 65535 CTAs along y and z
     d.kchunk = std::max(d.kchunk, (nz + 65534) / 65535);
     while (d.ty < 16 && ny > 65535 * d.ty) d.ty *= 2;
@@ -1700,12 +1709,12 @@ static int time_setting(ewf_handle *h, int steps, float *ms)
         return EWF_OK;
     }
     const step_fn fn = pick_step(h);
-    const int brief = std::min(short_graph(h), steps & ~1);
+    const int brief = std::min(short_graph(h), std::max(2, steps & ~1));
     if (brief > 0) {
         h->graph_dirty = true;  // no graph of another setting stays
         cudaGraphExec_t exec = nullptr;
         if ((st = ready_graph(h, fn, brief, &exec))) return st;
-        const int n = std::max(1, steps / brief);
+        const int n = std::max(4, steps / brief);  // (steps past the last one sample and inject nothing)
         cudaError_t e = cudaGraphLaunch(exec, h->stream);  // warm
         if (e == cudaSuccess) e = cudaEventRecord(h->ev0, h->stream);
         for (int q = 0; q < n && e == cudaSuccess; ++q) e = cudaGraphLaunch(exec, h->stream);
@@ -1777,7 +1786,7 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
     // two-kernel step: z-chunk x tile height (rows of 32 columns per CTA)
     const bool split = !h->wave && !h->fused;
     static const int ty_cand[] = {4, 8, 16};
-    // the rule's own setting is timed twice, and another one has to be faster by more than those two differ
+    // the rule's own setting is timed twice; on small grids another one has to be faster by more than those two differ
     const SplitShape by_size = split_shape(h->p.nx, h->p.ny, h->p.nz);
     float margin = 0.f;
     if (split) {
@@ -1787,7 +1796,7 @@ extern "C" int ewf_autotune(ewf_handle *h, int32_t nsteps, int32_t *kchunk)
         float t[2] = {};
         for (float &ms : t)
             if ((st = time_setting(h, steps, &ms))) return st;
-        margin = std::max(0.01f * std::min(t[0], t[1]), std::fabs(t[0] - t[1]));
+        if (short_graph(h)) margin = std::max(0.01f * std::min(t[0], t[1]), std::fabs(t[0] - t[1]));
         best = std::min(t[0], t[1]) - margin;
         best_k = h->kchunk;
         best_ty = h->ty;

@@ -1008,7 +1008,7 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
         int st = batch_ready(b);
         if (!st) st = ewf_batch_reset(b);
         if (st) return st;
-        const int brief = std::min(short_graph(b), steps & ~1), n = brief > 0 ? std::max(1, steps / brief) : 0;
+        const int brief = std::min(short_graph(b), std::max(2, steps & ~1)), n = std::max(4, steps / std::max(1, brief));  // (past the last step nothing is sampled or injected)
         cudaGraphExec_t exec = nullptr;
         if (brief > 0) {
             if ((st = ready_graph(b, brief, &exec))) return st;
@@ -1030,12 +1030,12 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
         *ms /= brief > 0 ? n * brief : std::max(1, steps);
         return (int)EWF_OK;
     };
-    // the setting by default is timed twice, and another one has to be faster by more than those two differ
+    // the setting by default is timed twice; with small chains another one has to be faster by more than those two differ
     apply(best_k, best_ty, best_own, best_pf);
     float t[2] = {}, ms = 0.f;
     for (float &x : t)
         if (int st = time(&x)) return st;
-    const float margin = std::max(0.01f * std::min(t[0], t[1]), std::fabs(t[0] - t[1]));
+    const float margin = short_graph(b) ? std::max(0.01f * std::min(t[0], t[1]), std::fabs(t[0] - t[1])) : 0.f;
     float best = std::min(t[0], t[1]) - margin;
     bool other = false;
     for (int own = 0; own < 2; ++own)

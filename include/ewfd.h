@@ -256,7 +256,7 @@ int ewf_staged_test_hold(int32_t plane, int32_t polls);
 int ewf_set_dependent_launch(ewf_handle *h, int32_t on);
 int ewf_get_dependent_launch(const ewf_handle *h, int32_t *on);
 /* Two-kernel step: the velocity kernel asks L2 for the input lines of the plane `planes` ahead
- * (0..8; 0 = off; by default 3 from 12 M cells on, else off; ewf_autotune picks it).  A hint: results do not depend on it. */
+ * (0..8; 0 = off; by default 2 from 12 M cells on, else off; ewf_autotune picks it).  A hint: results do not depend on it. */
 int ewf_set_l2_prefetch(ewf_handle *h, int32_t planes);
 int ewf_get_l2_prefetch(const ewf_handle *h, int32_t *planes);
 
@@ -363,7 +363,7 @@ int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk);
 int ewf_batch_set_tile(ewf_batch *b, int32_t tile_y);
 int ewf_batch_get_tile(const ewf_batch *b, int32_t *tile_y);
 /* The velocity kernels ask L2 for their state lines `planes` planes ahead (0..8; 0, the default: launches of
- * 12 M cells or more 3, others none; ewf_batch_autotune picks it).  A hint: results do not depend on it. */
+ * 12 M cells or more 2, others none; ewf_batch_autotune picks it).  A hint: results do not depend on it. */
 int ewf_batch_set_l2_prefetch(ewf_batch *b, int32_t planes);
 /* Launch form: 0 (default) -- the chains of launches too small to fill the GPU on up to eight parallel branches
  * (streams of the captured graph) balanced by cell-updates, then the others one after another; 1 -- all of them
