@@ -482,7 +482,8 @@ def main():
         kt = s.time_kernels(min(200, nt))
         if form == F.STEP_SPLIT:
             kb = KERNEL_BYTES[args.workload]
-            names = {"stress": "k_stress", "velocity": "k_velocity"}
+            pair = "_pair" if m.cells >= 4e5 else ""  # FP32 from 0.4 M cells on: two cells per thread
+            names = {"stress": "k_stress" + pair, "velocity": "k_velocity" + pair}
         else:  # one kernel does the whole step: its compulsory bytes are the one-pass step's
             kb = {"stress": STEP_BYTES[args.workload]}
             names = {"stress": "k_wave" if form == F.STEP_WAVE else ONEPASS_KERNELS[s.onepass()]}

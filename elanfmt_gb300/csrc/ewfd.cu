@@ -1235,6 +1235,7 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
         rf.it_wr = it_wr;
     }
     const bool pdl = h->pdl && !ev;  // kernels timed between events run as plain launches
+    // (FP64 has no packed arithmetic, and the pairs were not written for a weight per component)
     constexpr bool PAIRS = sizeof(T) == 4 && DAMP != DAMP_PERCOMP;
     const bool pair = PAIRS && h->pair;
     const dim3 pblk(PAIR_TX, pair_rows(h->ty)), pgrd(grd.x, (h->p.ny + pblk.y - 1) / pblk.y, grd.z);

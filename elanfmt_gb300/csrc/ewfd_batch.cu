@@ -118,6 +118,8 @@ float *bptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.base
 //   64^3 13 17 33 and 10 14 31        96^3 35 56 116 and 34 52 103      112^3 66 101 198 and 61 91 182
 //   128^3 92 136 260 and 84 126 251   144^3 142 206 396 and 142 213 426   160^3 182 265 513 and 186 278 556
 // and of 6 with a small isotropic model: 30^3 11.4 and 14.5, 40^3 16.1 and 17.9, 50^3 28.1 and 23.6, 64^3 40.3 and 30.7.
+// More of them change nothing: 64 of iso 50^3 180 and 129, 64^3 304 and 203, 80^3 667 and 369, of ortho 50^3 221 and 169, 64^3 361
+// and 279; 32 of iso 100^3 699 and 502, of ortho 100^3 821 and 738; 12 of ortho 128^3 520 and 488.
 constexpr double APART_FROM = 1e5, APART_TO = 2.5e6;
 
 float *sptr(const Prob &q, void *alloc) { return alloc ? (float *)alloc + q.sbase_off : nullptr; }

@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(split_max_threads<float>(), split_min_ctas<flo
                                                         min(k0 + p.a.kchunk, p.a.nz), p.rf);
 }
 
-// Receiver gather of one problem, all its right-hand sides: rows [row0, row0 + nrow) of the traces.
+// Receiver gather of one chain's right-hand sides: rows [row0, row0 + nrow) of the traces.
 template <typename T>
 __global__ void k_brecord(const StepArgs<T> a, const long long *__restrict__ rec_off, const int *__restrict__ rec_comp, int row0,
                           int nrow, double *__restrict__ traces, int nt, const int *it_rd)

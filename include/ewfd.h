@@ -318,8 +318,8 @@ int ewf_pack_field_noalloc(void *dst, int32_t dst_dtype_bytes, int32_t sx, int64
  * (src/FastWaveED_GPU3D_v1_DC_Earthquake_FULL_OK4_final/vizme_FastBiotED_GPU3D_OK_2024_final.m
  * :551-558, 579-582, 604-607).  sos: nsec rows of (b0 b1 b2 a0 a1 a2) as MATLAB and scipy lay
  * them out; each section is the direct form II transposed recursion from zero state.
- * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (a section of a trace per lane, or a trace per thread when there are many,
- * on `stream`), with the same bits. */
+ * ewf_sosfilt works on host arrays; ewf_sosfilt_device on device arrays (a section of a trace per
+ * lane, or a trace per thread when there are many, on `stream`), with the same bits. */
 #define EWF_SOS_MAX_SECTIONS 16
 int ewf_sosfilt(const double *sos, int32_t nsec, double *x, int64_t ntr, int64_t n);
 int ewf_sosfilt_device(const double *sos, int32_t nsec, double *x, int64_t ntr, int64_t n, void *stream);
@@ -333,9 +333,9 @@ int ewf_restore(ewf_handle *h, const char *path);
  * process): n problems -- models of any size and family -- each with n_rhs[i] right-hand sides
  * (independent source sets sharing the problem's model, e.g. the 6 elementary moment tensors of
  * a moment-tensor inversion), advanced together.  Per time step one stress and one velocity launch for
- * an RHS or, on large and very small models, for all of a problem's (materials read from HBM once), with
- * sources and receivers inside where the solver's own step has them there, replayed from a CUDA graph.  FP32; every problem runs the
- * same nt; state starts at zero.
+ * an RHS or, on large and very small models, for all of a problem's (materials read from HBM once), or
+ * for all tiny problems of one scheme, with sources and receivers inside where the solver's own step has
+ * them there, replayed from CUDA graphs.  FP32; every problem runs the same nt; state starts at zero.
  * ------------------------------------------------------------------------------------------- */
 typedef struct ewf_batch ewf_batch;
 int ewf_batch_create(int32_t n, const ewf_params *p, const int32_t *n_rhs, ewf_batch **out);
@@ -403,9 +403,9 @@ int ewf_mlp_adam_all(int32_t count, float *const *w, float *const *m, float *con
                      const size_t *n, const float *wd, float lr, float b1, float b2, float eps, int32_t step, void *stream);
 /* Synchronises and reports (then clears) a failed bounded wait of the GEMMs. */
 int ewf_mlp_status(void);
-/* Test hook of the failure path: with tile >= 0, the MMA issuer of the first CTA of every later
- * ewf_mlp_gemm launch withholds the accumulator-ready signal of its tile number `tile` (a signal
- * nothing else gives), and every mbarrier wait gives up after `polls` polls; the epilogue's wait
+/* Test hook of the failure path: with tile >= 0, the MMA issuers of the CTAs of every later GEMM launch whose first
+ * tiles lie in the first 128 x 256 of the product withhold the accumulator-ready signal of their tile number `tile`
+ * (a signal nothing else gives), and every mbarrier wait gives up after `polls` polls; the epilogue's wait
  * on that tile runs out, the launch still ends and ewf_mlp_status reports it.  tile < 0 restores
  * normal operation (default limit 2^22 polls). */
 int ewf_mlp_test_hold(int32_t tile, int32_t polls);
