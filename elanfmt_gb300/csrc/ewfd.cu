@@ -626,7 +626,7 @@ static void split_default_shape(ewf_handle *h)
     const SplitShape d = split_shape(h->p.nx, h->p.ny, h->p.nz);
     // 4, the shortest chunk that can be asked for, stands for the shorter ones of the rule too
     if (h->p.kchunk == 0 || h->p.kchunk == 4) h->kchunk = h->p.kchunk ? std::min(h->p.kchunk, d.kchunk) : d.kchunk;
-    h->ty = d.ty;
+    h->ty = h->p.kchunk >= 32 ? std::max(d.ty, 8) : d.ty;  // (long chunks: iso-het 97x83x71 in 64 planes 88 us a step with 4 rows, 67)
     h->l2pf = d.l2pf;
     h->pair = d.pair;
     h->stream_l2 = d.stream;
@@ -1237,7 +1237,7 @@ static void launch_step_t(const ewf_handle *h, const StepArgs<T> &a, cudaEvent_t
     const bool pdl = h->pdl && !ev;  // kernels timed between events run as plain launches
     // (FP64 has no packed arithmetic, and the pairs were not written for a weight per component)
     constexpr bool PAIRS = sizeof(T) == 4 && DAMP != DAMP_PERCOMP;
-    const bool pair = PAIRS && h->pair;
+    const bool pair = PAIRS && h->pair && enough_pairs(h->p.model, (double)h->p.nx * h->p.ny * h->p.nz, a.kchunk);
     const dim3 pblk(PAIR_TX, pair_rows(h->ty)), pgrd(grd.x, (h->p.ny + pblk.y - 1) / pblk.y, grd.z);
     if (ev) cudaEventRecord(ev[0], h->stream);
     if constexpr (PAIRS) {

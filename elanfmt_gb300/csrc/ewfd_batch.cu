@@ -658,7 +658,6 @@ static int build_tables(ewf_batch *b)
         const ewf_params &p = q.p;
         const SplitShape shape = split_shape(p.nx, p.ny, p.nz, c.R);
         c.ty = std::max(b->ty, shape.ty);
-        c.pair = shape.pair || c.R > 1;
         c.stream_l2 = shape.stream;
         c.a = all[c.prob].a;
         for (auto &f : c.a.f) f += c.r0 * (long long)q.box;
@@ -669,6 +668,7 @@ static int build_tables(ewf_batch *b)
         c.a.kchunk = split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
         if (q.kchunk > 0) c.a.kchunk = q.kchunk <= KCHUNK_BY_SIZE ? std::min(q.kchunk, c.a.kchunk) : q.kchunk;
         c.a.kchunk = std::max(c.a.kchunk, (p.nz + 65534) / 65535);  // a grid has at most 65535 CTAs along z
+        c.pair = c.R > 1 || (shape.pair && enough_pairs(p.model, together * p.nx * p.ny * p.nz, c.a.kchunk));
         std::vector<SrcEntry> ent;
         int before = 0;
         bool plane1 = false;

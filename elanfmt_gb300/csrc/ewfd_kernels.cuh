@@ -43,6 +43,13 @@ struct StepArgs {
     const T *w6[6];   // per-component weights of Vx/sxx, Vy/syy, Vz/szz, sxy, sxz, syz (box layout)
     long long sy;     // plane pitch of materials / damping, elements
     int sx;           // row pitch of materials / damping, elements
+    int fdiv;         // FP32: 1 if div_fast is verified for dx, dy, dz; FP64: its correction steps (1 or 2); 0: IEEE division
+    int vdamp_on;     // vdamp != 0 (an integer: a test of T takes the FP64 pipe in the FP64 form)
+    int bc1;          // 1: BC1 after the stress update (stress_store, inject_entry); 0: none
+    int smu_on;       // isotropic 1-D PML scheme: shear modulus smu instead of c66 on plane k = 1
+    int l2pf;         // two-kernel step: the velocity kernel asks L2 for its inputs this many planes ahead (0: off)
+    // (the extents and the spacings where the kernels' paired constant reads find them: the one-pass kernels take 1 to 18 %
+    // longer with the five integers above behind them)
     int nx, ny, nz;
     int bc1_rows;     // rows j < bc1_rows get the szz / sxz free-surface rule (OK4:279-281)
     int kchunk;       // planes per CTA
@@ -50,14 +57,9 @@ struct StepArgs {
     T c66, bx, by, bz;  // isotropic scalars (OK4:405-407)
     T c44, c55;         // per-component-weight scheme: shear moduli of yz and xz
     T third;            // (T)1/(T)3 of BC1
-    int fdiv;           // FP32: 1 if div_fast is verified for dx, dy, dz; FP64: its correction steps (1 or 2); 0: IEEE division
     T vdamp;            // linear velocity damping (16 km scheme), 0 = off
-    int vdamp_on;       // vdamp != 0 (an integer: a test of T takes the FP64 pipe in the FP64 form)
-    int bc1;            // 1: BC1 after the stress update (stress_store, inject_entry); 0: none
-    int smu_on;         // isotropic 1-D PML scheme: shear modulus smu instead of c66 on plane k = 1
     T smu;
     float one, minus_one;  // 1 and -1 (ewfd_pair.cuh)
-    int l2pf;           // two-kernel step: the velocity kernel asks L2 for its inputs this many planes ahead (0: off)
 };
 
 struct SrcEntry {
@@ -463,12 +465,15 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int i, int j
     T wz_k = T(0);
     if (DAMP == DAMP_PML1D) wz_k = ld(a.w1[2] + k0);
     StressIn<T, MODEL, DAMP> nxt;
-    stress_load_mat<T, MODEL, DAMP>(a, c, k0, nxt);
-    if (SRC) pdl_wait();  // nothing above depends on an earlier launch
+    if (SRC) {
+        stress_load_mat<T, MODEL, DAMP>(a, c, k0, nxt);
+        pdl_wait();  // nothing above depends on an earlier launch
+    }
     T vx_m = lds<COH>(a.f[0] + c - sy);  // Vx(k-1)
     T vy_m = lds<COH>(a.f[1] + c - sy);  // Vy(k-1)
     T vz_k = lds<COH>(a.f[2] + c);        // Vz(k)
     stress_load_state<T, MODEL, DAMP, COH>(a, c, nxt);
+    if (!SRC) stress_load_mat<T, MODEL, DAMP>(a, c, k0, nxt);
     // point sources on this column (SRC: the two-kernel step's stress kernel)
     bool src_col = false;
     T s_src = T(0);
@@ -486,16 +491,9 @@ __device__ __forceinline__ void stress_column(const StepArgs<T> &a, int i, int j
         stress_math<T, MODEL, DAMP>(a, q, cd, i, j, k, vx_m, vy_m, vz_k, wz_k, o, w_xy, w_xz, w_yz);
         stress_store<T, SRC>(a, c, sy, k, i, j, row_bc, o, w_xy, w_xz, w_yz);
         if (SRC && src_col && k >= ss.k0 && k <= ss.k1) {
-            if (ss.inl) {
-#pragma unroll
-                for (int e = 0; e < SRC_INLINE; ++e)
-                    if (e < ss.nsrc && ss.e[e].i == i && ss.e[e].j == j && fused_src_plane(ss.e[e].comp, ss.e[e].k) == k)
-                        inject_entry(a, ss.e[e], s_src, ss.order);
-            } else {
-                for (int e = 0; e < ss.nsrc; ++e) {
-                    const SrcEntry q_e = ss.src[e];
-                    if (q_e.i == i && q_e.j == j && fused_src_plane(q_e.comp, q_e.k) == k) inject_entry(a, q_e, s_src, ss.order);
-                }
+            for (int e = 0; e < ss.nsrc; ++e) {
+                const SrcEntry q_e = ss.inl ? ss.e[e] : ss.src[e];
+                if (q_e.i == i && q_e.j == j && fused_src_plane(q_e.comp, q_e.k) == k) inject_entry(a, q_e, s_src, ss.order);
             }
         }
         if (MODEL == MODEL_ISO && DAMP == DAMP_PML1D) wz_k = q.w;
@@ -515,7 +513,7 @@ template <typename T>
 constexpr int split_min_ctas() { return sizeof(T) == 4 ? 2 : 1; }
 
 template <typename T, int MODEL, int DAMP>
-__global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k_stress(const StepArgs<T> a, const StressSrc ss)
+__global__ void __launch_bounds__(split_max_threads<T>(), split_min_ctas<T>()) k_stress(const StepArgs<T> a, const __grid_constant__ StressSrc ss)
 {
     pdl_trigger();
     const int k0 = blockIdx.z * a.kchunk;
@@ -746,12 +744,15 @@ __device__ __forceinline__ void velocity_column(const StepArgs<T> &a, int i, int
 
     long long c = (long long)i + (long long)j * a.sx + (long long)k0 * sy;
     VelIn<T, MODEL, DAMP, KAHAN> nxt;
-    vel_load_mat<T, MODEL, DAMP, KAHAN>(a, c, k0, nxt);
-    if (REC) pdl_wait();  // nothing above depends on an earlier launch
+    if (REC) {
+        vel_load_mat<T, MODEL, DAMP, KAHAN>(a, c, k0, nxt);
+        pdl_wait();  // nothing above depends on an earlier launch
+    }
     T szz_m = lds<COH>(a.f[5] + c - sy);
     T sxz_k = lds<COH>(a.f[7] + c);
     T syz_k = lds<COH>(a.f[8] + c);
     vel_load_state<T, MODEL, DAMP, KAHAN, COH>(a, c, nxt);
+    if (!REC) vel_load_mat<T, MODEL, DAMP, KAHAN>(a, c, k0, nxt);
     if (KAHAN) {
 #pragma unroll
         for (int f = 0; f < 3; ++f) nxt.cp[f] = a.comp[f][c];

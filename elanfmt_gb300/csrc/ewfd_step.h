@@ -6,6 +6,7 @@
 
 #include <vector>
 
+#include "ewfd.h"
 #include "ewfd_kernels.cuh"
 
 // Sources for the stress kernel (false: the injection kernel applies them)
@@ -33,6 +34,16 @@ struct SplitShape {
     bool stream;
 };
 SplitShape split_shape(int nx, int ny, int nz, int R = 1);
+
+// Two cells per thread halve the threads: chunks longer than the rule's (a caller's own) can leave too few of them.  us per step of one
+// and of two cells by planes per chunk, where they part:
+//   iso 128^3  8 37.6 37.9  16 42.5 45.7  64 127 138     200x190x150  32 142 124  64 155 181     97x83x71  8 19.2 19.8  64 77 94
+//   iso-het 128^3  16 58.9 53.3  32 87.7 90.5     200x190x150  32 169 154  64 196 205     97x83x71  16 33.1 33.4  64 88 107
+//   ortho 128^3  16 63.1 51.7  32 96.6 88.9     97x83x71  8 24.7 24.3  16 39.6 39.1  32 59 71     80x80x70  8 20.8 23.9  16 25.7 41.6
+inline bool enough_pairs(int model, double cells, int kchunk)
+{
+    return cells / (2.0 * kchunk) >= (model == EWF_MODEL_ISO ? 7.5e4 : model == EWF_MODEL_ISO_HET ? 5e4 : 3e4);
+}
 
 // Buffers (16-byte aligned) set to zero in stream order, ZERO_GROUP of them per launch
 struct ZeroBuf {
