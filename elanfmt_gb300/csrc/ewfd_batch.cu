@@ -444,8 +444,10 @@ constexpr double BRANCH_CELLS = 6e5, BRANCH_SHARE = 1.1e6;
 // and of problems with a stress receiver each: iso 16^3  15 17.4 9.6   50 60 15.8   200 253 48     iso 28^3  50 74 31   200 277 147.
 constexpr double MANY_CELLS = 2e4, MANY_CELLS_2 = 2.8e4, MANY_ORTHO = 1.2e6;
 constexpr int MANY_MIN = 12, MANY_MIN_2 = 32;
-// A chunk that is asked for up to this many planes is the most that the rule by size may take, which takes no more than
-// 6 by itself: 8 asks for the rule, and stands for it where the autotuner chose it.
+// A chunk that is asked for is the most planes that the rule by size may take.  It takes no more than 6 by itself, and chains
+// want no more: one model after another, or few at a time, they do not fill the GPU in longer chunks.  us per step by the rule and in 16, 32 and 64
+// planes: 4 iso 100^3 63 137 186 293     6 iso 64^3 22 46 71 124     6 rhs of ortho 80^3 55 131 173 295     4 rhs of iso 144^3 221 232 239 251
+// (64 planes in the shared launches of before 147, 93, 266, 306).  8 stands for the rule where the autotuner returns it.
 constexpr int KCHUNK_BY_SIZE = 8;
 static int scheme(const ewf_params &p) { return p.model == EWF_MODEL_ISO ? 0 : p.damping == EWF_DAMP_W3D ? 1 : 2; }
 
@@ -666,7 +668,7 @@ static int build_tables(ewf_batch *b)
         // the problem's own size, and so: 6 iso 40^3 12.0 and 8.8, 16 iso 40^3 32.4 and 22.9, 8 iso 50^3 24.5 and
         // 16.8, 8 ortho 64^3 40.6 and 38.1, 8 iso 80^3 50.1 and 49.2.
         c.a.kchunk = split_shape(p.nx, p.ny, p.nz, (int)std::min(1e6, c.R * together)).kchunk;
-        if (q.kchunk > 0) c.a.kchunk = q.kchunk <= KCHUNK_BY_SIZE ? std::min(q.kchunk, c.a.kchunk) : q.kchunk;
+        if (q.kchunk > 0) c.a.kchunk = std::min(q.kchunk, c.a.kchunk);
         c.a.kchunk = std::max(c.a.kchunk, (p.nz + 65534) / 65535);  // a grid has at most 65535 CTAs along z
         c.pair = c.R > 1 || (shape.pair && enough_pairs(p.model, together * p.nx * p.ny * p.nz, c.a.kchunk));
         std::vector<SrcEntry> ent;
@@ -987,18 +989,16 @@ extern "C" int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int3
     return EWF_OK;
 }
 
-// Times `nsteps` steps for each (tile height, z-chunk) candidate with CUDA events, keeps the
+// Times `nsteps` steps for each launch form and tile height, then for each prefetch distance, with CUDA events, keeps the
 // fastest, and leaves the batch reset (the tuning steps advance the state).
 extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_out)
 {
     if (!b || nsteps < 1) return ewf_fail(EWF_ERR_ARG, "bad argument");
-    // planes per CTA: the rule by size, or one number for all problems
-    static const int cand[] = {KCHUNK_BY_SIZE, 12, 16, 24, 32};
     static const int ty_cand[] = {4, 8};
     const int steps = std::min(nsteps, b->nt - 1);
-    int best_k = KCHUNK_BY_SIZE, best_ty = 4, best_pf = 0, best_own = 0;
-    auto apply = [&](int kc, int ty, int own, int pf) {
-        for (auto &q : b->probs) q.kchunk = kc;
+    int best_ty = 4, best_pf = 0, best_own = 0;
+    auto apply = [&](int ty, int own, int pf) {
+        for (auto &q : b->probs) q.kchunk = KCHUNK_BY_SIZE;
         b->ty = ty;
         b->own = own;
         b->l2pf = pf;
@@ -1033,7 +1033,7 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
         return (int)EWF_OK;
     };
     // the setting by default is timed twice; with small chains another one has to be faster by more than those two differ
-    apply(best_k, best_ty, best_own, best_pf);
+    apply(best_ty, best_own, best_pf);
     float t[2] = {}, ms = 0.f;
     for (float &x : t)
         if (int st = time(&x)) return st;
@@ -1041,31 +1041,29 @@ extern "C" int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk_
     float best = std::min(t[0], t[1]) - margin;
     bool other = false;
     for (int own = 0; own < 2; ++own)
-        for (int ty : ty_cand)
-            for (int kc : cand) {
-                if (own == 0 && ty == 4 && kc == KCHUNK_BY_SIZE) continue;
-                apply(kc, ty, own, 0);
-                if (int st = time(&ms)) return st;
-                if (ms < best) {
-                    best = ms;
-                    best_k = kc;
-                    best_ty = ty;
-                    best_own = own;
-                    other = true;
-                }
+        for (int ty : ty_cand) {
+            if (own == 0 && ty == 4) continue;
+            apply(ty, own, 0);
+            if (int st = time(&ms)) return st;
+            if (ms < best) {
+                best = ms;
+                best_ty = ty;
+                best_own = own;
+                other = true;
             }
+        }
     if (other) best -= margin;
     for (int pf : {2, 3, 4}) {  // then the velocity kernels' L2 prefetch distance at that setting
-        apply(best_k, best_ty, best_own, pf);
+        apply(best_ty, best_own, pf);
         if (int st = time(&ms)) return st;
         if (ms < best) {
             best = ms;
             best_pf = pf;
         }
     }
-    apply(best_k, best_ty, best_own, best_pf);
+    apply(best_ty, best_own, best_pf);
     if (int st = batch_ready(b)) return st;
-    if (kchunk_out) *kchunk_out = best_k;
+    if (kchunk_out) *kchunk_out = KCHUNK_BY_SIZE;
     return ewf_batch_reset(b);
 }
 

@@ -123,8 +123,8 @@ typedef struct ewf_params {
     int32_t src_order;    /* ewf_src_order */
     int32_t over_y;       /* legacy OVERY: BC1 rows are j < min(nx, ny + over_y) (OK4:279-281) */
     int32_t nout;         /* progress line every nout steps (OK4:502-504); 0 = quiet */
-    int32_t kchunk;       /* planes per CTA of the z-marching kernels, from 4; 0 = by size.  Two-kernel step: with 4 (in a
-                             batch, up to 8) the rule by size may take fewer */
+    int32_t kchunk;       /* planes per CTA of the z-marching kernels, from 4; 0 = by size.  Two-kernel step: with 4 the
+                             rule by size may take fewer; in a batch kchunk is the most that it may take */
     int32_t graph_steps;  /* steps captured per CUDA graph; 0 = default (64; what is left of a run in graphs of 8 on
                              small grids), <0 = no graph */
     int32_t check_finite; /* 1: ewf_run checks the receiver traces for NaN/Inf */
@@ -354,9 +354,9 @@ int ewf_batch_last_run_ms(const ewf_batch *b, double *ms);
 /* traces of (prob, rhs): out[r*nt + it] for the problem's n_rec receivers */
 int ewf_batch_get_seismograms(ewf_batch *b, int32_t prob, int32_t rhs, double *out, size_t n);
 int ewf_batch_get_field(ewf_batch *b, int32_t prob, int32_t rhs, int32_t field, void *host, size_t n, int32_t dtype_bytes);
-/* the autotuner over the whole batch: launch form, z-chunk and CTA tile height, then the
- * velocity kernels' L2 prefetch distance (leaves the batch reset).  A batch made with *kchunk and set to what
- * the getters below return has the same setting. */
+/* the autotuner over the whole batch: launch form and CTA tile height, then the velocity kernels' L2 prefetch
+ * distance, with chunks by size (leaves the batch reset).  A batch made with *kchunk and set to what the getters
+ * below return has the same setting. */
 int ewf_batch_autotune(ewf_batch *b, int32_t nsteps, int32_t *kchunk);
 /* CTA tile height of every launch of the batch, in rows of 32 columns: 4 (default), 8 or 16
  * (kernels with two cells per thread take twice as many rows, 16 at most); results do not depend on it */
